@@ -43,6 +43,8 @@ _SIGNATURES = {
                                                    c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_float]),
     "b200_gemm_generic": ("gemm_generic", [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int,
                                            c_int, c_int, c_int, c_int, c_float, c_float, c_void_p, c_int]),
+    "b200_gemm_f32_tcgen05": ("gemm_f32_tcgen05", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int,
+                                                   c_int, c_float, c_float, c_void_p, c_int, c_void_p, c_int]),
     "b200_gemm_generic_batched": ("gemm_generic", [c_void_p, c_int, c_int, ctypes.c_longlong, c_void_p, c_int, c_int,
                                                    ctypes.c_longlong, c_void_p, c_int, c_int, ctypes.c_longlong, c_int, c_int,
                                                    c_int, c_int]),
@@ -383,7 +385,8 @@ def gemm_generic(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, epilogue: in
                  gate_args: tuple[float, float] = (0.0, 0.0), bias: torch.Tensor | None = None,
                  silu_columns: int = 0) -> None:
     """c = a @ w.T (store), c += a @ w.T (residual add, c float32) or c = act(gate) * up with
-    gate/up rows interleaved in w (act: SiLU, or GELU in its tanh form).  32-bit FMA accumulation, no tensor cores.
+    gate/up rows interleaved in w (act: SiLU, or GELU in its tanh form).  Sums of 32-bit precision: by FMA, or, for more
+    than a few rows of float32 operands, by ``gemm_f32_tcgen05``.
     ``bias`` float32 [w.shape[0]] joins every sum before the epilogue; the store epilogue passes the first ``silu_columns``
     results through SiLU."""
     _dev(a, w, c)
@@ -391,10 +394,38 @@ def gemm_generic(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, epilogue: in
     N = w.shape[0]
     assert w.shape[1] == K and a.stride(1) == 1 and w.stride(1) == 1 and c.stride(1) == 1
     assert c.shape[0] == M and c.shape[1] == (N // 2 if epilogue in GATED_EPILOGUES else N)
+    if M > 16 and a.dtype == w.dtype == c.dtype == torch.float32 and gemm_f32_tcgen05(a, w, c, epilogue, gate_args, bias, silu_columns):
+        return
     _check(_fn("b200_gemm_generic")(
         a.data_ptr(), dtype_code(a.dtype), a.stride(0), w.data_ptr(), dtype_code(w.dtype), w.stride(0), c.data_ptr(),
         dtype_code(c.dtype), c.stride(0), M, N, K, epilogue, float(gate_args[0]), float(gate_args[1]),
         _bias_ptr(bias, N), int(silu_columns), _stream()), "gemm_generic")
+
+
+def gemm_f32_tcgen05(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, epilogue: int = EPILOGUE_STORE,
+                     gate_args: tuple[float, float] = (0.0, 0.0), bias: torch.Tensor | None = None, silu_columns: int = 0,
+                     n_spans: int = 0) -> bool:
+    """``gemm_generic`` for float32 operands with float32's precision on the tensor cores: every number as the sum of three
+    bfloat16 numbers, partial sums of 64 products added in float32.  ``n_spans``: how often K is cut (0: the shape decides).
+    Returns False, having done nothing, for operands it does not take."""
+    M, K = a.shape
+    N = w.shape[0]
+    lib = library("gemm_f32_tcgen05")
+    lib.b200_gemm_f32_scratch.restype = ctypes.c_longlong
+    elements = lib.b200_gemm_f32_scratch(M, N, K, a.stride(0), w.stride(0))
+    if elements <= 0 or w.data_ptr() & 15 or a.stride(1) != 1 or w.stride(1) != 1:
+        return False
+    _dev(a, w, c)
+    assert a.dtype == w.dtype == c.dtype == torch.float32 and w.shape[1] == K and c.stride(1) == 1
+    assert tuple(c.shape) == (M, N // 2 if epilogue in GATED_EPILOGUES else N)
+    scratch = torch.empty(elements, dtype=torch.bfloat16, device=a.device)
+    status = _fn("b200_gemm_f32_tcgen05")(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), c.data_ptr(), c.stride(0), M, N, K,
+                                          epilogue, float(gate_args[0]), float(gate_args[1]), _bias_ptr(bias, N),
+                                          int(silu_columns), scratch.data_ptr(), int(n_spans), _stream())
+    if status == _UNSUPPORTED:
+        return False
+    _check(status, "gemm_generic")
+    return True
 
 
 def gemm_per_head(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor) -> None:

@@ -1,0 +1,89 @@
+"""The float32 run's kernels at the sizes where they can go wrong: the product on the tensor cores (edges of its tiles,
+cuts of K, every epilogue, rows off the 16-byte grid, sums that are not finite), the product for few rows, and the attention over tiles of queries."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+EPS = 2.0 ** -23
+
+
+def ops():
+    from gpullama3.java_b200.kernels import ops as o
+    return o
+
+
+def _epilogue(o, epilogue, sums, c0, silu):
+    if epilogue == o.EPILOGUE_STORE:
+        out = sums.clone()
+        out[:, :silu] = torch.nn.functional.silu(out[:, :silu])
+        return out
+    if epilogue == o.EPILOGUE_RESIDUAL_ADD:
+        return c0.double() + sums
+    g, u = sums[:, 0::2], sums[:, 1::2]
+    if epilogue == o.EPILOGUE_GATED_SILU:
+        return torch.nn.functional.silu(g) * u
+    if epilogue == o.EPILOGUE_GATED_GELU_TANH:
+        return torch.nn.functional.gelu(g, approximate="tanh") * u
+    g, u = g.clamp(max=1.5), u.clamp(-1.5, 1.5)
+    return g * torch.sigmoid(1.7 * g) * (u + 1)
+
+
+@pytest.mark.parametrize("M, N, K, spans", [(17, 64, 1024, 0), (64, 128, 512, 0), (65, 130, 1028, 0), (129, 258, 1032, 0), (130, 1000, 68, 0),
+                                            (300, 256, 4100, 0), (64, 300, 2048, 1), (200, 260, 1100, 3), (33, 514, 1024, 8)])
+@pytest.mark.parametrize("epilogue", [0, 1, 2, 3, 4])
+def test_products_on_the_tensor_cores_keep_32_bits(M, N, K, spans, epilogue):
+    """A sum of K products has K / 64 float32 additions of partial sums, and within a partial sum at most 24 truncated ones:
+    its error is below (K / 64 + 26) 2^-23 sum |a w| (two more for the terms left out and the bias).  The activations change
+    a value by less than 1.5 times its argument's error here, and round a few times themselves."""
+    o = ops()
+    g = torch.Generator().manual_seed(M + N + K)
+    a = torch.randn(M, K + 5, generator=g).cuda()[:, 1:K + 1]                       # rows off the 16-byte grid, of another stride
+    w = (torch.randn(N, K, generator=g) / math.sqrt(K)).cuda()
+    bias = torch.randn(N, generator=g).cuda()
+    columns = N // 2 if epilogue >= 2 else N
+    c = torch.randn(M, columns + 3, generator=g).cuda()
+    c0 = c.clone()
+    silu = 37 if epilogue == 0 else 0
+    assert o.gemm_f32_tcgen05(a, w, c[:, :columns], epilogue, (1.5, 1.7), bias, silu, n_spans=spans)
+    sums = a.double() @ w.double().t() + bias.double()
+    bound = (K / 64 + 26) * EPS * (a.double().abs() @ w.double().abs().t() + bias.abs().double())
+    ref = _epilogue(o, epilogue, sums, c0[:, :columns], silu)
+    if epilogue >= 2:
+        big = sums.abs().amax() + 2
+        bound = 1.5 * big * (bound[:, 0::2] + bound[:, 1::2]) + 16 * EPS * ref.abs()
+    else:
+        bound = 1.5 * bound + 16 * EPS * ref.abs()
+    assert bool(((c[:, :columns].double() - ref).abs() <= bound).all())
+    assert torch.equal(c[:, columns:], c0[:, columns:])
+    from gpullama3.java_b200.kernels.build import library
+    assert library("gemm_f32_tcgen05").b200_gemm_f32_tcgen05_status() == 0
+
+
+def test_products_whose_sums_are_not_finite():
+    """Infinities and NaN come out where the plain product has them: such sums are formed again by multiply-adds."""
+    o = ops()
+    g = torch.Generator().manual_seed(3)
+    a, w = torch.randn(100, 512, generator=g), torch.randn(200, 512, generator=g)
+    a[3, 7], a[50, 100], w[20, 30], a[11, 5], w[5, 5] = math.inf, math.nan, -math.inf, 3.4e38, 1e-3
+    a[60], a[61, 4] = math.nan, -3.39e38     # (the second rounds to an infinity as a bfloat16 number)
+    a, w = a.cuda(), w.cuda()
+    c = torch.empty(100, 200, device="cuda")
+    assert o.gemm_f32_tcgen05(a, w, c)
+    ref = torch.stack([o_row for o_row in (a.double().unsqueeze(1) * w.double().unsqueeze(0)).sum(-1)]).float()
+    assert torch.equal(torch.isnan(c), torch.isnan(ref)) and torch.equal(torch.isinf(c), torch.isinf(ref))
+    assert torch.equal(c[torch.isinf(c)], ref[torch.isinf(ref)])
+    ok = torch.isfinite(ref)
+    bound = 100 * EPS * (a.double().abs() @ w.double().abs().t())
+    assert bool(((c.double() - ref.double()).abs()[ok] <= bound[ok]).all())
+
+
+def test_products_that_stay_with_the_plain_kernels():
+    o = ops()
+    for M, N, K in ((16, 1024, 1024), (17, 1024, 1023), (17, 40, 2048), (100, 64, 64)):
+        a, w, c = torch.zeros(M, K, device="cuda"), torch.zeros(N, K, device="cuda"), torch.full((M, N), 7.0, device="cuda")
+        assert not o.gemm_f32_tcgen05(a, w, c) and bool((c == 7.0).all())
+        o.gemm_generic(a, w, c)
+        assert bool((c == 0).all())
