@@ -77,6 +77,9 @@ _SIGNATURES = {
     "b200_attention_decode_rope": ("attention_decode", [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
                                                         c_void_p, c_void_p, ctypes.c_longlong, c_int, c_int, c_int,
                                                         c_int, c_int, c_int, c_void_p, c_int, c_int, c_int]),
+    "b200_attention_prefill_f32": ("attention_prefill_f32", [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
+                                                             c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
+                                                             c_void_p, c_void_p, c_int, c_float]),
     "b200_attention_prefill_tc": ("attention_prefill_tcgen05", [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p,
                                                                 c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int,
                                                                 c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
@@ -361,6 +364,37 @@ def attention_paged(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, posit
         n_kv_heads, head_dim, int(window), int(n_splits), scratch.data_ptr() if scratch is not None else None,
         int(keep_first), int(chunk), ptr(slopes), ptr(sinks), ptr(gate), gate.stride(0) if gate is not None else 0,
         float(softcap), _stream()), "attention_paged")
+
+
+def attention_prefill_f32(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, cu_seqlens: torch.Tensor, kv_lens: torch.Tensor,
+                          page_table: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, n_seqs: int, max_q_len: int,
+                          n_heads: int, n_kv_heads: int, head_dim: int, window: int = 0, *, chunk: int = 0,
+                          slopes: torch.Tensor | None = None, sinks: torch.Tensor | None = None,
+                          gate: torch.Tensor | None = None, softcap: float = 0.0) -> bool:
+    """``attention_paged`` of float32 queries that lie sequence after sequence (``cu_seqlens`` int32 [n_seqs + 1]; ``kv_lens``
+    counts this pass's tokens), a tile of them at a time; the same terms without kept first positions.  Returns False,
+    having done nothing, for operands it does not take."""
+    if q.dtype != torch.float32 or head_dim not in (32, 64, 96, 128) or q_row_stride % 4 or q.data_ptr() & 15:
+        return False
+    _dev(q, out, cu_seqlens, kv_lens, page_table, k_pool, v_pool, slopes, sinks, gate)
+    assert out.is_contiguous() and out.shape[1] == n_heads * head_dim and out.dtype == q.dtype == k_pool.dtype == v_pool.dtype
+    assert k_pool.is_contiguous() and v_pool.is_contiguous() and page_table.is_contiguous()
+    assert tuple(k_pool.shape[1:]) == (n_kv_heads, PAGE_TOKENS, head_dim)
+    assert tuple(v_pool.shape[1:]) == (n_kv_heads, head_dim, PAGE_TOKENS)
+    assert cu_seqlens.dtype == kv_lens.dtype == page_table.dtype == torch.int32 and cu_seqlens.numel() == n_seqs + 1
+    for t in (slopes, sinks):
+        assert t is None or (t.dtype == torch.float32 and t.is_contiguous() and t.numel() == n_heads)
+    assert gate is None or (gate.dtype == q.dtype and gate.stride(1) == 1 and gate.shape[1] >= n_heads)
+    ptr = lambda t: t.data_ptr() if t is not None else None
+    status = _fn("b200_attention_prefill_f32")(
+        q.data_ptr(), q_row_stride, out.data_ptr(), cu_seqlens.data_ptr(), kv_lens.data_ptr(), page_table.data_ptr(),
+        page_table.shape[1], k_pool.data_ptr(), v_pool.data_ptr(), n_seqs, int(max_q_len), n_heads, n_kv_heads, head_dim,
+        int(window), int(chunk), ptr(slopes), ptr(sinks), ptr(gate), gate.stride(0) if gate is not None else 0, float(softcap),
+        _stream())
+    if status == _UNSUPPORTED:
+        return False
+    _check(status, "attention_paged")
+    return True
 
 
 # --------------------------------------------------------------------------- matrix products

@@ -255,13 +255,19 @@ def attend(shape, qkv: torch.Tensor, out: torch.Tensor, ctx: StepContext, table:
     (``slopes``, ``sinks``, ``softcap``) where it has any."""
     if fast.try_attention(qkv, out, ctx, table, cache, shape, gate):
         return
+    terms = dict(chunk=getattr(shape, "chunk", None) or 0, slopes=getattr(shape, "slopes", None), sinks=getattr(shape, "sinks", None),
+                 gate=gate, softcap=getattr(shape, "softcap", None) or 0.0)
+    # float32 prompts: a tile of a sequence's queries at a time
+    if not ctx.all_decode and not shape.keep_first and ops.attention_prefill_f32(
+            qkv, qkv.shape[1], out, ctx.cu_seqlens, ctx.kv_lens, table, cache.k, cache.v, ctx.n_seqs, ctx.max_q_len, shape.n_heads,
+            shape.n_kv_heads, shape.head_dim, shape.window or 0, **terms):
+        return
     rows = qkv.shape[0] * shape.n_heads
     reach = min(ctx.capacity(cache.group), _reach(shape) or ctx.capacity(cache.group))
     splits = 1 if rows >= 1024 else max(1, min(16, 1024 // rows, reach // 512))
     ops.attention_paged(qkv, qkv.shape[1], out, ctx.positions, ctx.seq_ids, table, cache.k, cache.v,
                         shape.n_heads, shape.n_kv_heads, shape.head_dim, shape.window or 0, n_splits=splits,
-                        keep_first=shape.keep_first, chunk=getattr(shape, "chunk", None) or 0, slopes=getattr(shape, "slopes", None), sinks=getattr(shape, "sinks", None),
-                        gate=gate, softcap=getattr(shape, "softcap", None) or 0.0)
+                        keep_first=shape.keep_first, **terms)
 
 
 VALUE_MIX_SOURCE = "value mix source"   # in a pass's ``ctx.extras``: the first value-mixing layer's own values [T, G dv]

@@ -87,3 +87,47 @@ def test_products_that_stay_with_the_plain_kernels():
         assert not o.gemm_f32_tcgen05(a, w, c) and bool((c == 7.0).all())
         o.gemm_generic(a, w, c)
         assert bool((c == 0).all())
+
+
+CUTS = [([5, 1, 100, 77], [5, 300, 100, 200]), ([70, 64, 65], [70, 64, 129]), ([130, 3], [400, 69])]
+
+
+@pytest.mark.parametrize("q_lens, kv_lens", CUTS)
+@pytest.mark.parametrize("H, G, D", [(6, 2, 32), (4, 4, 64), (8, 1, 64), (6, 3, 96), (6, 2, 128)])
+@pytest.mark.parametrize("terms", [{}, {"window": 33}, {"chunk": 48, "sinks": 1, "gate": 1}, {"slopes": 1, "softcap": 5.0, "window": 100, "sinks": 1},
+                                   {"odd_values": 1}, {"odd_values": 1, "window": 20}], ids=str)
+def test_attention_over_tiles_of_queries(q_lens, kv_lens, H, G, D, terms):
+    """Against the plain kernel.  Behind every sequence's end the pages hold NaN; with ``odd_values`` the last two positions of
+    the first sequence hold values that are not finite, which earlier queries must not see.  A score is a sum of D products of 2 normal numbers
+    by normal numbers over sqrt(D): its rounding is below (D / 2 + 4) 2^-24 2 sqrt(D) on either side, and a result moves by
+    at most twice that times the largest value."""
+    o = ops()
+    terms = dict(terms)
+    gen = torch.Generator("cuda").manual_seed(H * D)
+    rand = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    n, T, width = len(q_lens), sum(q_lens), max(-(-k // 64) for k in kv_lens)
+    table = torch.randperm(n * width, generator=gen, device="cuda").to(torch.int32).view(n, width)
+    k, v, q = rand(n * width, G, 64, D), rand(n * width, G, D, 64), rand(T, (H + 2 * G) * D) * 2
+    biggest = float(v.abs().max())
+    for i, length in enumerate(kv_lens):
+        if length % 64:
+            page = int(table[i, length // 64])
+            k[page, :, length % 64:], v[page, :, :, length % 64:] = math.nan, math.nan
+    if terms.pop("odd_values", 0):
+        last = kv_lens[0] - 1
+        v[int(table[0, last // 64]), :, 3, last % 64] = math.nan
+        v[int(table[0, (last - 1) // 64]), :, 5, (last - 1) % 64] = math.inf
+    window = terms.pop("window", 0)
+    for name, shape in (("slopes", (H,)), ("sinks", (H,)), ("gate", (T, H + 3))):
+        if terms.pop(name, 0):
+            terms[name] = rand(*shape) * (0.1 if name == "slopes" else 1.0)
+    positions = torch.cat([torch.arange(b - a, b) for a, b in zip(q_lens, kv_lens)]).to(torch.int32).cuda()
+    seq_ids = torch.repeat_interleave(torch.arange(n), torch.tensor(q_lens)).to(torch.int32).cuda()
+    cu = torch.tensor([0] + q_lens).cumsum(0).to(torch.int32).cuda()
+    lens = torch.tensor(kv_lens, dtype=torch.int32, device="cuda")
+    want, got = torch.empty(T, H * D, device="cuda"), torch.full((T, H * D), 7.0, device="cuda")
+    o.attention_paged(q, q.shape[1], want, positions, seq_ids, table, k, v, H, G, D, window, **terms)
+    assert o.attention_prefill_f32(q, q.shape[1], got, cu, lens, table, k, v, n, max(q_lens), H, G, D, window, **terms)
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
+    ok = torch.isfinite(want)
+    assert float((got - want)[ok].abs().max()) <= 2 * 2 * (D / 2 + 4) * 2.0 ** -24 * 2 * math.sqrt(D) * biggest
