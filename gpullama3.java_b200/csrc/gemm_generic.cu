@@ -197,72 +197,123 @@ template <> __device__ __forceinline__ float4 load4<__nv_bfloat16>(const __nv_bf
                        __uint_as_float(v.y & 0xffff0000u));
 }
 
-constexpr int kFewWarps = 8, kFewThreads = kFewWarps * 32, kFewRows = 4;
+// a weight is read once: not kept in L1, which holds the activations
+template <typename T> __device__ __forceinline__ float4 load4_once(const T* p);
+template <> __device__ __forceinline__ float4 load4_once<float>(const float* p) {
+    float4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+template <> __device__ __forceinline__ float4 load4_once<__nv_bfloat16>(const __nv_bfloat16* p) {
+    uint2 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16),
+                       __uint_as_float(v.y & 0xffff0000u));
+}
 
-// sum over the lanes of a warp by halving: afterwards v[0] of lane l is the sum of every lane's v[l] (31 exchanges
-// for 32 numbers, where a butterfly per number would need 160)
-__device__ __forceinline__ float reduce_by_halving(float (&v)[32], int lane) {
+constexpr int kFewWarps = 8, kFewThreads = kFewWarps * 32;
+constexpr int kFewRows = 8;               // weight rows of a CTA, in two groups of four
+constexpr int kFewSlice = kFewWarps * 128;   // elements of K that the CTA's warps take at a time, 128 each
+
+// Sums over the lanes of a warp of NV numbers by halving: afterwards lane l has the sum number l / (32 / NV) (31 exchanges
+// for 32 numbers, where a butterfly per number would need 160).
+template <int NV>
+__device__ __forceinline__ float reduce_by_halving(float (&v)[NV], int lane) {
 #pragma unroll
-    for (int half = 16; half >= 1; half >>= 1) {
-        const bool upper = (lane & half) != 0;
+    for (int half = NV / 2, bit = 16; half >= 1; half >>= 1, bit >>= 1) {
+        const bool upper = (lane & bit) != 0;
 #pragma unroll
         for (int i = 0; i < half; ++i) {
             const float send = upper ? v[i] : v[i + half];
             const float keep = upper ? v[i + half] : v[i];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, half);
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
         }
     }
+#pragma unroll
+    for (int bit = 16 / NV; bit >= 1; bit >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], bit);
     return v[0];
 }
 
-// A CTA owns four consecutive weight rows (two gate/up pairs of the gated epilogue); its eight warps split K between
-// them (a warp takes 128 elements of every 1024), so that a narrow output still gives every SM several CTAs and each
-// activation element loaded from L1 meets four weight rows.  MT tokens (8 or 16): 4 x MT sums per lane, summed over
-// the lanes by halving and over the warps in shared memory in warp order.  Still plain 32-bit FMA.
-template <typename TA, typename TW, typename TC, int MT>
-__global__ void __launch_bounds__(kFewThreads)
+// A CTA owns eight consecutive weight rows (four gate/up pairs of the gated epilogue); its eight warps take 128 elements of
+// every 1024 of K each.  A lane holds its four elements of all MT tokens in registers and carries the eight weight rows past
+// them, four rows at a time: 4 x MT sums of four products per lane, summed over the lanes by halving, over the slices of K
+// in a register and over the warps in shared memory in warp order.  Nine to sixteen tokens go in four parts (NH) past the same
+// weights.  Still plain 32-bit FMA.
+// Bound by the stream of the weights for up to four tokens (134 MB: 28 us, 4.7 TB/s; 43.5 us when every lane fetched the
+// activations again for every four rows), from eight on by the instructions of the products and the exchanges (134 MB at 8
+// tokens: 36 us against 46; at 16 tokens: 53 against 78; parts of 8 tokens there spill and take 65).  A slice of the eight rows (32 KB of float32 a CTA) is asked for before the dependency
+// wait, and a group's next slice as soon as its registers are free.
+// four products, the first two and the last two side by side in packed pairs of multiply-adds
+__device__ __forceinline__ float dot4_pairs(const float4& w, const float4& x) {
+    unsigned long long w01, w23, x01, x23;
+    float even, odd;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(w01) : "f"(w.x), "f"(w.y));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(w23) : "f"(w.z), "f"(w.w));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(x01) : "f"(x.x), "f"(x.y));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(x23) : "f"(x.z), "f"(x.w));
+    asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(w01) : "l"(x01));
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(w01) : "l"(w23), "l"(x23));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(even), "=f"(odd) : "l"(w01));
+    return even + odd;
+}
+
+template <typename TA, typename TW, typename TC, int MT, int NH>
+__global__ void __launch_bounds__(kFewThreads, 2)
 gemm_fewrows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W, int ldw, TC* __restrict__ C, int ldc,
                     int M, int N, int K, int epilogue, ProductExtras batch) {
+    constexpr int NV = 4 * MT;
     A += (size_t)blockIdx.z * batch.a;
     W += (size_t)blockIdx.z * batch.w;
     C += (size_t)blockIdx.z * batch.c;
-    __shared__ float part[kFewWarps][kFewRows * MT];
+    __shared__ float part[kFewWarps][NH * kFewRows * MT];   // of a warp: [half][row][token]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n0 = blockIdx.x * kFewRows;
-    const TW* w[kFewRows];
+    float4 wv[2][4];
+    auto load_group = [&](int g, int k) {   // rows beyond N are clamped: read, never stored
 #pragma unroll
-    for (int r = 0; r < kFewRows; ++r) w[r] = W + (size_t)min(n0 + r, N - 1) * ldw;   // clamped: read, never stored
-    float acc[kFewRows * MT];
+        for (int r = 0; r < 4; ++r)
+            wv[g][r] = k < K ? load4_once<TW>(W + (size_t)min(n0 + 4 * g + r, N - 1) * ldw + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    const int first = (warp * 32 + lane) * 4;
+    load_group(0, first);
+    load_group(1, first);
+    pdl_launch_dependents();
+    pdl_wait();
+    float total[NH][2];
 #pragma unroll
-    for (int i = 0; i < kFewRows * MT; ++i) acc[i] = 0.f;
-#pragma unroll 2
-    for (int k = (warp * 32 + lane) * 4; k < K; k += kFewWarps * 128) {
-        float4 wv[kFewRows];
+    for (int h = 0; h < NH; ++h) total[h][0] = total[h][1] = 0.f;
+    for (int k = first; k - first < K; k += kFewSlice) {   // (all lanes alike: the exchanges need the whole warp)
 #pragma unroll
-        for (int r = 0; r < kFewRows; ++r) wv[r] = load4<TW>(w[r] + k);
+        for (int h = 0; h < NH; ++h) {
+            float4 x[MT];
 #pragma unroll
-        for (int m = 0; m < MT; ++m) {
-            if (m < M) {
-                const float4 x = load4<TA>(A + (size_t)m * lda + k);
+            for (int m = 0; m < MT; ++m)
+                x[m] = k < K && h * MT + m < M ? load4<TA>(A + (size_t)(h * MT + m) * lda + k) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-                for (int r = 0; r < kFewRows; ++r)
-                    acc[r * MT + m] = fmaf(wv[r].w, x.w, fmaf(wv[r].z, x.z, fmaf(wv[r].y, x.y, fmaf(wv[r].x, x.x, acc[r * MT + m]))));
+            for (int g = 0; g < 2; ++g) {
+                float v[NV];
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+#pragma unroll
+                    for (int m = 0; m < MT; ++m)
+                        v[r * MT + m] = NH == 1 ? dot4_pairs(wv[g][r], x[m])
+                                                : fmaf(wv[g][r].w, x[m].w, fmaf(wv[g][r].z, x[m].z, fmaf(wv[g][r].y, x[m].y, wv[g][r].x * x[m].x)));
+                if (h == NH - 1) load_group(g, k + kFewSlice);
+                total[h][g] += reduce_by_halving<NV>(v, lane);
             }
         }
     }
-    // lane l ends up with sum number l (and l + 32 for 16 tokens) of this warp
+    if (lane % (32 / NV) == 0) {
 #pragma unroll
-    for (int b = 0; b < kFewRows * MT / 32; ++b) {
-        float v[32];
+        for (int h = 0; h < NH; ++h)
 #pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = acc[b * 32 + i];
-        part[warp][b * 32 + lane] = reduce_by_halving(v, lane);
+            for (int g = 0; g < 2; ++g) part[warp][(h * 2 + g) * NV + lane / (32 / NV)] = total[h][g];
     }
     __syncthreads();
-    // thread i < 4 * MT: row i / MT, token i % MT; the warps' sums are added in warp order
+    // thread i: half, row and token of sum number i; the warps' sums are added in warp order
     const int i = threadIdx.x;
-    if (i >= kFewRows * MT) return;
-    const int r = i / MT, m = i % MT, n = n0 + r;
+    if (i >= NH * kFewRows * MT) return;
+    const int r = i / MT % kFewRows, m = i / (MT * kFewRows) * MT + i % MT, n = n0 + r;
     float sum = 0.f;
 #pragma unroll
     for (int wp = 0; wp < kFewWarps; ++wp) sum += part[wp][i];
@@ -286,11 +337,10 @@ template <typename TA, typename TW, typename TC>
 static int launch_fewrows(const void* A, int lda, const void* W, int ldw, void* C, int ldc, int M, int N, int K, int epilogue,
                           int n_batch, ProductExtras batch, cudaStream_t stream) {
     const dim3 grid((N + kFewRows - 1) / kFewRows, 1, n_batch);
-    if (M <= 8)
-        gemm_fewrows_kernel<TA, TW, TC, 8><<<grid, kFewThreads, 0, stream>>>((const TA*)A, lda, (const TW*)W, ldw, (TC*)C, ldc, M, N, K, epilogue, batch);
-    else
-        gemm_fewrows_kernel<TA, TW, TC, 16><<<grid, kFewThreads, 0, stream>>>((const TA*)A, lda, (const TW*)W, ldw, (TC*)C, ldc, M, N, K, epilogue, batch);
-    return launch_status();
+    auto go = [&](auto kernel) {
+        return launch_pdl(kernel, grid, dim3(kFewThreads), 0, stream, (const TA*)A, lda, (const TW*)W, ldw, (TC*)C, ldc, M, N, K, epilogue, batch);
+    };
+    return M <= 4 ? go(gemm_fewrows_kernel<TA, TW, TC, 4, 1>) : M <= 8 ? go(gemm_fewrows_kernel<TA, TW, TC, 8, 1>) : go(gemm_fewrows_kernel<TA, TW, TC, 4, 4>);
 }
 
 }  // namespace b200

@@ -89,6 +89,32 @@ def test_products_that_stay_with_the_plain_kernels():
         assert bool((c == 0).all())
 
 
+@pytest.mark.parametrize("M", [1, 4, 5, 8, 9, 13, 16])
+@pytest.mark.parametrize("N, K", [(8, 1024), (10, 1028), (130, 2048), (6, 4), (1002, 8192), (24, 3000)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
+def test_products_of_few_rows(M, N, K, dtype):
+    """Below 4 + 5 + K / 1024 + 8 float32 additions to a sum, each of a half unit."""
+    o = ops()
+    g = torch.Generator().manual_seed(M * N + K)
+    a, w = torch.randn(M, K, generator=g).to(dtype).cuda(), (torch.randn(N, K, generator=g) / math.sqrt(K)).to(dtype).cuda()
+    bias = torch.randn(N, generator=g).cuda()
+    ref = a.double() @ w.double().t() + bias.double()
+    bound = (K / 1024 + 20) * EPS / 2 * (a.double().abs() @ w.double().abs().t() + bias.double().abs())
+    c = torch.empty(M, N, device="cuda")
+    o.gemm_generic(a, w, c, bias=bias)
+    assert bool(((c.double() - ref).abs() <= bound).all())
+    c0 = torch.randn(M, N, generator=g).cuda()
+    c = c0.clone()
+    o.gemm_generic(a, w, c, o.EPILOGUE_RESIDUAL_ADD, bias=bias)
+    assert bool(((c.double() - c0.double() - ref).abs() <= bound + EPS * (c0.abs().double() + ref.abs())).all())
+    h = torch.empty(M, N // 2, device="cuda")
+    o.gemm_generic(a, w, h, o.EPILOGUE_GATED_SILU, bias=bias)
+    gate, up = ref[:, 0::2], ref[:, 1::2]
+    want = torch.nn.functional.silu(gate) * up
+    slack = 1.2 * (bound[:, 0::2] * up.abs() + bound[:, 1::2] * gate.abs()) + 16 * EPS * want.abs() + 1e-9
+    assert bool(((h.double() - want).abs() <= slack).all())
+
+
 CUTS = [([5, 1, 100, 77], [5, 300, 100, 200]), ([70, 64, 65], [70, 64, 129]), ([130, 3], [400, 69])]
 
 
