@@ -79,6 +79,8 @@ attention_paged_kernel(const T* __restrict__ q, int q_row_stride, T* __restrict_
     float* red = s_s + kAttnThreads;        // [33]
     float* part = red + 33;                 // [4 warps][dim blocks * 32] partial outputs
 
+    pdl_launch_dependents();
+    pdl_wait();
     const int t = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = h / (n_heads / n_kv_heads);
     const int pos = positions[t];
@@ -209,6 +211,8 @@ template <typename T>
 __global__ void attention_paged_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                              T* __restrict__ out, int n_splits, int head_dim, int n_heads,
                                              const T* __restrict__ gate, int ld_gate) {
+    pdl_launch_dependents();
+    pdl_wait();
     const size_t row = blockIdx.x;
     const float gv = gate ? 1.0f / (1.0f + expf(-to_f32<T>(gate[(row / n_heads) * ld_gate + row % n_heads]))) : 1.f;
     const float* ml = part_ml + row * n_splits * 2;
@@ -247,11 +251,11 @@ extern "C" int b200_attention_paged(const void* q, int q_row_stride, void* out, 
     float* part_o = scratch;
     float* part_ml = scratch != nullptr ? scratch + (size_t)n_tokens * n_heads * n_splits * head_dim : nullptr;
     B200_DISPATCH_DTYPE(dtype, T,
-        b200::attention_paged_kernel<T><<<grid, b200::kAttnThreads, smem, stream>>>(
+        int st = b200::launch_pdl(b200::attention_paged_kernel<T>, grid, dim3(b200::kAttnThreads), smem, stream,
             (const T*)q, q_row_stride, (T*)out, positions, seq_ids, page_table, table_stride, (const T*)k_pool,
             (const T*)v_pool, n_heads, n_kv_heads, head_dim, window, part_o, part_ml, terms);
-        if (n_splits > 1)
-            b200::attention_paged_merge_kernel<T><<<n_tokens * n_heads, 64, 0, stream>>>(part_o, part_ml, (T*)out, n_splits, head_dim,
-                                                                                         n_heads, (const T*)gate, ld_gate));
-    return b200::launch_status();
+        if (st == 0 && n_splits > 1)
+            st = b200::launch_pdl(b200::attention_paged_merge_kernel<T>, dim3(n_tokens * n_heads), dim3(64), 0, stream, part_o, part_ml, (T*)out,
+                                  n_splits, head_dim, n_heads, (const T*)gate, ld_gate);
+        return st);
 }

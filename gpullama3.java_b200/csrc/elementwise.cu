@@ -20,6 +20,8 @@
 namespace b200 {
 
 __global__ void softcap_kernel(float* __restrict__ x, size_t n, float cap) {
+    pdl_launch_dependents();
+    pdl_wait();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         x[i] = cap * tanhf(x[i] / cap);
 }
@@ -257,8 +259,7 @@ extern "C" int b200_softcap_rows(float* x, long long n, float cap, cudaStream_t 
     if (n <= 0) return 0;
     if (!(cap > 0.f)) return b200::kErrBadArgument;
     const long long blocks = (n + 255) / 256;
-    b200::softcap_kernel<<<(int)(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, stream>>>(x, (size_t)n, cap);
-    return b200::launch_status();
+    return b200::launch_pdl(b200::softcap_kernel, dim3((int)(blocks < 148 * 16 ? blocks : 148 * 16)), dim3(256), 0, stream, x, (size_t)n, cap);
 }
 
 extern "C" int b200_gated_rmsnorm(const float* x, const float* w, const void* gate, int ld_gate, void* out, int dtype,

@@ -24,6 +24,8 @@ streams_combine_kernel(const float* __restrict__ x, float* out, const float* __r
     __shared__ float m_s[kMaxStreams * kMaxStreams], w_s[kMaxStreams];
     for (int i = threadIdx.x; i < s_in * s_out; i += kStreamThreads) m_s[i] = mix[i];
     for (int i = threadIdx.x; i < s_out; i += kStreamThreads) w_s[i] = (write != nullptr) ? write[i] : 0.f;
+    pdl_launch_dependents();
+    pdl_wait();
     __syncthreads();
     const int wv = width / VEC;
     for (size_t u = (size_t)blockIdx.x * kStreamThreads + threadIdx.x; u < n_units; u += (size_t)gridDim.x * kStreamThreads) {
@@ -89,6 +91,8 @@ streams_read_norm_kernel(const float* __restrict__ x, const float* __restrict__ 
     __shared__ float scratch[33];
     __shared__ float r_s[kMaxStreams];
     if (threadIdx.x < n_streams) r_s[threadIdx.x] = read[threadIdx.x];
+    pdl_launch_dependents();
+    pdl_wait();
     __syncthreads();
     const int r = blockIdx.x;
     const float* xr = x + (size_t)(rows ? rows[r] : r) * n_streams * width;
@@ -146,46 +150,55 @@ template <> struct StreamVec<1> {
     __device__ static void store(__nv_bfloat16* p, const float (&f)[1]) { p[0] = __float2bfloat16_rn(f[0]); }
 };
 
-// VEC columns per access (4 when the width and the pointers allow); a thread keeps the u of kStepKeep accesses in
-// registers (widths up to kStepKeep * VEC * 256) and forms u again from the new streams beyond that.
-constexpr int kStepKeep = 4;
+// A CTA of up to kStepThreads threads per token, VEC columns per access (4 when the width and the pointers allow).  A thread
+// asks for everything it reads of up to kStepKeep accesses before it writes anything (x is read and written through one pointer,
+// so the compiler cannot), keeps their u in registers (widths up to kStepKeep * VEC * kStepThreads) and forms u again from
+// the new streams beyond that.  S: the number of streams, or 0 for a number given at run time.
+// Bound by its bytes (2,048 tokens, three streams of 2,048: 142 MB in 36 us, launches by event; 50 us with 256 threads whose loads waited
+// for the stores before them).
+constexpr int kStepKeep = 2, kStepThreads = 512;
 
-template <typename TO, int VEC>
-__global__ void __launch_bounds__(kStreamThreads)
+template <typename TO, int VEC, int S>
+__global__ void __launch_bounds__(kStepThreads)
 streams_step_kernel(float* __restrict__ x, const float* __restrict__ mix, const float* __restrict__ write,
                     float* __restrict__ y, const float* __restrict__ read, const float* __restrict__ w,
-                    TO* __restrict__ out, int n_streams, int width, float eps) {
+                    TO* __restrict__ out, int streams, int width, float eps) {
+    constexpr int MAXS = S > 0 ? S : kMaxStreams;
+    const int n_streams = S > 0 ? S : streams, threads = blockDim.x;
     __shared__ float scratch[33];
     __shared__ float m_s[kMaxStreams * kMaxStreams], w_s[kMaxStreams], r_s[kMaxStreams];
-    for (int i = threadIdx.x; i < n_streams * n_streams; i += kStreamThreads) m_s[i] = mix[i];
+    for (int i = threadIdx.x; i < n_streams * n_streams; i += threads) m_s[i] = mix[i];   // (weights: before the wait)
     if (threadIdx.x < n_streams) {
         w_s[threadIdx.x] = write[threadIdx.x];
         r_s[threadIdx.x] = read != nullptr ? read[threadIdx.x] : 0.f;
     }
+    pdl_launch_dependents();
+    pdl_wait();
     __syncthreads();
     const size_t t = blockIdx.x;
     float* xr = x + t * n_streams * width;
     float* yr = y + t * width;
     const int units = width / VEC;
-    float keep[kStepKeep][VEC];
     float ss = 0.f;
-    auto column = [&](int c, float (&u)[VEC]) {
-        float in[kMaxStreams][VEC], yv[VEC], zero[VEC];
+    auto fetch = [&](int c, float (&in)[MAXS][VEC], float (&yv)[VEC]) {
 #pragma unroll
-        for (int a = 0; a < kMaxStreams; ++a)
+        for (int a = 0; a < MAXS; ++a)
             if (a < n_streams) StreamVec<VEC>::load(xr + (size_t)a * width + c, in[a]);
         StreamVec<VEC>::load(yr + c, yv);
+    };
+    auto mixed = [&](int c, const float (&in)[MAXS][VEC], const float (&yv)[VEC], float (&u)[VEC]) {
+        float zero[VEC];
 #pragma unroll
         for (int e = 0; e < VEC; ++e) zero[e] = u[e] = 0.f;
         StreamVec<VEC>::store(yr + c, zero);
 #pragma unroll
-        for (int j = 0; j < kMaxStreams; ++j) {
+        for (int j = 0; j < MAXS; ++j) {
             if (j >= n_streams) break;
             float acc[VEC];
 #pragma unroll
             for (int e = 0; e < VEC; ++e) acc[e] = 0.f;
 #pragma unroll
-            for (int a = 0; a < kMaxStreams; ++a) {
+            for (int a = 0; a < MAXS; ++a) {
                 if (a >= n_streams) break;
                 const float m = m_s[a * n_streams + j];
 #pragma unroll
@@ -199,18 +212,28 @@ streams_step_kernel(float* __restrict__ x, const float* __restrict__ mix, const 
             StreamVec<VEC>::store(xr + (size_t)j * width + c, acc);
         }
     };
+    float in[kStepKeep][MAXS][VEC], yv[kStepKeep][VEC], wv[kStepKeep][VEC], keep[kStepKeep][VEC];
 #pragma unroll
     for (int k = 0; k < kStepKeep; ++k) {
-        const int unit = k * kStreamThreads + threadIdx.x;
+        const int unit = k * threads + threadIdx.x;
+        if (unit < units) {
+            fetch(unit * VEC, in[k], yv[k]);
+            if (read != nullptr) StreamVec<VEC>::load(w + unit * VEC, wv[k]);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kStepKeep; ++k) {
+        const int unit = k * threads + threadIdx.x;
 #pragma unroll
         for (int e = 0; e < VEC; ++e) keep[k][e] = 0.f;
-        if (unit < units) column(unit * VEC, keep[k]);
+        if (unit < units) mixed(unit * VEC, in[k], yv[k], keep[k]);
 #pragma unroll
         for (int e = 0; e < VEC; ++e) ss += keep[k][e] * keep[k][e];
     }
-    for (int unit = kStepKeep * kStreamThreads + threadIdx.x; unit < units; unit += kStreamThreads) {
+    for (int unit = kStepKeep * threads + threadIdx.x; unit < units; unit += threads) {
         float u[VEC];
-        column(unit * VEC, u);
+        fetch(unit * VEC, in[0], yv[0]);
+        mixed(unit * VEC, in[0], yv[0], u);
 #pragma unroll
         for (int e = 0; e < VEC; ++e) ss += u[e] * u[e];
     }
@@ -220,18 +243,17 @@ streams_step_kernel(float* __restrict__ x, const float* __restrict__ mix, const 
     TO* o = out + t * width;
 #pragma unroll
     for (int k = 0; k < kStepKeep; ++k) {
-        const int unit = k * kStreamThreads + threadIdx.x;
+        const int unit = k * threads + threadIdx.x;
         if (unit < units) {
-            float wv[VEC], res[VEC];
-            StreamVec<VEC>::load(w + unit * VEC, wv);
+            float res[VEC];
 #pragma unroll
-            for (int e = 0; e < VEC; ++e) res[e] = wv[e] * (scale * keep[k][e]);
+            for (int e = 0; e < VEC; ++e) res[e] = wv[k][e] * (scale * keep[k][e]);
             StreamVec<VEC>::store(o + unit * VEC, res);
         }
     }
-    for (int unit = kStepKeep * kStreamThreads + threadIdx.x; unit < units; unit += kStreamThreads) {
-        float wv[VEC], res[VEC];   // beyond the kept columns u is formed again from the new streams (this thread wrote them)
-        StreamVec<VEC>::load(w + unit * VEC, wv);
+    for (int unit = kStepKeep * threads + threadIdx.x; unit < units; unit += threads) {
+        float wb[VEC], res[VEC];   // beyond the kept columns u is formed again from the new streams (this thread wrote them)
+        StreamVec<VEC>::load(w + unit * VEC, wb);
 #pragma unroll
         for (int e = 0; e < VEC; ++e) res[e] = 0.f;
         for (int j = 0; j < n_streams; ++j) {
@@ -241,9 +263,17 @@ streams_step_kernel(float* __restrict__ x, const float* __restrict__ mix, const 
             for (int e = 0; e < VEC; ++e) res[e] += r_s[j] * xv[e];
         }
 #pragma unroll
-        for (int e = 0; e < VEC; ++e) res[e] = wv[e] * (scale * res[e]);
+        for (int e = 0; e < VEC; ++e) res[e] = wb[e] * (scale * res[e]);
         StreamVec<VEC>::store(o + unit * VEC, res);
     }
+}
+
+template <typename TO, int VEC, int S>
+static int launch_streams_step(float* x, const float* mix, const float* write, float* y, const float* read, const float* w, void* out,
+                               int n_tokens, int n_streams, int width, float eps, cudaStream_t stream) {
+    const int units = (width / VEC + 31) / 32 * 32, threads = units < kStepThreads ? units : kStepThreads;
+    return launch_pdl(streams_step_kernel<TO, VEC, S>, dim3(n_tokens), dim3(threads), 0, stream, x, mix, write, y, read, w, (TO*)out,
+                      n_streams, width, eps);
 }
 
 }  // namespace b200
@@ -256,9 +286,14 @@ extern "C" int b200_streams_step(float* x, const float* mix, const float* write,
     if (read != nullptr && (w == nullptr || out == nullptr)) return b200::kErrBadArgument;
     const bool vec = width % 4 == 0 && (((uintptr_t)x | (uintptr_t)y | (uintptr_t)w | (uintptr_t)out) & 15) == 0;
     B200_DISPATCH_DTYPE(out_dtype, TO,
-        if (vec) b200::streams_step_kernel<TO, 4><<<n_tokens, b200::kStreamThreads, 0, stream>>>(x, mix, write, y, read, w, (TO*)out, n_streams, width, eps);
-        else b200::streams_step_kernel<TO, 1><<<n_tokens, b200::kStreamThreads, 0, stream>>>(x, mix, write, y, read, w, (TO*)out, n_streams, width, eps));
-    return b200::launch_status();
+        auto go = [&](auto launch) { return launch(x, mix, write, y, read, w, out, n_tokens, n_streams, width, eps, stream); };
+        if (!vec) return go(b200::launch_streams_step<TO, 1, 0>);
+        switch (n_streams) {
+            case 2: return go(b200::launch_streams_step<TO, 4, 2>);
+            case 3: return go(b200::launch_streams_step<TO, 4, 3>);
+            case 4: return go(b200::launch_streams_step<TO, 4, 4>);
+            default: return go(b200::launch_streams_step<TO, 4, 0>);
+        });
 }
 
 extern "C" int b200_streams_combine(const float* x, float* out, const float* mix, const float* write, const float* y,
@@ -270,9 +305,8 @@ extern "C" int b200_streams_combine(const float* x, float* out, const float* mix
     const size_t units = (size_t)n_tokens * width / (vec ? 4 : 1);
     const int grid = (int)((units + b200::kStreamThreads - 1) / b200::kStreamThreads < 148 * 16
                                ? (units + b200::kStreamThreads - 1) / b200::kStreamThreads : 148 * 16);
-    if (vec) b200::streams_combine_kernel<4><<<grid, b200::kStreamThreads, 0, stream>>>(x, out, mix, write, y, s_in, s_out, width, units);
-    else b200::streams_combine_kernel<1><<<grid, b200::kStreamThreads, 0, stream>>>(x, out, mix, write, y, s_in, s_out, width, units);
-    return b200::launch_status();
+    return b200::launch_pdl(vec ? b200::streams_combine_kernel<4> : b200::streams_combine_kernel<1>, dim3(grid), dim3(b200::kStreamThreads), 0,
+                            stream, x, out, mix, write, y, s_in, s_out, width, units);
 }
 
 extern "C" int b200_streams_read_norm(const float* x, const float* read, const float* w, void* out, int out_dtype,
@@ -281,7 +315,6 @@ extern "C" int b200_streams_read_norm(const float* x, const float* read, const f
     if (n_rows <= 0) return 0;
     if (n_streams < 1 || n_streams > b200::kMaxStreams || width < 1) return b200::kErrUnsupportedSize;
     B200_DISPATCH_DTYPE(out_dtype, TO,
-        b200::streams_read_norm_kernel<TO><<<n_rows, b200::kStreamThreads, 0, stream>>>(x, read, w, (TO*)out, rows,
-                                                                                       n_streams, width, eps));
-    return b200::launch_status();
+        return b200::launch_pdl(b200::streams_read_norm_kernel<TO>, dim3(n_rows), dim3(b200::kStreamThreads), 0, stream, x, read, w, (TO*)out,
+                                rows, n_streams, width, eps));
 }
