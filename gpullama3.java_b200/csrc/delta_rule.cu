@@ -267,6 +267,8 @@ causal_conv_single_kernel(const TI* __restrict__ x, int ld_x, const float* __res
                           float* __restrict__ state, size_t slot_stride, const int* __restrict__ slots,
                           const int* __restrict__ seq_ids, TO* __restrict__ out, int ld_out, int channels, int taps,
                           int activation, int add_input, int update_state) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int t = blockIdx.y;
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
     if (c >= channels) return;
@@ -345,6 +347,8 @@ __device__ __forceinline__ float softplus(float x) { return x > 20.f ? x : log1p
 template <typename T>
 __global__ void __launch_bounds__(128)
 delta_rule_prepare_kernel(PrepareArgs a) {
+    pdl_launch_dependents();
+    pdl_wait();
     const long long unit = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (unit >= (long long)a.n_tokens * a.heads) return;
@@ -414,6 +418,8 @@ __device__ __forceinline__ float silu_of(float z) { return z / (1.0f + expf(-z))
 template <typename T>
 __global__ void __launch_bounds__(128)
 linear_scan_prepare_kernel(LinearPrepareArgs a) {
+    pdl_launch_dependents();
+    pdl_wait();
     const long long unit = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (unit >= (long long)a.n_tokens * a.heads) return;
@@ -492,6 +498,8 @@ struct GatedPrepareArgs {
 template <typename T>
 __global__ void __launch_bounds__(128)
 gated_scan_prepare_kernel(GatedPrepareArgs a) {
+    pdl_launch_dependents();
+    pdl_wait();
     const long long unit = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (unit >= (long long)a.n_tokens * a.heads) return;
@@ -551,6 +559,8 @@ template <int RPT, int R, bool LINEAR>
 __global__ void __launch_bounds__(kScanThreads)
 delta_rule_scan_kernel(ScanArgs a) {
     extern __shared__ __align__(16) float smem[];
+    pdl_launch_dependents();
+    pdl_wait();
     constexpr int dpad = R * RPT, cols = kScanThreads / R;
     const int per_chunk = kChunk * a.row;
 
@@ -649,8 +659,9 @@ static int launch_scan(const ScanArgs& a, int n_seqs, cudaStream_t stream) {
         if (e != 0) return e;
     }
     dim3 grid((a.d_v + cols - 1) / cols, a.heads, n_seqs);
-    kernel<<<grid, kScanThreads, smem, stream>>>(a);
-    return launch_status();
+    // an early start for steps of a token or so a sequence: the CTAs of a long walk would settle unevenly over the SMs beside the
+    // predecessor's (2,048 tokens, 32 heads: 1.03 ms instead of 0.49)
+    return launch_pdl_cluster(kernel, grid, dim3(kScanThreads), smem, stream, dim3(1, 1, 1), a.n_tokens < 4 * n_seqs, a);
 }
 
 template <int RPT, bool LINEAR>
@@ -677,6 +688,332 @@ static int launch_scan_rows(const ScanArgs& a, int rpt, int lanes, int n_seqs, c
     return kErrUnsupportedSize;
 }
 
+// ---------------------------------------------------------------------------------------------------------------
+// The delta rule over long runs of tokens, kDeltaRun tokens at a time (key size 64).  The scan above is one chain of steps, a
+// token each, that no pipe of the GPU is busy with; a run of C tokens from a state S0 is instead a few small products.  With G_t
+// the product of the run's decays up to and with token t (per key channel), and j < t <= C:
+//     A[t, j] = beta_t sum_d k_t[d] k_j[d] G_t[d] / G_j[d]        B[t, j] = sum_d q_t[d] k_j[d] G_t[d] / G_j[d]   (and j = t)
+//     (1 + A) U = beta (V - (G k) S0)                             O = (G q) S0 + B U
+//     S_C = G_C S0 + sum_j (G_C / G_j k_j) u_j^T
+// (the form in which DeltaNet and its gated relatives are trained: Yang et al., "Parallelizing Linear Transformers with the
+// Delta Rule over Sequence Length", 2024).  The quotients are never formed as quotients: G_t / G_j is carried along as the product of the
+// decays between, so that nothing overflows however strong they are.
+//   delta_run_parts   a CTA per (run, head), all at once: the rows that the scan has prepared for it, here in shared memory; A and
+//                     B; (1 + A)^-1 applied to beta G k and beta V by forward substitution.  Leaves a row per token: G q,
+//                     (G_C / G_j) k, W = (1 + A)^-1 beta G k, U0 = (1 + A)^-1 beta V; B and G_C behind all rows.
+//   delta_run_carry   a CTA per (head, 16 columns, sequence) walks the runs: U = U0 - W S, O = (G q) S + B U, S <- G_C S + k^T U.
+// All sums are 32-bit multiply-adds.  A token that is not finite reaches itself and later tokens only, as in the scan.
+// Bound by latency and issue: 2,048 tokens, 32 heads of 64 by 64: 262 us (prepare and scan: 498); error against 64 bits 1.6e-7 of the
+// norm for the results, 1.3e-7 for the state (scan: 1.5e-7 and 1.2e-7).
+constexpr int kDeltaRun = 32, kDeltaKey = 64, kDeltaCols = 16;
+constexpr int kDeltaPitch = kDeltaKey + 4;
+
+struct DeltaRunArgs {
+    PrepareArgs in;         // what the rows are made of; rows: [heads, T, row], written here
+    float* b;               // [heads, T, kDeltaRun]
+    float* decay;           // [heads, runs, kDeltaKey]
+    float* state;
+    size_t slot_stride;
+    const int* slots;
+    const int* cu_seqlens;
+    float* out;             // [T, heads d_v]
+    int n_seqs, most_runs;
+};
+
+// run number `run` of the packed step: its first token and how many it has (0: there is no such run)
+__device__ __forceinline__ int delta_run_at(const DeltaRunArgs& a, int run, int& first) {
+    for (int s = 0; s < a.n_seqs; ++s) {
+        const int begin = a.cu_seqlens[s], n = a.cu_seqlens[s + 1] - begin, runs = (n + kDeltaRun - 1) / kDeltaRun;
+        if (run < runs) {
+            first = begin + run * kDeltaRun;
+            return min(kDeltaRun, n - run * kDeltaRun);
+        }
+        run -= runs;
+    }
+    return 0;
+}
+
+struct DeltaPartsSmem {
+    float q[kDeltaRun][kDeltaPitch], k[kDeltaRun][kDeltaPitch], g[kDeltaRun][kDeltaPitch];
+    float part[4][2][kDeltaRun][kDeltaRun + 1];   // per warp: its 16 channels' sums for A and B
+    float a[kDeltaRun][kDeltaRun + 4];
+    float beta[kDeltaRun];
+};
+
+template <typename T>
+__global__ void __launch_bounds__(128, 3)
+delta_run_parts_kernel(DeltaRunArgs a) {
+    extern __shared__ __align__(16) float smem[];
+    auto& sm = *reinterpret_cast<DeltaPartsSmem*>(smem);
+    const PrepareArgs& in = a.in;
+    const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const float neg_rate = -expf(in.a_log[h]);      // (weights: before the wait)
+    float bias[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) bias[e] = in.dt_bias[in.decay_per_head ? (size_t)h : (size_t)h * kDeltaKey + 32 * e + lane];
+    pdl_launch_dependents();
+    pdl_wait();
+    int first = 0;
+    const int m = delta_run_at(a, blockIdx.x, first);
+    if (m == 0) return;
+    const int kvh = h / (in.heads / in.kv_heads);
+    const T* qr = (const T*)in.qkv + (size_t)first * in.ld_qkv + (size_t)kvh * kDeltaKey;
+    const T* kr0 = qr + (size_t)in.kv_heads * kDeltaKey;
+    const T* vr = (const T*)in.qkv + (size_t)first * in.ld_qkv + 2 * (size_t)in.kv_heads * kDeltaKey + (size_t)h * in.d_v;
+    const T* dr = (const T*)in.decay + (size_t)first * in.ld_decay + (in.decay_per_head ? (size_t)h : (size_t)h * kDeltaKey);
+    float* rows = in.rows + ((size_t)h * in.n_tokens + first) * in.row;
+    // ---- unit rows of q and k, decays: eight tokens a warp, two channels a lane.  Tokens beyond the run's end: nothing, and no decay.
+#pragma unroll 2
+    for (int i = 0; i < kDeltaRun / 4; ++i) {
+        const int t = warp * (kDeltaRun / 4) + i;
+        float q[2], k[2], z[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            q[e] = t < m ? to_f32<T>(qr[(size_t)t * in.ld_qkv + 32 * e + lane]) : 0.f;
+            k[e] = t < m ? to_f32<T>(kr0[(size_t)t * in.ld_qkv + 32 * e + lane]) : 0.f;
+            z[e] = t < m ? to_f32<T>(dr[(size_t)t * in.ld_decay + (in.decay_per_head ? 0 : 32 * e + lane)]) : 0.f;
+        }
+        const float fq = in.q_scale / sqrtf(warp_sum(q[0] * q[0] + q[1] * q[1]) + in.unit_eps);
+        const float fk = 1.0f / sqrtf(warp_sum(k[0] * k[0] + k[1] * k[1]) + in.unit_eps);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            sm.q[t][32 * e + lane] = q[e] * fq;
+            sm.k[t][32 * e + lane] = k[e] * fk;
+            sm.g[t][32 * e + lane] = t < m ? expf(neg_rate * softplus(z[e] + bias[e])) : 1.f;
+        }
+    }
+    if (tid < kDeltaRun)
+        sm.beta[tid] = tid < m ? 1.0f / (1.0f + expf(-to_f32<T>(((const T*)in.beta)[(size_t)(first + tid) * in.ld_beta + h]))) : 0.f;
+    __syncthreads();
+    // ---- A and B: lane j carries k_j times the decays since, 16 channels a warp (lanes j > t hold nothing that is used)
+    {
+        const int d0 = warp * 16;
+        float kr[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) kr[i] = 0.f;
+#pragma unroll 2
+        for (int t = 0; t < m; ++t) {
+            float sa[2] = {0.f, 0.f}, sb[2] = {0.f, 0.f};
+#pragma unroll
+            for (int i = 0; i < 16; i += 4) {
+                const float4 g4 = *reinterpret_cast<const float4*>(&sm.g[t][d0 + i]), k4 = *reinterpret_cast<const float4*>(&sm.k[t][d0 + i]);
+                const float4 q4 = *reinterpret_cast<const float4*>(&sm.q[t][d0 + i]);
+                const float gv[4] = {g4.x, g4.y, g4.z, g4.w}, kv[4] = {k4.x, k4.y, k4.z, k4.w}, qv[4] = {q4.x, q4.y, q4.z, q4.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    kr[i + e] = lane == t ? kv[e] : kr[i + e] * gv[e];
+                    sa[e & 1] = fmaf(kv[e], kr[i + e], sa[e & 1]);
+                    sb[e & 1] = fmaf(qv[e], kr[i + e], sb[e & 1]);
+                }
+            }
+            sm.part[warp][0][t][lane] = sa[0] + sa[1];
+            sm.part[warp][1][t][lane] = sb[0] + sb[1];
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < m * kDeltaRun; i += 128) {
+        const int t = i / kDeltaRun, j = i % kDeltaRun;
+        const float sa = (sm.part[0][0][t][j] + sm.part[1][0][t][j]) + (sm.part[2][0][t][j] + sm.part[3][0][t][j]);
+        const float sb = (sm.part[0][1][t][j] + sm.part[1][1][t][j]) + (sm.part[2][1][t][j] + sm.part[3][1][t][j]);
+        sm.a[t][j] = j < t ? sm.beta[t] * sa : 0.f;
+        a.b[((size_t)h * in.n_tokens + first + t) * kDeltaRun + j] = j <= t ? sb : 0.f;
+    }
+    // ---- the first 64 threads: G forward (rows of q and k times it); the others: the decays still to come
+    const int c = tid % kDeltaKey;
+    float x[kDeltaRun];
+    if (tid < kDeltaKey) {
+        float decay = 1.f;
+#pragma unroll
+        for (int t = 0; t < kDeltaRun; ++t) {
+            decay *= sm.g[t][c];
+            if (t < m) rows[(size_t)t * in.row + c] = sm.q[t][c] * decay;
+            x[t] = sm.beta[t] * (sm.k[t][c] * decay);
+        }
+        a.decay[((size_t)h * a.most_runs + blockIdx.x) * kDeltaKey + c] = decay;
+    } else {
+        float decay = 1.f;
+#pragma unroll
+        for (int t = kDeltaRun - 1; t >= 0; --t) {
+            if (t < m) rows[(size_t)t * in.row + kDeltaKey + c] = sm.k[t][c] * decay;
+            decay *= sm.g[t][c];
+        }
+    }
+    __syncthreads();   // A is complete
+    // ---- forward substitution, a column a thread: the 64 columns of beta G k, then those of beta V
+    for (int col = tid; col < kDeltaKey + in.d_v; col += 128) {
+        float* dst = rows + 2 * kDeltaKey + col;
+        if (col >= kDeltaKey) {
+#pragma unroll
+            for (int t = 0; t < kDeltaRun; ++t) x[t] = t < m ? sm.beta[t] * to_f32<T>(vr[(size_t)t * in.ld_qkv + col - kDeltaKey]) : 0.f;
+        }
+#pragma unroll
+        for (int t = 0; t < kDeltaRun; ++t) {
+            float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int j = 0; j < t; j += 4) {
+                const float4 a4 = *reinterpret_cast<const float4*>(&sm.a[t][j]);
+                const float av[4] = {a4.x, a4.y, a4.z, a4.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) if (j + e < t) s[e] = fmaf(av[e], x[j + e], s[e]);
+            }
+            if (t < m) {
+                x[t] -= (s[0] + s[1]) + (s[2] + s[3]);
+                dst[(size_t)t * in.row] = x[t];
+            }
+        }
+    }
+}
+
+constexpr int kCarryThreads = 256;
+
+struct DeltaCarrySmem {
+    float q[2][kDeltaRun][kDeltaKey], k[2][kDeltaRun][kDeltaKey], w[2][kDeltaRun][kDeltaKey];
+    float u0[2][kDeltaRun][kDeltaCols], b[2][kDeltaRun][kDeltaRun], decay[2][kDeltaKey];
+    float s[kDeltaCols][kDeltaPitch];         // the state's columns
+    float u[kDeltaCols][kDeltaRun + 4];
+};
+
+__device__ __forceinline__ void fma4(float2& acc, const float4& x, const float4& y) {   // even and odd products side by side
+    unsigned long long x01, x23, y01, y23, &c = reinterpret_cast<unsigned long long&>(acc);
+    asm("mov.b64 %0, {%1, %2};" : "=l"(x01) : "f"(x.x), "f"(x.y));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(x23) : "f"(x.z), "f"(x.w));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(y01) : "f"(y.x), "f"(y.y));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(y23) : "f"(y.z), "f"(y.w));
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(x01), "l"(y01));
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(x23), "l"(y23));
+}
+
+// Thread (column tx, group ty of 16): tokens 2 ty, 2 ty + 1 of a run, rows 4 ty .. + 3 of the state's column.
+__global__ void __launch_bounds__(kCarryThreads)
+delta_run_carry_kernel(DeltaRunArgs a) {
+    extern __shared__ __align__(16) float smem[];
+    auto& sm = *reinterpret_cast<DeltaCarrySmem*>(smem);
+    pdl_launch_dependents();
+    pdl_wait();
+    const int h = blockIdx.y, seq = blockIdx.z, col0 = blockIdx.x * kDeltaCols, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int d_v = a.in.d_v, row = a.in.row;
+    const int begin = a.cu_seqlens[seq], n = a.cu_seqlens[seq + 1] - begin, runs = (n + kDeltaRun - 1) / kDeltaRun;
+    if (n <= 0) return;
+    int run0 = 0;
+    for (int s = 0; s < seq; ++s) run0 += (a.cu_seqlens[s + 1] - a.cu_seqlens[s] + kDeltaRun - 1) / kDeltaRun;
+    float* S_g = a.state + (size_t)a.slots[seq] * a.slot_stride + (size_t)h * kDeltaKey * d_v + col0 + tx;
+    float S[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) S[i] = S_g[(size_t)(4 * ty + i) * d_v];
+    *reinterpret_cast<float4*>(&sm.s[tx][4 * ty]) = make_float4(S[0], S[1], S[2], S[3]);
+    const size_t token0 = (size_t)h * a.in.n_tokens + begin;
+    // (tokens beyond a short run's end: rows of its last token, whose results are not used)
+    auto fetch = [&](int run, int buf) {
+        const int base = run * kDeltaRun, m = min(kDeltaRun, n - base);
+        const float* rows = a.in.rows + (token0 + base) * row;
+#pragma unroll
+        for (int i = 0; i < kDeltaRun * kDeltaKey / 4 / kCarryThreads; ++i) {
+            const int t = tid / (kDeltaKey / 4) + i * (kCarryThreads / (kDeltaKey / 4)), d = tid % (kDeltaKey / 4) * 4;
+            const float* r = rows + (size_t)min(t, m - 1) * row + d;
+            copy_async_16(&sm.w[buf][t][d], r + 2 * kDeltaKey);
+            copy_async_16(&sm.q[buf][t][d], r);
+            copy_async_16(&sm.k[buf][t][d], r + kDeltaKey);
+        }
+        const int tb = tid / (kDeltaRun / 4), jb = tid % (kDeltaRun / 4) * 4;
+        copy_async_16(&sm.b[buf][tb][jb], a.b + (token0 + base + min(tb, m - 1)) * kDeltaRun + jb);
+        if (tid < kDeltaRun * kDeltaCols / 4) {
+            const int t = tid / (kDeltaCols / 4), c = tid % (kDeltaCols / 4) * 4;
+            copy_async_16(&sm.u0[buf][t][c], rows + (size_t)min(t, m - 1) * row + 3 * kDeltaKey + col0 + c);
+        } else if (tid < kDeltaRun * kDeltaCols / 4 + kDeltaKey / 4) {
+            const int d = (tid - kDeltaRun * kDeltaCols / 4) * 4;
+            copy_async_16(&sm.decay[buf][d], a.decay + ((size_t)h * a.most_runs + run0 + run) * kDeltaKey + d);
+        }
+        copy_async_commit();
+    };
+    fetch(0, 0);
+    const int t0 = 2 * ty;
+    for (int run = 0; run < runs; ++run) {
+        const int buf = run & 1, m = min(kDeltaRun, n - run * kDeltaRun);
+        copy_async_wait<0>();
+        __syncthreads();       // this run's rows and the state's columns are there; the other buffer has been read
+        if (run + 1 < runs) fetch(run + 1, buf ^ 1);
+        // ---- U and the state's part of O
+        float2 ws[2], qs[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) ws[i] = qs[i] = make_float2(0.f, 0.f);
+#pragma unroll 8
+        for (int d = 0; d < kDeltaKey; d += 4) {
+            const float4 s4 = *reinterpret_cast<const float4*>(&sm.s[tx][d]);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                fma4(ws[i], *reinterpret_cast<const float4*>(&sm.w[buf][t0 + i][d]), s4);
+                fma4(qs[i], *reinterpret_cast<const float4*>(&sm.q[buf][t0 + i][d]), s4);
+            }
+        }
+        float u[2], o[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            u[i] = t0 + i < m ? sm.u0[buf][t0 + i][tx] - (ws[i].x + ws[i].y) : 0.f;
+            o[i] = qs[i].x + qs[i].y;
+        }
+        *reinterpret_cast<float2*>(&sm.u[tx][t0]) = make_float2(u[0], u[1]);
+        __syncthreads();
+        // ---- the state first (the next run waits for it)
+        float4 add = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 g4 = *reinterpret_cast<const float4*>(&sm.decay[buf][4 * ty]);
+#pragma unroll
+        for (int j = 0; j < kDeltaRun; j += 4) {
+            const float4 u4 = *reinterpret_cast<const float4*>(&sm.u[tx][j]);
+            const float uv[4] = {u4.x, u4.y, u4.z, u4.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float4 k4 = *reinterpret_cast<const float4*>(&sm.k[buf][j + e][4 * ty]);
+                add.x = fmaf(k4.x, uv[e], add.x); add.y = fmaf(k4.y, uv[e], add.y);
+                add.z = fmaf(k4.z, uv[e], add.z); add.w = fmaf(k4.w, uv[e], add.w);
+            }
+        }
+        S[0] = fmaf(S[0], g4.x, add.x); S[1] = fmaf(S[1], g4.y, add.y); S[2] = fmaf(S[2], g4.z, add.z); S[3] = fmaf(S[3], g4.w, add.w);
+        *reinterpret_cast<float4*>(&sm.s[tx][4 * ty]) = make_float4(S[0], S[1], S[2], S[3]);   // (last read before the barrier above)
+        // ---- O: whole fours of earlier tokens, then the rest one by one (no token is weighted that comes later)
+        const int whole = t0 & ~3;
+        float2 bu[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) bu[i] = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j < kDeltaRun - 4; j += 4) {
+            if (j < whole) {
+                const float4 u4 = *reinterpret_cast<const float4*>(&sm.u[tx][j]);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) fma4(bu[i], *reinterpret_cast<const float4*>(&sm.b[buf][t0 + i][j]), u4);
+            }
+        }
+        const float4 u4 = *reinterpret_cast<const float4*>(&sm.u[tx][whole]);
+        const float uv[4] = {u4.x, u4.y, u4.z, u4.w};
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const float4 b4 = *reinterpret_cast<const float4*>(&sm.b[buf][t0 + i][whole]);
+            const float bv[4] = {b4.x, b4.y, b4.z, b4.w};
+            float s = bu[i].x + bu[i].y;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) if (whole + j <= t0 + i) s = fmaf(bv[j], uv[j], s);
+            if (t0 + i < m) a.out[((size_t)begin + run * kDeltaRun + t0 + i) * a.in.heads * d_v + (size_t)h * d_v + col0 + tx] = o[i] + s;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) S_g[(size_t)(4 * ty + i) * d_v] = S[i];
+}
+
+template <typename T>
+static int launch_delta_runs(const DeltaRunArgs& a, cudaStream_t stream) {
+    static bool configured = false;
+    if (!configured) {
+        if (cudaFuncSetAttribute(delta_run_parts_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DeltaPartsSmem)) != cudaSuccess ||
+            cudaFuncSetAttribute(delta_run_carry_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DeltaCarrySmem)) != cudaSuccess)
+            return (int)cudaGetLastError();
+        configured = true;
+    }
+    const int st = launch_pdl(delta_run_parts_kernel<T>, dim3(a.most_runs, a.in.heads), dim3(128), sizeof(DeltaPartsSmem), stream, a);
+    if (st != 0) return st;
+    // (no early start: its long CTAs would settle two and three to an SM beside the predecessor's)
+    return launch_pdl_cluster(delta_run_carry_kernel, dim3(a.in.d_v / kDeltaCols, a.in.heads, a.n_seqs), dim3(kCarryThreads),
+                              sizeof(DeltaCarrySmem), stream, dim3(1, 1, 1), false, a);
+}
+
 }  // namespace b200
 
 extern "C" int b200_causal_conv_silu(const void* x, int ld_x, const float* w, float* state, long long slot_stride,
@@ -701,13 +1038,11 @@ extern "C" int b200_causal_conv_silu(const void* x, int ld_x, const float* w, fl
         const dim3 grid_s(((wide4 ? channels / 4 : channels) + 127) / 128, n_tokens);
         B200_DISPATCH_DTYPE(dtype, T,
             if (wide4)
-                b200::causal_conv_single_kernel<T, T, 4><<<grid_s, 128, 0, stream>>>((const T*)x, ld_x, w, nullptr, state, (size_t)slot_stride,
-                                                                                   slots, seq_ids, (T*)out, ld_out, channels, taps, 1, 0,
-                                                                                   update_state);
+                b200::launch_pdl(b200::causal_conv_single_kernel<T, T, 4>, grid_s, dim3(128), 0, stream, (const T*)x, ld_x, w, nullptr,
+                                 state, (size_t)slot_stride, slots, seq_ids, (T*)out, ld_out, channels, taps, 1, 0, update_state);
             else
-                b200::causal_conv_single_kernel<T, T, 1><<<grid_s, 128, 0, stream>>>((const T*)x, ld_x, w, nullptr, state, (size_t)slot_stride,
-                                                                                   slots, seq_ids, (T*)out, ld_out, channels, taps, 1, 0,
-                                                                                   update_state));
+                b200::launch_pdl(b200::causal_conv_single_kernel<T, T, 1>, grid_s, dim3(128), 0, stream, (const T*)x, ld_x, w, nullptr,
+                                 state, (size_t)slot_stride, slots, seq_ids, (T*)out, ld_out, channels, taps, 1, 0, update_state));
         return b200::launch_status();
     }
     if (runs) {
@@ -760,13 +1095,11 @@ extern "C" int b200_causal_conv(const void* x, int ld_x, int in_dtype, const flo
         B200_DISPATCH_DTYPE(in_dtype, TI,
             B200_DISPATCH_DTYPE2(out_dtype, TO,
                 if (wide4)
-                    b200::causal_conv_single_kernel<TI, TO, 4><<<grid_s, 128, 0, stream>>>((const TI*)x, ld_x, w, bias, state, (size_t)slot_stride,
-                                                                                         slots, seq_ids, (TO*)out, ld_out, channels, taps,
-                                                                                         activation, add_input, update_state);
+                    b200::launch_pdl(b200::causal_conv_single_kernel<TI, TO, 4>, grid_s, dim3(128), 0, stream, (const TI*)x, ld_x, w, bias,
+                                 state, (size_t)slot_stride, slots, seq_ids, (TO*)out, ld_out, channels, taps, activation, add_input, update_state);
                 else
-                    b200::causal_conv_single_kernel<TI, TO, 1><<<grid_s, 128, 0, stream>>>((const TI*)x, ld_x, w, bias, state, (size_t)slot_stride,
-                                                                                         slots, seq_ids, (TO*)out, ld_out, channels, taps,
-                                                                                         activation, add_input, update_state)));
+                    b200::launch_pdl(b200::causal_conv_single_kernel<TI, TO, 1>, grid_s, dim3(128), 0, stream, (const TI*)x, ld_x, w, bias,
+                                 state, (size_t)slot_stride, slots, seq_ids, (TO*)out, ld_out, channels, taps, activation, add_input, update_state)));
         return b200::launch_status();
     }
     B200_DISPATCH_DTYPE(in_dtype, TI,
@@ -820,11 +1153,24 @@ extern "C" int b200_delta_rule_row(int d_k, int d_v) {
     return (3 * rpt * lanes + d_v + 3 + 3) / 4 * 4;
 }
 
+// Floats of scratch behind those rows with which b200_delta_rule_scan takes runs of tokens instead of a token at a time; 0: it
+// does not.  Key size 64, whole tiles of columns.  The scan takes as long as its longest sequence (0.24 us a token) or, with warps
+// enough to fill the GPU, 0.105 us a token of 32 heads of 64 in all; runs take 0.11 us a token in all and half the scan's time for a
+// sequence alone.  Measured, scan and runs, 32 heads of 64: 1 x 64 tokens 21 and 25 us, 1 x 96 29 and 27, 1 x 2,048 498 and 262, 2 x
+// 512 160 and 122, 8 x 256 246 and 230, 16 x 128 218 and 232, 64 x 40 272 and 434.
+extern "C" long long b200_delta_rule_runs_scratch(int n_tokens, int n_seqs, int longest, int heads, int d_k, int d_v) {
+    if (n_tokens <= 0 || n_seqs <= 0 || d_k != b200::kDeltaKey || d_v % b200::kDeltaCols != 0) return 0;
+    if (longest < 96 || (long long)n_tokens * heads * d_v > 4096ll * longest) return 0;
+    const long long runs = n_tokens / b200::kDeltaRun + n_seqs;
+    return (long long)heads * ((long long)n_tokens * b200::kDeltaRun + runs * b200::kDeltaKey);
+}
+
 extern "C" int b200_delta_rule_scan(const void* qkv, int ld_qkv, const void* beta, int ld_beta, const void* decay,
                                     int ld_decay, const float* dt_bias, const float* a_log, float* state,
                                     long long slot_stride, const int* slots, const int* cu_seqlens, float* out,
-                                    float* scratch, int dtype, int n_tokens, int n_seqs, int heads, int kv_heads, int d_k,
-                                    int d_v, float q_scale, float unit_eps, int decay_per_head, cudaStream_t stream) {
+                                    float* scratch, float* runs_scratch, int dtype, int n_tokens, int n_seqs, int heads,
+                                    int kv_heads, int d_k, int d_v, float q_scale, float unit_eps, int decay_per_head,
+                                    cudaStream_t stream) {
     if (n_seqs <= 0 || n_tokens <= 0) return 0;
     if (heads < 1 || kv_heads < 1 || heads % kv_heads || d_k < 1 || d_v < 1 || n_seqs > 65535 || heads > 65535 || !scratch)
         return b200::kErrBadArgument;
@@ -834,9 +1180,17 @@ extern "C" int b200_delta_rule_scan(const void* qkv, int ld_qkv, const void* bet
     if ((uintptr_t)scratch % 16) return b200::kErrBadArgument;
     b200::PrepareArgs p = {qkv, ld_qkv, beta, ld_beta, decay, ld_decay, dt_bias, a_log, scratch, n_tokens, heads, kv_heads,
                            d_k, d_v, rpt * lanes, row, q_scale, unit_eps, decay_per_head ? 1 : 0};
+    if (runs_scratch != nullptr && rpt * lanes == b200::kDeltaKey && d_v % b200::kDeltaCols == 0) {
+        if ((uintptr_t)runs_scratch % 16) return b200::kErrBadArgument;
+        const int runs = n_tokens / b200::kDeltaRun + n_seqs;
+        const b200::DeltaRunArgs r = {p, runs_scratch, runs_scratch + (size_t)heads * n_tokens * b200::kDeltaRun, state, (size_t)slot_stride,
+                                      slots, cu_seqlens, out, n_seqs, runs};
+        B200_DISPATCH_DTYPE(dtype, T, return b200::launch_delta_runs<T>(r, stream));
+    }
     const long long units = (long long)n_tokens * heads;
     B200_DISPATCH_DTYPE(dtype, T,
-        b200::delta_rule_prepare_kernel<T><<<(unsigned)((units + 3) / 4), 128, 0, stream>>>(p));
+        const int st = b200::launch_pdl(b200::delta_rule_prepare_kernel<T>, dim3((unsigned)((units + 3) / 4)), dim3(128), 0, stream, p);
+        if (st != 0) return st);
     b200::ScanArgs a = {scratch, state, (size_t)slot_stride, slots, cu_seqlens, out, n_tokens, heads, d_k, d_v, row, -1, 0};
     return b200::launch_scan_rows<false>(a, rpt, lanes, n_seqs, stream);
 }
@@ -864,7 +1218,8 @@ extern "C" int b200_linear_scan(const void* q, int ld_q, const void* k, int ld_k
                                  step_scales_value ? 1 : 0, qk_silu, v_silu, pairs, inv_freq, positions};
     const long long units = (long long)n_tokens * heads;
     B200_DISPATCH_DTYPE(dtype, T,
-        b200::linear_scan_prepare_kernel<T><<<(unsigned)((units + 3) / 4), 128, 0, stream>>>(p));
+        const int st = b200::launch_pdl(b200::linear_scan_prepare_kernel<T>, dim3((unsigned)((units + 3) / 4)), dim3(128), 0, stream, p);
+        if (st != 0) return st);
     b200::ScanArgs a = {scratch, state, (size_t)slot_stride, slots, cu_seqlens, out, n_tokens, heads, d_k, d_v, row, -1, 0};
     return b200::launch_scan_rows<true>(a, rpt, lanes, n_seqs, stream);
 }
@@ -885,7 +1240,8 @@ extern "C" int b200_gated_scan(const void* q, int ld_q, const void* k, int ld_k,
                                 rpt * lanes, row, q_scale};
     const long long units = (long long)n_tokens * heads;
     B200_DISPATCH_DTYPE(dtype, T,
-        b200::gated_scan_prepare_kernel<T><<<(unsigned)((units + 3) / 4), 128, 0, stream>>>(p));
+        const int st = b200::launch_pdl(b200::gated_scan_prepare_kernel<T>, dim3((unsigned)((units + 3) / 4)), dim3(128), 0, stream, p);
+        if (st != 0) return st);
     b200::ScanArgs a = {scratch, state, (size_t)slot_stride, slots, cu_seqlens, out, n_tokens, heads, d_k, d_v + 1, row, sum_off, sum_stride};
     return b200::launch_scan_rows<true>(a, rpt, lanes, n_seqs, stream);
 }

@@ -131,8 +131,8 @@ _SIGNATURES = {
     "b200_causal_conv_silu": ("delta_rule", [c_void_p, c_int, c_void_p, c_void_p, ctypes.c_longlong, c_void_p, c_void_p,
                                              c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int]),
     "b200_delta_rule_scan": ("delta_rule", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
-                                            ctypes.c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
-                                            c_int, c_int, c_int, c_int, c_float, c_float, c_int]),
+                                            ctypes.c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
+                                            c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_int]),
     "b200_moe_route": ("moe", [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                                c_int, c_int, c_float, c_void_p, c_int, c_void_p, c_float]),
     "b200_moe_rows": ("moe", [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
@@ -1534,12 +1534,13 @@ def delta_rule_supported(d_k: int) -> bool:
 def delta_rule_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, dt_bias: torch.Tensor,
                     a_log: torch.Tensor, state: torch.Tensor, slots: torch.Tensor, cu_seqlens: torch.Tensor,
                     out: torch.Tensor, heads: int, kv_heads: int, d_k: int, d_v: int, q_scale: float,
-                    unit_eps: float, alloc=None, decay_per_head: bool = False) -> None:
+                    unit_eps: float, alloc=None, decay_per_head: bool = False, longest: int | None = None) -> None:
     """The gated delta rule over a packed step.  qkv [T, 2 kv_heads d_k + heads d_v] (after the convolution), beta
     [T, >= heads] and decay [T, >= heads d_k] as the projections leave them, state float32 [slots, >= heads d_k d_v]
     (updated in place), out float32 [T, heads d_v].  ``decay_per_head``: decay [T, >= heads] and dt_bias [heads], one
     decay for all key channels of a head.  ``alloc(shape, dtype)``: where the scan's scratch (a row of
-    32-bit numbers per token and head) comes from."""
+    32-bit numbers per token and head, and for long sequences a few dozen more) comes from.  ``longest``: the most tokens of
+    one sequence, where the caller knows it: long ones are taken in runs of tokens."""
     _dev(qkv, beta, decay, dt_bias, a_log, state, slots, cu_seqlens, out)
     assert qkv.dtype == beta.dtype == decay.dtype and qkv.stride(1) == beta.stride(1) == decay.stride(1) == 1
     assert dt_bias.dtype == a_log.dtype == state.dtype == out.dtype == torch.float32 and out.is_contiguous()
@@ -1548,12 +1549,18 @@ def delta_rule_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, 
     assert state.shape[1] >= heads * d_k * d_v and out.shape[1] == heads * d_v and out.shape[0] == qkv.shape[0]
     lib = library("delta_rule")
     shape = (heads, qkv.shape[0], int(lib.b200_delta_rule_row(c_int(d_k), c_int(d_v))))
-    scratch = alloc(shape, torch.float32) if alloc is not None else torch.empty(shape, dtype=torch.float32, device=qkv.device)
+    if alloc is None:
+        alloc = lambda shape, dtype: torch.empty(shape, dtype=dtype, device=qkv.device)
+    scratch = alloc(shape, torch.float32)
+    lib.b200_delta_rule_runs_scratch.restype = ctypes.c_longlong
+    n_tokens, n_seqs = qkv.shape[0], slots.numel()
+    more = lib.b200_delta_rule_runs_scratch(n_tokens, n_seqs, longest or -(-n_tokens // n_seqs), heads, d_k, d_v) if n_seqs else 0
+    runs_scratch = alloc((more,), torch.float32) if more else None
     _check(_fn("b200_delta_rule_scan")(qkv.data_ptr(), qkv.stride(0), beta.data_ptr(), beta.stride(0), decay.data_ptr(),
                                        decay.stride(0), dt_bias.data_ptr(), a_log.data_ptr(), state.data_ptr(),
                                        state.stride(0), slots.data_ptr(), cu_seqlens.data_ptr(), out.data_ptr(),
-                                       scratch.data_ptr(), dtype_code(qkv.dtype), qkv.shape[0], slots.numel(), heads,
-                                       kv_heads, d_k, d_v, float(q_scale), float(unit_eps),
+                                       scratch.data_ptr(), runs_scratch.data_ptr() if more else None, dtype_code(qkv.dtype),
+                                       n_tokens, n_seqs, heads, kv_heads, d_k, d_v, float(q_scale), float(unit_eps),
                                        1 if decay_per_head else 0, _stream()), "delta_rule_scan")
 
 
