@@ -118,26 +118,37 @@ attention_paged_kernel(const T* __restrict__ q, int q_row_stride, T* __restrict_
     const int vecs = head_dim / E;           // 16-byte pieces per key row
 
     for (int base = lo; base <= last; base += kAttnThreads) {
-        // ---- scores of this warp's 32 keys, eight keys per step
+        // ---- scores of this warp's 32 keys: eight keys per load, four loads (a lane's four keys) side by side
         const int wbase = base + warp * 32;
-#pragma unroll 1
-        for (int k8 = 0; k8 < 32; k8 += 8) {
-            const int key = wbase + k8 + (lane >> 2);
-            float dot = 0.f;
-            if (key <= last) {
-                const int j = key < n_keep ? key : key + shift;
-                const T* kr = k_pool + (size_t)pages[j / kPageTokens] * page_stride + head_off +
-                              (size_t)(j % kPageTokens) * head_dim;
-                for (int v = sub; v < vecs; v += 4) {
-                    float f[E];
-                    Vec16<T>::load(kr + v * E, f);
+        const T* kr[4];
+        float dot[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-                    for (int e = 0; e < E; ++e) dot += q_s[v * E + e] * f[e];
+        for (int i = 0; i < 4; ++i) {
+            const int key = wbase + 8 * i + (lane >> 2), j = key < n_keep ? key : key + shift;
+            kr[i] = key <= last ? k_pool + (size_t)pages[j / kPageTokens] * page_stride + head_off + (size_t)(j % kPageTokens) * head_dim : nullptr;
+        }
+#pragma unroll 2
+        for (int v = sub; v < vecs; v += 4) {
+            float f[4][E];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (kr[i] != nullptr) {
+                    Vec16<T>::load(kr[i] + v * E, f[i]);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < E; ++e) f[i][e] = 0.f;
                 }
             }
-            dot += __shfl_xor_sync(0xffffffffu, dot, 1);
-            dot += __shfl_xor_sync(0xffffffffu, dot, 2);
-            if (sub == 0) s_s[warp * 32 + k8 + (lane >> 2)] = dot;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int e = 0; e < E; ++e) dot[i] += q_s[v * E + e] * f[i][e];
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            dot[i] += __shfl_xor_sync(0xffffffffu, dot[i], 1);
+            dot[i] += __shfl_xor_sync(0xffffffffu, dot[i], 2);
+            if (sub == 0) s_s[warp * 32 + 8 * i + (lane >> 2)] = dot[i];
         }
         __syncwarp();
         const int key = base + tid;          // from here on a thread is a key

@@ -234,15 +234,6 @@ __device__ __forceinline__ float reduce_by_halving(float (&v)[NV], int lane) {
     return v[0];
 }
 
-// A CTA owns eight consecutive weight rows (four gate/up pairs of the gated epilogue); its eight warps take 128 elements of
-// every 1024 of K each.  A lane holds its four elements of all MT tokens in registers and carries the eight weight rows past
-// them, four rows at a time: 4 x MT sums of four products per lane, summed over the lanes by halving, over the slices of K
-// in a register and over the warps in shared memory in warp order.  Nine to sixteen tokens go in four parts (NH) past the same
-// weights.  Still plain 32-bit FMA.
-// Bound by the stream of the weights for up to four tokens (134 MB: 28 us, 4.7 TB/s; 43.5 us when every lane fetched the
-// activations again for every four rows), from eight on by the instructions of the products and the exchanges (134 MB at 8
-// tokens: 36 us against 46; at 16 tokens: 53 against 78; parts of 8 tokens there spill and take 65).  A slice of the eight rows (32 KB of float32 a CTA) is asked for before the dependency
-// wait, and a group's next slice as soon as its registers are free.
 // four products, the first two and the last two side by side in packed pairs of multiply-adds
 __device__ __forceinline__ float dot4_pairs(const float4& w, const float4& x) {
     unsigned long long w01, w23, x01, x23;
@@ -257,6 +248,16 @@ __device__ __forceinline__ float dot4_pairs(const float4& w, const float4& x) {
     return even + odd;
 }
 
+// A CTA owns eight consecutive weight rows (four gate/up pairs of the gated epilogue); its eight warps take 128 elements of
+// every 1024 of K each.  A lane holds its four elements of all MT tokens in registers and carries the eight weight rows past
+// them, four rows at a time: 4 x MT sums of four products per lane, summed over the lanes by halving, over the slices of K
+// in a register and over the warps in shared memory in warp order.  Nine to sixteen tokens go in four parts (NH) past the same
+// weights.  Still plain 32-bit FMA.
+// Bound by the stream of the weights for up to four tokens (134 MB: 28 us, 4.7 TB/s; 43.5 us when every lane fetched the
+// activations again for every four rows), from eight on by the instructions of the products and the exchanges (134 MB at 8
+// tokens: 36 us against 46; at 16 tokens: 53 against 78; parts of 8 tokens there spill and take 65).  A slice of the eight rows (32 KB
+// of float32 a CTA) is asked for before the dependency wait, and a group's next slice as soon as its registers are free.  (Sums kept over
+// all slices, so that the lanes exchange once a CTA, need the activations again for the second group: 48 us at 8 tokens.)
 template <typename TA, typename TW, typename TC, int MT, int NH>
 __global__ void __launch_bounds__(kFewThreads, 2)
 gemm_fewrows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W, int ldw, TC* __restrict__ C, int ldc,

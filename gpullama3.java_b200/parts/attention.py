@@ -264,7 +264,8 @@ def attend(shape, qkv: torch.Tensor, out: torch.Tensor, ctx: StepContext, table:
         return
     rows = qkv.shape[0] * shape.n_heads
     reach = min(ctx.capacity(cache.group), _reach(shape) or ctx.capacity(cache.group))
-    splits = 1 if rows >= 1024 else max(1, min(16, 1024 // rows, reach // 512))
+    # spans of at least one tile of 128 keys, up to two thousand CTAs (of which a GPU holds some 1,800 at a time)
+    splits = 1 if rows >= 2048 else max(1, min(16, 2048 // rows, reach // 128))
     ops.attention_paged(qkv, qkv.shape[1], out, ctx.positions, ctx.seq_ids, table, cache.k, cache.v,
                         shape.n_heads, shape.n_kv_heads, shape.head_dim, shape.window or 0, n_splits=splits,
                         keep_first=shape.keep_first, **terms)
