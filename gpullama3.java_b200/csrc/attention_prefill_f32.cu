@@ -13,9 +13,10 @@
 // padded by four floats, so that 16 lanes that read 16 rows meet no bank twice.  Keys and values have one buffer each, refilled
 // (cp.async) as soon as they are read: the next page's keys arrive during the softmax and the output, its values during
 // the next scores.  Two or three CTAs share an SM and fill each other's waits.
-// Bound by the multiply-add units and their operands from shared memory: 2,048 tokens, 32 heads of 64: 0.73 ms = 24 TFLOP/s of
-// needed work (the plain kernel: 4.32 ms); eight prompts of 256: 127 us (773); 64 tokens behind 1,984: 261 us (330).  Sums over 32
-// dimensions and over a page at a time keep the error at the plain kernel's (3e-7 of the norm; one chain over all keys: 7e-7, no faster).
+// Bound by the multiply-add units and their operands from shared memory: 2,048 tokens, 32 heads of 64: 0.53 ms = 32 TFLOP/s of
+// needed work (the plain kernel: 4.32 ms; 0.73 with the tiles of one head after those of another, an SM's share of the work then 0.74 to 1.36
+// of the mean); eight prompts of 256: 125 us (773); 64 tokens behind 1,984: 264 us (330).  Sums over 32 dimensions and over a page at a
+// time keep the error at the plain kernel's (3e-7 of the norm; one chain over all keys: 7e-7, no faster).
 //
 // Terms as in the plain kernel (window, chunk, slopes, sinks, gate, softcap; not keep_first).  Values of keys past a
 // sequence's end are read as zeros.  A key that some row of the tile must not see has probability 0 there, and 0 times a value that is
@@ -68,12 +69,13 @@ attention_prefill_f32_kernel(const PrefillF32Args a) {
     extern __shared__ __align__(16) float smem_f[];
     auto& sm = *reinterpret_cast<PrefillF32Smem<D, RT>*>(smem_f);
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int g = blockIdx.y, seq = blockIdx.z, group = a.n_heads / a.n_kv_heads;
+    // tiles in order of falling length over all kv heads: the long ones start together and the short ones fill the end
+    const int g = blockIdx.x % a.n_kv_heads, seq = blockIdx.y, group = a.n_heads / a.n_kv_heads;
     pdl_launch_dependents();
     pdl_wait();
     const int begin = a.cu_seqlens[seq], q_len = a.cu_seqlens[seq + 1] - begin, kv_len = a.kv_lens[seq];
     const int n_rows = q_len * group;
-    const int row0 = (int)(gridDim.x - 1 - blockIdx.x) * BQ;    // the rows with the most keys first
+    const int row0 = ((int)gridDim.x / a.n_kv_heads - 1 - (int)blockIdx.x / a.n_kv_heads) * BQ;
     if (row0 >= n_rows) return;
     const int pos0 = kv_len - q_len;                             // position of the sequence's first token of the pass
     const int* pages = a.page_table + (size_t)seq * a.table_stride;
@@ -265,7 +267,7 @@ static int launch_prefill_f32(const PrefillF32Args& a, int n_seqs, int max_q_len
         configured = true;
     }
     const long long rows = (long long)max_q_len * (a.n_heads / a.n_kv_heads);
-    return launch_pdl(kernel, dim3((unsigned)((rows + BQ - 1) / BQ), a.n_kv_heads, n_seqs), dim3(kPfThreads), smem, stream, a);
+    return launch_pdl(kernel, dim3((unsigned)((rows + BQ - 1) / BQ) * a.n_kv_heads, n_seqs), dim3(kPfThreads), smem, stream, a);
 }
 
 }  // namespace b200
@@ -283,7 +285,7 @@ extern "C" int b200_attention_prefill_f32(const void* q, int q_row_stride, void*
     if (!(softcap >= 0.f) || chunk < 0 || (chunk > 0 && window > 0)) return kErrBadArgument;
     if (n_kv_heads <= 0 || n_heads % n_kv_heads != 0) return kErrBadArgument;
     if (q_row_stride % 4 != 0 || (((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool) & 15)) return kErrUnsupportedSize;
-    if (n_seqs > 65535 || n_kv_heads > 65535 || (long long)max_q_len * (n_heads / n_kv_heads) > 0x7fffff00ll) return kErrUnsupportedSize;
+    if (n_seqs > 65535 || (long long)max_q_len * n_heads > 0x7fffff00ll) return kErrUnsupportedSize;
     PrefillF32Args a = {};
     a.q = (const float*)q; a.out = (float*)out; a.cu_seqlens = cu_seqlens; a.kv_lens = kv_lens; a.page_table = page_table;
     a.k_pool = (const float*)k_pool; a.v_pool = (const float*)v_pool; a.slopes = slopes; a.sinks = sinks; a.gate = (const float*)gate;
