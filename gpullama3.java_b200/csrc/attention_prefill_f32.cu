@@ -18,6 +18,9 @@
 // of the mean); eight prompts of 256: 125 us (773); 64 tokens behind 1,984: 264 us (330).  Sums over 32 dimensions and over a page at a
 // time keep the error at the plain kernel's (3e-7 of the norm; one chain over all keys: 7e-7, no faster).
 //
+// Decode steps (one token a sequence) take the same kernel with one or two rows a group and their pages cut into spans, merged by a
+// second kernel: 8 sequences of 500 keys, 32 heads of 64: 20 us a layer, launches by event (35 with the plain kernel in spans of a tile).
+//
 // Terms as in the plain kernel (window, chunk, slopes, sinks, gate, softcap; not keep_first).  Values of keys past a
 // sequence's end are read as zeros.  A key that some row of the tile must not see has probability 0 there, and 0 times a value that is
 // not finite is not 0: a page with such keys and such values is summed key by key, over the keys each row sees.
@@ -41,6 +44,8 @@ struct PrefillF32Args {
     const float* gate;
     int q_row_stride, table_stride, n_heads, n_kv_heads, window, chunk, ld_gate;
     float softcap;
+    float* part_o;          // SPANS: [row][span][D] sums, row = token * n_heads + head
+    float* part_ml;         // SPANS: [row][span][2] maximum and sum of exponentials
 };
 
 __device__ __forceinline__ void fma_pair(float2& acc, float ax, float ay, float bx, float by) {
@@ -62,8 +67,10 @@ struct PrefillF32Smem {
     float p[8 * RT][kPfPitch];
 };
 
-template <int D, int RT>
-__global__ void __launch_bounds__(kPfThreads, D <= 64 ? 3 : 2)
+// SPANS: the pages are shared out among gridDim.z CTAs, which leave unnormalised results (decode steps: one row of queries per
+// sequence and kv head, RT = 1 or 2, and nothing else to fill the GPU with).
+template <int D, int RT, bool SPANS>
+__global__ void __launch_bounds__(kPfThreads, SPANS ? 4 : D <= 64 ? 3 : 2)
 attention_prefill_f32_kernel(const PrefillF32Args a) {
     constexpr int BQ = 8 * RT, DJ = D / 16;
     extern __shared__ __align__(16) float smem_f[];
@@ -83,7 +90,13 @@ attention_prefill_f32_kernel(const PrefillF32Args a) {
     auto first_of = [&](int pos) { return a.chunk > 0 ? pos - pos % a.chunk : a.window > 0 ? max(0, pos - a.window + 1) : 0; };
     const int pos_lo = pos0 + row0 / group, pos_hi = pos0 + min(row0 + BQ - 1, n_rows - 1) / group;
     const int first_lo = first_of(pos_lo), first_hi = first_of(pos_hi);
-    const int page_end = pos_hi / kPageTokens + 1;
+    int page = first_lo / kPageTokens, page_end = pos_hi / kPageTokens + 1;
+    const int span = SPANS ? blockIdx.z : 0, n_spans = SPANS ? gridDim.z : 1;
+    if (SPANS) {
+        const int each = (page_end - page + n_spans - 1) / n_spans;
+        page += span * each;
+        page_end = min(page_end, page + each);     // (a span may be empty)
+    }
 
     auto fetch_keys = [&](int page) {
         const float* src = a.k_pool + (size_t)pages[page] * page_stride + head_off;
@@ -97,10 +110,9 @@ attention_prefill_f32_kernel(const PrefillF32Args a) {
             copy16_async(&sm.v[c / 16][key], src + (size_t)c * 4, 4 * min(4, max(0, kv_len - page * kPageTokens - key)));
         }
     };
-    int page = first_lo / kPageTokens;
-    fetch_keys(page);
+    if (!SPANS || page < page_end) fetch_keys(page);
     asm volatile("cp.async.commit_group;" ::: "memory");
-    fetch_values(page);
+    if (!SPANS || page < page_end) fetch_values(page);
     asm volatile("cp.async.commit_group;" ::: "memory");
     for (int c = tid; c < BQ * D / 4; c += kPfThreads) {
         const int r = min(row0 + c / (D / 4), n_rows - 1), d = c % (D / 4) * 4;
@@ -112,8 +124,8 @@ attention_prefill_f32_kernel(const PrefillF32Args a) {
 #pragma unroll
     for (int i = 0; i < RT; ++i) {
         const int r = min(row0 + ty * RT + i, n_rows - 1);
-        m_run[i] = a.sinks ? a.sinks[g * group + r % group] : -INFINITY;
-        l_run[i] = a.sinks && tx == 0 ? 1.f : 0.f;
+        m_run[i] = a.sinks && span == 0 ? a.sinks[g * group + r % group] : -INFINITY;
+        l_run[i] = a.sinks && span == 0 && tx == 0 ? 1.f : 0.f;
 #pragma unroll
         for (int j = 0; j < DJ; ++j) o[i][j] = 0.f;
     }
@@ -195,7 +207,7 @@ attention_prefill_f32_kernel(const PrefillF32Args a) {
         __syncthreads();
         // ---- output
         int odd_values = 0;
-        if (masked) {
+        if (min(base + kPageTokens, kv_len) - 1 > pos_lo || base < first_hi) {   // keys of the sequence that some row must not see
             bool bad = false;
             for (int c = tid; c < D * kPageTokens; c += kPfThreads) bad |= !isfinite(sm.v[c / kPageTokens][c % kPageTokens]);
             odd_values = __syncthreads_or(bad);
@@ -249,6 +261,13 @@ attention_prefill_f32_kernel(const PrefillF32Args a) {
         const int r = row0 + ty * RT + i;
         if (r >= n_rows) continue;
         const int t = begin + r / group, h = g * group + r % group;
+        if (SPANS) {
+            const size_t part = ((size_t)t * a.n_heads + h) * n_spans + span;
+#pragma unroll
+            for (int j = 0; j < DJ; ++j) a.part_o[part * D + tx + 16 * j] = o[i][j];
+            if (tx == 0) { a.part_ml[part * 2] = m_run[i]; a.part_ml[part * 2 + 1] = l; }
+            continue;
+        }
         const float gate = a.gate ? 1.0f / (1.0f + expf(-a.gate[(size_t)t * a.ld_gate + h])) : 1.f;
         float* dst = a.out + ((size_t)t * a.n_heads + h) * D;
 #pragma unroll
@@ -256,11 +275,70 @@ attention_prefill_f32_kernel(const PrefillF32Args a) {
     }
 }
 
+// out[row] = sum_s o_s exp(m_s - m) / sum_s l_s exp(m_s - m) over the spans of a (token, head) row, in span order; a thread per
+// dimension, everything asked for at once
+constexpr int kMostSpans = 16;
+
+__global__ void __launch_bounds__(128)
+attention_spans_merge_f32_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, float* __restrict__ out,
+                                 int n_spans, int head_dim, int n_heads, const float* __restrict__ gate, int ld_gate) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const size_t row = blockIdx.x;
+    const int d = threadIdx.x;
+    if (d >= head_dim) return;
+    const float* ml = part_ml + row * n_spans * 2;
+    float ms[kMostSpans], ls[kMostSpans], po[kMostSpans];
+#pragma unroll
+    for (int s = 0; s < kMostSpans; ++s) {
+        const bool in = s < n_spans;
+        ms[s] = in ? ml[2 * s] : -INFINITY;
+        ls[s] = in ? ml[2 * s + 1] : 0.f;
+        po[s] = in ? part_o[(row * n_spans + s) * head_dim + d] : 0.f;
+    }
+    const float gv = gate ? 1.0f / (1.0f + expf(-gate[(row / n_heads) * ld_gate + row % n_heads])) : 1.f;
+    float m = -INFINITY;
+#pragma unroll
+    for (int s = 0; s < kMostSpans; ++s) m = fmaxf(m, ms[s]);
+    float l = 0.f, acc = 0.f;
+#pragma unroll
+    for (int s = 0; s < kMostSpans; ++s) {
+        if (s >= n_spans) break;
+        const float f = ms[s] == -INFINITY ? 0.f : expf(ms[s] - m);
+        l += ls[s] * f;
+        acc += po[s] * f;
+    }
+    out[row * head_dim + d] = acc / l * gv;
+}
+
+template <int D, int RT>
+static int launch_spans_f32(PrefillF32Args a, int n_seqs, int n_spans, float* scratch, cudaStream_t stream) {
+    const size_t smem = sizeof(PrefillF32Smem<D, RT>);
+    auto kernel = attention_prefill_f32_kernel<D, RT, true>;
+    static bool configured = false;
+    if (!configured) {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return (int)cudaGetLastError();
+        configured = true;
+    }
+    a.part_o = scratch;
+    a.part_ml = scratch + (size_t)n_seqs * a.n_heads * n_spans * D;
+    const int st = launch_pdl(kernel, dim3(a.n_kv_heads, n_seqs, n_spans), dim3(kPfThreads), smem, stream, a);
+    if (st != 0) return st;
+    return launch_pdl(attention_spans_merge_f32_kernel, dim3((unsigned)(n_seqs * a.n_heads)), dim3(D <= 64 ? 64 : 128), 0, stream, a.part_o, a.part_ml,
+                      a.out, n_spans, D, a.n_heads, a.gate, a.ld_gate);
+}
+
+template <int D>
+static int spans_f32_of(const PrefillF32Args& a, int n_seqs, int n_spans, float* scratch, cudaStream_t stream) {
+    if (a.n_heads / a.n_kv_heads <= 8) return launch_spans_f32<D, 1>(a, n_seqs, n_spans, scratch, stream);
+    return launch_spans_f32<D, 2>(a, n_seqs, n_spans, scratch, stream);
+}
+
 template <int D, int RT>
 static int launch_prefill_f32(const PrefillF32Args& a, int n_seqs, int max_q_len, cudaStream_t stream) {
     constexpr int BQ = 8 * RT;
     const size_t smem = sizeof(PrefillF32Smem<D, RT>);
-    auto kernel = attention_prefill_f32_kernel<D, RT>;
+    auto kernel = attention_prefill_f32_kernel<D, RT, false>;
     static bool configured = false;
     if (!configured) {
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return (int)cudaGetLastError();
@@ -272,14 +350,25 @@ static int launch_prefill_f32(const PrefillF32Args& a, int n_seqs, int max_q_len
 
 }  // namespace b200
 
+// How many spans of pages a decode step's attention is cut into (every sequence brings one token, `reach` keys at most), or 0: the
+// plain kernel has it (more heads to a kv head than a tile of this kernel's has rows).  About five CTAs an SM, a page each at least.
+extern "C" int b200_attention_decode_f32_spans(int n_seqs, int n_heads, int n_kv_heads, int reach) {
+    if (n_seqs <= 0 || n_kv_heads <= 0 || n_heads / n_kv_heads > 16) return 0;
+    const long long ctas = (long long)n_seqs * n_kv_heads;
+    const long long want = (5ll * b200::device_sm_count() + ctas - 1) / ctas, pages = ((long long)reach + b200::kPageTokens - 1) / b200::kPageTokens;
+    const long long spans = want < pages ? want : pages;
+    return (int)(spans < 1 ? 1 : spans > b200::kMostSpans ? b200::kMostSpans : spans);
+}
+
 // Queries: the first n_heads head_dim elements of rows of q_row_stride elements, packed sequence after sequence
 // (cu_seqlens); kv_lens counts each sequence's keys with this pass's.  head_dim 32, 64, 96 or 128; other sizes, rows off the 16-byte
-// grid and more than 65,535 sequences are left to the plain kernel (kErrUnsupportedSize).
+// grid and more than 65,535 sequences are left to the plain kernel (kErrUnsupportedSize).  n_spans > 0: every sequence brings one
+// token, whose keys are cut into so many spans (at most 16; scratch: n_seqs n_heads n_spans (head_dim + 2) floats).
 extern "C" int b200_attention_prefill_f32(const void* q, int q_row_stride, void* out, const int* cu_seqlens, const int* kv_lens,
                                           const int* page_table, int table_stride, const void* k_pool, const void* v_pool,
                                           int n_seqs, int max_q_len, int n_heads, int n_kv_heads, int head_dim, int window,
                                           int chunk, const float* slopes, const float* sinks, const void* gate, int ld_gate,
-                                          float softcap, cudaStream_t stream) {
+                                          float softcap, int n_spans, float* scratch, cudaStream_t stream) {
     using namespace b200;
     if (n_seqs <= 0 || max_q_len <= 0) return 0;
     if (!(softcap >= 0.f) || chunk < 0 || (chunk > 0 && window > 0)) return kErrBadArgument;
@@ -291,6 +380,16 @@ extern "C" int b200_attention_prefill_f32(const void* q, int q_row_stride, void*
     a.k_pool = (const float*)k_pool; a.v_pool = (const float*)v_pool; a.slopes = slopes; a.sinks = sinks; a.gate = (const float*)gate;
     a.q_row_stride = q_row_stride; a.table_stride = table_stride; a.n_heads = n_heads; a.n_kv_heads = n_kv_heads;
     a.window = window; a.chunk = chunk; a.ld_gate = ld_gate; a.softcap = softcap;
+    if (n_spans > 0) {
+        if (max_q_len != 1 || n_spans > kMostSpans || scratch == nullptr || n_heads / n_kv_heads > 16) return kErrBadArgument;
+        switch (head_dim) {
+            case 32: return spans_f32_of<32>(a, n_seqs, n_spans, scratch, stream);
+            case 64: return spans_f32_of<64>(a, n_seqs, n_spans, scratch, stream);
+            case 96: return spans_f32_of<96>(a, n_seqs, n_spans, scratch, stream);
+            case 128: return spans_f32_of<128>(a, n_seqs, n_spans, scratch, stream);
+            default: return kErrUnsupportedSize;
+        }
+    }
     switch (head_dim) {
         case 32: return launch_prefill_f32<32, 8>(a, n_seqs, max_q_len, stream);
         case 64: return launch_prefill_f32<64, 8>(a, n_seqs, max_q_len, stream);

@@ -3,8 +3,8 @@
 // A is [M, K] (activations, row-major, row stride lda), W is [N, K] (a weight as the reference
 // stores it: one row per output, core/model/tensor/FloatTensor.java:98-100 of the reference
 // project).  Three kernels: tiles of 128 x 128 for prompts, of 64 x 64 for fewer than 128 rows, and a weight-streaming one for a decode step's few rows
-// (further down).  This is the kernel of the true 32-bit path (no tensor cores, no reduced-precision
-// matrix mode) and the fallback of the bfloat16 path for sizes or storage types the tensor-core
+// (further down).  These are the kernels of the true 32-bit path for few rows and for small products
+// (gemm_f32_tcgen05.cu has the rest) and the fallback of the bfloat16 path for sizes or storage types the tensor-core
 // kernels refuse.  Epilogues:
 //   0  store         C[M, N] = acc                       (C of type TC)
 //   1  residual add  C[M, N] += acc                      (C is the 32-bit residual stream)

@@ -3,7 +3,7 @@
 ``try_gemm`` and ``try_attention`` run the specialised sm_100a kernel that fits the operands and
 return True, or return False when no specialised kernel takes these storage types or sizes (the
 caller then runs the plain kernel, which takes every size).  The true 32-bit run never comes
-here with anything but float32 operands and therefore always takes the plain kernels."""
+here with anything but float32 operands and therefore always takes the kernels of ``ops`` that keep 32 bits."""
 from __future__ import annotations
 
 import torch

@@ -79,7 +79,7 @@ _SIGNATURES = {
                                                         c_int, c_int, c_int, c_void_p, c_int, c_int, c_int]),
     "b200_attention_prefill_f32": ("attention_prefill_f32", [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
                                                              c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
-                                                             c_void_p, c_void_p, c_int, c_float]),
+                                                             c_void_p, c_void_p, c_int, c_float, c_int, c_void_p]),
     "b200_attention_prefill_tc": ("attention_prefill_tcgen05", [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p,
                                                                 c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int,
                                                                 c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
@@ -370,10 +370,11 @@ def attention_prefill_f32(q: torch.Tensor, q_row_stride: int, out: torch.Tensor,
                           page_table: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, n_seqs: int, max_q_len: int,
                           n_heads: int, n_kv_heads: int, head_dim: int, window: int = 0, *, chunk: int = 0,
                           slopes: torch.Tensor | None = None, sinks: torch.Tensor | None = None,
-                          gate: torch.Tensor | None = None, softcap: float = 0.0) -> bool:
+                          gate: torch.Tensor | None = None, softcap: float = 0.0, n_spans: int = 0) -> bool:
     """``attention_paged`` of float32 queries that lie sequence after sequence (``cu_seqlens`` int32 [n_seqs + 1]; ``kv_lens``
-    counts this pass's tokens), a tile of them at a time; the same terms without kept first positions.  Returns False,
-    having done nothing, for operands it does not take."""
+    counts this pass's tokens), a tile of them at a time; the same terms without kept first positions.  ``n_spans`` > 0: a decode
+    step (``max_q_len`` 1) whose keys are cut into so many spans (``attention_decode_f32_spans``), merged by a second kernel.
+    Returns False, having done nothing, for operands it does not take."""
     if q.dtype != torch.float32 or head_dim not in (32, 64, 96, 128) or q_row_stride % 4 or q.data_ptr() & 15:
         return False
     _dev(q, out, cu_seqlens, kv_lens, page_table, k_pool, v_pool, slopes, sinks, gate)
@@ -385,16 +386,23 @@ def attention_prefill_f32(q: torch.Tensor, q_row_stride: int, out: torch.Tensor,
     for t in (slopes, sinks):
         assert t is None or (t.dtype == torch.float32 and t.is_contiguous() and t.numel() == n_heads)
     assert gate is None or (gate.dtype == q.dtype and gate.stride(1) == 1 and gate.shape[1] >= n_heads)
+    scratch = torch.empty(n_seqs * n_heads * n_spans * (head_dim + 2), dtype=torch.float32, device=q.device) if n_spans > 0 else None
     ptr = lambda t: t.data_ptr() if t is not None else None
     status = _fn("b200_attention_prefill_f32")(
         q.data_ptr(), q_row_stride, out.data_ptr(), cu_seqlens.data_ptr(), kv_lens.data_ptr(), page_table.data_ptr(),
         page_table.shape[1], k_pool.data_ptr(), v_pool.data_ptr(), n_seqs, int(max_q_len), n_heads, n_kv_heads, head_dim,
         int(window), int(chunk), ptr(slopes), ptr(sinks), ptr(gate), gate.stride(0) if gate is not None else 0, float(softcap),
-        _stream())
+        int(n_spans), ptr(scratch), _stream())
     if status == _UNSUPPORTED:
         return False
     _check(status, "attention_paged")
     return True
+
+
+def attention_decode_f32_spans(n_seqs: int, n_heads: int, n_kv_heads: int, reach: int) -> int:
+    """Into how many spans ``attention_prefill_f32`` cuts a decode step's keys (``reach``: the most one token sees); 0: the
+    step is one for ``attention_paged``."""
+    return int(library("attention_prefill_f32").b200_attention_decode_f32_spans(n_seqs, n_heads, n_kv_heads, int(reach)))
 
 
 # --------------------------------------------------------------------------- matrix products

@@ -257,13 +257,15 @@ def attend(shape, qkv: torch.Tensor, out: torch.Tensor, ctx: StepContext, table:
         return
     terms = dict(chunk=getattr(shape, "chunk", None) or 0, slopes=getattr(shape, "slopes", None), sinks=getattr(shape, "sinks", None),
                  gate=gate, softcap=getattr(shape, "softcap", None) or 0.0)
-    # float32 prompts: a tile of a sequence's queries at a time
-    if not ctx.all_decode and not shape.keep_first and ops.attention_prefill_f32(
+    reach = min(ctx.capacity(cache.group), _reach(shape) or ctx.capacity(cache.group))
+    # float32: a tile of a sequence's queries at a time, decode steps in spans of pages
+    tiled = qkv.dtype == torch.float32 and not shape.keep_first
+    spans = ops.attention_decode_f32_spans(ctx.n_seqs, shape.n_heads, shape.n_kv_heads, reach) if tiled and ctx.all_decode else 0
+    if (tiled and (spans or not ctx.all_decode) and ops.attention_prefill_f32(
             qkv, qkv.shape[1], out, ctx.cu_seqlens, ctx.kv_lens, table, cache.k, cache.v, ctx.n_seqs, ctx.max_q_len, shape.n_heads,
-            shape.n_kv_heads, shape.head_dim, shape.window or 0, **terms):
+            shape.n_kv_heads, shape.head_dim, shape.window or 0, n_spans=spans, **terms)):
         return
     rows = qkv.shape[0] * shape.n_heads
-    reach = min(ctx.capacity(cache.group), _reach(shape) or ctx.capacity(cache.group))
     # spans of at least one tile of 128 keys, up to two thousand CTAs (of which a GPU holds some 1,800 at a time)
     splits = 1 if rows >= 2048 else max(1, min(16, 2048 // rows, reach // 128))
     ops.attention_paged(qkv, qkv.shape[1], out, ctx.positions, ctx.seq_ids, table, cache.k, cache.v,

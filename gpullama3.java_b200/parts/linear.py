@@ -1,7 +1,7 @@
 """A weight matrix [out, in] and the choice of kernel that multiplies activations with it.
 
-The kernels are chosen by precision and size only (the true 32-bit run always takes the plain FMA
-kernel; the bfloat16 run takes a tensor-core kernel where one accepts the sizes), never by
+The kernels are chosen by precision and size only (the true 32-bit run takes FMA kernels, or for
+more than a few rows a tensor-core kernel that keeps 32 bits; the bfloat16 run takes a tensor-core kernel where one accepts the sizes), never by
 model."""
 from __future__ import annotations
 

@@ -118,16 +118,8 @@ def test_products_of_few_rows(M, N, K, dtype):
 CUTS = [([5, 1, 100, 77], [5, 300, 100, 200]), ([70, 64, 65], [70, 64, 129]), ([130, 3], [400, 69])]
 
 
-@pytest.mark.parametrize("q_lens, kv_lens", CUTS)
-@pytest.mark.parametrize("H, G, D", [(6, 2, 32), (4, 4, 64), (8, 1, 64), (6, 3, 96), (6, 2, 128)])
-@pytest.mark.parametrize("terms", [{}, {"window": 33}, {"chunk": 48, "sinks": 1, "gate": 1}, {"slopes": 1, "softcap": 5.0, "window": 100, "sinks": 1},
-                                   {"odd_values": 1}, {"odd_values": 1, "window": 20}], ids=str)
-def test_attention_over_tiles_of_queries(q_lens, kv_lens, H, G, D, terms):
-    """Against the plain kernel.  Behind every sequence's end the pages hold NaN; with ``odd_values`` the last two positions of
-    the first sequence hold values that are not finite, which earlier queries must not see.  A score is a sum of D products of 2 normal numbers
-    by normal numbers over sqrt(D): its rounding is below (D / 2 + 4) 2^-24 2 sqrt(D) on either side, and a result moves by
-    at most twice that times the largest value."""
-    o = ops()
+def attention_problem(q_lens, kv_lens, H, G, D, terms):
+    """Queries, a paged cache that holds NaN behind every sequence's end, and the terms by name with their tensors."""
     terms = dict(terms)
     gen = torch.Generator("cuda").manual_seed(H * D)
     rand = lambda *s: torch.randn(*s, generator=gen, device="cuda")
@@ -151,9 +143,43 @@ def test_attention_over_tiles_of_queries(q_lens, kv_lens, H, G, D, terms):
     seq_ids = torch.repeat_interleave(torch.arange(n), torch.tensor(q_lens)).to(torch.int32).cuda()
     cu = torch.tensor([0] + q_lens).cumsum(0).to(torch.int32).cuda()
     lens = torch.tensor(kv_lens, dtype=torch.int32, device="cuda")
-    want, got = torch.empty(T, H * D, device="cuda"), torch.full((T, H * D), 7.0, device="cuda")
-    o.attention_paged(q, q.shape[1], want, positions, seq_ids, table, k, v, H, G, D, window, **terms)
-    assert o.attention_prefill_f32(q, q.shape[1], got, cu, lens, table, k, v, n, max(q_lens), H, G, D, window, **terms)
+    return q, k, v, table, positions, seq_ids, cu, lens, window, terms, biggest
+
+
+def close_enough(got, want, D, biggest):
+    """A score is a sum of D products of 2 normal numbers by normal numbers over sqrt(D): its rounding is below (D / 2 + 4) 2^-24 2 sqrt(D)
+    on either side, and a result moves by at most twice that times the largest value."""
     assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
     ok = torch.isfinite(want)
     assert float((got - want)[ok].abs().max()) <= 2 * 2 * (D / 2 + 4) * 2.0 ** -24 * 2 * math.sqrt(D) * biggest
+
+
+@pytest.mark.parametrize("q_lens, kv_lens", CUTS)
+@pytest.mark.parametrize("H, G, D", [(6, 2, 32), (4, 4, 64), (8, 1, 64), (6, 3, 96), (6, 2, 128)])
+@pytest.mark.parametrize("terms", [{}, {"window": 33}, {"chunk": 48, "sinks": 1, "gate": 1}, {"slopes": 1, "softcap": 5.0, "window": 100, "sinks": 1},
+                                   {"odd_values": 1}, {"odd_values": 1, "window": 20}], ids=str)
+def test_attention_over_tiles_of_queries(q_lens, kv_lens, H, G, D, terms):
+    """Against the plain kernel; with ``odd_values`` the last two positions of the first sequence hold values that are not finite,
+    which earlier queries must not see."""
+    o = ops()
+    q, k, v, table, positions, seq_ids, cu, lens, window, terms, biggest = attention_problem(q_lens, kv_lens, H, G, D, terms)
+    want, got = torch.empty(len(positions), H * D, device="cuda"), torch.full((len(positions), H * D), 7.0, device="cuda")
+    o.attention_paged(q, q.shape[1], want, positions, seq_ids, table, k, v, H, G, D, window, **terms)
+    assert o.attention_prefill_f32(q, q.shape[1], got, cu, lens, table, k, v, len(q_lens), max(q_lens), H, G, D, window, **terms)
+    close_enough(got, want, D, biggest)
+
+
+@pytest.mark.parametrize("kv_lens, n_spans", [([1, 64, 65, 300], 1), ([1, 64, 65, 300], 3), ([1030, 5], 16), ([700], 5)])
+@pytest.mark.parametrize("H, G, D", [(6, 2, 32), (4, 4, 64), (8, 1, 64), (16, 1, 64), (12, 1, 96), (6, 2, 128)])
+@pytest.mark.parametrize("terms", [{}, {"window": 33}, {"chunk": 48, "sinks": 1, "gate": 1}, {"slopes": 1, "softcap": 5.0, "window": 100, "sinks": 1},
+                                   {"odd_values": 1}], ids=str)
+def test_attention_of_decode_steps_in_spans(kv_lens, n_spans, H, G, D, terms):
+    o = ops()
+    q_lens = [1] * len(kv_lens)
+    if terms.get("odd_values") and kv_lens[0] < 2:
+        kv_lens = kv_lens[::-1]
+    q, k, v, table, positions, seq_ids, cu, lens, window, terms, biggest = attention_problem(q_lens, kv_lens, H, G, D, terms)
+    want, got = torch.empty(len(q_lens), H * D, device="cuda"), torch.full((len(q_lens), H * D), 7.0, device="cuda")
+    o.attention_paged(q, q.shape[1], want, positions, seq_ids, table, k, v, H, G, D, window, **terms)
+    assert o.attention_prefill_f32(q, q.shape[1], got, cu, lens, table, k, v, len(q_lens), 1, H, G, D, window, n_spans=n_spans, **terms)
+    close_enough(got, want, D, biggest)
