@@ -31,6 +31,8 @@
 // It also runs a memory whose gates another kernel made (gated_scan): S <- g S + b k v^T per head and token with g and b of every
 // token given as logarithms and running maxima, and beside S a vector n that takes the keys alone (a column of values that are all
 // one, kept in its own place of the slot); the read-outs come with n . q behind them.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace b200 {
@@ -693,30 +695,36 @@ static int launch_scan_rows(const ScanArgs& a, int rpt, int lanes, int n_seqs, c
 // token each, that no pipe of the GPU is busy with; a run of C tokens from a state S0 is instead a few small products.  With G_t
 // the product of the run's decays up to and with token t (per key channel), and j < t <= C:
 //     A[t, j] = beta_t sum_d k_t[d] k_j[d] G_t[d] / G_j[d]        B[t, j] = sum_d q_t[d] k_j[d] G_t[d] / G_j[d]   (and j = t)
-//     (1 + A) U = beta (V - (G k) S0)                             O = (G q) S0 + B U
-//     S_C = G_C S0 + sum_j (G_C / G_j k_j) u_j^T
+//     W = (1 + A)^-1 beta G k      U0 = (1 + A)^-1 beta V         U = U0 - W S0
+//     O = (G q) S0 + B U = B U0 + (G q - B W) S0                  S_C = G_C S0 + sum_j (G_C / G_j k_j) u_j^T
 // (the form in which DeltaNet and its gated relatives are trained: Yang et al., "Parallelizing Linear Transformers with the
 // Delta Rule over Sequence Length", 2024).  The quotients are never formed as quotients: G_t / G_j is carried along as the product of the
 // decays between, so that nothing overflows however strong they are.
 //   delta_run_parts   a CTA per (run, head), all at once: the rows that the scan has prepared for it, here in shared memory; A and
-//                     B; (1 + A)^-1 applied to beta G k and beta V by forward substitution.  Leaves a row per token: G q,
-//                     (G_C / G_j) k, W = (1 + A)^-1 beta G k, U0 = (1 + A)^-1 beta V; B and G_C behind all rows.
-//   delta_run_carry   a CTA per (head, 16 columns, sequence) walks the runs: U = U0 - W S, O = (G q) S + B U, S <- G_C S + k^T U.
-// All sums are 32-bit multiply-adds.  A token that is not finite reaches itself and later tokens only, as in the scan.
-// Bound by latency and issue: 2,048 tokens, 32 heads of 64 by 64: 262 us (prepare and scan: 498); error against 64 bits 1.6e-7 of the
-// norm for the results, 1.3e-7 for the state (scan: 1.5e-7 and 1.2e-7).
+//                     B; W and U0 by forward substitution.  Leaves a row per token: G q - B W, (G_C / G_j) k, W, U0; G_C behind
+//                     all rows, and B U0 where the results go.
+//   delta_run_carry   a CTA per (head, 16 columns, sequence) walks the runs: U = U0 - W S, O += (G q - B W) S, S <- G_C S + k^T U.
+// A token's results differ from the scan's by the order of sums alone, but B U and (G q) S0 can be large and cancel, and A's and
+// B's errors go through a triangular solve: with 32-bit sums in the first kernel the results were 5 % (independent keys) to 23 %
+// (keys of one sign) further from 64 bits than the scan's.  So the first kernel, which is all at once and waits for nothing, computes in
+// 64 bits and rounds what it leaves; the walk's sums are 32-bit multiply-adds.  A token that is not finite reaches itself and
+// later tokens only, as in the scan.
+// Bound by what shared memory answers in the first kernel (every operand is read by all lanes alike) and by latency in the second: 2,048
+// tokens, 32 heads of 64 by 64: 251 us (prepare and scan: 497; with 32-bit sums in the first kernel, its rows by rows, 261); error
+// against 64 bits 1.24e-7 of the norm for the results and 1.25e-7 for the state (scan: 1.52e-7 and 1.27e-7), with keys and queries of one
+// sign 0.88e-7 and 1.26e-7 (1.09e-7 and 1.27e-7).
 constexpr int kDeltaRun = 32, kDeltaKey = 64, kDeltaCols = 16;
 constexpr int kDeltaPitch = kDeltaKey + 4;
+constexpr int kDeltaBlock = 4;   // tokens whose sums for A and B meet at a time
 
 struct DeltaRunArgs {
     PrepareArgs in;         // what the rows are made of; rows: [heads, T, row], written here
-    float* b;               // [heads, T, kDeltaRun]
     float* decay;           // [heads, runs, kDeltaKey]
     float* state;
     size_t slot_stride;
     const int* slots;
     const int* cu_seqlens;
-    float* out;             // [T, heads d_v]
+    float* out;             // [T, heads d_v], 16-byte aligned
     int n_seqs, most_runs;
 };
 
@@ -733,11 +741,11 @@ __device__ __forceinline__ int delta_run_at(const DeltaRunArgs& a, int run, int&
     return 0;
 }
 
-struct DeltaPartsSmem {
-    float q[kDeltaRun][kDeltaPitch], k[kDeltaRun][kDeltaPitch], g[kDeltaRun][kDeltaPitch];
-    float part[4][2][kDeltaRun][kDeltaRun + 1];   // per warp: its 16 channels' sums for A and B
-    float a[kDeltaRun][kDeltaRun + 4];
-    float beta[kDeltaRun];
+struct DeltaPartsSmem {   // (rows are read by all lanes alike or by neighbouring lanes: no padding; three CTAs share an SM)
+    double q[kDeltaRun][kDeltaKey], k[kDeltaRun][kDeltaKey], g[kDeltaRun][kDeltaKey];
+    double part[4][2][kDeltaBlock][kDeltaRun];    // per warp: its 16 channels' sums for A and B
+    double at[kDeltaRun][kDeltaRun + 2], bt[kDeltaRun][kDeltaRun + 2];   // A and B by columns
+    double beta[kDeltaRun];
 };
 
 template <typename T>
@@ -762,103 +770,139 @@ delta_run_parts_kernel(DeltaRunArgs a) {
     const T* vr = (const T*)in.qkv + (size_t)first * in.ld_qkv + 2 * (size_t)in.kv_heads * kDeltaKey + (size_t)h * in.d_v;
     const T* dr = (const T*)in.decay + (size_t)first * in.ld_decay + (in.decay_per_head ? (size_t)h : (size_t)h * kDeltaKey);
     float* rows = in.rows + ((size_t)h * in.n_tokens + first) * in.row;
-    // ---- unit rows of q and k, decays: eight tokens a warp, two channels a lane.  Tokens beyond the run's end: nothing, and no decay.
-#pragma unroll 2
-    for (int i = 0; i < kDeltaRun / 4; ++i) {
-        const int t = warp * (kDeltaRun / 4) + i;
-        float q[2], k[2], z[2];
+    // ---- unit rows of q and k, decays (32-bit, as the scan's): eight tokens a warp, two channels a lane, all asked for before the
+    // first is used.  Tokens beyond the run's end: nothing, and no decay.
+    {
+        constexpr int kEach = kDeltaRun / 4;
+        float q[kEach][2], k[kEach][2], z[kEach][2];
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            q[e] = t < m ? to_f32<T>(qr[(size_t)t * in.ld_qkv + 32 * e + lane]) : 0.f;
-            k[e] = t < m ? to_f32<T>(kr0[(size_t)t * in.ld_qkv + 32 * e + lane]) : 0.f;
-            z[e] = t < m ? to_f32<T>(dr[(size_t)t * in.ld_decay + (in.decay_per_head ? 0 : 32 * e + lane)]) : 0.f;
+        for (int i = 0; i < kEach; ++i) {
+            const int t = warp * kEach + i;
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                q[i][e] = t < m ? to_f32<T>(qr[(size_t)t * in.ld_qkv + 32 * e + lane]) : 0.f;
+                k[i][e] = t < m ? to_f32<T>(kr0[(size_t)t * in.ld_qkv + 32 * e + lane]) : 0.f;
+                z[i][e] = t < m ? to_f32<T>(dr[(size_t)t * in.ld_decay + (in.decay_per_head ? 0 : 32 * e + lane)]) : 0.f;
+            }
         }
-        const float fq = in.q_scale / sqrtf(warp_sum(q[0] * q[0] + q[1] * q[1]) + in.unit_eps);
-        const float fk = 1.0f / sqrtf(warp_sum(k[0] * k[0] + k[1] * k[1]) + in.unit_eps);
+        // lane i: the factor that makes q (i < 8) or k of the warp's token i % 8 a unit vector
+        float square = 1.f;
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            sm.q[t][32 * e + lane] = q[e] * fq;
-            sm.k[t][32 * e + lane] = k[e] * fk;
-            sm.g[t][32 * e + lane] = t < m ? expf(neg_rate * softplus(z[e] + bias[e])) : 1.f;
+        for (int i = 0; i < kEach; ++i) {
+            const float sq = warp_sum(q[i][0] * q[i][0] + q[i][1] * q[i][1]), sk = warp_sum(k[i][0] * k[i][0] + k[i][1] * k[i][1]);
+            if (lane == i) square = sq;
+            if (lane == kEach + i) square = sk;
+        }
+        const float factor = (lane < kEach ? in.q_scale : 1.0f) / sqrtf(square + in.unit_eps);
+#pragma unroll
+        for (int i = 0; i < kEach; ++i) {
+            const int t = warp * kEach + i;
+            const float fq = __shfl_sync(0xffffffffu, factor, i), fk = __shfl_sync(0xffffffffu, factor, kEach + i);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                sm.q[t][32 * e + lane] = q[i][e] * fq;
+                sm.k[t][32 * e + lane] = k[i][e] * fk;
+                sm.g[t][32 * e + lane] = t < m ? expf(neg_rate * softplus(z[i][e] + bias[e])) : 1.f;
+            }
         }
     }
     if (tid < kDeltaRun)
         sm.beta[tid] = tid < m ? 1.0f / (1.0f + expf(-to_f32<T>(((const T*)in.beta)[(size_t)(first + tid) * in.ld_beta + h]))) : 0.f;
     __syncthreads();
-    // ---- A and B: lane j carries k_j times the decays since, 16 channels a warp (lanes j > t hold nothing that is used)
+    // ---- A and B: lane l of a half warp carries k_l and k_(l + 16) times the decays since, eight of the warp's 16 channels each half
+    // (what bounds this is shared memory, which answers a read for all lanes alike no faster than one for each: two halves with
+    // channels of their own need half the reads).  Sums with tokens to come hold nothing that is used; below token 16 the second
+    // key is yet to come altogether.
     {
-        const int d0 = warp * 16;
-        float kr[16];
+        const int half = lane >> 4, d0 = warp * 16 + half * 8, j0 = lane & 15;
+        double kr[2][8];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) kr[i] = 0.f;
-#pragma unroll 2
-        for (int t = 0; t < m; ++t) {
-            float sa[2] = {0.f, 0.f}, sb[2] = {0.f, 0.f};
+        for (int i = 0; i < 8; ++i) kr[0][i] = kr[1][i] = 0.0;
+        auto step = [&](int t, int tt, auto both) {
+            constexpr int n = decltype(both)::value ? 2 : 1;
+            double sa[2][2] = {{0.0, 0.0}, {0.0, 0.0}}, sb[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
 #pragma unroll
-            for (int i = 0; i < 16; i += 4) {
-                const float4 g4 = *reinterpret_cast<const float4*>(&sm.g[t][d0 + i]), k4 = *reinterpret_cast<const float4*>(&sm.k[t][d0 + i]);
-                const float4 q4 = *reinterpret_cast<const float4*>(&sm.q[t][d0 + i]);
-                const float gv[4] = {g4.x, g4.y, g4.z, g4.w}, kv[4] = {k4.x, k4.y, k4.z, k4.w}, qv[4] = {q4.x, q4.y, q4.z, q4.w};
+            for (int i = 0; i < 8; i += 2) {
+                const double2 g2 = *reinterpret_cast<const double2*>(&sm.g[t][d0 + i]), k2 = *reinterpret_cast<const double2*>(&sm.k[t][d0 + i]);
+                const double2 q2 = *reinterpret_cast<const double2*>(&sm.q[t][d0 + i]);
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    kr[i + e] = lane == t ? kv[e] : kr[i + e] * gv[e];
-                    sa[e & 1] = fmaf(kv[e], kr[i + e], sa[e & 1]);
-                    sb[e & 1] = fmaf(qv[e], kr[i + e], sb[e & 1]);
+                for (int c = 0; c < n; ++c) {
+                    const bool own = j0 + 16 * c == t;
+                    kr[c][i] = own ? k2.x : kr[c][i] * g2.x;
+                    kr[c][i + 1] = own ? k2.y : kr[c][i + 1] * g2.y;
+                    sa[c][0] = fma(k2.x, kr[c][i], sa[c][0]); sa[c][1] = fma(k2.y, kr[c][i + 1], sa[c][1]);
+                    sb[c][0] = fma(q2.x, kr[c][i], sb[c][0]); sb[c][1] = fma(q2.y, kr[c][i + 1], sb[c][1]);
                 }
             }
-            sm.part[warp][0][t][lane] = sa[0] + sa[1];
-            sm.part[warp][1][t][lane] = sb[0] + sb[1];
-        }
-    }
-    __syncthreads();
-    for (int i = tid; i < m * kDeltaRun; i += 128) {
-        const int t = i / kDeltaRun, j = i % kDeltaRun;
-        const float sa = (sm.part[0][0][t][j] + sm.part[1][0][t][j]) + (sm.part[2][0][t][j] + sm.part[3][0][t][j]);
-        const float sb = (sm.part[0][1][t][j] + sm.part[1][1][t][j]) + (sm.part[2][1][t][j] + sm.part[3][1][t][j]);
-        sm.a[t][j] = j < t ? sm.beta[t] * sa : 0.f;
-        a.b[((size_t)h * in.n_tokens + first + t) * kDeltaRun + j] = j <= t ? sb : 0.f;
-    }
-    // ---- the first 64 threads: G forward (rows of q and k times it); the others: the decays still to come
-    const int c = tid % kDeltaKey;
-    float x[kDeltaRun];
-    if (tid < kDeltaKey) {
-        float decay = 1.f;
+            // lane l keeps the sum with token l: its half's channels and, from the other half, theirs
+            const double a0 = sa[0][0] + sa[0][1], a1 = sa[1][0] + sa[1][1], b0 = sb[0][0] + sb[0][1], b1 = sb[1][0] + sb[1][1];
+            const double a_other = __shfl_xor_sync(0xffffffffu, half ? a0 : a1, 16), b_other = __shfl_xor_sync(0xffffffffu, half ? b0 : b1, 16);
+            sm.part[warp][0][tt][lane] = (half ? a1 : a0) + a_other;
+            sm.part[warp][1][tt][lane] = (half ? b1 : b0) + b_other;
+        };
+        for (int t0 = 0; t0 < m; t0 += kDeltaBlock) {
 #pragma unroll
-        for (int t = 0; t < kDeltaRun; ++t) {
-            decay *= sm.g[t][c];
-            if (t < m) rows[(size_t)t * in.row + c] = sm.q[t][c] * decay;
-            x[t] = sm.beta[t] * (sm.k[t][c] * decay);
-        }
-        a.decay[((size_t)h * a.most_runs + blockIdx.x) * kDeltaKey + c] = decay;
-    } else {
-        float decay = 1.f;
-#pragma unroll
-        for (int t = kDeltaRun - 1; t >= 0; --t) {
-            if (t < m) rows[(size_t)t * in.row + kDeltaKey + c] = sm.k[t][c] * decay;
-            decay *= sm.g[t][c];
-        }
-    }
-    __syncthreads();   // A is complete
-    // ---- forward substitution, a column a thread: the 64 columns of beta G k, then those of beta V
-    for (int col = tid; col < kDeltaKey + in.d_v; col += 128) {
-        float* dst = rows + 2 * kDeltaKey + col;
-        if (col >= kDeltaKey) {
-#pragma unroll
-            for (int t = 0; t < kDeltaRun; ++t) x[t] = t < m ? sm.beta[t] * to_f32<T>(vr[(size_t)t * in.ld_qkv + col - kDeltaKey]) : 0.f;
-        }
-#pragma unroll
-        for (int t = 0; t < kDeltaRun; ++t) {
-            float s[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (int j = 0; j < t; j += 4) {
-                const float4 a4 = *reinterpret_cast<const float4*>(&sm.a[t][j]);
-                const float av[4] = {a4.x, a4.y, a4.z, a4.w};
-#pragma unroll
-                for (int e = 0; e < 4; ++e) if (j + e < t) s[e] = fmaf(av[e], x[j + e], s[e]);
+            for (int tt = 0; tt < kDeltaBlock; ++tt) {
+                if (t0 >= 16) step(t0 + tt, tt, std::true_type{});
+                else step(t0 + tt, tt, std::false_type{});
             }
-            if (t < m) {
-                x[t] -= (s[0] + s[1]) + (s[2] + s[3]);
-                dst[(size_t)t * in.row] = x[t];
+            __syncthreads();
+            const int tt = warp, t = t0 + tt;   // (a warp per token of the block)
+            static_assert(kDeltaBlock == 4, "a warp per token of a block");
+            const double sa = (sm.part[0][0][tt][lane] + sm.part[1][0][tt][lane]) + (sm.part[2][0][tt][lane] + sm.part[3][0][tt][lane]);
+            const double sb = (sm.part[0][1][tt][lane] + sm.part[1][1][tt][lane]) + (sm.part[2][1][tt][lane] + sm.part[3][1][tt][lane]);
+            sm.at[lane][t] = lane < t ? sm.beta[t] * sa : 0.0;
+            sm.bt[lane][t] = lane <= t ? sb : 0.0;
+            __syncthreads();
+        }
+    }
+    // ---- the last 64 threads: keys times the decays still to come
+    if (tid >= kDeltaKey) {
+        const int c = tid - kDeltaKey;
+        double decay = 1.0;
+#pragma unroll 4
+        for (int t = kDeltaRun - 1; t >= 0; --t) {
+            if (t < m) rows[(size_t)t * in.row + kDeltaKey + c] = (float)(sm.k[t][c] * decay);
+            decay *= sm.g[t][c];
+        }
+        a.decay[((size_t)h * a.most_runs + blockIdx.x) * kDeltaKey + c] = (float)decay;
+    }
+    // ---- forward substitution, a column a thread: the 64 columns of beta G k, then those of beta V.  A token that is finished is taken
+    // out of all later ones (independent sums: 64-bit multiply-adds answer slowly), and B times it out of r.
+    for (int col = tid; col < kDeltaKey + in.d_v; col += 128) {
+        const bool key = col < kDeltaKey;
+        const int v_col = col - kDeltaKey;
+        double x[kDeltaRun], r[kDeltaRun];
+        if (key) {
+            double decay = 1.0;
+#pragma unroll
+            for (int t = 0; t < kDeltaRun; ++t) {
+                decay *= sm.g[t][col];
+                r[t] = sm.q[t][col] * decay;
+                x[t] = sm.beta[t] * (sm.k[t][col] * decay);
+            }
+        } else {
+#pragma unroll
+            for (int t = 0; t < kDeltaRun; ++t) {
+                r[t] = 0.0;
+                x[t] = t < m ? sm.beta[t] * (double)to_f32<T>(vr[(size_t)t * in.ld_qkv + v_col]) : 0.0;
+            }
+        }
+        float* dst = rows + 2 * kDeltaKey + col;                                               // W, U0
+        float* dst_b = key ? rows + col : a.out + (size_t)first * in.heads * in.d_v + (size_t)h * in.d_v + v_col;   // G q - B W, B U0
+        const size_t step_b = key ? (size_t)in.row : (size_t)in.heads * in.d_v;
+#pragma unroll
+        for (int j = 0; j < kDeltaRun; ++j) {
+            if (j >= m) break;
+            r[j] = fma(-sm.bt[j][j], x[j], r[j]);
+            dst[(size_t)j * in.row] = (float)x[j];
+            dst_b[(size_t)j * step_b] = (float)(key ? r[j] : -r[j]);
+#pragma unroll
+            for (int t = (j + 1) & ~1; t < kDeltaRun; t += 2) {
+                const double2 a2 = *reinterpret_cast<const double2*>(&sm.at[j][t]), b2 = *reinterpret_cast<const double2*>(&sm.bt[j][t]);
+                if (t > j) { x[t] = fma(-a2.x, x[j], x[t]); r[t] = fma(-b2.x, x[j], r[t]); }
+                x[t + 1] = fma(-a2.y, x[j], x[t + 1]);
+                r[t + 1] = fma(-b2.y, x[j], r[t + 1]);
             }
         }
     }
@@ -868,7 +912,7 @@ constexpr int kCarryThreads = 256;
 
 struct DeltaCarrySmem {
     float q[2][kDeltaRun][kDeltaKey], k[2][kDeltaRun][kDeltaKey], w[2][kDeltaRun][kDeltaKey];
-    float u0[2][kDeltaRun][kDeltaCols], b[2][kDeltaRun][kDeltaRun], decay[2][kDeltaKey];
+    float u0[2][kDeltaRun][kDeltaCols], o0[2][kDeltaRun][kDeltaCols], decay[2][kDeltaKey];
     float s[kDeltaCols][kDeltaPitch];         // the state's columns
     float u[kDeltaCols][kDeltaRun + 4];
 };
@@ -901,7 +945,8 @@ delta_run_carry_kernel(DeltaRunArgs a) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) S[i] = S_g[(size_t)(4 * ty + i) * d_v];
     *reinterpret_cast<float4*>(&sm.s[tx][4 * ty]) = make_float4(S[0], S[1], S[2], S[3]);
-    const size_t token0 = (size_t)h * a.in.n_tokens + begin;
+    const size_t token0 = (size_t)h * a.in.n_tokens + begin, out_row = (size_t)a.in.heads * d_v;
+    float* out = a.out + (size_t)begin * out_row + (size_t)h * d_v + col0;
     // (tokens beyond a short run's end: rows of its last token, whose results are not used)
     auto fetch = [&](int run, int buf) {
         const int base = run * kDeltaRun, m = min(kDeltaRun, n - base);
@@ -914,15 +959,13 @@ delta_run_carry_kernel(DeltaRunArgs a) {
             copy_async_16(&sm.q[buf][t][d], r);
             copy_async_16(&sm.k[buf][t][d], r + kDeltaKey);
         }
-        const int tb = tid / (kDeltaRun / 4), jb = tid % (kDeltaRun / 4) * 4;
-        copy_async_16(&sm.b[buf][tb][jb], a.b + (token0 + base + min(tb, m - 1)) * kDeltaRun + jb);
-        if (tid < kDeltaRun * kDeltaCols / 4) {
-            const int t = tid / (kDeltaCols / 4), c = tid % (kDeltaCols / 4) * 4;
+        static_assert(kCarryThreads == 2 * kDeltaRun * kDeltaCols / 4, "a thread per 16 bytes of U0 and of B U0");
+        const int t = tid % (kCarryThreads / 2) / (kDeltaCols / 4), c = tid % (kDeltaCols / 4) * 4;
+        if (tid < kCarryThreads / 2)
             copy_async_16(&sm.u0[buf][t][c], rows + (size_t)min(t, m - 1) * row + 3 * kDeltaKey + col0 + c);
-        } else if (tid < kDeltaRun * kDeltaCols / 4 + kDeltaKey / 4) {
-            const int d = (tid - kDeltaRun * kDeltaCols / 4) * 4;
-            copy_async_16(&sm.decay[buf][d], a.decay + ((size_t)h * a.most_runs + run0 + run) * kDeltaKey + d);
-        }
+        else
+            copy_async_16(&sm.o0[buf][t][c], out + (size_t)(base + min(t, m - 1)) * out_row + c);
+        if (tid < kDeltaKey / 4) copy_async_16(&sm.decay[buf][tid * 4], a.decay + ((size_t)h * a.most_runs + run0 + run) * kDeltaKey + tid * 4);
         copy_async_commit();
     };
     fetch(0, 0);
@@ -932,7 +975,7 @@ delta_run_carry_kernel(DeltaRunArgs a) {
         copy_async_wait<0>();
         __syncthreads();       // this run's rows and the state's columns are there; the other buffer has been read
         if (run + 1 < runs) fetch(run + 1, buf ^ 1);
-        // ---- U and the state's part of O
+        // ---- U, and the state's part of O
         float2 ws[2], qs[2];
 #pragma unroll
         for (int i = 0; i < 2; ++i) ws[i] = qs[i] = make_float2(0.f, 0.f);
@@ -945,15 +988,15 @@ delta_run_carry_kernel(DeltaRunArgs a) {
                 fma4(qs[i], *reinterpret_cast<const float4*>(&sm.q[buf][t0 + i][d]), s4);
             }
         }
-        float u[2], o[2];
+        float u[2];
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             u[i] = t0 + i < m ? sm.u0[buf][t0 + i][tx] - (ws[i].x + ws[i].y) : 0.f;
-            o[i] = qs[i].x + qs[i].y;
+            if (t0 + i < m) out[(size_t)(run * kDeltaRun + t0 + i) * out_row + tx] = sm.o0[buf][t0 + i][tx] + (qs[i].x + qs[i].y);
         }
         *reinterpret_cast<float2*>(&sm.u[tx][t0]) = make_float2(u[0], u[1]);
         __syncthreads();
-        // ---- the state first (the next run waits for it)
+        // ---- the state
         float4 add = make_float4(0.f, 0.f, 0.f, 0.f);
         const float4 g4 = *reinterpret_cast<const float4*>(&sm.decay[buf][4 * ty]);
 #pragma unroll
@@ -969,30 +1012,6 @@ delta_run_carry_kernel(DeltaRunArgs a) {
         }
         S[0] = fmaf(S[0], g4.x, add.x); S[1] = fmaf(S[1], g4.y, add.y); S[2] = fmaf(S[2], g4.z, add.z); S[3] = fmaf(S[3], g4.w, add.w);
         *reinterpret_cast<float4*>(&sm.s[tx][4 * ty]) = make_float4(S[0], S[1], S[2], S[3]);   // (last read before the barrier above)
-        // ---- O: whole fours of earlier tokens, then the rest one by one (no token is weighted that comes later)
-        const int whole = t0 & ~3;
-        float2 bu[2];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) bu[i] = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int j = 0; j < kDeltaRun - 4; j += 4) {
-            if (j < whole) {
-                const float4 u4 = *reinterpret_cast<const float4*>(&sm.u[tx][j]);
-#pragma unroll
-                for (int i = 0; i < 2; ++i) fma4(bu[i], *reinterpret_cast<const float4*>(&sm.b[buf][t0 + i][j]), u4);
-            }
-        }
-        const float4 u4 = *reinterpret_cast<const float4*>(&sm.u[tx][whole]);
-        const float uv[4] = {u4.x, u4.y, u4.z, u4.w};
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const float4 b4 = *reinterpret_cast<const float4*>(&sm.b[buf][t0 + i][whole]);
-            const float bv[4] = {b4.x, b4.y, b4.z, b4.w};
-            float s = bu[i].x + bu[i].y;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) if (whole + j <= t0 + i) s = fmaf(bv[j], uv[j], s);
-            if (t0 + i < m) a.out[((size_t)begin + run * kDeltaRun + t0 + i) * a.in.heads * d_v + (size_t)h * d_v + col0 + tx] = o[i] + s;
-        }
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) S_g[(size_t)(4 * ty + i) * d_v] = S[i];
@@ -1155,14 +1174,18 @@ extern "C" int b200_delta_rule_row(int d_k, int d_v) {
 
 // Floats of scratch behind those rows with which b200_delta_rule_scan takes runs of tokens instead of a token at a time; 0: it
 // does not.  Key size 64, whole tiles of columns.  The scan takes as long as its longest sequence (0.24 us a token) or, with warps
-// enough to fill the GPU, 0.105 us a token of 32 heads of 64 in all; runs take 0.11 us a token in all and half the scan's time for a
-// sequence alone.  Measured, scan and runs, 32 heads of 64: 1 x 64 tokens 21 and 25 us, 1 x 96 29 and 27, 1 x 2,048 498 and 262, 2 x
-// 512 160 and 122, 8 x 256 246 and 230, 16 x 128 218 and 232, 64 x 40 272 and 434.
+// enough to fill the GPU, 0.105 us a token of 32 heads of 64 in all; runs take 0.11 us a token in all, a third to a half of the scan's time
+// for a sequence alone, and some 10 us to start with, more where many heads start at once.  Measured, scan and runs, in us: 32 heads of 64: 1 x 96
+// tokens 28 and 32, 1 x 128 35 and 35, 1 x 200 53 and 41, 1 x 2,048 497 and 251, 2 x 512 160 and 123; 64 heads: 1 x 96 36 and 37, 1 x 512 160
+// and 123; 8 heads: 1 x 96 27 and 25, 4 x 256 66 and 43, 8 x 128 45 and 43, 8 x 256 83 and 75, 8 x 1,024 323 and 241; 4 heads of 128
+// columns: 1 x 96 27 and 27, 8 x 128 42 and 45, 8 x 256 78 and 59; with twice the work for the longest sequence's length (32 heads: 4 x 256,
+// 8 x 256) runs were 6 % faster at most when they had 32-bit sums.
 extern "C" long long b200_delta_rule_runs_scratch(int n_tokens, int n_seqs, int longest, int heads, int d_k, int d_v) {
     if (n_tokens <= 0 || n_seqs <= 0 || d_k != b200::kDeltaKey || d_v % b200::kDeltaCols != 0) return 0;
-    if (longest < 96 || (long long)n_tokens * heads * d_v > 4096ll * longest) return 0;
+    const long long work = (long long)n_tokens * heads * d_v;
+    if (longest < 96 || work > 4096ll * longest || (longest < 160 && work > 1024ll * longest)) return 0;
     const long long runs = n_tokens / b200::kDeltaRun + n_seqs;
-    return (long long)heads * ((long long)n_tokens * b200::kDeltaRun + runs * b200::kDeltaKey);
+    return (long long)heads * runs * b200::kDeltaKey;
 }
 
 extern "C" int b200_delta_rule_scan(const void* qkv, int ld_qkv, const void* beta, int ld_beta, const void* decay,
@@ -1180,11 +1203,10 @@ extern "C" int b200_delta_rule_scan(const void* qkv, int ld_qkv, const void* bet
     if ((uintptr_t)scratch % 16) return b200::kErrBadArgument;
     b200::PrepareArgs p = {qkv, ld_qkv, beta, ld_beta, decay, ld_decay, dt_bias, a_log, scratch, n_tokens, heads, kv_heads,
                            d_k, d_v, rpt * lanes, row, q_scale, unit_eps, decay_per_head ? 1 : 0};
-    if (runs_scratch != nullptr && rpt * lanes == b200::kDeltaKey && d_v % b200::kDeltaCols == 0) {
+    if (runs_scratch != nullptr && rpt * lanes == b200::kDeltaKey && d_v % b200::kDeltaCols == 0 && (uintptr_t)out % 16 == 0) {
         if ((uintptr_t)runs_scratch % 16) return b200::kErrBadArgument;
         const int runs = n_tokens / b200::kDeltaRun + n_seqs;
-        const b200::DeltaRunArgs r = {p, runs_scratch, runs_scratch + (size_t)heads * n_tokens * b200::kDeltaRun, state, (size_t)slot_stride,
-                                      slots, cu_seqlens, out, n_seqs, runs};
+        const b200::DeltaRunArgs r = {p, runs_scratch, state, (size_t)slot_stride, slots, cu_seqlens, out, n_seqs, runs};
         B200_DISPATCH_DTYPE(dtype, T, return b200::launch_delta_runs<T>(r, stream));
     }
     const long long units = (long long)n_tokens * heads;
