@@ -13,10 +13,13 @@
 // padded by four floats, so that 16 lanes that read 16 rows meet no bank twice.  Keys and values have one buffer each, refilled
 // (cp.async) as soon as they are read: the next page's keys arrive during the softmax and the output, its values during
 // the next scores.  Two or three CTAs share an SM and fill each other's waits.
-// Bound by the multiply-add units and their operands from shared memory: 2,048 tokens, 32 heads of 64: 0.53 ms = 32 TFLOP/s of
-// needed work (the plain kernel: 4.32 ms; 0.73 with the tiles of one head after those of another, an SM's share of the work then 0.74 to 1.36
-// of the mean); eight prompts of 256: 125 us (773); 64 tokens behind 1,984: 264 us (330).  Sums over 32 dimensions and over a page at a
-// time keep the error at the plain kernel's (3e-7 of the norm; one chain over all keys: 7e-7, no faster).
+// Bound by the multiply-add units and their operands from shared memory: 2,048 tokens, 32 heads of 64: 0.57 ms = 30 TFLOP/s of
+// needed work (the plain kernel: 4.32 ms; 0.73 with the tiles of one head after those of another, an SM's share of the work then 0.74 to
+// 1.36 of the mean); eight prompts of 256: 115 us (763).
+// Sums are kept short, a score's over 16 dimensions, then two such sums, then 32 dimensions after 32, an output's over 32 keys, then a page
+// (half as long with heads of 32), and what a page's addition into a row's output rounds off joins the next.  The error is then below the
+// plain kernel's, which adds trees of 32 (200 tokens behind 1,600, heads of 64: 1.61e-7 of the norm against 1.89e-7).  Sums over 32 dimensions
+// and 64 keys with nothing kept are 8 % faster and leave 2.1e-7, one chain over all keys 7e-7.
 //
 // Decode steps (one token a sequence) take the same kernel with one or two rows a group and their pages cut into spans, merged by a
 // second kernel: 8 sequences of 500 keys, 32 heads of 64: 20 us a layer, launches by event (35 with the plain kernel in spans of a tile).
@@ -73,6 +76,7 @@ template <int D, int RT, bool SPANS>
 __global__ void __launch_bounds__(kPfThreads, SPANS ? 4 : D <= 64 ? 3 : 2)
 attention_prefill_f32_kernel(const PrefillF32Args a) {
     constexpr int BQ = 8 * RT, DJ = D / 16;
+    constexpr int DIMS = D <= 32 ? 8 : 16, KEYS = D <= 32 ? 16 : 32;   // dimensions and keys whose products are added up by themselves
     extern __shared__ __align__(16) float smem_f[];
     auto& sm = *reinterpret_cast<PrefillF32Smem<D, RT>*>(smem_f);
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
@@ -120,14 +124,14 @@ attention_prefill_f32_kernel(const PrefillF32Args a) {
             a.q + (size_t)(begin + r / group) * a.q_row_stride + (size_t)(g * group + r % group) * D + d);
     }
     float m_run[RT], l_run[RT];      // l_run: this lane's share of the row's sum
-    float o[RT][DJ];
+    float o[RT][DJ], rest[RT][DJ];   // rest: what the additions into o have rounded off
 #pragma unroll
     for (int i = 0; i < RT; ++i) {
         const int r = min(row0 + ty * RT + i, n_rows - 1);
         m_run[i] = a.sinks && span == 0 ? a.sinks[g * group + r % group] : -INFINITY;
         l_run[i] = a.sinks && span == 0 && tx == 0 ? 1.f : 0.f;
 #pragma unroll
-        for (int j = 0; j < DJ; ++j) o[i][j] = 0.f;
+        for (int j = 0; j < DJ; ++j) o[i][j] = rest[i][j] = 0.f;
     }
     const float sqrt_d = sqrtf((float)D);
 
@@ -136,37 +140,45 @@ attention_prefill_f32_kernel(const PrefillF32Args a) {
         const bool masked = base + kPageTokens - 1 > pos_lo || base < first_hi;    // some row must not see some key
         asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncthreads();
-        // ---- scores: 32 dimensions at a time (short chains of additions), sums over even and odd ones side by side
+        // ---- scores: sums over even and odd dimensions of DIMS side by side, then of 32 dimensions, then of 32 after 32
         float sc[RT][4];
 #pragma unroll
         for (int d0 = 0; d0 < D; d0 += 32) {
-            float2 s2[RT][4];
+            float sum[RT][4];
 #pragma unroll
-            for (int i = 0; i < RT; ++i)
+            for (int part = 0; part < 32 / DIMS; ++part) {
+                float2 s2[RT][4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) s2[i][j] = make_float2(0.f, 0.f);
+                for (int i = 0; i < RT; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) s2[i][j] = make_float2(0.f, 0.f);
 #pragma unroll 2
-            for (int d = d0; d < d0 + 32; d += 4) {
-                float4 kv[4];
+                for (int d = d0 + DIMS * part; d < d0 + DIMS * (part + 1); d += 4) {
+                    float4 kv[4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) kv[j] = *reinterpret_cast<const float4*>(&sm.k[tx + 16 * j][d]);
+                    for (int j = 0; j < 4; ++j) kv[j] = *reinterpret_cast<const float4*>(&sm.k[tx + 16 * j][d]);
 #pragma unroll
-                for (int i = 0; i < RT; ++i) {
-                    const float4 qv = *reinterpret_cast<const float4*>(&sm.q[ty * RT + i][d]);
+                    for (int i = 0; i < RT; ++i) {
+                        const float4 qv = *reinterpret_cast<const float4*>(&sm.q[ty * RT + i][d]);
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        fma_pair(s2[i][j], qv.x, qv.y, kv[j].x, kv[j].y);
-                        fma_pair(s2[i][j], qv.z, qv.w, kv[j].z, kv[j].w);
+                        for (int j = 0; j < 4; ++j) {
+                            fma_pair(s2[i][j], qv.x, qv.y, kv[j].x, kv[j].y);
+                            fma_pair(s2[i][j], qv.z, qv.w, kv[j].z, kv[j].w);
+                        }
                     }
                 }
+#pragma unroll
+                for (int i = 0; i < RT; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float both = s2[i][j].x + s2[i][j].y;
+                        sum[i][j] = part == 0 ? both : sum[i][j] + both;
+                    }
             }
 #pragma unroll
             for (int i = 0; i < RT; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float part = s2[i][j].x + s2[i][j].y;
-                    sc[i][j] = d0 == 0 ? part : sc[i][j] + part;
-                }
+                for (int j = 0; j < 4; ++j) sc[i][j] = d0 == 0 ? sum[i][j] : sc[i][j] + sum[i][j];
         }
         __syncthreads();
         if (page + 1 < page_end) fetch_keys(page + 1);
@@ -201,7 +213,7 @@ attention_prefill_f32_kernel(const PrefillF32Args a) {
             }
             l_run[i] = l_run[i] * corr + sum;
 #pragma unroll
-            for (int j = 0; j < DJ; ++j) o[i][j] *= corr;
+            for (int j = 0; j < DJ; ++j) { o[i][j] *= corr; rest[i][j] *= corr; }
         }
         asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncthreads();
@@ -223,31 +235,47 @@ attention_prefill_f32_kernel(const PrefillF32Args a) {
                     for (int j = 0; j < DJ; ++j) o[i][j] = fmaf(p, sm.v[tx + 16 * j][key], o[i][j]);
                 }
             }
-        } else {   // a page's sums by themselves, then into the row's: chains of 32 additions and one per page
-            float2 o2[RT][DJ];
+        } else {   // a page's sums by themselves, KEYS keys at a time, then into the row's with what that rounds off kept (Kahan, 1965)
+            float sum[RT][DJ];
 #pragma unroll
             for (int i = 0; i < RT; ++i)
 #pragma unroll
-                for (int j = 0; j < DJ; ++j) o2[i][j] = make_float2(0.f, 0.f);
+                for (int j = 0; j < DJ; ++j) sum[i][j] = 0.f;
+#pragma unroll 1
+            for (int key0 = 0; key0 < kPageTokens; key0 += KEYS) {
+                float2 o2[RT][DJ];
+#pragma unroll
+                for (int i = 0; i < RT; ++i)
+#pragma unroll
+                    for (int j = 0; j < DJ; ++j) o2[i][j] = make_float2(0.f, 0.f);
 #pragma unroll 2
-            for (int key = 0; key < kPageTokens; key += 4) {
-                float4 vv[DJ];
+                for (int key = key0; key < key0 + KEYS; key += 4) {
+                    float4 vv[DJ];
 #pragma unroll
-                for (int j = 0; j < DJ; ++j) vv[j] = *reinterpret_cast<const float4*>(&sm.v[tx + 16 * j][key]);
+                    for (int j = 0; j < DJ; ++j) vv[j] = *reinterpret_cast<const float4*>(&sm.v[tx + 16 * j][key]);
 #pragma unroll
-                for (int i = 0; i < RT; ++i) {
-                    const float4 pv = *reinterpret_cast<const float4*>(&sm.p[ty * RT + i][key]);
+                    for (int i = 0; i < RT; ++i) {
+                        const float4 pv = *reinterpret_cast<const float4*>(&sm.p[ty * RT + i][key]);
 #pragma unroll
-                    for (int j = 0; j < DJ; ++j) {
-                        fma_pair(o2[i][j], pv.x, pv.y, vv[j].x, vv[j].y);
-                        fma_pair(o2[i][j], pv.z, pv.w, vv[j].z, vv[j].w);
+                        for (int j = 0; j < DJ; ++j) {
+                            fma_pair(o2[i][j], pv.x, pv.y, vv[j].x, vv[j].y);
+                            fma_pair(o2[i][j], pv.z, pv.w, vv[j].z, vv[j].w);
+                        }
                     }
                 }
+#pragma unroll
+                for (int i = 0; i < RT; ++i)
+#pragma unroll
+                    for (int j = 0; j < DJ; ++j) sum[i][j] += o2[i][j].x + o2[i][j].y;
             }
 #pragma unroll
             for (int i = 0; i < RT; ++i)
 #pragma unroll
-                for (int j = 0; j < DJ; ++j) o[i][j] += o2[i][j].x + o2[i][j].y;
+                for (int j = 0; j < DJ; ++j) {
+                    const float add = sum[i][j] + rest[i][j], total = o[i][j] + add, lost = add - (total - o[i][j]);
+                    o[i][j] = total;
+                    rest[i][j] = lost == lost ? lost : 0.f;   // (nothing is kept of an infinite sum)
+                }
         }
         __syncthreads();
         if (page + 1 < page_end) fetch_values(page + 1);
@@ -391,8 +419,8 @@ extern "C" int b200_attention_prefill_f32(const void* q, int q_row_stride, void*
         }
     }
     switch (head_dim) {
-        case 32: return launch_prefill_f32<32, 8>(a, n_seqs, max_q_len, stream);
-        case 64: return launch_prefill_f32<64, 8>(a, n_seqs, max_q_len, stream);
+        case 32: return launch_prefill_f32<32, 4>(a, n_seqs, max_q_len, stream);
+        case 64: return launch_prefill_f32<64, 4>(a, n_seqs, max_q_len, stream);
         case 96: return launch_prefill_f32<96, 4>(a, n_seqs, max_q_len, stream);
         case 128: return launch_prefill_f32<128, 4>(a, n_seqs, max_q_len, stream);
         default: return kErrUnsupportedSize;
