@@ -265,9 +265,7 @@ def attend(shape, qkv: torch.Tensor, out: torch.Tensor, ctx: StepContext, table:
             qkv, qkv.shape[1], out, ctx.cu_seqlens, ctx.kv_lens, table, cache.k, cache.v, ctx.n_seqs, ctx.max_q_len, shape.n_heads,
             shape.n_kv_heads, shape.head_dim, shape.window or 0, n_spans=spans, **terms)):
         return
-    rows = qkv.shape[0] * shape.n_heads
-    # spans of at least one tile of 128 keys, up to two thousand CTAs (of which a GPU holds some 1,800 at a time)
-    splits = 1 if rows >= 2048 else max(1, min(16, 2048 // rows, reach // 128))
+    splits = ops.attention_paged_spans(qkv.shape[0] * shape.n_heads, reach, ops.sm_count(qkv.device))
     ops.attention_paged(qkv, qkv.shape[1], out, ctx.positions, ctx.seq_ids, table, cache.k, cache.v,
                         shape.n_heads, shape.n_kv_heads, shape.head_dim, shape.window or 0, n_splits=splits,
                         keep_first=shape.keep_first, **terms)
