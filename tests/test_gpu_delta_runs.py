@@ -99,8 +99,9 @@ def test_numbers_that_are_not_finite_reach_later_tokens_only(what):
 @pytest.mark.parametrize("kind", ["independent", "activated", "one sign", "weak decay", "dependent keys", "strong decay"])
 def test_runs_are_no_further_from_64_bits_than_the_token_chain(kind, per_head):
     """The norm of all errors against the recurrence in 64 bits, over 500,000 results: what a token at a time leaves, and what runs leave.
-    The states' errors are 65,000 numbers that mostly stem from the same roundings on both sides (unit rows, decays, the state's own);
-    their norms differ by chance by up to one in a hundred, so that a fiftieth is allowed.  Queries and keys of one sign make B U and
+    The states' errors are 65,000 numbers that mostly stem from the same roundings on both sides (unit rows, decays, the state's own):
+    their norms differ by chance by up to one in a hundred, and a run's 32 writes to a state, of alternating signs where keys have one sign, are
+    added up before they join it (a fiftieth more there): a twentieth is allowed.  Queries and keys of one sign make B U and
     (G q) S large and of opposite signs; keys that nearly depend on each other, written with full strength, make the triangular system stiff."""
     lengths, H, dv = [500], 16, 64
     p = problem(lengths, H, H, dv, torch.float32, per_head, kind == "strong decay")
@@ -127,4 +128,4 @@ def test_runs_are_no_further_from_64_bits_than_the_token_chain(kind, per_head):
         got = torch.stack([state[s, :live].view(H, 64, dv) for s in p["slots"]])
         errors.append([float((g.double() - w).norm()) for g, w in ((out, want), (got, states))])
     (runs, runs_state), (chain, chain_state) = errors
-    assert runs <= chain and runs_state <= 1.02 * chain_state
+    assert runs <= chain and runs_state <= 1.05 * chain_state
