@@ -1,7 +1,7 @@
 // Causal grouped-query attention of prompt tokens over the paged cache in float32, a tile of queries at a time.
 //
 // The same sums as the plain kernel (attention_generic.cu: one CTA per token and query head, which reads every key for every
-// query), for passes that bring many tokens of a sequence: a CTA owns BQ rows, a row being a (token, query head) of one kv
+// query), for queries that share keys: a CTA owns BQ rows, a row being a (token, query head) of one kv
 // head, so that a page of keys and values fetched once serves all of them.  Scores, softmax and sums stay 32-bit
 // multiply-adds (inference/InferenceCore.java:106-145 of the reference project).
 //
@@ -21,8 +21,9 @@
 // plain kernel's, which adds trees of 32 (200 tokens behind 1,600, heads of 64: 1.61e-7 of the norm against 1.89e-7).  Sums over 32 dimensions
 // and 64 keys with nothing kept are 8 % faster and leave 2.1e-7, one chain over all keys 7e-7.
 //
-// Decode steps (one token a sequence) take the same kernel with one or two rows a group and their pages cut into spans, merged by a
-// second kernel: 8 sequences of 500 keys, 32 heads of 64: 20 us a layer, launches by event (35 with the plain kernel in spans of a tile).
+// Few queries: one, two or four rows a group, and the pages of a tile cut into spans, merged by a second kernel (the plan that picks both is
+// with the caller).  8 sequences of 500 keys decoded, 32 heads of 64: 11.5 us (25 with the plain kernel in spans of a tile); 2 tokens
+// behind 2,000 keys: 10 us, 16 tokens: 31 (plain 37 and 110; a single tile of 64 rows without spans: 251 and 252).
 //
 // Terms as in the plain kernel (window, chunk, slopes, sinks, gate, softcap; not keep_first).  Values of keys past a
 // sequence's end are read as zeros.  A key that some row of the tile must not see has probability 0 there, and 0 times a value that is
@@ -47,8 +48,8 @@ struct PrefillF32Args {
     const float* gate;
     int q_row_stride, table_stride, n_heads, n_kv_heads, window, chunk, ld_gate;
     float softcap;
-    float* part_o;          // SPANS: [row][span][D] sums, row = token * n_heads + head
-    float* part_ml;         // SPANS: [row][span][2] maximum and sum of exponentials
+    float* part_o;          // with spans: [row][span][D] sums, row = token * n_heads + head
+    float* part_ml;         // with spans: [row][span][2] maximum and sum of exponentials
 };
 
 __device__ __forceinline__ void fma_pair(float2& acc, float ax, float ay, float bx, float by) {
@@ -70,10 +71,9 @@ struct PrefillF32Smem {
     float p[8 * RT][kPfPitch];
 };
 
-// SPANS: the pages are shared out among gridDim.z CTAs, which leave unnormalised results (decode steps: one row of queries per
-// sequence and kv head, RT = 1 or 2, and nothing else to fill the GPU with).
-template <int D, int RT, bool SPANS>
-__global__ void __launch_bounds__(kPfThreads, SPANS ? 4 : D <= 64 ? 3 : 2)
+// gridDim.z > 1: a tile's pages are shared out among so many CTAs, which leave unnormalised results.
+template <int D, int RT>
+__global__ void __launch_bounds__(kPfThreads, RT <= 2 ? 4 : D <= 64 ? 3 : 2)
 attention_prefill_f32_kernel(const PrefillF32Args a) {
     constexpr int BQ = 8 * RT, DJ = D / 16;
     constexpr int DIMS = D <= 32 ? 8 : 16, KEYS = D <= 32 ? 16 : 32;   // dimensions and keys whose products are added up by themselves
@@ -95,8 +95,8 @@ attention_prefill_f32_kernel(const PrefillF32Args a) {
     const int pos_lo = pos0 + row0 / group, pos_hi = pos0 + min(row0 + BQ - 1, n_rows - 1) / group;
     const int first_lo = first_of(pos_lo), first_hi = first_of(pos_hi);
     int page = first_lo / kPageTokens, page_end = pos_hi / kPageTokens + 1;
-    const int span = SPANS ? blockIdx.z : 0, n_spans = SPANS ? gridDim.z : 1;
-    if (SPANS) {
+    const int span = blockIdx.z, n_spans = gridDim.z;
+    if (n_spans > 1) {
         const int each = (page_end - page + n_spans - 1) / n_spans;
         page += span * each;
         page_end = min(page_end, page + each);     // (a span may be empty)
@@ -114,9 +114,9 @@ attention_prefill_f32_kernel(const PrefillF32Args a) {
             copy16_async(&sm.v[c / 16][key], src + (size_t)c * 4, 4 * min(4, max(0, kv_len - page * kPageTokens - key)));
         }
     };
-    if (!SPANS || page < page_end) fetch_keys(page);
+    if (page < page_end) fetch_keys(page);
     asm volatile("cp.async.commit_group;" ::: "memory");
-    if (!SPANS || page < page_end) fetch_values(page);
+    if (page < page_end) fetch_values(page);
     asm volatile("cp.async.commit_group;" ::: "memory");
     for (int c = tid; c < BQ * D / 4; c += kPfThreads) {
         const int r = min(row0 + c / (D / 4), n_rows - 1), d = c % (D / 4) * 4;
@@ -289,7 +289,7 @@ attention_prefill_f32_kernel(const PrefillF32Args a) {
         const int r = row0 + ty * RT + i;
         if (r >= n_rows) continue;
         const int t = begin + r / group, h = g * group + r % group;
-        if (SPANS) {
+        if (n_spans > 1) {
             const size_t part = ((size_t)t * a.n_heads + h) * n_spans + span;
 #pragma unroll
             for (int j = 0; j < DJ; ++j) a.part_o[part * D + tx + 16 * j] = o[i][j];
@@ -340,63 +340,45 @@ attention_spans_merge_f32_kernel(const float* __restrict__ part_o, const float* 
 }
 
 template <int D, int RT>
-static int launch_spans_f32(PrefillF32Args a, int n_seqs, int n_spans, float* scratch, cudaStream_t stream) {
+static int launch_prefill_f32(PrefillF32Args a, int n_seqs, int max_q_len, int n_tokens, int n_spans, float* scratch, cudaStream_t stream) {
+    constexpr int BQ = 8 * RT;
     const size_t smem = sizeof(PrefillF32Smem<D, RT>);
-    auto kernel = attention_prefill_f32_kernel<D, RT, true>;
+    auto kernel = attention_prefill_f32_kernel<D, RT>;
     static bool configured = false;
     if (!configured) {
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return (int)cudaGetLastError();
         configured = true;
     }
     a.part_o = scratch;
-    a.part_ml = scratch + (size_t)n_seqs * a.n_heads * n_spans * D;
-    const int st = launch_pdl(kernel, dim3(a.n_kv_heads, n_seqs, n_spans), dim3(kPfThreads), smem, stream, a);
-    if (st != 0) return st;
-    return launch_pdl(attention_spans_merge_f32_kernel, dim3((unsigned)(n_seqs * a.n_heads)), dim3(D <= 64 ? 64 : 128), 0, stream, a.part_o, a.part_ml,
+    a.part_ml = n_spans > 1 ? scratch + (size_t)n_tokens * a.n_heads * n_spans * D : nullptr;
+    const long long rows = (long long)max_q_len * (a.n_heads / a.n_kv_heads);
+    const int st = launch_pdl(kernel, dim3((unsigned)((rows + BQ - 1) / BQ) * a.n_kv_heads, n_seqs, n_spans), dim3(kPfThreads), smem, stream, a);
+    if (st != 0 || n_spans == 1) return st;
+    return launch_pdl(attention_spans_merge_f32_kernel, dim3((unsigned)(n_tokens * a.n_heads)), dim3(D <= 64 ? 64 : 128), 0, stream, a.part_o, a.part_ml,
                       a.out, n_spans, D, a.n_heads, a.gate, a.ld_gate);
 }
 
 template <int D>
-static int spans_f32_of(const PrefillF32Args& a, int n_seqs, int n_spans, float* scratch, cudaStream_t stream) {
-    if (a.n_heads / a.n_kv_heads <= 8) return launch_spans_f32<D, 1>(a, n_seqs, n_spans, scratch, stream);
-    return launch_spans_f32<D, 2>(a, n_seqs, n_spans, scratch, stream);
-}
-
-template <int D, int RT>
-static int launch_prefill_f32(const PrefillF32Args& a, int n_seqs, int max_q_len, cudaStream_t stream) {
-    constexpr int BQ = 8 * RT;
-    const size_t smem = sizeof(PrefillF32Smem<D, RT>);
-    auto kernel = attention_prefill_f32_kernel<D, RT, false>;
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return (int)cudaGetLastError();
-        configured = true;
+static int prefill_f32_of(const PrefillF32Args& a, int n_seqs, int max_q_len, int n_tokens, int tile, int n_spans, float* scratch, cudaStream_t stream) {
+    switch (tile) {
+        case 8: return launch_prefill_f32<D, 1>(a, n_seqs, max_q_len, n_tokens, n_spans, scratch, stream);
+        case 16: return launch_prefill_f32<D, 2>(a, n_seqs, max_q_len, n_tokens, n_spans, scratch, stream);
+        case 32: return launch_prefill_f32<D, 4>(a, n_seqs, max_q_len, n_tokens, n_spans, scratch, stream);
     }
-    const long long rows = (long long)max_q_len * (a.n_heads / a.n_kv_heads);
-    return launch_pdl(kernel, dim3((unsigned)((rows + BQ - 1) / BQ) * a.n_kv_heads, n_seqs), dim3(kPfThreads), smem, stream, a);
+    return kErrBadArgument;
 }
 
 }  // namespace b200
 
-// How many spans of pages a decode step's attention is cut into (every sequence brings one token, `reach` keys at most), or 0: the
-// plain kernel has it (more heads to a kv head than a tile of this kernel's has rows).  About five CTAs an SM, a page each at least.
-extern "C" int b200_attention_decode_f32_spans(int n_seqs, int n_heads, int n_kv_heads, int reach) {
-    if (n_seqs <= 0 || n_kv_heads <= 0 || n_heads / n_kv_heads > 16) return 0;
-    const long long ctas = (long long)n_seqs * n_kv_heads;
-    const long long want = (5ll * b200::device_sm_count() + ctas - 1) / ctas, pages = ((long long)reach + b200::kPageTokens - 1) / b200::kPageTokens;
-    const long long spans = want < pages ? want : pages;
-    return (int)(spans < 1 ? 1 : spans > b200::kMostSpans ? b200::kMostSpans : spans);
-}
-
 // Queries: the first n_heads head_dim elements of rows of q_row_stride elements, packed sequence after sequence
 // (cu_seqlens); kv_lens counts each sequence's keys with this pass's.  head_dim 32, 64, 96 or 128; other sizes, rows off the 16-byte
-// grid and more than 65,535 sequences are left to the plain kernel (kErrUnsupportedSize).  n_spans > 0: every sequence brings one
-// token, whose keys are cut into so many spans (at most 16; scratch: n_seqs n_heads n_spans (head_dim + 2) floats).
+// grid and more than 65,535 sequences are left to the plain kernel (kErrUnsupportedSize).  tile: rows of a tile, 8, 16 or 32.
+// n_spans > 1: every tile's keys are cut into so many spans (at most 16; scratch: n_tokens n_heads n_spans (head_dim + 2) floats).
 extern "C" int b200_attention_prefill_f32(const void* q, int q_row_stride, void* out, const int* cu_seqlens, const int* kv_lens,
                                           const int* page_table, int table_stride, const void* k_pool, const void* v_pool,
-                                          int n_seqs, int max_q_len, int n_heads, int n_kv_heads, int head_dim, int window,
+                                          int n_seqs, int max_q_len, int n_tokens, int n_heads, int n_kv_heads, int head_dim, int window,
                                           int chunk, const float* slopes, const float* sinks, const void* gate, int ld_gate,
-                                          float softcap, int n_spans, float* scratch, cudaStream_t stream) {
+                                          float softcap, int tile, int n_spans, float* scratch, cudaStream_t stream) {
     using namespace b200;
     if (n_seqs <= 0 || max_q_len <= 0) return 0;
     if (!(softcap >= 0.f) || chunk < 0 || (chunk > 0 && window > 0)) return kErrBadArgument;
@@ -408,21 +390,12 @@ extern "C" int b200_attention_prefill_f32(const void* q, int q_row_stride, void*
     a.k_pool = (const float*)k_pool; a.v_pool = (const float*)v_pool; a.slopes = slopes; a.sinks = sinks; a.gate = (const float*)gate;
     a.q_row_stride = q_row_stride; a.table_stride = table_stride; a.n_heads = n_heads; a.n_kv_heads = n_kv_heads;
     a.window = window; a.chunk = chunk; a.ld_gate = ld_gate; a.softcap = softcap;
-    if (n_spans > 0) {
-        if (max_q_len != 1 || n_spans > kMostSpans || scratch == nullptr || n_heads / n_kv_heads > 16) return kErrBadArgument;
-        switch (head_dim) {
-            case 32: return spans_f32_of<32>(a, n_seqs, n_spans, scratch, stream);
-            case 64: return spans_f32_of<64>(a, n_seqs, n_spans, scratch, stream);
-            case 96: return spans_f32_of<96>(a, n_seqs, n_spans, scratch, stream);
-            case 128: return spans_f32_of<128>(a, n_seqs, n_spans, scratch, stream);
-            default: return kErrUnsupportedSize;
-        }
-    }
+    if (n_spans < 1 || n_spans > kMostSpans || (n_spans > 1 && scratch == nullptr)) return kErrBadArgument;
     switch (head_dim) {
-        case 32: return launch_prefill_f32<32, 4>(a, n_seqs, max_q_len, stream);
-        case 64: return launch_prefill_f32<64, 4>(a, n_seqs, max_q_len, stream);
-        case 96: return launch_prefill_f32<96, 4>(a, n_seqs, max_q_len, stream);
-        case 128: return launch_prefill_f32<128, 4>(a, n_seqs, max_q_len, stream);
+        case 32: return prefill_f32_of<32>(a, n_seqs, max_q_len, n_tokens, tile, n_spans, scratch, stream);
+        case 64: return prefill_f32_of<64>(a, n_seqs, max_q_len, n_tokens, tile, n_spans, scratch, stream);
+        case 96: return prefill_f32_of<96>(a, n_seqs, max_q_len, n_tokens, tile, n_spans, scratch, stream);
+        case 128: return prefill_f32_of<128>(a, n_seqs, max_q_len, n_tokens, tile, n_spans, scratch, stream);
         default: return kErrUnsupportedSize;
     }
 }

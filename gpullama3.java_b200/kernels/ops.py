@@ -16,6 +16,7 @@ PAGE_TOKENS = 64  # must equal b200::kPageTokens
 # what the plain kernels, which take every size the others refuse, are built for
 HEAD_DIM_STEP, MAX_HEAD_DIM = 16, 512   # attention_generic.cu
 MAX_ROTARY_DIM = 512                    # rope_cache.cu
+F32_TILE_HEAD_DIMS = (32, 64, 96, 128)  # attention_prefill_f32.cu
 
 _DTYPE_CODE = {torch.float32: F32, torch.bfloat16: BF16}
 
@@ -79,8 +80,8 @@ _SIGNATURES = {
                                                         c_void_p, c_void_p, ctypes.c_longlong, c_int, c_int, c_int,
                                                         c_int, c_int, c_int, c_void_p, c_int, c_int, c_int]),
     "b200_attention_prefill_f32": ("attention_prefill_f32", [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
-                                                             c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
-                                                             c_void_p, c_void_p, c_int, c_float, c_int, c_void_p]),
+                                                             c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
+                                                             c_void_p, c_void_p, c_void_p, c_int, c_float, c_int, c_int, c_void_p]),
     "b200_attention_prefill_tc": ("attention_prefill_tcgen05", [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p,
                                                                 c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int,
                                                                 c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
@@ -383,12 +384,13 @@ def attention_prefill_f32(q: torch.Tensor, q_row_stride: int, out: torch.Tensor,
                           page_table: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, n_seqs: int, max_q_len: int,
                           n_heads: int, n_kv_heads: int, head_dim: int, window: int = 0, *, chunk: int = 0,
                           slopes: torch.Tensor | None = None, sinks: torch.Tensor | None = None,
-                          gate: torch.Tensor | None = None, softcap: float = 0.0, n_spans: int = 0) -> bool:
+                          gate: torch.Tensor | None = None, softcap: float = 0.0, tile: int = 0, n_spans: int = 0, alloc=None) -> bool:
     """``attention_paged`` of float32 queries that lie sequence after sequence (``cu_seqlens`` int32 [n_seqs + 1]; ``kv_lens``
-    counts this pass's tokens), a tile of them at a time; the same terms without kept first positions.  ``n_spans`` > 0: a decode
-    step (``max_q_len`` 1) whose keys are cut into so many spans (``attention_decode_f32_spans``), merged by a second kernel.
-    Returns False, having done nothing, for operands it does not take."""
-    if q.dtype != torch.float32 or head_dim not in (32, 64, 96, 128) or q_row_stride % 4 or q.data_ptr() & 15:
+    counts this pass's tokens), a tile of them at a time; the same terms without kept first positions.  ``n_spans`` > 1: a tile's
+    keys are cut into so many spans (``attention_f32_plan``), merged by a second kernel; their scratch comes from ``alloc(shape, dtype)``
+    when given (None from it: no spans).  ``tile``: rows of a tile, 8, 16 or 32 (0: 32).  Returns False, having done nothing, for
+    operands it does not take."""
+    if q.dtype != torch.float32 or head_dim not in F32_TILE_HEAD_DIMS or q_row_stride % 4 or q.data_ptr() & 15:
         return False
     _dev(q, out, cu_seqlens, kv_lens, page_table, k_pool, v_pool, slopes, sinks, gate)
     assert out.is_contiguous() and out.shape[1] == n_heads * head_dim and out.dtype == q.dtype == k_pool.dtype == v_pool.dtype
@@ -399,23 +401,67 @@ def attention_prefill_f32(q: torch.Tensor, q_row_stride: int, out: torch.Tensor,
     for t in (slopes, sinks):
         assert t is None or (t.dtype == torch.float32 and t.is_contiguous() and t.numel() == n_heads)
     assert gate is None or (gate.dtype == q.dtype and gate.stride(1) == 1 and gate.shape[1] >= n_heads)
-    scratch = torch.empty(n_seqs * n_heads * n_spans * (head_dim + 2), dtype=torch.float32, device=q.device) if n_spans > 0 else None
+    n_tokens, n_spans, scratch = out.shape[0], max(1, int(n_spans)), None
+    if n_spans > 1:
+        shape = (n_tokens * n_heads * n_spans * (head_dim + 2),)
+        scratch = alloc(shape, torch.float32) if alloc is not None else torch.empty(shape, dtype=torch.float32, device=q.device)
+        if scratch is None:
+            n_spans = 1
     ptr = lambda t: t.data_ptr() if t is not None else None
     status = _fn("b200_attention_prefill_f32")(
         q.data_ptr(), q_row_stride, out.data_ptr(), cu_seqlens.data_ptr(), kv_lens.data_ptr(), page_table.data_ptr(),
-        page_table.shape[1], k_pool.data_ptr(), v_pool.data_ptr(), n_seqs, int(max_q_len), n_heads, n_kv_heads, head_dim,
+        page_table.shape[1], k_pool.data_ptr(), v_pool.data_ptr(), n_seqs, int(max_q_len), n_tokens, n_heads, n_kv_heads, head_dim,
         int(window), int(chunk), ptr(slopes), ptr(sinks), ptr(gate), gate.stride(0) if gate is not None else 0, float(softcap),
-        int(n_spans), ptr(scratch), _stream())
+        int(tile) or 32, n_spans, ptr(scratch), _stream())
     if status == _UNSUPPORTED:
         return False
     _check(status, "attention_paged")
     return True
 
 
-def attention_decode_f32_spans(n_seqs: int, n_heads: int, n_kv_heads: int, reach: int) -> int:
-    """Into how many spans ``attention_prefill_f32`` cuts a decode step's keys (``reach``: the most one token sees); 0: the
-    step is one for ``attention_paged``."""
-    return int(library("attention_prefill_f32").b200_attention_decode_f32_spans(n_seqs, n_heads, n_kv_heads, int(reach)))
+# What a float32 attention launch takes, in microseconds, fitted to 7,000 measured launches (heads of 32 to 128, 1 to 16 query heads to a
+# kv head, 1 to 64 sequences of 1 to 256 tokens behind 0 to 8,000): per tile of ``attention_prefill_f32`` the time a page takes a CTA
+# that has the SM to itself (a constant and a share per 64 dimensions) and the time it takes of an SM that is full (per 64 dimensions);
+# the same for 128 keys of one row of the plain kernel (tile 0).
+_F32_PAGE = {8: (0.83, 1.04, 1.44), 16: (1.15, 1.46, 1.77), 32: (2.50, 1.49, 2.57), 0: (1.11, 2.29, 0.99)}
+_F32_MOST_SPANS, _F32_MOST_PARTS = 16, 1 << 25   # (spans' unnormalised results: 128 MB at most)
+
+
+def attention_f32_plan(q_lens: list[int], kv_lens: list[int], n_heads: int, n_kv_heads: int, head_dim: int, reach: int,
+                       sms: int) -> tuple[int, int]:
+    """How a float32 pass is attended whose sequences bring ``q_lens`` tokens to ``kv_lens`` keys each (this pass's among them; a
+    token sees ``reach`` at most): (rows of a tile, spans of keys) for ``attention_prefill_f32``, or (0, 0): by ``attention_paged``.
+
+    Small tiles and many spans fill the GPU where there are few queries, large tiles read keys and values less often, spans cost a
+    second launch and their results' way through memory: of each tile with one, two and four spans and with CTAs for two and a half
+    rounds of SMs and for five, the one that the figures above say is fastest (4 % above the fastest measured on the mean, 41 % at most; 2 tokens behind 8,000,
+    32 heads of 64 over 8: 24 us, one tile of 64 rows without spans 967).  The plain kernel reads keys and values for every query head anew,
+    which one or two heads to a kv head can afford (8 sequences of 2,000 keys decoded, 32 heads of 64: 69 us, 97 in tiles of 8)."""
+    group, wide = n_heads // n_kv_heads, head_dim / 64
+    longest = -(-min(reach, max(kv_lens)) // PAGE_TOKENS)
+    pages = [min(reach, kv - q / 2) / PAGE_TOKENS + 0.5 for q, kv in zip(q_lens, kv_lens)]
+    best = (math.inf, 0, 0)
+    for tile, (alone, alone_wide, full) in _F32_PAGE.items():
+        if tile == 0:
+            if group > 2:
+                continue
+            rows, each, work = sum(q_lens) * n_heads, (longest + 1) // 2, sum(q * n_heads * (p / 2 + 0.5) for q, p in zip(q_lens, pages))
+            options = {attention_paged_spans(rows, min(reach, max(kv_lens)), sms)}
+        else:
+            tiles = [-(-q * group // tile) * n_kv_heads for q in q_lens]
+            each, work = longest, sum(t * p for t, p in zip(tiles, pages))
+            most = min(_F32_MOST_SPANS, longest)
+            options = {min(most, n) for n in (1, 2, 4)} | {max(1, min(most, n * sms // (2 * sum(tiles)))) for n in (5, 10)}
+        for spans in sorted(options):
+            if tile and spans > 1 and sum(q_lens) * n_heads * spans * (head_dim + 2) > _F32_MOST_PARTS:
+                continue
+            latency = -(-each // spans) * (alone + alone_wide * wide)
+            through = work * full * wide / sms
+            cost = max(latency, through) + 0.66 * min(latency, through)
+            if spans > 1:   # (a twentieth more, so that what is equal by these figures stays in one launch)
+                cost = 1.05 * cost + 1.0 + (5.75e-6 * sum(q_lens) * n_heads * spans * head_dim if tile else 0.0)
+            best = min(best, (cost, tile, spans if tile else 0))
+    return best[1:]
 
 
 # --------------------------------------------------------------------------- matrix products

@@ -258,13 +258,20 @@ def attend(shape, qkv: torch.Tensor, out: torch.Tensor, ctx: StepContext, table:
     terms = dict(chunk=getattr(shape, "chunk", None) or 0, slopes=getattr(shape, "slopes", None), sinks=getattr(shape, "sinks", None),
                  gate=gate, softcap=getattr(shape, "softcap", None) or 0.0)
     reach = min(ctx.capacity(cache.group), _reach(shape) or ctx.capacity(cache.group))
-    # float32: a tile of a sequence's queries at a time, decode steps in spans of pages
-    tiled = qkv.dtype == torch.float32 and not shape.keep_first
-    spans = ops.attention_decode_f32_spans(ctx.n_seqs, shape.n_heads, shape.n_kv_heads, reach) if tiled and ctx.all_decode else 0
-    if (tiled and (spans or not ctx.all_decode) and ops.attention_prefill_f32(
-            qkv, qkv.shape[1], out, ctx.cu_seqlens, ctx.kv_lens, table, cache.k, cache.v, ctx.n_seqs, ctx.max_q_len, shape.n_heads,
-            shape.n_kv_heads, shape.head_dim, shape.window or 0, n_spans=spans, **terms)):
-        return
+    if qkv.dtype == torch.float32 and not shape.keep_first and shape.head_dim in ops.F32_TILE_HEAD_DIMS:
+        # a tile of a sequence's queries at a time, the keys of few tiles in spans of pages; a decode step's launches must be right
+        # for sequences of any length up to the step's capacity
+        key = ("float32 attention", shape.n_heads, shape.n_kv_heads, shape.head_dim, reach)
+        plan = ctx.extras.get(key)
+        if plan is None:
+            kv_lens = [reach] * ctx.n_seqs if ctx.all_decode else [s + q for s, q in zip(ctx.start_pos, ctx.q_lens)]
+            plan = ctx.extras[key] = ops.attention_f32_plan(ctx.q_lens, kv_lens, shape.n_heads, shape.n_kv_heads, shape.head_dim, reach,
+                                                            ops.sm_count(qkv.device))
+        tile, spans = plan
+        if tile and ops.attention_prefill_f32(qkv, qkv.shape[1], out, ctx.cu_seqlens, ctx.kv_lens, table, cache.k, cache.v, ctx.n_seqs,
+                                              ctx.max_q_len, shape.n_heads, shape.n_kv_heads, shape.head_dim, shape.window or 0, tile=tile,
+                                              n_spans=spans, alloc=ctx.empty, **terms):
+            return
     splits = ops.attention_paged_spans(qkv.shape[0] * shape.n_heads, reach, ops.sm_count(qkv.device))
     ops.attention_paged(qkv, qkv.shape[1], out, ctx.positions, ctx.seq_ids, table, cache.k, cache.v,
                         shape.n_heads, shape.n_kv_heads, shape.head_dim, shape.window or 0, n_splits=splits,

@@ -185,6 +185,22 @@ def test_attention_of_decode_steps_in_spans(kv_lens, n_spans, H, G, D, terms):
     close_enough(got, want, D, biggest)
 
 
+@pytest.mark.parametrize("q_lens, kv_lens", [([5, 1, 100, 77], [5, 300, 100, 500]), ([2], [1030]), ([3, 3, 1], [64, 65, 700])])
+@pytest.mark.parametrize("H, G, D", [(6, 2, 32), (4, 4, 64), (16, 1, 64), (6, 3, 96), (6, 2, 128)])
+@pytest.mark.parametrize("tile, n_spans", [(8, 1), (8, 5), (16, 3), (32, 1), (32, 16)])
+@pytest.mark.parametrize("terms", [{}, {"chunk": 48, "sinks": 1, "gate": 1}, {"slopes": 1, "softcap": 5.0, "window": 100, "sinks": 1}, {"odd_values": 1}],
+                         ids=str)
+def test_attention_over_tiles_in_spans(q_lens, kv_lens, H, G, D, tile, n_spans, terms):
+    """Tiles of every size, their keys whole and in spans (some of them empty), against the plain kernel."""
+    o = ops()
+    q, k, v, table, positions, seq_ids, cu, lens, window, terms, biggest = attention_problem(q_lens, kv_lens, H, G, D, terms)
+    want, got = torch.empty(len(positions), H * D, device="cuda"), torch.full((len(positions), H * D), 7.0, device="cuda")
+    o.attention_paged(q, q.shape[1], want, positions, seq_ids, table, k, v, H, G, D, window, **terms)
+    assert o.attention_prefill_f32(q, q.shape[1], got, cu, lens, table, k, v, len(q_lens), max(q_lens), H, G, D, window, tile=tile, n_spans=n_spans,
+                                   **terms)
+    close_enough(got, want, D, biggest)
+
+
 def attention_in_64_bits(q, k, v, table, q_lens, kv_lens, H, G, D):
     out, at = [], 0
     for i, (n, length) in enumerate(zip(q_lens, kv_lens)):
@@ -199,8 +215,8 @@ def attention_in_64_bits(q, k, v, table, q_lens, kv_lens, H, G, D):
 
 
 @pytest.mark.parametrize("H, G, D", [(32, 8, 32), (32, 8, 64), (24, 8, 96), (24, 8, 128)])
-@pytest.mark.parametrize("q_len, kv_len", [(300, 300), (200, 1800)])
-def test_attention_over_tiles_is_no_further_from_64_bits_than_the_plain_kernel(H, G, D, q_len, kv_len):
+@pytest.mark.parametrize("q_len, kv_len, tile, n_spans", [(300, 300, 32, 1), (200, 1800, 32, 1), (64, 2000, 32, 8), (16, 2000, 16, 16), (12, 1200, 8, 1)])
+def test_attention_over_tiles_is_no_further_from_64_bits_than_the_plain_kernel(H, G, D, q_len, kv_len, tile, n_spans):
     """The norm of all errors (100,000 results and more, so that it moves by less than a fiftieth by chance) with every key unmasked where
     causality allows, queries as large as a norm leaves them."""
     o = ops()
@@ -209,5 +225,35 @@ def test_attention_over_tiles_is_no_further_from_64_bits_than_the_plain_kernel(H
     want = attention_in_64_bits(q, k, v, table, [q_len], [kv_len], H, G, D)
     plain, got = torch.empty(q_len, H * D, device="cuda"), torch.empty(q_len, H * D, device="cuda")
     o.attention_paged(q, q.shape[1], plain, positions, seq_ids, table, k, v, H, G, D)
-    assert o.attention_prefill_f32(q, q.shape[1], got, cu, lens, table, k, v, 1, q_len, H, G, D)
+    assert o.attention_prefill_f32(q, q.shape[1], got, cu, lens, table, k, v, 1, q_len, H, G, D, tile=tile, n_spans=n_spans)
     assert float((got.double() - want).norm()) <= 1.02 * float((plain.double() - want).norm())
+
+
+@pytest.mark.parametrize("q_lens, kv_lens", [([2], [700]), ([3, 1, 40], [3, 900, 40]), ([1] * 3, [900, 65, 1]), ([1] * 30, [500] * 30), ([150, 2], [150, 300])])
+@pytest.mark.parametrize("H, G, D", [(8, 2, 64), (4, 4, 64), (6, 1, 128), (4, 2, 48)])
+def test_attend_of_float32_passes(q_lens, kv_lens, H, G, D):
+    """Through the choice of kernel, tile and spans that a model's mixers make; 48 has no tiles."""
+    from types import SimpleNamespace
+
+    from gpullama3.java_b200.parts.attention import attend
+
+    q, k, v, table, positions, seq_ids, cu, lens, _, _, biggest = attention_problem(q_lens, kv_lens, H, G, D, {})
+    for i, length in enumerate(kv_lens):      # (no NaN behind the ends: the plain computation here would meet them)
+        if length % 64:
+            page = int(table[i, length // 64])
+            k[page, :, length % 64:], v[page, :, :, length % 64:] = 0.0, 0.0
+    asked = []
+
+    def empty(shape, dtype):
+        asked.append(tuple(shape))
+        return torch.empty(shape, dtype=dtype, device="cuda")
+
+    ctx = SimpleNamespace(n_seqs=len(q_lens), q_lens=q_lens, start_pos=[b - a for a, b in zip(q_lens, kv_lens)], max_q_len=max(q_lens),
+                          all_decode=max(q_lens) == 1, positions=positions, seq_ids=seq_ids, cu_seqlens=cu, kv_lens=lens, extras={}, empty=empty,
+                          capacity=lambda group: max(kv_lens))
+    shape = SimpleNamespace(n_heads=H, n_kv_heads=G, head_dim=D, window=None, keep_first=0)
+    out = torch.full((sum(q_lens), H * D), 7.0, device="cuda")
+    attend(shape, q, out, ctx, table, SimpleNamespace(k=k, v=v, group=0))
+    close_enough(out, attention_in_64_bits(q, k, v, table, q_lens, kv_lens, H, G, D).float(), D, biggest)
+    if D != 48 and q_lens == [2]:
+        assert ctx.extras and asked      # (two tokens behind 698: their keys go in spans, whose scratch the step gives)
