@@ -188,7 +188,8 @@ gemm_generic_big_kernel(const TA* __restrict__ A, int lda, const TW* __restrict_
 // ---------------------------------------------------------------------------------------------
 // The same product for a decode step's few rows (M <= 16): tiles of 64 tokens would leave the FMA units idle and
 // read every weight through shared memory for nothing.  Here the weight rows are streamed 16 bytes per lane, every
-// element meeting all M tokens' activations (which stay in L1); see gemm_fewrows_kernel.
+// element meeting all M tokens' activations, which a lane holds in registers (gemm_fewrows_kernel) or fetches from L1
+// (gemm_fourrows_kernel).
 template <typename T> __device__ __forceinline__ float4 load4(const T* p);
 template <> __device__ __forceinline__ float4 load4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
 template <> __device__ __forceinline__ float4 load4<__nv_bfloat16>(const __nv_bfloat16* p) {
@@ -334,9 +335,94 @@ gemm_fewrows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W,
     }
 }
 
+// The same for at most eight tokens with half as many rows a CTA and the activations fetched from L1 for every four weight rows: sums are
+// kept over all of K and exchanged once, and tokens that are not there cost nothing.  Faster where the kernel above has fewer CTAs than
+// the GPU has SMs and K is long (an SM's share is then one CTA's chain of slices: 8 tokens, 128 x 2,048 in float32: 2.7 us against 4.2), and
+// for bfloat16 weights, whose multiply-adds and exchanges take longer than their stream (5 tokens, 16,384 x 2,048: 33 us against 44);
+// fourrows_wins draws the line.  Four rows of sums for up to eight tokens are the 32 numbers that a warp sums by halving.
+constexpr int kFourRows = 4, kFourTokens = 8;
+
+template <typename TA, typename TW, typename TC>
+__global__ void __launch_bounds__(kFewThreads)
+gemm_fourrows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W, int ldw, TC* __restrict__ C, int ldc,
+                     int M, int N, int K, int epilogue, ProductExtras batch) {
+    constexpr int MT = kFourTokens;
+    pdl_launch_dependents();
+    pdl_wait();
+    A += (size_t)blockIdx.z * batch.a;
+    W += (size_t)blockIdx.z * batch.w;
+    C += (size_t)blockIdx.z * batch.c;
+    __shared__ float part[kFewWarps][kFourRows * MT];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n0 = blockIdx.x * kFourRows;
+    const TW* w[kFourRows];
+#pragma unroll
+    for (int r = 0; r < kFourRows; ++r) w[r] = W + (size_t)min(n0 + r, N - 1) * ldw;   // clamped: read, never stored
+    float acc[kFourRows * MT];
+#pragma unroll
+    for (int i = 0; i < kFourRows * MT; ++i) acc[i] = 0.f;
+#pragma unroll 2
+    for (int k = (warp * 32 + lane) * 4; k < K; k += kFewSlice) {
+        float4 wv[kFourRows];
+#pragma unroll
+        for (int r = 0; r < kFourRows; ++r) wv[r] = load4<TW>(w[r] + k);
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+            if (m < M) {
+                const float4 x = load4<TA>(A + (size_t)m * lda + k);
+#pragma unroll
+                for (int r = 0; r < kFourRows; ++r)
+                    acc[r * MT + m] = fmaf(wv[r].w, x.w, fmaf(wv[r].z, x.z, fmaf(wv[r].y, x.y, fmaf(wv[r].x, x.x, acc[r * MT + m]))));
+            }
+        }
+    }
+    part[warp][lane] = reduce_by_halving<kFourRows * MT>(acc, lane);   // lane l: sum number l
+    __syncthreads();
+    // thread i < 32: row i / MT, token i % MT; the warps' sums are added in warp order
+    const int i = threadIdx.x;
+    if (i >= kFourRows * MT) return;
+    const int r = i / MT, m = i % MT, n = n0 + r;
+    float sum = 0.f;
+#pragma unroll
+    for (int wp = 0; wp < kFewWarps; ++wp) sum += part[wp][i];
+    if (batch.bias && n < N) sum += batch.bias[n];
+    if (epilogue >= 2) {
+        float up = 0.f;   // the gate row's thread also adds up the up row (the next row of the CTA)
+        if ((r & 1) == 0) {
+#pragma unroll
+            for (int wp = 0; wp < kFewWarps; ++wp) up += part[wp][i + MT];
+            if (batch.bias && n + 1 < N) up += batch.bias[n + 1];
+            if (m < M && n + 1 < N) C[(size_t)m * ldc + n / 2] = from_f32<TC>(gated_pair(sum, up, epilogue, batch.gate_limit, batch.gate_slope));
+        }
+    } else if (m < M && n < N) {
+        TC* c = C + (size_t)m * ldc + n;
+        if (epilogue == 1) *c = from_f32<TC>(to_f32<TC>(*c) + sum);
+        else *c = from_f32<TC>(stored(batch, n, sum));
+    }
+}
+
+// Measured with weights from memory, M 1 to 16, N 32 to 28,672, K 64 to 14,336.  Up to one slice of K the kernel of eight rows is never
+// slower.  float32 weights: four rows win below 384 weight rows (1.4 times at 128 x 2,048), from five tokens on as long as eight rows make
+// fewer CTAs than there are SMs (1.3 times at 1,024 x 2,048; 0.75 at 2,048 x 2,048).  bfloat16 weights: four rows win (1.1 to 1.5 times)
+// except for four tokens, which fill the other kernel's registers, where eight rows make one round of CTAs (0.7 at 2,048 x 2,048), and for
+// three or eight tokens over a long K (0.8 at 4,096 x 14,336).
+static bool fourrows_wins(int M, int N, int K, bool bf16_weights) {
+    if (M > kFourTokens || K <= kFewSlice) return false;
+    const int ctas = (N + kFewRows - 1) / kFewRows, sms = device_sm_count();
+    if (!bf16_weights) return M <= 4 ? N < 384 : ctas <= sms;
+    return M != 4 && !(ctas > sms && ctas <= 2 * sms) && !(K >= 8192 && (M == 3 || M >= 7));
+}
+
 template <typename TA, typename TW, typename TC>
 static int launch_fewrows(const void* A, int lda, const void* W, int ldw, void* C, int ldc, int M, int N, int K, int epilogue,
                           int n_batch, ProductExtras batch, cudaStream_t stream) {
+    if (fourrows_wins(M, N, K, sizeof(TW) == 2)) {
+        // (an early start for grids that leave room on the SMs: about one round of CTAs would settle unevenly beside the predecessor's, 8 tokens,
+        // 4,096 x 4,096: 26.0 us instead of 22.5)
+        const dim3 grid((N + kFourRows - 1) / kFourRows, 1, n_batch);
+        return launch_pdl_cluster(gemm_fourrows_kernel<TA, TW, TC>, grid, dim3(kFewThreads), 0, stream, dim3(1, 1, 1), (long long)grid.x * n_batch <= 2 * device_sm_count(),
+                                  (const TA*)A, lda, (const TW*)W, ldw, (TC*)C, ldc, M, N, K, epilogue, batch);
+    }
     const dim3 grid((N + kFewRows - 1) / kFewRows, 1, n_batch);
     auto go = [&](auto kernel) {
         return launch_pdl(kernel, grid, dim3(kFewThreads), 0, stream, (const TA*)A, lda, (const TW*)W, ldw, (TC*)C, ldc, M, N, K, epilogue, batch);
