@@ -289,6 +289,7 @@ extern "C" int b200_streams_step(float* x, const float* mix, const float* write,
         auto go = [&](auto launch) { return launch(x, mix, write, y, read, w, out, n_tokens, n_streams, width, eps, stream); };
         if (!vec) return go(b200::launch_streams_step<TO, 1, 0>);
         switch (n_streams) {
+            case 1: return go(b200::launch_streams_step<TO, 4, 1>);
             case 2: return go(b200::launch_streams_step<TO, 4, 2>);
             case 3: return go(b200::launch_streams_step<TO, 4, 3>);
             case 4: return go(b200::launch_streams_step<TO, 4, 4>);

@@ -223,6 +223,31 @@ def test_streams_step(streams, width, T):
 
 
 @DTYPES
+@pytest.mark.parametrize("streams, width, T", [(1, 2048, 3), (2, 4100, 2), (4, 2500, 3), (4, 4100, 2), (5, 64, 9), (8, 30, 4), (6, 4104, 2), (8, 4100, 2),
+                                               (3, 4100, 2), (3, 1027, 2), (8, 1030, 2)])
+def test_streams_step_in_every_form(dtype, streams, width, T):
+    """Every number of streams that has a kernel of its own and the general one, rows in one and in two accesses a thread and beyond the
+    columns that a thread keeps (4,096 by fours, 1,024 one by one), with and without the read, results in either type.  A result is a sum
+    of up to nine products and a norm: some twenty roundings, and one to bfloat16."""
+    xs = _rand(T, streams, width, seed=2).cuda()
+    lst = [xs[:, a].cpu().to(F) for a in range(streams)]
+    W = {"h.mix": _rand(streams, streams, seed=4).to(F), "h.out": _rand(streams, seed=5).to(F)}
+    read, nw = _rand(streams, seed=3), _rand(width, seed=6) * 0.3
+    y = _rand(T, width, seed=7).cuda()
+    ref = plain.connect(lst, W, "h.", y.cpu().to(F))
+    silent = xs.clone()
+    ops.streams_step(silent, W["h.mix"].float().cuda(), W["h.out"].float().cuda(), y.clone())
+    out = torch.full((T, width), 9.0, dtype=dtype, device="cuda")
+    ops.streams_step(xs, W["h.mix"].float().cuda(), W["h.out"].float().cuda(), y, read.cuda(), (1 + nw).cuda(), out, 1e-5)
+    assert torch.equal(silent, xs) and float(y.abs().max()) == 0.0
+    for j in range(streams):
+        torch.testing.assert_close(xs[:, j].cpu().to(F), ref[j], rtol=2e-5, atol=2e-5)
+    u = sum(read[a].to(F) * ref[a] for a in range(streams))
+    slack = 2.0 ** -8 if dtype == torch.bfloat16 else 0.0
+    torch.testing.assert_close(out.cpu().to(F), plain.offset_norm(u, nw.to(F), 1e-5), rtol=5e-5 + slack, atol=5e-5)
+
+
+@DTYPES
 def test_head_rows_into_cache_pages(dtype):
     """Keys as rows and values transposed, each at its token's position in the page its sequence's table names."""
     T, G, dk, dv, D, n_pages = 7, 2, 24, 16, 32, 5
