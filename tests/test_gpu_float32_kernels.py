@@ -15,6 +15,25 @@ def ops():
     return o
 
 
+def split_in_three(x):
+    """The three bfloat16 parts of 2^24 x, in 64 bits."""
+    x, parts = x.float() * 2.0 ** 24, []
+    for _ in range(3):
+        parts.append(x.to(torch.bfloat16).float())
+        x = x - parts[-1]
+    return [p.double() * 2.0 ** -24 for p in parts]
+
+
+TERMS = [(2, 0), (0, 2), (1, 1), (1, 0), (0, 1), (0, 0)]
+NORM = 3.0e-7      # of a product's errors; the kernel leaves 1.0e-7 to 1.3e-7 below K = 5,000
+SHAPES = [(17, 64, 1024), (64, 128, 512), (129, 258, 1032), (300, 256, 4100), (100, 130, 2048)]
+
+
+def operands(M, N, K):
+    g = torch.Generator().manual_seed(M * N + K)
+    return torch.randn(M, K, generator=g), torch.randn(N, K, generator=g) / math.sqrt(K)
+
+
 def _epilogue(o, epilogue, sums, c0, silu):
     if epilogue == o.EPILOGUE_STORE:
         out = sums.clone()
@@ -257,3 +276,15 @@ def test_attend_of_float32_passes(q_lens, kv_lens, H, G, D):
     close_enough(out, attention_in_64_bits(q, k, v, table, q_lens, kv_lens, H, G, D).float(), D, biggest)
     if D != 48 and q_lens == [2]:
         assert ctx.extras and asked      # (two tokens behind 698: their keys go in spans, whose scratch the step gives)
+
+
+@pytest.mark.parametrize("M, N, K, tensor_cores", [(64, 1024, 64, False), (100, 2048, 64, False), (127, 512, 128, False), (64, 512, 128, True),
+                                                   (100, 512, 192, True), (128, 1024, 64, True), (17, 1024, 124, False)])
+def test_products_of_a_short_k_go_where_they_are_faster(M, N, K, tensor_cores):
+    o = ops()
+    a, w = operands(M, N, K)
+    a, w, c = a.cuda(), w.cuda(), torch.full((M, N), 7.0, device="cuda")
+    assert o.gemm_f32_tcgen05(a, w, c) == tensor_cores
+    o.gemm_generic(a, w, c)
+    want = a.double() @ w.double().t()
+    assert float((c.double() - want).norm() / want.norm()) < (NORM if tensor_cores else K * EPS)
