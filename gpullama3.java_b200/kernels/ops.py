@@ -764,6 +764,13 @@ def sm_count(device) -> int:
     return n
 
 
+def gemm_f32_tcgen05_status() -> int:
+    """0 when every wait inside the float32 product on the tensor cores completed since the last call; synchronises."""
+    lib = library("gemm_f32_tcgen05")
+    lib.b200_gemm_f32_tcgen05_status.restype = c_int
+    return int(lib.b200_gemm_f32_tcgen05_status())
+
+
 def gemm_skinny_status() -> int:
     lib = library("gemm_skinny_tcgen05")
     lib.b200_gemm_skinny_status.restype = c_int
