@@ -170,14 +170,14 @@ def test_replay_cuts_at_real_layer_sizes(sized, tmp_path, dtype, cut):
     run_in_process(model, steps, tmp_path, max_live_tokens(steps))
     after = ops.launches_by_kernel()
     ran = {k for k in after if after[k] != before.get(k, 0)}
+    if dtype == torch.float32:
+        assert ops.gemm_f32_tcgen05_status() == 0
     if dtype == torch.bfloat16:
         assert ops.gemm_tcgen05_status() == 0 and ops.attention_prefill_tc_status() == 0
         assert not ({"gemm_generic", "attention_paged", "attention_prefill"} & ran), ran
         assert {"gemm_tcgen05", "attention_prefill_tc"} <= ran, ran
         if cut != "whole":
             assert {"attention_decode_rope", "gemm_decode_linked"} <= ran, ran
-    else:
-        assert ops.gemm_f32_tcgen05_status() == 0
         else:   # the long prompts rotate and fill the cache in the projection's epilogue, the short ones in a kernel of its own
             assert {"gemm_tcgen05_qkv_rope", "rope_angles", "rope_cache_write"} <= ran, ran
         hidden, inner = cfg["hidden_size"], cfg["intermediate_size"]
