@@ -2,9 +2,11 @@
 // 5th-generation tensor cores.
 //
 // A float32 number is the sum of three bfloat16 numbers, x = x0 + x1 + x2 (each the nearest to what is left: 3 x 8 bits hold
-// the 24 bits of the mantissa, so the split loses nothing).  A product of two such sums has nine terms; the six whose orders
-// of magnitude add up to 2 or less (a2 w0, a0 w2, a1 w1, a1 w0, a0 w1, a0 w0) are multiplied, exactly, by the bfloat16 tensor
-// cores; the three left out are below 2^-26 of the product each, less than a float32 multiply-add's own rounding.  What costs precision on tensor cores is the
+// the 24 bits of the mantissa).  Both operands are split times 2^24, which loses nothing: the third part has room in bfloat16's
+// exponents down to the smallest subnormal number (unscaled, numbers below 2^-109 would lose it), and sums are scaled back, exactly,
+// in the epilogue.  A product of two such sums has nine terms; the six whose orders of magnitude add up to 2 or less (a2 w0, a0 w2,
+// a1 w1, a1 w0, a0 w1, a0 w0) are multiplied, exactly, by the bfloat16 tensor cores; of the three left out a1 w2 and a2 w1 reach
+// 2^-25 of the product, all together 2^-24, a float32 multiply-add's own rounding.  What costs precision on tensor cores is the
 // accumulation, whose additions are truncated: so an accumulator in tensor memory lives for 64 elements of K only (its small
 // terms first, its four large additions last) and is then added, rounded to nearest, into float32 registers.  A sum of K products so has K / 64
 // ordinary float32 additions where the plain kernel's chain of multiply-adds has K.
@@ -25,8 +27,9 @@
 // Few tiles (few tokens or a narrow output): K is cut into spans, one CTA each, which form a cluster; their sums meet in
 // distributed shared memory and are added in span order.
 //
-// What is not finite: the split of an infinity or of a number that rounds to one leaves NaN where the plain sum may be
-// infinite.  A sum that comes out not finite is therefore formed again from the float32 operands with plain multiply-adds.
+// What is not finite: the split of an infinity or of a number that rounds to one (from 2^104 on) leaves NaN where the plain sum may be
+// finite or infinite, and scaled sums are infinite from 2^80 on.  A sum that comes out not finite is therefore formed again from the
+// float32 operands with plain multiply-adds.
 //
 // Bound: six bfloat16 products per float32 product under the power limit, i.e. a sixth of the 1,375 TFLOP/s that bfloat16
 // products sustain (229), or the stream of the weights for few tokens.  Measured: 2,048 x 16,384 x 2,048 in 0.69 ms = 200 TFLOP/s
@@ -113,8 +116,16 @@ __device__ __forceinline__ void tmem_ld_x16(uint32_t taddr, float (&v)[16]) {
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// x, y -> their three bfloat16 parts as pairs (x in the low half)
+constexpr float kF32Up = 16777216.f;                        // operands are split times 2^24 ...
+constexpr float kF32Down = 1.f / (kF32Up * kF32Up);         // ... and sums carry 2^48
+
+// x, y -> the three bfloat16 parts of 2^24 x and 2^24 y as pairs (x in the low half)
 __device__ __forceinline__ void split_pair(float x, float y, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
+    unsigned long long xy, up;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(xy) : "f"(x), "f"(y));
+    asm("mov.b64 %0, {%1, %1};" : "=l"(up) : "f"(kF32Up));
+    asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(xy) : "l"(up));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(xy));
     __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
     p0 = *reinterpret_cast<uint32_t*>(&h);
     x -= __uint_as_float(p0 << 16);
@@ -172,11 +183,12 @@ __device__ __noinline__ float gated_f32(float gate, float up, int epilogue, floa
 }
 __device__ __noinline__ float silu_f32(float s) { return s / (1.0f + expf(-s)); }
 
-// One sum per lane, lanes being neighbouring columns n of row m of C (n - lane a multiple of 32): epilogue and store.  All
+// One sum (times 2^48) per lane, lanes being neighbouring columns n of row m of C (n - lane a multiple of 32): epilogue and store.  All
 // lanes of the warp call it.  EPI: 0 store, 1 residual add, 2 the gated ones.
 template <int EPI>
 __device__ __forceinline__ void finish_sum(float s, int m, int n, const F32Args& p) {
     const bool live = m < p.M && n < p.N;
+    s *= kF32Down;
     if (live && !isfinite(s)) s = plain_sum(p.A + (size_t)m * p.lda, p.W + (size_t)n * p.ldw, p.K);
     if (p.bias != nullptr && live) s += p.bias[n];
     if (EPI == 2) {

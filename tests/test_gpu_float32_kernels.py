@@ -300,3 +300,28 @@ def test_every_term_of_a_product_is_there(M, N, K):
     want = a.double() @ w.double().t()
     assert float((c.double() - want).norm() / want.norm()) < NORM
     assert o.gemm_f32_tcgen05_status() == 0
+
+
+@pytest.mark.parametrize("a_exponent, w_exponent", [(-100, 0), (-115, 20), (-125, 40), (-140, 60), (0, -105), (60, -122), (-60, -50), (60, -30)])
+def test_products_of_small_numbers_keep_32_bits(a_exponent, w_exponent):
+    """Down to subnormal numbers, whose bits the split must not lose either."""
+    o = ops()
+    a, w = operands(70, 200, 600)
+    a, w = torch.ldexp(a, torch.tensor(float(a_exponent))).cuda(), torch.ldexp(w, torch.tensor(float(w_exponent))).cuda()
+    c = torch.empty(70, 200, device="cuda")
+    assert o.gemm_f32_tcgen05(a, w, c)
+    want = a.double() @ w.double().t()
+    assert float((c.double() - want).norm() / want.norm()) < NORM
+
+
+@pytest.mark.parametrize("a_exponent, w_exponent", [(110, -90), (70, 20), (-30, 110), (60, 60)])
+def test_products_of_large_numbers(a_exponent, w_exponent):
+    """Numbers that leave no room for the scale and sums that leave none for its square are summed by multiply-adds: below K roundings."""
+    o = ops()
+    a, w = operands(40, 130, 600)
+    a, w = torch.ldexp(a, torch.tensor(float(a_exponent))).cuda(), torch.ldexp(w, torch.tensor(float(w_exponent))).cuda()
+    c = torch.empty(40, 130, device="cuda")
+    assert o.gemm_f32_tcgen05(a, w, c)
+    want = a.double() @ w.double().t()
+    assert bool(torch.isfinite(c).all())
+    assert bool(((c.double() - want).abs() <= 600 * EPS * (a.double().abs() @ w.double().abs().t())).all())
