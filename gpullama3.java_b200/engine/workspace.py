@@ -40,9 +40,16 @@ class Workspace:
         self.capacity = nbytes
 
     def reset(self) -> None:
-        """A new pass begins: everything is free again; grow if the last pass did not fit."""
+        """A new pass begins: everything is free again; grow if the last pass did not fit (and the device has the memory: what
+        does not fit then comes from the allocator once more)."""
         if self._wanted > self.capacity:
-            self._allocate(int(self._wanted * 1.25) + _ALIGN)
+            before = self.capacity
+            try:
+                self._allocate(int(self._wanted * 1.25) + _ALIGN)
+            except torch.OutOfMemoryError:
+                self.capacity = 0
+                if before:
+                    self._allocate(before)
         self._top = 0
         self._wanted = 0
 
@@ -72,3 +79,16 @@ class Workspace:
             self.overflowed += 1
             return torch.empty(shape, dtype=dtype, device=self.device)
         return block.narrow(0, start // size, numel).view(shape)
+
+    def spare(self, shape, dtype: torch.dtype, keep: bool = False) -> torch.Tensor | None:
+        """The piece that ``take`` would hand out next, without taking it (with ``keep``: taken): memory for launches made before the
+        next ``take``.  None where neither the block nor the allocator has room; what the pass wants is then left as it was."""
+        top, wanted = self._top, self._wanted
+        try:
+            piece = self.take(shape, dtype)
+        except torch.OutOfMemoryError:
+            self._top, self._wanted = top, wanted
+            return None
+        if not keep:
+            self._top = top
+        return piece

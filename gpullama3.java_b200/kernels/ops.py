@@ -484,18 +484,20 @@ def _bias_ptr(bias: torch.Tensor | None, n: int):
 
 def gemm_generic(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, epilogue: int = EPILOGUE_STORE,
                  gate_args: tuple[float, float] = (0.0, 0.0), bias: torch.Tensor | None = None,
-                 silu_columns: int = 0) -> None:
+                 silu_columns: int = 0, scratch=None) -> None:
     """c = a @ w.T (store), c += a @ w.T (residual add, c float32) or c = act(gate) * up with
     gate/up rows interleaved in w (act: SiLU, or GELU in its tanh form).  Sums of 32-bit precision: by FMA, or, for more
     than a few rows of float32 operands, by ``gemm_f32_tcgen05``.
     ``bias`` float32 [w.shape[0]] joins every sum before the epilogue; the store epilogue passes the first ``silu_columns``
-    results through SiLU."""
+    results through SiLU.  ``scratch(shape, dtype)``: where memory for this product alone comes from, if not from the allocator
+    (None from it: the product does without)."""
     _dev(a, w, c)
     M, K = a.shape
     N = w.shape[0]
     assert w.shape[1] == K and a.stride(1) == 1 and w.stride(1) == 1 and c.stride(1) == 1
     assert c.shape[0] == M and c.shape[1] == (N // 2 if epilogue in GATED_EPILOGUES else N)
-    if M > 16 and a.dtype == w.dtype == c.dtype == torch.float32 and gemm_f32_tcgen05(a, w, c, epilogue, gate_args, bias, silu_columns):
+    if (M > 16 and a.dtype == w.dtype == c.dtype == torch.float32
+            and gemm_f32_tcgen05(a, w, c, epilogue, gate_args, bias, silu_columns, scratch=scratch)):
         return
     _check(_fn("b200_gemm_generic")(
         a.data_ptr(), dtype_code(a.dtype), a.stride(0), w.data_ptr(), dtype_code(w.dtype), w.stride(0), c.data_ptr(),
@@ -505,10 +507,11 @@ def gemm_generic(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, epilogue: in
 
 def gemm_f32_tcgen05(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, epilogue: int = EPILOGUE_STORE,
                      gate_args: tuple[float, float] = (0.0, 0.0), bias: torch.Tensor | None = None, silu_columns: int = 0,
-                     n_spans: int = 0) -> bool:
+                     n_spans: int = 0, scratch=None) -> bool:
     """``gemm_generic`` for float32 operands with float32's precision on the tensor cores: every number as the sum of three
     bfloat16 numbers, partial sums of 64 products added in float32.  ``n_spans``: how often K is cut (0: the shape decides).
-    Returns False, having done nothing, for operands it does not take."""
+    ``scratch(shape, dtype)``: where the split activations go, 6 bytes an element (None: the allocator).  Returns False, having done
+    nothing, for operands it does not take and where there is no memory for these."""
     M, K = a.shape
     N = w.shape[0]
     lib = library("gemm_f32_tcgen05")
@@ -519,10 +522,15 @@ def gemm_f32_tcgen05(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, epilogue
     _dev(a, w, c)
     assert a.dtype == w.dtype == c.dtype == torch.float32 and w.shape[1] == K and c.stride(1) == 1
     assert tuple(c.shape) == (M, N // 2 if epilogue in GATED_EPILOGUES else N)
-    scratch = torch.empty(elements, dtype=torch.bfloat16, device=a.device)
+    try:
+        planes = scratch((elements,), torch.bfloat16) if scratch is not None else torch.empty(elements, dtype=torch.bfloat16, device=a.device)
+    except torch.OutOfMemoryError:
+        planes = None
+    if planes is None:
+        return False
     status = _fn("b200_gemm_f32_tcgen05")(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), c.data_ptr(), c.stride(0), M, N, K,
                                           epilogue, float(gate_args[0]), float(gate_args[1]), _bias_ptr(bias, N),
-                                          int(silu_columns), scratch.data_ptr(), int(n_spans), _stream())
+                                          int(silu_columns), planes.data_ptr(), int(n_spans), _stream())
     if status == _UNSUPPORTED:
         return False
     _check(status, "gemm_generic")

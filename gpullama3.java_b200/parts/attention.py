@@ -28,7 +28,7 @@ from ..cache.sequence_cache import KVCacheNeed, KVView
 from ..config.base import ConfigError
 from ..kernels import fast, ops
 from ..weights.loader import ParamSpec
-from .base import Mixer, PositionEncoding, StepContext, register_mixer
+from .base import Mixer, PositionEncoding, StepContext, register_mixer, scratch_of
 from .linear import Linear
 
 
@@ -186,7 +186,7 @@ class GroupedQueryAttention(Mixer):
             if writes_cache and self.shares_cache:
                 raise ConfigError("a mixer without key and value projections cannot write a cache entry")
             # (the rows of a layer whose values later layers mix with theirs outlive the block: they come from the allocator)
-            raw = self.qkv.store(x, ctx.dtype, ctx.empty if self.value_mix != "source" else None)
+            raw = self.qkv.store(x, ctx.dtype, ctx.empty if self.value_mix != "source" else None, scratch_of(ctx))
             mix = None
             if self.value_mix == "source":
                 ctx.extras[VALUE_MIX_SOURCE] = raw[:, self.value_off:self.value_off + self.n_kv_heads * self.value_dim]
@@ -209,12 +209,12 @@ class GroupedQueryAttention(Mixer):
             # a prompt pass: projection, rotation and cache write as one product where its epilogue can do all three
             qkv = ctx.empty((x.shape[0], self.qkv.out_features), ctx.dtype)
             if not fast.try_projection_with_rope(x, self.qkv.weight, qkv, ctx, table, cache, self, writes_cache):
-                self.qkv.into(x, qkv)
+                self.qkv.into(x, qkv, scratch_of(ctx))
                 ops.rope_cache_write(qkv, ctx.positions, ctx.seq_ids, table, self.position.inverse_frequencies(x.device),
                                      cache.k, cache.v, self.n_heads, self.n_kv_heads, self.head_dim,
                                      self.position.rotary_dim, self.position.pairing, write_cache=writes_cache)
         else:
-            qkv = self.qkv.store(x, ctx.dtype, ctx.empty)  # [T, q_dim + 2 kv_dim]; queries are rotated in place below
+            qkv = self.qkv.store(x, ctx.dtype, ctx.empty, scratch_of(ctx))  # [T, q_dim + 2 kv_dim]; queries are rotated in place below
             # a decode step: one kernel rotates, writes the cache and attends, where the sizes allow
             attended = fast.try_decode_attention_with_rope(qkv, out, ctx, table, cache, self, writes_cache)
             if not attended:
@@ -224,7 +224,7 @@ class GroupedQueryAttention(Mixer):
         gate = raw[:, self.gate_off:self.gate_off + self.n_heads] if self.output_gate else None
         if not attended:
             attend(self, qkv, out, ctx, table, cache, gate)
-        return self.o.add_to(out, residual, then_norm)
+        return self.o.add_to(out, residual, then_norm, scratch_of(ctx))
 
 
 def plan_decode_attention(shape, ctx: StepContext, cache: KVView) -> tuple[int, bool]:
@@ -270,7 +270,7 @@ def attend(shape, qkv: torch.Tensor, out: torch.Tensor, ctx: StepContext, table:
         tile, spans = plan
         if tile and ops.attention_prefill_f32(qkv, qkv.shape[1], out, ctx.cu_seqlens, ctx.kv_lens, table, cache.k, cache.v, ctx.n_seqs,
                                               ctx.max_q_len, shape.n_heads, shape.n_kv_heads, shape.head_dim, shape.window or 0, tile=tile,
-                                              n_spans=spans, alloc=ctx.empty, **terms):
+                                              n_spans=spans, alloc=scratch_of(ctx), **terms):
             return
     splits = ops.attention_paged_spans(qkv.shape[0] * shape.n_heads, reach, ops.sm_count(qkv.device))
     ops.attention_paged(qkv, qkv.shape[1], out, ctx.positions, ctx.seq_ids, table, cache.k, cache.v,

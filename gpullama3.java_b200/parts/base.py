@@ -58,8 +58,25 @@ class StepContext:
             return self.workspace.take(shape, dtype)
         return torch.empty(tuple(shape), dtype=dtype, device=self.device)
 
+    def scratch(self, shape, dtype: torch.dtype) -> torch.Tensor | None:
+        """Memory for the launches that the caller makes before it asks for anything else; None where there is none left (for a
+        caller that can do without).  What comes from the workspace may be handed out again right away, since kernels run in stream
+        order; not in a decode step, in which parts may run beside one another on streams of their own: there it stays taken
+        until the block has run."""
+        if self.workspace is not None:
+            return self.workspace.spare(shape, dtype, keep=self.all_decode)
+        try:
+            return torch.empty(tuple(shape), dtype=dtype, device=self.device)
+        except torch.OutOfMemoryError:
+            return None
+
     def capacity(self, group: int) -> int:
         return self.kv_capacity[group] if group < len(self.kv_capacity) else self.max_kv_len
+
+
+def scratch_of(ctx):
+    """``ctx.scratch``, for parts that hand it to their products; None (the allocator) for a stand-in of a step that has none."""
+    return getattr(ctx, "scratch", None)
 
 
 @dataclass

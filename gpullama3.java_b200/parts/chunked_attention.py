@@ -22,7 +22,7 @@ from ..config.base import ConfigError
 from ..kernels import ops
 from ..weights.loader import ParamSpec
 from .attention import attend, kernel_head_dim, plan_decode_attention
-from .base import Mixer, OpenEnded, PositionEncoding, StepContext, register_mixer
+from .base import Mixer, OpenEnded, PositionEncoding, StepContext, register_mixer, scratch_of
 from .linear import Linear
 from .position import PAIRING_CODES
 
@@ -143,7 +143,7 @@ class ChunkedAttention(Mixer, OpenEnded):
         return ctx.all_decode and self.qkv is not None and self.qkv.links_with(ctx.n_tokens, ctx.dtype)
 
     def rows_into(self, x, ctx: StepContext, cache: KVView, rows, writes_cache=True, mul=1.0):
-        self.rows_from(self.qkv.store(x, ctx.dtype, ctx.empty), ctx, cache, rows, writes_cache, mul)
+        self.rows_from(self.qkv.store(x, ctx.dtype, ctx.empty, scratch_of(ctx)), ctx, cache, rows, writes_cache, mul)
 
     def rows_from(self, raw, ctx: StepContext, cache: KVView, rows, writes_cache=True, mul=1.0):
         H, dv, D, T = self.heads, self.value_dim, self.row_dim, raw.shape[0]
@@ -159,7 +159,7 @@ class ChunkedAttention(Mixer, OpenEnded):
     def forward(self, x, ctx: StepContext, cache: KVView, residual, writes_cache=True, then_norm=None):
         rows = ctx.empty((x.shape[0], self.open_columns()), ctx.dtype)
         self.rows_into(x, ctx, cache, rows, writes_cache)
-        return self.o.add_to(rows, residual, then_norm)
+        return self.o.add_to(rows, residual, then_norm, scratch_of(ctx))
 
 
 register_mixer("chunked_attention", ChunkedAttention)

@@ -21,7 +21,7 @@ from ..cache.sequence_cache import StateNeed, StateView
 from ..config.base import ConfigError
 from ..kernels import ops
 from ..weights.loader import ParamSpec
-from .base import Mixer, StepContext, register_mixer
+from .base import Mixer, StepContext, register_mixer, scratch_of
 from .linear import Linear
 
 
@@ -95,18 +95,18 @@ class ChannelDeltaRule(Mixer):
     def forward(self, x, ctx: StepContext, cache: StateView, residual, writes_cache=True, then_norm=None):
         H, G, dk, dv, T = self.n_heads, self.n_kv_heads, self.key_dim, self.value_dim, x.shape[0]
         state = cache.data                                                    # [slots, S of every head | convolution inputs]
-        proj = self.inputs.store(x, ctx.dtype, ctx.empty)
+        proj = self.inputs.store(x, ctx.dtype, ctx.empty, scratch_of(ctx))
         qkv = ctx.empty((T, self.channels), ctx.dtype)
         ops.causal_conv_silu(proj, self.conv_weight, state[:, self.state_floats:], ctx.slots_dev, ctx.seq_ids,
                              ctx.cu_seqlens, qkv, self.channels, update_state=writes_cache)
-        decay = self.a2.store(proj[:, self.a1_off:self.a1_off + self.decay_rank], ctx.dtype, ctx.empty)   # [T, H dk]
-        gate = self.g2.store(proj[:, self.g1_off:self.g1_off + self.gate_rank], ctx.dtype, ctx.empty)     # [T, H dv]
+        decay = self.a2.store(proj[:, self.a1_off:self.a1_off + self.decay_rank], ctx.dtype, ctx.empty, scratch_of(ctx))   # [T, H dk]
+        gate = self.g2.store(proj[:, self.g1_off:self.g1_off + self.gate_rank], ctx.dtype, ctx.empty, scratch_of(ctx))     # [T, H dv]
         o = ctx.empty((T, H * dv), torch.float32)
         ops.delta_rule_scan(qkv, proj[:, self.beta_off:], decay, self.dt_bias, self.a_log, state, ctx.slots_dev,
                             ctx.cu_seqlens, o, H, G, dk, dv, dk ** -0.5, self.unit_eps, alloc=ctx.empty, longest=ctx.max_q_len)
         gated = ctx.empty((T, H * dv), ctx.dtype)
         ops.gated_rmsnorm(o, self.norm_weight, gate, gated, H, dv, self.norm_eps)
-        return self.o.add_to(gated, residual, then_norm)
+        return self.o.add_to(gated, residual, then_norm, scratch_of(ctx))
 
 
 class HeadDeltaRule(Mixer):
@@ -178,7 +178,7 @@ class HeadDeltaRule(Mixer):
     def forward(self, x, ctx: StepContext, cache: StateView, residual, writes_cache=True, then_norm=None):
         H, G, dk, dv, T = self.n_heads, self.n_kv_heads, self.key_dim, self.value_dim, x.shape[0]
         state = cache.data
-        proj = self.inputs.store(x, ctx.dtype, ctx.empty)
+        proj = self.inputs.store(x, ctx.dtype, ctx.empty, scratch_of(ctx))
         qkv = ctx.empty((T, self.channels), ctx.dtype)
         ops.causal_conv_silu(proj, self.conv_weight, state[:, self.state_floats:], ctx.slots_dev, ctx.seq_ids,
                              ctx.cu_seqlens, qkv, self.channels, update_state=writes_cache)
@@ -188,7 +188,7 @@ class HeadDeltaRule(Mixer):
                             decay_per_head=True, longest=ctx.max_q_len)
         gated = ctx.empty((T, H * dv), ctx.dtype)
         ops.gated_rmsnorm(o, self.norm_weight, proj[:, self.gate_off:], gated, H, dv, self.norm_eps, self.gate_activation)
-        return self.o.add_to(gated, residual, then_norm)
+        return self.o.add_to(gated, residual, then_norm, scratch_of(ctx))
 
 
 register_mixer("channel_delta", ChannelDeltaRule)

@@ -10,7 +10,7 @@ import torch
 from ..config.base import ConfigError
 from ..kernels import ops
 from ..weights.loader import ParamSpec
-from .base import FeedForward, OpenEnded, StepContext, register_feed_forward
+from .base import FeedForward, OpenEnded, StepContext, register_feed_forward, scratch_of
 from .linear import Linear
 
 
@@ -62,15 +62,15 @@ class SwiGLUFeedForward(FeedForward, OpenEnded):
 
     def rows_into(self, x, ctx: StepContext, cache, rows, writes_cache=True, mul=1.0):
         assert mul == 1.0
-        self.gate_up.gated_into(x, rows, self.activation, self.gate_args)
+        self.gate_up.gated_into(x, rows, self.activation, self.gate_args, scratch_of(ctx))
 
     def takes_scaled_rows(self, ctx: StepContext) -> bool:
         return (ctx.all_decode and self.activation in ("silu", "gelu_tanh")
                 and self.gate_up.links_with(ctx.n_tokens, ctx.dtype))
 
     def forward(self, x, ctx: StepContext, residual, then_norm=None):
-        h = self.gate_up.gated(x, ctx.dtype, ctx.empty, self.activation, self.gate_args)  # [T, intermediate]
-        return self.down.add_to(h, residual, then_norm)
+        h = self.gate_up.gated(x, ctx.dtype, ctx.empty, self.activation, self.gate_args, scratch_of(ctx))  # [T, intermediate]
+        return self.down.add_to(h, residual, then_norm, scratch_of(ctx))
 
 
 class DenseFeedForward(FeedForward):
@@ -108,9 +108,9 @@ class DenseFeedForward(FeedForward):
         return self.down_bias
 
     def forward(self, x, ctx: StepContext, residual, then_norm=None, add_result_bias: bool = True):
-        u = self.up.store(x, ctx.dtype, ctx.empty)
+        u = self.up.store(x, ctx.dtype, ctx.empty, scratch_of(ctx))
         ops.bias_act_rows(u, self.up_bias, self.activation)
-        self.down.add_to(u, residual)
+        self.down.add_to(u, residual, scratch=scratch_of(ctx))
         if add_result_bias and self.down_bias is not None:
             ops.add_row(residual, self.down_bias)
         return None

@@ -27,7 +27,7 @@ from ..cache.sequence_cache import EntryNeeds, StateNeed
 from ..config.base import ConfigError
 from ..kernels import ops
 from ..weights.loader import ParamSpec
-from .base import Block, FirstRead, StepContext, all_parts, register_block
+from .base import Block, FirstRead, StepContext, all_parts, register_block, scratch_of
 from .linear import Linear
 
 SUBLAYER_RESULT = "gated residual sublayer result"   # in a pass's ``ctx.extras``: float32 [T, width], zero between uses
@@ -249,10 +249,10 @@ class GatedResidualBlock(Block):
             x = self._join(y, x, 1, self.feed_forward_norm, residual, ctx, y_bias=y_bias, cast=cast_behind("feed_forward"),
                            **mix_behind("feed_forward"))
         if self.side_dim:
-            a = self.side_gate.store(x, ctx.dtype, ctx.empty)
+            a = self.side_gate.store(x, ctx.dtype, ctx.empty, scratch_of(ctx))
             g = ctx.empty((T, self.side_k), ctx.dtype)
             ops.token_gate_rows(a, ctx.tokens, self.side_table, g, self.side_dim)
-            self.side_proj.add_to(g, y)
+            self.side_proj.add_to(g, y, scratch=scratch_of(ctx))
             ops.gated_norm_step(y, self.side_norm, None, residual, self.side_eps, center=False, cast=cast_behind("side"),
                                 **mix_behind("side"))
         return StreamRows(last, ahead[4] if ahead is not None else None)
@@ -262,7 +262,7 @@ class GatedResidualBlock(Block):
         stream; returns ``cast``, which then holds the updated stream in the run's type."""
         bias = getattr(norm, "bias", None)
         w = norm.weight if norm.weight.dtype == torch.float32 else norm.group_form()[0]
-        r = self.gates[which].store(x, torch.float32, ctx.empty)    # (the gate's logits leave their product in 32 bits)
+        r = self.gates[which].store(x, torch.float32, ctx.empty, scratch_of(ctx))    # (the gate's logits leave their product in 32 bits)
         ops.gated_norm_step(y, w, bias, residual, norm.eps, gate=r, gate_bias=self.gate_biases[which], y_bias=y_bias, cast=cast,
                             center=bias is not None, **mix)
         return cast

@@ -32,7 +32,7 @@ from ..config.base import ConfigError
 from ..kernels import ops
 from ..weights.loader import ParamSpec
 from .attention import attend, kernel_head_dim
-from .base import Mixer, OpenEnded, StepContext, register_mixer
+from .base import Mixer, OpenEnded, StepContext, register_mixer, scratch_of
 from .linear import Linear
 from .position import PAIRING_CODES
 
@@ -179,7 +179,7 @@ class LatentAttention(Mixer, OpenEnded):
         return ctx.all_decode and self.down is not None and self.down.links_with(ctx.n_tokens, ctx.dtype)
 
     def rows_into(self, x, ctx: StepContext, cache: KVView, rows, writes_cache=True, mul=1.0):
-        self.rows_from(self.down.store(x, ctx.dtype, ctx.empty), ctx, cache, rows, writes_cache, mul)
+        self.rows_from(self.down.store(x, ctx.dtype, ctx.empty, scratch_of(ctx)), ctx, cache, rows, writes_cache, mul)
 
     def rows_from(self, raw, ctx: StepContext, cache: KVView, rows, writes_cache=True, mul=1.0):
         """``raw`` [T, queries (or q_rank) | kv_rank + rot_dim | gate]."""
@@ -192,7 +192,7 @@ class LatentAttention(Mixer, OpenEnded):
         if self.q_rank is not None:
             c_q = ctx.empty((T, self.q_pad), ctx.dtype)
             ops.head_rows(raw, c_q, self.query_segment, self.norm_eps, None, self.norm_weights)
-            q = self.uq.store(c_q[:, :self.q_rank], ctx.dtype, ctx.empty)     # [T, H dk]
+            q = self.uq.store(c_q[:, :self.q_rank], ctx.dtype, ctx.empty, scratch_of(ctx))     # [T, H dk]
         else:
             q = ctx.empty((T, H * (dk + dr)), ctx.dtype)
             ops.head_rows(raw, q, self.query_segment, self.norm_eps, None, None, rotary=self._rotary(ctx))
@@ -220,7 +220,7 @@ class LatentAttention(Mixer, OpenEnded):
     def forward(self, x, ctx: StepContext, cache: KVView, residual, writes_cache=True, then_norm=None):
         rows = ctx.empty((x.shape[0], self.open_columns()), ctx.dtype)
         self.rows_into(x, ctx, cache, rows, writes_cache)
-        return self.o.add_to(rows, residual, then_norm)
+        return self.o.add_to(rows, residual, then_norm, scratch_of(ctx))
 
 
 register_mixer("latent_attention", LatentAttention)

@@ -22,31 +22,32 @@ class Linear:
         self.bias = bias.to(device=weight.device, dtype=torch.float32).contiguous() if bias is not None else None
         self.out_features, self.in_features = weight.shape
 
-    def _run(self, a, c: torch.Tensor, epilogue: int, gate_args=(0.0, 0.0)) -> None:
+    def _run(self, a, c: torch.Tensor, epilogue: int, gate_args=(0.0, 0.0), scratch=None) -> None:
         if isinstance(a, ScaledRows):  # only handed to a product that said it links (links_with)
             ops.gemm_decode_linked(a.data, self.weight, c, epilogue, row_factors=(a.partials, a.eps, a.dim),
                                    bias=self.bias, silu_columns=self.silu_columns)
             return
         if fast.try_gemm(a, self.weight, c, epilogue, gate_args, self.bias, self.silu_columns):
             return
-        ops.gemm_generic(a, self.weight, c, epilogue, gate_args, self.bias, self.silu_columns)
+        ops.gemm_generic(a, self.weight, c, epilogue, gate_args, self.bias, self.silu_columns, scratch)
 
     def links_with(self, n_rows: int, dtype: torch.dtype) -> bool:
         """Whether this product can be one half of a split norm for ``n_rows`` rows of ``dtype``."""
         return dtype == torch.bfloat16 and ops.gemm_decode_links(n_rows, self.weight)
 
-    def store(self, a: torch.Tensor, out_dtype: torch.dtype, alloc=None) -> torch.Tensor:
-        """a @ W.T as a new [T, out] tensor (from ``alloc(shape, dtype)`` when given, a step's ``ctx.empty``)."""
+    def store(self, a: torch.Tensor, out_dtype: torch.dtype, alloc=None, scratch=None) -> torch.Tensor:
+        """a @ W.T as a new [T, out] tensor (from ``alloc(shape, dtype)`` when given, a step's ``ctx.empty``).  ``scratch``, here
+        and below: where memory for the product alone comes from, a step's ``ctx.scratch`` (None: the allocator)."""
         shape = (a.shape[0], self.out_features)
         c = alloc(shape, out_dtype) if alloc is not None else torch.empty(shape, dtype=out_dtype, device=a.device)
-        self._run(a, c, ops.EPILOGUE_STORE)
+        self._run(a, c, ops.EPILOGUE_STORE, scratch=scratch)
         return c
 
-    def into(self, a: torch.Tensor, c: torch.Tensor) -> None:
+    def into(self, a: torch.Tensor, c: torch.Tensor, scratch=None) -> None:
         """c = a @ W.T into a tensor the caller brings."""
-        self._run(a, c, ops.EPILOGUE_STORE)
+        self._run(a, c, ops.EPILOGUE_STORE, scratch=scratch)
 
-    def add_to(self, a: torch.Tensor, residual: torch.Tensor, then_norm=None) -> ScaledRows | None:
+    def add_to(self, a: torch.Tensor, residual: torch.Tensor, then_norm=None, scratch=None) -> ScaledRows | None:
         """residual += a @ W.T, the sum kept in float32.  With ``then_norm`` (a norm that has a row-factor form)
         and a product that links, the same kernel also leaves that norm of the new residual as ScaledRows; a ``then_norm``
         that stands for two norms of the same rows (``second_form``) gets the rows under both weights."""
@@ -63,23 +64,23 @@ class Linear:
                                    emit_second=(second(), act2) if second is not None else None, bias=self.bias)
             rows = ScaledRows(act, partials, eps, dim)
             return (rows, ScaledRows(act2, partials, eps, dim)) if second is not None else rows
-        self._run(a, residual, ops.EPILOGUE_RESIDUAL_ADD)
+        self._run(a, residual, ops.EPILOGUE_RESIDUAL_ADD, scratch=scratch)
         return None
 
-    def gated_into(self, a: torch.Tensor, c: torch.Tensor, activation: str = "silu", gate_args=(0.0, 0.0)) -> None:
+    def gated_into(self, a: torch.Tensor, c: torch.Tensor, activation: str = "silu", gate_args=(0.0, 0.0), scratch=None) -> None:
         """``gated`` into a tensor the caller brings."""
-        self._run(a, c, ops.GATED_EPILOGUE_OF[activation], gate_args)
+        self._run(a, c, ops.GATED_EPILOGUE_OF[activation], gate_args, scratch)
 
     def gated_silu(self, a: torch.Tensor, out_dtype: torch.dtype, alloc=None) -> torch.Tensor:
         """W holds gate and up rows interleaved; returns silu(gate) * up as [T, out/2]."""
         return self.gated(a, out_dtype, alloc, "silu")
 
     def gated(self, a: torch.Tensor, out_dtype: torch.dtype, alloc=None, activation: str = "silu",
-              gate_args=(0.0, 0.0)) -> torch.Tensor:
+              gate_args=(0.0, 0.0), scratch=None) -> torch.Tensor:
         """W holds gate and up rows interleaved; returns act(gate) * up as [T, out/2] (``activation``: ``silu`` or
         ``gelu_tanh``), or with ``clamped_sigmoid`` g' sigmoid(slope g') (u' + 1) of the clamped pair (``gate_args`` =
         (limit, slope)); all applied in the product's epilogue."""
         shape = (a.shape[0], self.out_features // 2)
         c = alloc(shape, out_dtype) if alloc is not None else torch.empty(shape, dtype=out_dtype, device=a.device)
-        self._run(a, c, ops.GATED_EPILOGUE_OF[activation], gate_args)
+        self._run(a, c, ops.GATED_EPILOGUE_OF[activation], gate_args, scratch)
         return c

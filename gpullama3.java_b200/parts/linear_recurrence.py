@@ -40,7 +40,7 @@ from ..cache.sequence_cache import StateNeed, StateView
 from ..config.base import ConfigError
 from ..kernels import ops
 from ..weights.loader import ParamSpec
-from .base import Mixer, OpenEnded, PositionEncoding, StepContext, register_mixer
+from .base import Mixer, OpenEnded, PositionEncoding, StepContext, register_mixer, scratch_of
 from .linear import Linear
 from .position import PAIRING_CODES
 
@@ -105,15 +105,15 @@ class GatedLinearAttention(Mixer):
 
     def forward(self, x, ctx: StepContext, cache: StateView, residual, writes_cache=True, then_norm=None):
         H, dk, dv, T = self.n_heads, self.key_dim, self.value_dim, x.shape[0]
-        proj = self.inputs.store(x, ctx.dtype, ctx.empty)
-        decay = self.a2.store(proj[:, self.a1_off:self.a1_off + self.decay_rank], ctx.dtype, ctx.empty)    # [T, H dk]
+        proj = self.inputs.store(x, ctx.dtype, ctx.empty, scratch_of(ctx))
+        decay = self.a2.store(proj[:, self.a1_off:self.a1_off + self.decay_rank], ctx.dtype, ctx.empty, scratch_of(ctx))    # [T, H dk]
         o = ctx.empty((T, H * dv), torch.float32)
         ops.linear_scan(proj[:, self.q_off:], proj[:, self.k_off:], proj[:, self.v_off:], decay, cache.data, ctx.slots_dev,
                         ctx.cu_seqlens, o, H, H, dk, dv, decay_kind=ops.DECAY_SIGMOID_POWER, decay_bias=self.decay_bias,
                         power=1.0 / self.tau, q_scale=dk ** -0.5, alloc=ctx.empty)
         gated = ctx.empty((T, H * dv), ctx.dtype)
         ops.gated_rmsnorm(o, self.norm_weight, proj[:, self.g_off:], gated, H, dv, self.norm_eps, "silu")
-        return self.o.add_to(gated, residual, then_norm)
+        return self.o.add_to(gated, residual, then_norm, scratch_of(ctx))
 
 
 class StateSpaceDuality(Mixer):
@@ -165,7 +165,7 @@ class StateSpaceDuality(Mixer):
     def forward(self, x, ctx: StepContext, cache: StateView, residual, writes_cache=True, then_norm=None):
         H, G, N, dv, T, gn = self.n_heads, self.n_groups, self.state_dim, self.value_dim, x.shape[0], self.n_groups * self.state_dim
         state = cache.data                                                    # [slots, S of every head | convolution inputs]
-        proj = self.inputs.store(x, ctx.dtype, ctx.empty)
+        proj = self.inputs.store(x, ctx.dtype, ctx.empty, scratch_of(ctx))
         xbc = ctx.empty((T, self.channels), ctx.dtype)
         ops.causal_conv(proj[:, self.conv_off:], self.conv_weight, state[:, self.state_floats:], ctx.slots_dev, ctx.seq_ids,
                         ctx.cu_seqlens, xbc, self.channels, bias=self.conv_bias, activation="silu", update_state=writes_cache)
@@ -176,7 +176,7 @@ class StateSpaceDuality(Mixer):
         gated = ctx.empty((T, self.inner), ctx.dtype)
         ops.gated_rmsnorm(o, self.norm_weight, proj[:, self.z_off:], gated, self.norm_groups, self.inner // self.norm_groups,
                           self.norm_eps, "silu", gate_first=True)
-        return self.o.add_to(gated, residual, then_norm)
+        return self.o.add_to(gated, residual, then_norm, scratch_of(ctx))
 
 
 class FixedDecayAttention(Mixer, OpenEnded):
@@ -248,7 +248,7 @@ class FixedDecayAttention(Mixer, OpenEnded):
         return ctx.all_decode and self.inputs is not None and self.inputs.links_with(ctx.n_tokens, ctx.dtype)
 
     def rows_into(self, x, ctx: StepContext, cache: StateView, rows, writes_cache=True, mul=1.0):
-        self._recur(self.inputs.store(x, ctx.dtype, ctx.empty), ctx, cache, rows, mul, silu=False)   # (activated by the product)
+        self._recur(self.inputs.store(x, ctx.dtype, ctx.empty, scratch_of(ctx)), ctx, cache, rows, mul, silu=False)   # (activated by the product)
 
     def rows_from(self, raw, ctx: StepContext, cache: StateView, rows, writes_cache=True, mul=1.0):
         self._recur(raw, ctx, cache, rows, mul, silu=self.silu)
@@ -280,7 +280,7 @@ class FixedDecayAttention(Mixer, OpenEnded):
     def forward(self, x, ctx: StepContext, cache: StateView, residual, writes_cache=True, then_norm=None):
         rows = ctx.empty((x.shape[0], self.open_columns()), ctx.dtype)
         self.rows_into(x, ctx, cache, rows, writes_cache)
-        return self.o.add_to(rows, residual, then_norm)
+        return self.o.add_to(rows, residual, then_norm, scratch_of(ctx))
 
 
 class MatrixMemory(Mixer, OpenEnded):
@@ -334,7 +334,7 @@ class MatrixMemory(Mixer, OpenEnded):
         return ctx.all_decode and self.inputs is not None and self.inputs.links_with(ctx.n_tokens, ctx.dtype)
 
     def rows_into(self, x, ctx: StepContext, cache: StateView, rows, writes_cache=True, mul=1.0):
-        self.rows_from(self.inputs.store(x, ctx.dtype, ctx.empty), ctx, cache, rows, writes_cache, mul)
+        self.rows_from(self.inputs.store(x, ctx.dtype, ctx.empty, scratch_of(ctx)), ctx, cache, rows, writes_cache, mul)
 
     def rows_from(self, raw, ctx: StepContext, cache: StateView, rows, writes_cache=True, mul=1.0):
         assert mul == 1.0
@@ -352,7 +352,7 @@ class MatrixMemory(Mixer, OpenEnded):
     def forward(self, x, ctx: StepContext, cache: StateView, residual, writes_cache=True, then_norm=None):
         rows = ctx.empty((x.shape[0], self.open_columns()), ctx.dtype)
         self.rows_into(x, ctx, cache, rows, writes_cache)
-        return self.o.add_to(rows, residual, then_norm)
+        return self.o.add_to(rows, residual, then_norm, scratch_of(ctx))
 
 
 register_mixer("mlstm", MatrixMemory)

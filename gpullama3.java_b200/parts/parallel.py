@@ -24,7 +24,7 @@ import torch
 from ..config.base import ConfigError
 from ..cache.sequence_cache import EntryNeeds
 from ..kernels import ops
-from .base import Block, Mixer, OpenEnded, StepContext, all_parts, register_block, register_mixer
+from .base import Block, Mixer, OpenEnded, StepContext, all_parts, register_block, register_mixer, scratch_of
 from .linear import Linear
 
 
@@ -157,8 +157,8 @@ class ParallelBlock(Block):
         n = self.columns[0]
         if self.feed_forward is None:
             self.mixer.rows_into(h, ctx, cache, rows, writes_cache)
-            return self.out.add_to(rows, residual, then_norm)
-        raw = self.inputs.store(h, ctx.dtype, ctx.empty) if self.inputs is not None else None
+            return self.out.add_to(rows, residual, then_norm, scratch_of(ctx))
+        raw = self.inputs.store(h, ctx.dtype, ctx.empty, scratch_of(ctx)) if self.inputs is not None else None
 
         def mix():
             if raw is not None:
@@ -181,7 +181,7 @@ class ParallelBlock(Block):
         else:
             mix()
             feed_forward()
-        return self.out.add_to(rows, residual, then_norm)
+        return self.out.add_to(rows, residual, then_norm, scratch_of(ctx))
 
 
 class ParallelMixers(Mixer, OpenEnded):
@@ -237,7 +237,7 @@ class ParallelMixers(Mixer, OpenEnded):
         return ctx.all_decode and self.inputs is not None and self.inputs.links_with(ctx.n_tokens, ctx.dtype)
 
     def rows_into(self, x, ctx: StepContext, cache, rows, writes_cache=True, mul=1.0):
-        self.rows_from(self.inputs.store(x, ctx.dtype, ctx.empty), ctx, cache, rows, writes_cache, mul)
+        self.rows_from(self.inputs.store(x, ctx.dtype, ctx.empty, scratch_of(ctx)), ctx, cache, rows, writes_cache, mul)
 
     def rows_from(self, raw, ctx: StepContext, cache, rows, writes_cache=True, mul=1.0):
         at, col = 0, 0
@@ -249,7 +249,7 @@ class ParallelMixers(Mixer, OpenEnded):
     def forward(self, x, ctx: StepContext, cache, residual, writes_cache=True, then_norm=None):
         rows = ctx.empty((x.shape[0], self.open_columns()), ctx.dtype)
         self.rows_into(x, ctx, cache, rows, writes_cache)
-        return self.o.add_to(rows, residual, then_norm)
+        return self.o.add_to(rows, residual, then_norm, scratch_of(ctx))
 
 
 register_block("parallel", ParallelBlock)

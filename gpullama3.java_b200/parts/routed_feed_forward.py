@@ -31,7 +31,7 @@ import torch
 from ..config.base import ConfigError
 from ..kernels import ops
 from ..weights.loader import ParamSpec
-from .base import FeedForward, OpenEnded, StepContext, register_feed_forward
+from .base import FeedForward, OpenEnded, StepContext, register_feed_forward, scratch_of
 from .linear import Linear
 
 
@@ -176,13 +176,13 @@ class RoutedFeedForward(FeedForward, OpenEnded):
                 runs = [(e, bounds[e], bounds[e + 1]) for e in range(self.n_experts) if bounds[e + 1] > bounds[e]]
                 for e, lo, hi in runs:
                     if self.gated:
-                        self.up[e].gated_into(xs[lo:hi], y[lo:hi], self.activation, self.gate_args)
+                        self.up[e].gated_into(xs[lo:hi], y[lo:hi], self.activation, self.gate_args, scratch_of(ctx))
                     else:
-                        self.up[e].into(xs[lo:hi], y[lo:hi])
+                        self.up[e].into(xs[lo:hi], y[lo:hi], scratch_of(ctx))
                 if not self.gated:
                     ops.bias_act_rows(y, None, self.activation)
                 for e, lo, hi in runs:
-                    self.down[e].into(y[lo:hi], o[lo:hi])
+                    self.down[e].into(y[lo:hi], o[lo:hi], scratch_of(ctx))
         ops.moe_combine(o, place, weights, residual)
 
     # ---- the shared expert: rows before a last product
@@ -198,7 +198,7 @@ class RoutedFeedForward(FeedForward, OpenEnded):
         return weight
 
     def rows_into(self, x, ctx: StepContext, cache, rows, writes_cache=True, mul=1.0):
-        self.rows_from(self.shared_up.store(x, ctx.dtype, ctx.empty), ctx, cache, rows, writes_cache, mul)
+        self.rows_from(self.shared_up.store(x, ctx.dtype, ctx.empty, scratch_of(ctx)), ctx, cache, rows, writes_cache, mul)
 
     def rows_from(self, raw, ctx: StepContext, cache, rows, writes_cache=True, mul=1.0):
         assert mul == 1.0
@@ -209,7 +209,7 @@ class RoutedFeedForward(FeedForward, OpenEnded):
         if self.shared_size:
             rows = ctx.empty((x.shape[0], self.shared_size), ctx.dtype)
             self.rows_into(x, ctx, None, rows)
-            self.shared_down.add_to(rows, residual)
+            self.shared_down.add_to(rows, residual, scratch=scratch_of(ctx))
         return None
 
 

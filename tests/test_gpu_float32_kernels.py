@@ -268,7 +268,7 @@ def test_attend_of_float32_passes(q_lens, kv_lens, H, G, D):
         return torch.empty(shape, dtype=dtype, device="cuda")
 
     ctx = SimpleNamespace(n_seqs=len(q_lens), q_lens=q_lens, start_pos=[b - a for a, b in zip(q_lens, kv_lens)], max_q_len=max(q_lens),
-                          all_decode=max(q_lens) == 1, positions=positions, seq_ids=seq_ids, cu_seqlens=cu, kv_lens=lens, extras={}, empty=empty,
+                          all_decode=max(q_lens) == 1, positions=positions, seq_ids=seq_ids, cu_seqlens=cu, kv_lens=lens, extras={}, scratch=empty,
                           capacity=lambda group: max(kv_lens))
     shape = SimpleNamespace(n_heads=H, n_kv_heads=G, head_dim=D, window=None, keep_first=0)
     out = torch.full((sum(q_lens), H * D), 7.0, device="cuda")
@@ -325,3 +325,41 @@ def test_products_of_large_numbers(a_exponent, w_exponent):
     want = a.double() @ w.double().t()
     assert bool(torch.isfinite(c).all())
     assert bool(((c.double() - want).abs() <= 600 * EPS * (a.double().abs() @ w.double().abs().t())).all())
+
+
+def test_a_float32_prompt_asks_nothing_of_the_allocator_once_its_workspace_fits(monkeypatch):
+    """The split activations of the products and the spans of attention come from the pass's workspace; without memory to spare the products are
+    made by multiply-adds and the keys are not cut."""
+    from gpullama3.java_b200.engine.api import Engine, SequenceInput
+    from gpullama3.java_b200.parts.base import StepContext
+
+    config = {"architectures": ["LlamaForCausalLM"], "num_hidden_layers": 2, "hidden_size": 256, "num_attention_heads": 4, "num_key_value_heads": 2,
+              "head_dim": 64, "intermediate_size": 768, "vocab_size": 512, "rope_theta": 10000.0, "rms_norm_eps": 1e-5, "tie_word_embeddings": False,
+              "max_position_embeddings": 1024}
+    engine = Engine.from_random(config, 3, dtype="float32", max_tokens=64 * 12, max_batch=1)
+    engine.step_fn.use_graphs = False
+
+    def prompt():
+        slot = engine.cache.acquire()
+        engine.step([SequenceInput(slot, list(range(400)), [])])
+        out = engine.step([SequenceInput(slot, list(range(20)), [19])])
+        engine.cache.release(slot)
+        return out.clone()
+
+    want = prompt()
+    prompt()
+    asked, empty = [], torch.empty
+
+    def counted(*args, **kwargs):
+        t = empty(*args, **kwargs)
+        if t.is_cuda:
+            asked.append(t.numel())
+        return t
+
+    monkeypatch.setattr(torch, "empty", counted)
+    assert torch.equal(prompt(), want)
+    assert max(asked, default=0) <= want.numel()      # (the logits)
+    monkeypatch.setattr(StepContext, "scratch", lambda self, shape, dtype: None)
+    without = prompt()
+    assert not torch.equal(without, want)
+    torch.testing.assert_close(without, want, rtol=1e-4, atol=1e-4 * float(want.abs().max()))
