@@ -391,7 +391,8 @@ def run_8b(peaks, layers, warmup, steps=512, prefill=True):
 
 
 def run_1b_f32(peaks, layers, warmup, context, batch):
-    """The 1B shape in true float32 (plain FMA kernels, float32 weights and cache): prefill 2,048, decode at ``batch``."""
+    """The 1B shape in true float32 (float32 weights and cache; prompts' products as bfloat16 parts of float32 numbers on the tensor cores,
+    everything else by 32-bit multiply-adds): prefill 2,048, decode at ``batch``."""
     cfg, full = model_config("1b", layers)
     engine = make_engine(cfg, "float32", batch * context + 4096, batch)
     try:
@@ -402,7 +403,7 @@ def run_1b_f32(peaks, layers, warmup, context, batch):
         dec = decode_record(cfg, 4, [n + warmup for n in lengths], times, peaks, launches)
     finally:
         drop(engine)
-    log(f"1B float32: prefill 2048 {pre['ms']} ms ({pre['tflops']} TFLOP/s of FMA); decode b{batch} {dec['ms_per_step']} ms/step "
+    log(f"1B float32: prefill 2048 {pre['ms']} ms ({pre['tflops']} TFLOP/s); decode b{batch} {dec['ms_per_step']} ms/step "
         f"({dec['tokens_per_s']:.0f} tok/s, frac {dec['frac']})")
     return {"layers": cfg["num_hidden_layers"], "layers_full": full, "prefill": pre, "decode": dec}
 

@@ -22,8 +22,8 @@
 // and 64 keys with nothing kept are 8 % faster and leave 2.1e-7, one chain over all keys 7e-7.
 //
 // Few queries: one, two or four rows a group, and the pages of a tile cut into spans, merged by a second kernel (the plan that picks both is
-// with the caller).  8 sequences of 500 keys decoded, 32 heads of 64: 11.5 us (25 with the plain kernel in spans of a tile); 2 tokens
-// behind 2,000 keys: 10 us, 16 tokens: 31 (plain 37 and 110; a single tile of 64 rows without spans: 251 and 252).
+// with the caller).  8 sequences of 500 keys decoded, 32 heads of 64: 12 us (25 with the plain kernel in spans of a tile); 2 tokens
+// behind 2,000 keys: 10 us, 16 tokens: 21 (plain 37 and 110; a single tile of 64 rows without spans: 251 and 252).
 //
 // Terms as in the plain kernel (window, chunk, slopes, sinks, gate, softcap; not keep_first).  Values of keys past a
 // sequence's end are read as zeros.  A key that some row of the tile must not see has probability 0 there, and 0 times a value that is

@@ -436,7 +436,7 @@ def attention_f32_plan(q_lens: list[int], kv_lens: list[int], n_heads: int, n_kv
     second launch and their results' way through memory: of each tile with one, two and four spans and with CTAs for two and a half
     rounds of SMs and for five, the one that the figures above say is fastest (4 % above the fastest measured on the mean, 41 % at most; 2 tokens behind 8,000,
     32 heads of 64 over 8: 24 us, one tile of 64 rows without spans 967).  The plain kernel reads keys and values for every query head anew,
-    which one or two heads to a kv head can afford (8 sequences of 2,000 keys decoded, 32 heads of 64: 69 us, 97 in tiles of 8)."""
+    which one or two heads to a kv head can afford (8 sequences of 2,000 keys decoded, 32 heads of 64: 64 us, 97 in tiles of 8)."""
     group, wide = n_heads // n_kv_heads, head_dim / 64
     longest = -(-min(reach, max(kv_lens)) // PAGE_TOKENS)
     pages = [min(reach, kv - q / 2) / PAGE_TOKENS + 0.5 for q, kv in zip(q_lens, kv_lens)]
@@ -1621,7 +1621,7 @@ def delta_rule_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, 
     [T, >= heads] and decay [T, >= heads d_k] as the projections leave them, state float32 [slots, >= heads d_k d_v]
     (updated in place), out float32 [T, heads d_v].  ``decay_per_head``: decay [T, >= heads] and dt_bias [heads], one
     decay for all key channels of a head.  ``alloc(shape, dtype)``: where the scan's scratch (a row of
-    32-bit numbers per token and head, and for long sequences a few dozen more) comes from.  ``longest``: the most tokens of
+    32-bit numbers per token and head, and for long sequences two more) comes from.  ``longest``: the most tokens of
     one sequence, where the caller knows it: long ones are taken in runs of tokens."""
     _dev(qkv, beta, decay, dt_bias, a_log, state, slots, cu_seqlens, out)
     assert qkv.dtype == beta.dtype == decay.dtype and qkv.stride(1) == beta.stride(1) == decay.stride(1) == 1
