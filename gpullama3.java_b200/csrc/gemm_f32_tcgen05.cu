@@ -480,12 +480,9 @@ static int launch_f32(const __nv_bfloat16* planes, int padded, F32Args p, int n_
 
 // Whether (and with how many bfloat16 elements of scratch) the product goes to the tensor cores: 0, no.
 // Left to the plain kernels: few rows (they stream the weights as fast), rows that TMA cannot address, and products so
-// small that the second launch and the epilogue cost more than they save.  The plain kernel takes 7.7 us up to 127 rows at K = 64 and 12.8
-// at K = 128, this one 8 to 9 and 9 to 10 in tiles of 64 tokens, 13.6 and 14.9 in tiles of 128; from 128 rows on the plain kernel takes 19
-// and 28.
+// small that the second launch costs more than it saves.
 extern "C" long long b200_gemm_f32_scratch(int M, int N, int K, int lda, int ldw) {
     if (M <= 16 || K < 64 || K % 4 != 0 || ldw % 4 != 0 || lda < K || N < 64 || (long long)N * K < 65536) return 0;
-    if (M < 128 && K < (M <= 64 ? 128 : 192)) return 0;
     if (3ll * M > 0x7fffffffll) return 0;
     return 3ll * M * ((K + 7) / 8 * 8);
 }
@@ -518,7 +515,9 @@ extern "C" int b200_gemm_f32_tcgen05(const void* A, int lda, const void* W, int 
     p.lda = lda; p.ldw = ldw; p.ldc = ldc; p.M = M; p.N = N; p.K = K;
     p.epilogue = epilogue; p.silu_cols = silu_cols; p.gate_limit = gate_limit; p.gate_slope = gate_slope;
     const auto planes = (const __nv_bfloat16*)scratch;
-    if (M <= 64)
+    // Tiles of 64 tokens also for 65 to 127 over a short K, where the epilogue is most of the time: 2,048 columns, K = 64: 9.2 us (13.7 in
+    // tiles of 128, plain kernel 8.0 with twice the error); 512 columns, K = 128: 10.3 (14.9, 12.8).
+    if (M <= 64 || (M < 128 && K <= 192))
         return epilogue == 0 ? launch_f32<64, 4, 0>(planes, padded, p, n_spans, stream)
              : epilogue == 1 ? launch_f32<64, 4, 1>(planes, padded, p, n_spans, stream)
                              : launch_f32<64, 4, 2>(planes, padded, p, n_spans, stream);
