@@ -337,7 +337,7 @@ gemm_fewrows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W,
 
 // The same for at most eight tokens with half as many rows a CTA and the activations fetched from L1 for every four weight rows: sums are
 // kept over all of K and exchanged once, and tokens that are not there cost nothing.  Faster where the kernel above has fewer CTAs than
-// the GPU has SMs and K is long (an SM's share is then one CTA's chain of slices: 8 tokens, 128 x 2,048 in float32: 2.7 us against 4.2), and
+// the GPU has SMs and K is long (an SM's share is then one CTA's chain of slices: 8 tokens, 128 x 2,048 in float32: 3.2 us against 4.2), and
 // for bfloat16 weights, whose multiply-adds and exchanges take longer than their stream (5 tokens, 16,384 x 2,048: 33 us against 44);
 // fourrows_wins draws the line.  Four rows of sums for up to eight tokens are the 32 numbers that a warp sums by halving.
 constexpr int kFourRows = 4, kFourTokens = 8;
@@ -371,8 +371,12 @@ gemm_fourrows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W
             if (m < M) {
                 const float4 x = load4<TA>(A + (size_t)m * lda + k);
 #pragma unroll
-                for (int r = 0; r < kFourRows; ++r)
-                    acc[r * MT + m] = fmaf(wv[r].w, x.w, fmaf(wv[r].z, x.z, fmaf(wv[r].y, x.y, fmaf(wv[r].x, x.x, acc[r * MT + m]))));
+                for (int r = 0; r < kFourRows; ++r) {
+                    // (32-bit weights: four products by themselves, then one addition, as the kernel above; 16-bit ones, whose products are
+                    // exact, are bound by the instructions)
+                    if constexpr (sizeof(TW) == 4) acc[r * MT + m] += dot4_pairs(wv[r], x);
+                    else acc[r * MT + m] = fmaf(wv[r].w, x.w, fmaf(wv[r].z, x.z, fmaf(wv[r].y, x.y, fmaf(wv[r].x, x.x, acc[r * MT + m]))));
+                }
             }
         }
     }
@@ -402,8 +406,8 @@ gemm_fourrows_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W
 }
 
 // Measured with weights from memory, M 1 to 16, N 32 to 28,672, K 64 to 14,336.  Up to one slice of K the kernel of eight rows is never
-// slower.  float32 weights: four rows win below 384 weight rows (1.4 times at 128 x 2,048), from five tokens on as long as eight rows make
-// fewer CTAs than there are SMs (1.3 times at 1,024 x 2,048; 0.75 at 2,048 x 2,048).  bfloat16 weights: four rows win (1.1 to 1.5 times)
+// slower.  float32 weights: four rows win below 384 weight rows (1.3 times at 128 x 2,048), from five tokens on as long as eight rows make
+// fewer CTAs than there are SMs (1.14 times at 1,024 x 2,048; 0.75 at 2,048 x 2,048).  bfloat16 weights: four rows win (1.1 to 1.5 times)
 // except for four tokens, which fill the other kernel's registers, where eight rows make one round of CTAs (0.7 at 2,048 x 2,048), and for
 // three or eight tokens over a long K (0.8 at 4,096 x 14,336).
 static bool fourrows_wins(int M, int N, int K, bool bf16_weights) {
