@@ -710,7 +710,7 @@ static int launch_scan_rows(const ScanArgs& a, int rpt, int lanes, int n_seqs, c
 // 64 bits and rounds what it leaves; the walk's sums are 32-bit multiply-adds.  A token that is not finite reaches itself and
 // later tokens only, as in the scan.
 // Bound by what shared memory answers in the first kernel (every operand is read by all lanes alike) and by latency in the second: 2,048
-// tokens, 32 heads of 64 by 64: 251 us (prepare and scan: 497; with 32-bit sums in the first kernel, its rows by rows, 261); error
+// tokens, 32 heads of 64 by 64: 251 us (prepare and scan: 497; with 32-bit sums in the first kernel, every lane reading all channels, 261); error
 // against 64 bits 1.24e-7 of the norm for the results and 1.25e-7 for the state (scan: 1.52e-7 and 1.27e-7), with keys and queries of one
 // sign 0.88e-7 and 1.26e-7 (1.09e-7 and 1.27e-7).
 constexpr int kDeltaRun = 32, kDeltaKey = 64, kDeltaCols = 16;
