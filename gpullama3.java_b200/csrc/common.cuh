@@ -114,35 +114,55 @@ inline bool pdl_enabled() {
     return on == 1;
 }
 
-// The general form: CTAs grouped into thread-block clusters of `cluster` (1, 1, 1: no clusters), and
+// How a kernel is launched beyond its grid: CTAs grouped into thread-block clusters of `cluster` (1, 1, 1: no clusters), and
 // `early_start` false for a kernel that should find the GPU empty.  A long kernel whose grid just fills the
 // SMs is such a kernel: started early, its CTAs settle wherever the predecessor's CTAs leave room, unevenly, and
 // the SMs that got more of them finish late.
+// `shared_percent` (-1: the driver's choice): how much of an SM's memory should be shared memory rather than L1.  A kernel that streams
+// through registers lives on L1, whose lines hold what is in flight, but an SM whose last kernel had most of its memory as shared
+// memory keeps that split for it unless the launch says otherwise.
+struct LaunchForm {
+    dim3 cluster = dim3(1, 1, 1);
+    bool early_start = true;
+    int shared_percent = -1;
+};
+constexpr int kStreamingSharedPercent = 28;   // 64 KB of shared memory: the resident CTAs of the streaming kernels; the rest is L1
+
 template <typename... KArgs, typename... Args>
-inline int launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                              dim3 cluster, bool early_start, Args... args) {
+inline int launch_pdl_as(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const LaunchForm& form, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
+    cudaLaunchAttribute attr[3];
     int n = 0;
-    if (cluster.x * cluster.y * cluster.z > 1) {
+    if (form.cluster.x * form.cluster.y * form.cluster.z > 1) {
         attr[n].id = cudaLaunchAttributeClusterDimension;
-        attr[n].val.clusterDim.x = cluster.x;
-        attr[n].val.clusterDim.y = cluster.y;
-        attr[n].val.clusterDim.z = cluster.z;
+        attr[n].val.clusterDim.x = form.cluster.x;
+        attr[n].val.clusterDim.y = form.cluster.y;
+        attr[n].val.clusterDim.z = form.cluster.z;
         ++n;
     }
-    if (pdl_enabled() && early_start) {
+    if (pdl_enabled() && form.early_start) {
         attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[n].val.programmaticStreamSerializationAllowed = 1;
+        ++n;
+    }
+    if (form.shared_percent >= 0) {
+        attr[n].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        attr[n].val.sharedMemCarveout = (unsigned int)form.shared_percent;
         ++n;
     }
     cfg.attrs = attr;
     cfg.numAttrs = n;
     return (int)cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+inline int launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                              dim3 cluster, bool early_start, Args... args) {
+    return launch_pdl_as(kernel, grid, block, smem, stream, LaunchForm{cluster, early_start}, args...);
 }
 
 template <typename... KArgs, typename... Args>

@@ -34,6 +34,7 @@ namespace b200 {
 
 constexpr int kDecodeWarps = 8;
 constexpr int kDecodeThreads = kDecodeWarps * 32;
+constexpr int kHeadRows = 32768;   // weight rows from which a product counts as an output head
 
 __device__ __forceinline__ uint4 load_stream(const void* p) {
     uint4 v;
@@ -269,8 +270,12 @@ static int launch_u(const __nv_bfloat16* a, int lda, const __nv_bfloat16* w, int
             configured = true;
         }
     }
-    return launch_pdl(kernel, dim3((N + ROWS - 1) / ROWS), dim3(kDecodeThreads), smem, stream, a, lda, w, ldw, (TC*)C, ldc,
-                      M, N, K, link);
+    // An output head reads long enough to be worth an SM's change from the prompt kernels' split of its memory, which leaves L1, where
+    // this kernel's loads are, a few KB (128,256 x 2,048 behind a prompt of 45 tokens: 120 us without, 79 with).
+    LaunchForm form;
+    if (N >= kHeadRows && smem <= 12 * 1024) form.shared_percent = kStreamingSharedPercent;
+    return launch_pdl_as(kernel, dim3((N + ROWS - 1) / ROWS), dim3(kDecodeThreads), smem, stream, form, a, lda, w, ldw, (TC*)C, ldc,
+                         M, N, K, link);
 }
 
 template <int MT, int NT, int EPI, typename TC>
