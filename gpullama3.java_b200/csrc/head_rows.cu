@@ -178,7 +178,7 @@ head_rows_kernel(const T* __restrict__ src, int ld_src, T* __restrict__ dst, int
     head_row<T>(src, ld_src, dst, ld_dst, bias, weight, segs.seg[s], t, row, lane, eps, 0.f, cache, mix);
 }
 
-// For launches of many tokens whose rows lie on a grid of eights (turned over halves or not at all; no norm over a whole
+// For launches of many tokens whose rows lie on a grid of eights (turned over halves or not at all, with or without angles; no norm over a whole
 // segment, no mixing): a CTA takes kTile tokens, makes their angles once, and its warps take (row, tokens) in turn.  G
 // lanes share a row, each with one piece of it in registers: four pairs (u[0..3], v[0..3]) of a turned part, or eight
 // numbers behind it; a warp's 32 / G rows are the same row of neighbouring tokens, so that values, which lie transposed in
@@ -221,7 +221,7 @@ head_rows_tile_kernel(const T* __restrict__ src, int ld_src, T* __restrict__ dst
     __syncthreads();
     pdl_wait();
     const int tasks = segs.total_rows * (kTile / RPW);
-    for (int task = threadIdx.x >> 5; task < tasks; task += kTileThreads / 32) {
+    for (int task = (int)blockIdx.y * (kTileThreads / 32) + (threadIdx.x >> 5); task < tasks; task += (int)gridDim.y * (kTileThreads / 32)) {
         int s = 0, row = task / (kTile / RPW);
         const int tt = (task % (kTile / RPW)) * RPW + lane / G, t = t0 + tt;
         while (s + 1 < segs.n && row >= segs.seg[s].n_rows) {
@@ -275,9 +275,10 @@ head_rows_tile_kernel(const T* __restrict__ src, int ld_src, T* __restrict__ dst
         if (g.target != 0) {
             const int pos = cache.positions[t];
             const size_t page = cache.page_table[(size_t)cache.seq_ids[t] * cache.table_stride + pos / kPageTokens];
-            const size_t head = (page * g.n_rows + row) * kPageTokens * g.d_pad;
+            const int dim = g.cache_dim >= 0 ? g.cache_dim : g.d_pad, first = g.cache_dim >= 0 ? g.dst_off : 0;
+            const size_t head = (page * g.n_rows + row) * kPageTokens * dim;
             if (g.target == 2) {          // a row per dimension, positions side by side
-                T* vp = (T*)cache.v_pool + head + (pos % kPageTokens);
+                T* vp = (T*)cache.v_pool + head + (size_t)first * kPageTokens + (pos % kPageTokens);
                 if (c0 < g.d_pad) {
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
@@ -287,7 +288,7 @@ head_rows_tile_kernel(const T* __restrict__ src, int ld_src, T* __restrict__ dst
                 }
                 continue;
             }
-            o = (T*)cache.k_pool + head + (size_t)(pos % kPageTokens) * g.d_pad;
+            o = (T*)cache.k_pool + head + (size_t)(pos % kPageTokens) * dim + first;
         }
         if (c0 < g.d_pad) {
             Piece<T>::store(o + c0, z);
@@ -399,20 +400,27 @@ extern "C" int b200_head_rows(const void* src, int ld_src, void* dst, int ld_dst
     }
     // many tokens on a grid of eights: tiles of tokens
     int n_freqs = 0, lanes = 8;
-    bool tiles = n_tokens >= 256 && ld_src % 4 == 0 && (dst == nullptr || ld_dst % 4 == 0) && positions != nullptr;
+    bool tiles = n_tokens >= 256 && ld_src % 4 == 0 && (dst == nullptr || ld_dst % 4 == 0);
     const size_t el = dtype == b200::kF32 ? 4 : 2;
     tiles = tiles && (uintptr_t)src % (4 * el) == 0 && (uintptr_t)dst % (4 * el) == 0 && (uintptr_t)k_pool % (4 * el) == 0;
     for (int i = 0; i < n_segments && tiles; ++i) {
         const b200::RowSegment& g = segs.seg[i];
         const int n = g.rotate == 2 ? g.pairs : 0;
-        tiles = g.rotate != 1 && g.mix_off < 0 && g.lead == 0 && g.cache_dim < 0 && g.d % 8 == 0 && g.d_pad % 8 == 0 && n % 4 == 0 &&
+        tiles = g.rotate != 1 && g.mix_off < 0 && g.lead == 0 && g.d % 8 == 0 && g.d_pad % 8 == 0 && n % 4 == 0 &&
+                (g.cache_dim < 0 || g.cache_dim % 4 == 0) &&
                 g.d_pad <= 256 && g.src_off % 4 == 0 && g.dst_off % 4 == 0 && (g.src_stride < 0 || g.src_stride % 4 == 0) &&
                 (g.dst_stride < 0 || g.dst_stride % 4 == 0);
         if (n > 0 && g.freq_off + n > n_freqs) n_freqs = g.freq_off + n;
         while (tiles && lanes * 8 < g.d_pad) lanes *= 2;
     }
-    if (tiles && n_freqs > 0 && n_freqs <= b200::kTileFreqs) {
-        const dim3 tile_grid((n_tokens + b200::kTile - 1) / b200::kTile);
+    if (tiles && n_freqs <= b200::kTileFreqs) {
+        // Without angles a tile's CTAs share nothing, so its rows are cut among as many of them (grid.y) as give every SM eight (2,048 tokens,
+        // 48 rows of 64 with keys and values into their pages: 44 us with a warp a row, 13 so).
+        const int tiles_x = (n_tokens + b200::kTile - 1) / b200::kTile;
+        const int tasks = segs.total_rows * b200::kTile * lanes / 32, warps = b200::kTileThreads / 32;
+        int ny = n_freqs > 0 ? 1 : 8 * b200::device_sm_count() / tiles_x;
+        ny = ny < 1 ? 1 : ny > (tasks + warps - 1) / warps ? (tasks + warps - 1) / warps : ny;
+        const dim3 tile_grid(tiles_x, ny);
         const size_t smem = sizeof(float2) * b200::kTile * n_freqs;
 #define B200_TILE(G)                                                                                                               \
         B200_DISPATCH_DTYPE(dtype, T,                                                                                              \
