@@ -427,7 +427,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 }
 
 // ---------------------------------------------------------------------------------------------
-// The pair kernel (head_dim 64 or 128, no window): one CTA owns 256 consecutive query tokens as two tiles of 128
+// The pair kernel (head_dim 64 or 128): one CTA owns 256 consecutive query tokens as two tiles of 128
 // and keeps both in flight.  Each tile has its own S and O in tensor memory and its own warpgroup of
 // softmax threads, ONE thread per query row: the thread reads its row of S (128 scores) into registers in
 // one go, so the maximum, the exponentials and the sum need no exchange between threads and no second
@@ -502,13 +502,17 @@ __device__ __forceinline__ void umma_bf16_a_tmem(uint32_t tmem_d, uint32_t tmem_
 // another in one stream.
 __device__ unsigned int g_pair_ctl[4];
 
-template <int D, bool TERMS>
+// WIN: compiled with a window or `chunk`.  Both tiles then start at the block that holds the first key of the pair's first row; what
+// of it lies below a row's own first key is masked as what lies above its position is (for the second tile that is a block more
+// than it needs, in nine at a window of 1,024).  2,048 tokens, 32 heads of 64, window 1,024: 62.6 us with a tile a CTA, 48.5 so.
+template <int D, bool TERMS, bool WIN>
 __global__ void __launch_bounds__(kPairThreads, 1)
 attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                               const __grid_constant__ CUtensorMap map_v, __nv_bfloat16* __restrict__ out,
                               const int* __restrict__ cu_seqlens, const int* __restrict__ kv_lens,
                               const int* __restrict__ page_table, int table_stride, int n_heads, int n_kv_heads,
-                              int k_rows_total, int v_rows_total, int n_seqs, int n_pairs, const float* __restrict__ sinks, FaTerms terms) {
+                              int k_rows_total, int v_rows_total, int n_seqs, int n_pairs, const float* __restrict__ sinks, FaTerms terms,
+                              int window, int chunk) {
     static_assert(D == 64 || D == 128, "the pair kernel is laid out for head_dim 64 and 128");
     // Tensor memory, 512 columns.  Tile t: S in columns 128 t, O in 256 + D t.  P (bfloat16 pairs, 64 columns): with
     // head_dim 64 in columns 384 + 64 t; with head_dim 128 nothing is left, so P overwrites the first half of S, which
@@ -580,8 +584,11 @@ attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
             const int kv_len = kv_lens[seq], start = kv_len - q_len;
             // tile t: rows q0 + 128 t .. ; its key blocks are 0 .. nb[t] - 1 (causal), nb[1] = 0 when the tile has no rows
             const int rows0 = min(kFaRows, q_len - q0), rows1 = max(0, min(kFaRows, q_len - q0 - kFaRows));
-            const int nb0 = (start + q0 + rows0 - 1) / kFaKeys + 1;
-            const int nb1 = rows1 > 0 ? (start + q0 + kFaRows + rows1 - 1) / kFaKeys + 1 : 0;
+            // (with WIN counted from block blk0, where the first row's keys start)
+            auto first_key = [&](int pos) { return !WIN ? 0 : chunk > 0 ? pos - pos % chunk : max(0, pos - window + 1); };
+            const int blk0 = WIN ? first_key(start + q0) / kFaKeys : 0;
+            const int nb0 = (start + q0 + rows0 - 1) / kFaKeys + 1 - blk0;
+            const int nb1 = rows1 > 0 ? (start + q0 + kFaRows + rows1 - 1) / kFaKeys + 1 - blk0 : 0;
             const int nb = max(nb0, nb1);
 
             if (ROLE == 0 && warp == kPairTmaWarp && lane == 0) {
@@ -602,7 +609,7 @@ attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
                     mbar_expect_tx(&sm.kv_full[s], 2 * (64 * D * 2) + 2 * (D * 64 * 2));
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
-                        const int lp = j * 2 + h;  // logical page; pages the sequence does not have are read as zeros
+                        const int lp = (blk0 + j) * 2 + h;  // logical page; pages the sequence does not have are read as zeros
                         const bool have = lp < n_pages_seq;
                         const int page = have ? pages[lp] : 0;
 #pragma unroll
@@ -688,6 +695,7 @@ attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
                 const int rows_t = t == 0 ? rows0 : rows1, nbt = t == 0 ? nb0 : nb1;
                 const int p_first = start + q0 + kFaRows * t;
                 const int pos = p_first + min(r, max(rows_t, 1) - 1);  // rows past the end mirror the last one (never stored)
+                const int lo_key = first_key(pos), lo_last = first_key(p_first + max(rows_t, 1) - 1);
                 const float scale_log2 = 1.4426950408889634f / sqrtf((float)D);
                 const uint32_t tmem_s = tmem + 128 * t, tmem_o = tmem + 256 + D * t, tmem_p = D == 64 ? tmem + 384 + 64 * t : tmem_s;
                 const float cap_qk = TERMS ? terms.softcap * sqrtf((float)D) : 0.f, cap_log2 = TERMS && cap_qk > 0.f ? 2.885390081777927f / cap_qk : 0.f;
@@ -709,15 +717,16 @@ attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     __syncwarp();
                     if (lane == 0) mbar_arrive_fa(&sm.s_free[t]);
-                    const int base = j * kFaKeys;
-                    const bool masked = base + kFaKeys - 1 > p_first;  // the block reaches beyond the tile's first row
+                    const int base = (blk0 + j) * kFaKeys;
+                    // the block reaches beyond the tile's first row, or below the last row's first key
+                    const bool masked = base + kFaKeys - 1 > p_first || (WIN && base < lo_last);
                     float m_blk = -INFINITY;
                     if (masked) {
 #pragma unroll
                         for (int c = 0; c < 4; ++c)
 #pragma unroll
                             for (int i = 0; i < 32; ++i)
-                                if (base + c * 32 + i <= pos) m_blk = fmaxf(m_blk, __uint_as_float(sr[c][i]));
+                                if (base + c * 32 + i <= pos && (!WIN || base + c * 32 + i >= lo_key)) m_blk = fmaxf(m_blk, __uint_as_float(sr[c][i]));
                     } else {
                         float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
@@ -772,15 +781,15 @@ attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
                     }
                     // probabilities as bfloat16 pairs into this row's lane of P: key k of the block in column k / 2
                     float l4[4] = {0.f, 0.f, 0.f, 0.f};
-                    if (masked) {  // the few blocks on the diagonal: every key is compared with the row's position
+                    if (masked) {  // the few blocks on the mask's edges: every key is compared with the row's bounds
 #pragma unroll
                         for (int c = 0; c < 4; ++c) {
                             uint32_t pk[16];
 #pragma unroll
                             for (int i = 0; i < 32; i += 2) {
                                 const int key = base + c * 32 + i;
-                                const float p0 = key <= pos ? ex2(fmaf(__uint_as_float(sr[c][i]), scale_log2, -m_scaled)) : 0.f;
-                                const float p1 = key + 1 <= pos ? ex2(fmaf(__uint_as_float(sr[c][i + 1]), scale_log2, -m_scaled)) : 0.f;
+                                const float p0 = key <= pos && (!WIN || key >= lo_key) ? ex2(fmaf(__uint_as_float(sr[c][i]), scale_log2, -m_scaled)) : 0.f;
+                                const float p1 = key + 1 <= pos && (!WIN || key + 1 >= lo_key) ? ex2(fmaf(__uint_as_float(sr[c][i + 1]), scale_log2, -m_scaled)) : 0.f;
                                 __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
                                 l4[c] += p0 + p1;
                                 pk[i / 2] = *reinterpret_cast<uint32_t*>(&h);
@@ -831,10 +840,10 @@ attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
                     l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
                     __syncwarp();
                     if (lane == 0) mbar_arrive_fa(&sm.exp_turn[1 - t]);  // the other tile's turn
-                    if ((j + 1) * kFaKeys > kv_len) {  // the block holds the sequence's end: see zero_values_beyond_end
+                    if (base + kFaKeys > kv_len) {  // the block holds the sequence's end: see zero_values_beyond_end
                         const int g = kv_base + j, s = g % PairStages<D>::value;  // (both tiles may do this: they write the same zeros)
                         if (mbar_wait(&sm.kv_full[s], (g / PairStages<D>::value) & 1, abort_flag))
-                            zero_values_beyond_end<D>(sm.v[s][0], sm.v[s][1], kv_len - j * kFaKeys, quarter * 32 + lane, 128);
+                            zero_values_beyond_end<D>(sm.v[s][0], sm.v[s][1], kv_len - base, quarter * 32 + lane, 128);
                         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     }
                     // P is in tensor memory and S has been read: the MMA thread may go on
@@ -952,14 +961,14 @@ static int launch_fa(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
 }  // namespace b200
 
 namespace b200 {
-template <int D, bool TERMS>
-static int launch_pair(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, void* out, const int* cu_seqlens,
+template <int D, bool TERMS, bool WIN>
+static int launch_pair_of(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, void* out, const int* cu_seqlens,
                        const int* kv_lens, const int* page_table, int table_stride, int n_seqs, int max_q_len, int n_heads,
-                       int n_kv_heads, int k_rows, int v_rows, const float* sinks, FaTerms terms, cudaStream_t stream) {
+                       int n_kv_heads, int k_rows, int v_rows, const float* sinks, FaTerms terms, int window, int chunk, cudaStream_t stream) {
     const size_t smem = sizeof(PairSmem<D>) + 1024;
     static bool configured = false;
     if (!configured) {
-        if (cudaFuncSetAttribute(attention_prefill_pair_kernel<D, TERMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        if (cudaFuncSetAttribute(attention_prefill_pair_kernel<D, TERMS, WIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
             return (int)cudaGetLastError();
         configured = true;
     }
@@ -972,9 +981,18 @@ static int launch_pair(const CUtensorMap& mq, const CUtensorMap& mk, const CUten
     if (e != cudaSuccess) return (int)e;
     if (dev < 0 || dev >= 64) return kErrBadArgument;
     const int grid = (int)(units < n_sms ? units : n_sms);  // one CTA per SM; each takes units until none are left
-    return launch_pdl(attention_prefill_pair_kernel<D, TERMS>, dim3(grid), dim3(kPairThreads), smem, stream, mq, mk, mv,
+    return launch_pdl(attention_prefill_pair_kernel<D, TERMS, WIN>, dim3(grid), dim3(kPairThreads), smem, stream, mq, mk, mv,
                       (__nv_bfloat16*)out, cu_seqlens, kv_lens, page_table, table_stride, n_heads, n_kv_heads, k_rows, v_rows,
-                      n_seqs, n_pairs, sinks, terms);
+                      n_seqs, n_pairs, sinks, terms, window, chunk);
+}
+
+template <int D, bool TERMS>
+static int launch_pair(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, void* out, const int* cu_seqlens,
+                       const int* kv_lens, const int* page_table, int table_stride, int n_seqs, int max_q_len, int n_heads,
+                       int n_kv_heads, int k_rows, int v_rows, const float* sinks, FaTerms terms, int window, int chunk, cudaStream_t stream) {
+    auto go = window > 0 || chunk > 0 ? launch_pair_of<D, TERMS, true> : launch_pair_of<D, TERMS, false>;
+    return go(mq, mk, mv, out, cu_seqlens, kv_lens, page_table, table_stride, n_seqs, max_q_len, n_heads, n_kv_heads, k_rows, v_rows,
+              sinks, terms, window, chunk, stream);
 }
 }  // namespace b200
 
@@ -1004,13 +1022,18 @@ extern "C" int b200_attention_prefill_tc(const void* q, int q_row_stride, int n_
     const bool more = softcap > 0.f || gate != nullptr;
 #define B200_GO(F, D, T, ...)                                                                                                  \
     F<D, T>(mq, mk, mv, out, cu_seqlens, kv_lens, page_table, table_stride, n_seqs, max_q_len, n_heads, n_kv_heads, __VA_ARGS__, stream)
-    // tiles in pairs when there are enough pairs to give every SM one (fewer: the single-tile kernel fills more SMs)
-    if (window <= 0 && chunk <= 0 && (long long)((max_q_len + 2 * kFaRows - 1) / (2 * kFaRows)) * n_heads * n_seqs >= device_sm_count()) {
+    // Tiles in pairs when there are enough pairs to give every SM one (fewer: the single-tile kernel fills more SMs).  A mask that hides
+    // early keys costs a pair its second tile's first block, which counts where few blocks are seen; heads of 64, two of whose
+    // single-tile CTAs share an SM, go in pairs from 768 keys on (2,048 tokens, 32 heads, a tile a CTA / in pairs: window 512 42.9 / 45.5 us,
+    // 1,024 62.6 / 48.5; 8,192 tokens, window 4,096: 568 / 363), heads of 128 always (window 128: 43.9 / 38.9, 1,024: 92.7 / 60.9).
+    const int reach = window > 0 ? window : chunk;
+    const bool pairs = reach == 0 || head_dim == 128 || reach >= 768;
+    if (pairs && (long long)((max_q_len + 2 * kFaRows - 1) / (2 * kFaRows)) * n_heads * n_seqs >= device_sm_count()) {
         if (head_dim == 64)
-            return more || sinks != nullptr ? B200_GO(launch_pair, 64, true, (int)k_rows, (int)v_rows, sinks, terms)
-                                            : B200_GO(launch_pair, 64, false, (int)k_rows, (int)v_rows, sinks, terms);
-        return more || sinks != nullptr ? B200_GO(launch_pair, 128, true, (int)k_rows, (int)v_rows, sinks, terms)
-                                        : B200_GO(launch_pair, 128, false, (int)k_rows, (int)v_rows, sinks, terms);
+            return more || sinks != nullptr ? B200_GO(launch_pair, 64, true, (int)k_rows, (int)v_rows, sinks, terms, window, chunk)
+                                            : B200_GO(launch_pair, 64, false, (int)k_rows, (int)v_rows, sinks, terms, window, chunk);
+        return more || sinks != nullptr ? B200_GO(launch_pair, 128, true, (int)k_rows, (int)v_rows, sinks, terms, window, chunk)
+                                        : B200_GO(launch_pair, 128, false, (int)k_rows, (int)v_rows, sinks, terms, window, chunk);
     }
     if (head_dim == 64)
         return more ? B200_GO(launch_fa, 64, true, window, chunk, sinks, (int)k_rows, (int)v_rows, terms)

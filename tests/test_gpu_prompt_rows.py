@@ -1,0 +1,119 @@
+"""Prompt forms of the kernels between a mixer's products: stream connections through a ring of stages, head rows in tiles without
+angles, output norms of several rows a warp, convolutions over runs, and windows in the attention over pairs of tiles."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def ops():
+    from gpullama3.java_b200.kernels import ops as o
+    return o
+
+
+@pytest.mark.parametrize("streams, width, T", [(3, 2048, 592), (3, 2048, 2048), (1, 64, 700), (2, 4096, 601), (4, 2052, 777), (8, 300, 600), (5, 260, 595)])
+@pytest.mark.parametrize("reads", [True, False])
+def test_streams_step_through_a_ring(streams, width, T, reads):
+    """The same bits as the kernel of fewer tokens, which takes the rows in pieces."""
+    o = ops()
+    g = torch.Generator("cuda").manual_seed(T + width)
+    randn = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    x, y, mix, write, read, w = randn(T, streams, width), randn(T, width), randn(streams, streams), randn(streams), randn(streams), randn(width)
+
+    def run(piece):
+        xs, ys, out = x.clone(), y.clone(), torch.zeros(T, width, dtype=torch.bfloat16, device="cuda")
+        for at in range(0, T, piece):
+            part = slice(at, min(T, at + piece))
+            o.streams_step(xs[part], mix, write, ys[part], *((read, w, out[part], 1e-6) if reads else ()))
+        return xs, ys, out
+    whole, pieces = run(T), run(300)
+    for a, b in zip(whole, pieces):
+        assert torch.equal(a, b)
+    assert not whole[1].any()
+    from gpullama3.java_b200.kernels.build import library
+    assert library("streams").b200_streams_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32], ids=["bf16", "f32"])
+@pytest.mark.parametrize("H, G, d, D, T", [(32, 8, 64, 64, 300), (3, 1, 40, 64, 257), (2, 2, 128, 128, 2048), (5, 5, 248, 256, 256)])
+def test_head_rows_of_many_tokens_without_angles(H, G, d, D, T, dtype):
+    """Queries with bias, norm and factor to a buffer widened with zeros, keys and values into their pages."""
+    o = ops()
+    g = torch.Generator("cuda").manual_seed(T + d)
+    randn = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    raw = randn(T, (H + 2 * G) * d).to(dtype)
+    bias, weight = randn((H + 2 * G) * d), randn(2 * d)
+    W = -(-(T + 5) // 64)
+    table = torch.randperm(W + 2, generator=torch.Generator().manual_seed(T))[:W].to(torch.int32).view(1, W).cuda()
+    positions = torch.arange(5, T + 5, dtype=torch.int32, device="cuda")
+    k_pool, v_pool = (torch.full(s, 3.0, dtype=dtype, device="cuda") for s in ((W + 2, G, 64, D), (W + 2, G, D, 64)))
+    seg = o.head_row_segment
+    segments = o.head_row_segments(seg(0, H, d, 0, D, 0, True, 0, 0.25), seg(H * d, G, d, 0, D, H * d, True, d, target=o.TO_CACHE_KEYS),
+                                   seg((H + G) * d, G, d, 0, D, (H + G) * d, False, -1, target=o.TO_CACHE_VALUES))
+    dst = torch.full((T, H * D), 5.0, dtype=dtype, device="cuda")
+    o.head_rows(raw, dst, segments, 1e-6, bias, weight, cache=(positions, torch.zeros_like(positions), table, k_pool, v_pool))
+    z = raw.double() + bias.double()
+    unit = lambda r: r / torch.sqrt((r * r).mean(-1, keepdim=True) + 1e-6)
+    pad = lambda r: torch.nn.functional.pad(r, (0, D - d))
+    q = pad(unit(z[:, :H * d].view(T, H, d)) * weight[:d].double() * 0.25).reshape(T, -1)
+    k = pad(unit(z[:, H * d:(H + G) * d].view(T, G, d)) * weight[d:].double())
+    v = pad(z[:, (H + G) * d:].view(T, G, d))
+    page, at = table[0].long()[positions.long() // 64], positions.long() % 64
+    tol = dict(rtol=2.0 ** -8, atol=1e-6) if dtype == torch.bfloat16 else dict(rtol=2e-6, atol=2e-6)
+    torch.testing.assert_close(dst.double(), q, **tol)
+    torch.testing.assert_close(k_pool[page, :, at].double(), k, **tol)
+    torch.testing.assert_close(v_pool[page, :, :, at].double(), v, **tol)
+    untouched = torch.ones(W + 2, 64, dtype=torch.bool, device="cuda")
+    untouched[page, at] = False
+    assert bool((k_pool.permute(0, 2, 1, 3)[untouched] == 3.0).all()) and bool((v_pool.permute(0, 3, 1, 2)[untouched] == 3.0).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32], ids=["bf16", "f32"])
+@pytest.mark.parametrize("H, d, T", [(32, 64, 257), (3, 128, 2731), (5, 32, 1639)])
+@pytest.mark.parametrize("activation, gate_first, per_row", [("sigmoid", False, False), ("silu", True, True)])
+def test_gated_norm_of_many_rows(H, d, T, dtype, activation, gate_first, per_row):
+    o = ops()
+    g = torch.Generator("cuda").manual_seed(T + d)
+    randn = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    x, w, wide = randn(T, H * d), randn(H * d if per_row else d), randn(T, H * d + 16).to(dtype)
+    gate, out = wide[:, 8:8 + H * d], torch.zeros(T, H * d + 8, dtype=dtype, device="cuda")
+    o.gated_rmsnorm(x, w, gate, out[:, :H * d], H, d, 1e-5, activation, gate_first, 0.5)
+    z = gate.double().view(T, H, d)
+    act = torch.sigmoid(z) if activation == "sigmoid" else z * torch.sigmoid(z)
+    v = x.double().view(T, H, d) * (act if gate_first else 1.0)
+    want = v * torch.rsqrt((v * v).mean(-1, keepdim=True) + 1e-5) * w.double().view(H if per_row else 1, d) * 0.5 * (1.0 if gate_first else act)
+    tol = dict(rtol=2.0 ** -8, atol=1e-6) if dtype == torch.bfloat16 else dict(rtol=3e-6, atol=1e-6)
+    torch.testing.assert_close(out[:, :H * d].double(), want.reshape(T, -1), **tol)
+    assert not out[:, H * d:].any()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("T, start, window, chunk", [(1024, 0, 100, 0), (1300, 77, 256, 0), (1025, 0, 1, 0), (2000, 3, 1000, 0), (1100, 60, 0, 300),
+                                                     (1024, 0, 0, 128), (1500, 0, 4000, 0), (1400, 129, 129, 0)])
+def test_windows_over_pairs_of_tiles(D, T, start, window, chunk):
+    """Enough tiles that the kernel over pairs takes them: windows and runs of positions that begin and end anywhere in a block,
+    shorter than a tile and longer than the sequence."""
+    o = ops()
+    H, G = 40, 8
+    g = torch.Generator("cuda").manual_seed(T + window + chunk)
+    kv = start + T
+    W = -(-kv // 64)
+    table = torch.randperm(W + 2, generator=torch.Generator().manual_seed(T))[:W].to(torch.int32).view(1, W).cuda()
+    randn = lambda *s: torch.randn(*s, generator=g, device="cuda").to(torch.bfloat16)
+    q, k_pool, v_pool = randn(T, H * D), randn(W + 2, G, 64, D), randn(W + 2, G, D, 64)
+    cu, kl = torch.tensor([0, T], dtype=torch.int32, device="cuda"), torch.tensor([kv], dtype=torch.int32, device="cuda")
+    out = torch.empty(T, H * D, dtype=torch.bfloat16, device="cuda")
+    assert o.attention_prefill_tc(q, H * D, out, cu, kl, table, k_pool, v_pool, 1, T, H, G, D, window, chunk=chunk)
+    assert o.attention_prefill_tc_status() == 0
+    k = k_pool[table[0].long()].permute(1, 0, 2, 3).reshape(G, W * 64, D)[:, :kv].double()
+    v = v_pool[table[0].long()].permute(1, 0, 3, 2).reshape(G, W * 64, D)[:, :kv].double()
+    pos, key = torch.arange(start, kv, device="cuda")[:, None], torch.arange(kv, device="cuda")[None]
+    hidden = (key > pos) | ((key < pos - pos % chunk) if chunk else (key <= pos - window))
+    want = torch.empty(T, H, D, dtype=torch.float64, device="cuda")
+    for h in range(H):
+        s = (q[:, h * D:(h + 1) * D].double() @ k[h // 5].T / math.sqrt(D)).masked_fill(hidden, -math.inf)
+        want[:, h] = s.softmax(-1) @ v[h // 5]
+    # probabilities and results rounded to bfloat16: 2^-9 each of the values' unit spread, a little more where few keys are seen
+    torch.testing.assert_close(out.double(), want.reshape(T, -1), rtol=2.0 ** -7, atol=2.0 ** -7)
