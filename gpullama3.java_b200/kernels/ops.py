@@ -142,6 +142,9 @@ _SIGNATURES = {
     "b200_moe_group": ("moe", [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p]),
     "b200_moe_gather": ("moe", [c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int]),
     "b200_moe_combine": ("moe", [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int]),
+    "b200_delta_rule_step": ("delta_rule", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p,
+                                            ctypes.c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
+                                            c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int]),
     "b200_differential_heads": ("elementwise", [c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                                                 c_float, c_float, c_float]),
     "b200_gated_norm_step": ("gated_residual", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -1743,3 +1746,26 @@ def moe_combine(o: torch.Tensor, place: torch.Tensor, weights: torch.Tensor, res
     assert o.shape[0] == T * top and o.shape[1] == residual.shape[1] and residual.shape[0] == T
     _check(_fn("b200_moe_combine")(o.data_ptr(), place.data_ptr(), weights.data_ptr(), residual.data_ptr(), T,
                                    residual.shape[1], top, _stream()), "moe_combine")
+def delta_rule_step(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor,
+                    state: torch.Tensor, slots: torch.Tensor, norm_weight: torch.Tensor, gate: torch.Tensor, out: torch.Tensor, heads: int,
+                    kv_heads: int, d_k: int, d_v: int, q_scale: float, unit_eps: float, eps: float, decay_per_head: bool = False,
+                    activation: str = "sigmoid") -> bool:
+    """``delta_rule_scan`` of one token per sequence and ``gated_rmsnorm`` of its results, out [T, heads d_v] of qkv's type, in one
+    launch.  Returns False, having done nothing, for sizes it does not take (heads other than 64 by 64)."""
+    if d_k != 64 or d_v != 64:
+        return False
+    _dev(qkv, beta, decay, dt_bias, a_log, state, slots, norm_weight, gate, out)
+    T = qkv.shape[0]
+    assert slots.numel() == T == out.shape[0] == gate.shape[0] and out.shape[1] == heads * d_v and out.stride(1) == gate.stride(1) == 1
+    assert qkv.dtype == beta.dtype == decay.dtype == gate.dtype == out.dtype and qkv.stride(1) == beta.stride(1) == decay.stride(1) == 1
+    assert dt_bias.dtype == a_log.dtype == state.dtype == norm_weight.dtype == torch.float32 and norm_weight.numel() == d_v
+    assert dt_bias.numel() == (heads if decay_per_head else heads * d_k) and a_log.numel() == heads and state.stride(1) == 1
+    assert decay.shape[1] >= (heads if decay_per_head else heads * d_k) and state.shape[1] >= heads * d_k * d_v and gate.shape[1] >= heads * d_v
+    _check(_fn("b200_delta_rule_step")(
+        qkv.data_ptr(), qkv.stride(0), beta.data_ptr(), beta.stride(0), decay.data_ptr(), decay.stride(0), dtype_code(qkv.dtype),
+        dt_bias.data_ptr(), a_log.data_ptr(), state.data_ptr(), state.stride(0), slots.data_ptr(), norm_weight.data_ptr(), gate.data_ptr(),
+        gate.stride(0), out.data_ptr(), out.stride(0), T, heads, kv_heads, d_k, d_v, float(q_scale), float(unit_eps), float(eps),
+        1 if decay_per_head else 0, GATE_ACTIVATIONS[activation], _stream()), "delta_rule_step")
+    return True
+
+

@@ -101,10 +101,13 @@ class ChannelDeltaRule(Mixer):
                              ctx.cu_seqlens, qkv, self.channels, update_state=writes_cache)
         decay = self.a2.store(proj[:, self.a1_off:self.a1_off + self.decay_rank], ctx.dtype, ctx.empty, scratch_of(ctx))   # [T, H dk]
         gate = self.g2.store(proj[:, self.g1_off:self.g1_off + self.gate_rank], ctx.dtype, ctx.empty, scratch_of(ctx))     # [T, H dv]
+        gated = ctx.empty((T, H * dv), ctx.dtype)
+        if ctx.all_decode and ops.delta_rule_step(qkv, proj[:, self.beta_off:], decay, self.dt_bias, self.a_log, state, ctx.slots_dev,
+                                                  self.norm_weight, gate, gated, H, G, dk, dv, dk ** -0.5, self.unit_eps, self.norm_eps):
+            return self.o.add_to(gated, residual, then_norm, scratch_of(ctx))
         o = ctx.empty((T, H * dv), torch.float32)
         ops.delta_rule_scan(qkv, proj[:, self.beta_off:], decay, self.dt_bias, self.a_log, state, ctx.slots_dev,
                             ctx.cu_seqlens, o, H, G, dk, dv, dk ** -0.5, self.unit_eps, alloc=ctx.empty, longest=ctx.max_q_len)
-        gated = ctx.empty((T, H * dv), ctx.dtype)
         ops.gated_rmsnorm(o, self.norm_weight, gate, gated, H, dv, self.norm_eps)
         return self.o.add_to(gated, residual, then_norm, scratch_of(ctx))
 
@@ -182,12 +185,16 @@ class HeadDeltaRule(Mixer):
         qkv = ctx.empty((T, self.channels), ctx.dtype)
         ops.causal_conv_silu(proj, self.conv_weight, state[:, self.state_floats:], ctx.slots_dev, ctx.seq_ids,
                              ctx.cu_seqlens, qkv, self.channels, update_state=writes_cache)
+        gated, gate = ctx.empty((T, H * dv), ctx.dtype), proj[:, self.gate_off:]
+        if ctx.all_decode and ops.delta_rule_step(qkv, proj[:, self.beta_off:], proj[:, self.decay_off:], self.dt_bias, self.a_log, state,
+                                                  ctx.slots_dev, self.norm_weight, gate, gated, H, G, dk, dv, dk ** -0.5, self.unit_eps,
+                                                  self.norm_eps, True, self.gate_activation):
+            return self.o.add_to(gated, residual, then_norm, scratch_of(ctx))
         o = ctx.empty((T, H * dv), torch.float32)
         ops.delta_rule_scan(qkv, proj[:, self.beta_off:], proj[:, self.decay_off:], self.dt_bias, self.a_log, state,
                             ctx.slots_dev, ctx.cu_seqlens, o, H, G, dk, dv, dk ** -0.5, self.unit_eps, alloc=ctx.empty,
                             decay_per_head=True, longest=ctx.max_q_len)
-        gated = ctx.empty((T, H * dv), ctx.dtype)
-        ops.gated_rmsnorm(o, self.norm_weight, proj[:, self.gate_off:], gated, H, dv, self.norm_eps, self.gate_activation)
+        ops.gated_rmsnorm(o, self.norm_weight, gate, gated, H, dv, self.norm_eps, self.gate_activation)
         return self.o.add_to(gated, residual, then_norm, scratch_of(ctx))
 
 
