@@ -171,7 +171,7 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride, _
                         const int* __restrict__ kv_lens, const int* __restrict__ page_table, int table_stride,
                         __nv_bfloat16* __restrict__ k_pool, __nv_bfloat16* __restrict__ v_pool,
                         float* __restrict__ part_o, float* __restrict__ part_ml, int n_heads, int n_kv_heads,
-                        int window, int n_splits, RopeArgs rope, DecodeTerms given) {
+                        int window, int n_splits, RopeArgs rope, DecodeTerms given, int pool_heads) {
     constexpr int D = KB * 32;
     const DecodeTerms terms = TERMS ? given : DecodeTerms{0, 0, nullptr, nullptr, nullptr, 0, 0.f};
     constexpr int NJ = D / 8;  // output tiles of 8 dims
@@ -219,8 +219,9 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride, _
     const int blk_end = min(blk_begin + per_split, n_blocks);
     auto block_of = [&](int v) { return v < kept_blocks ? v : v + shift; };
     const int* pages = page_table + (size_t)seq * table_stride;
-    const size_t page_stride = (size_t)n_kv_heads * kPageTokens * D;
-    const size_t head_off = (size_t)kvh * kPageTokens * D;
+    // (a cache of fewer kv heads than the queries are grouped by: groups pool_heads apart share one)
+    const size_t page_stride = (size_t)pool_heads * kPageTokens * D;
+    const size_t head_off = (size_t)(kvh % pool_heads) * kPageTokens * D;
 
     const int first_page = blk_begin + warp < blk_end ? pages[block_of(blk_begin + warp) * 32 / kPageTokens] : 0;
     if (FUSED) {
@@ -615,12 +616,14 @@ static int launch_attention_decode(const void* q, int q_row_stride, void* out, c
                                    int table_stride, void* k_pool, void* v_pool, float* scratch, long long scratch_floats,
                                    int n_seqs, int n_heads, int n_kv_heads, int head_dim, int window, int n_splits,
                                    bool fused, RopeArgs rope, bool early_start, cudaStream_t stream,
-                                   DecodeTerms terms = DecodeTerms{0, 0, nullptr, nullptr, nullptr, 0, 0.f}) {
+                                   DecodeTerms terms = DecodeTerms{0, 0, nullptr, nullptr, nullptr, 0, 0.f}, int pool_heads = 0) {
     if (n_seqs <= 0) return 0;
     if (!(terms.softcap >= 0.f)) return kErrBadArgument;
     if (terms.keep_first < 0 || (terms.keep_first > 0 && window <= 0)) return kErrBadArgument;
     if (terms.chunk < 0 || (terms.chunk > 0 && (window > 0 || terms.keep_first > 0))) return kErrBadArgument;
     if (n_kv_heads <= 0 || n_heads % n_kv_heads != 0 || n_splits < 1) return kErrBadArgument;
+    if (pool_heads == 0) pool_heads = n_kv_heads;
+    if (pool_heads < 0 || n_kv_heads % pool_heads != 0) return kErrBadArgument;
     const int group = n_heads / n_kv_heads;
     if (group > 16 || head_dim % 32 != 0 || head_dim < 32 || head_dim > 128 || q_row_stride % 8 != 0) return kErrUnsupportedSize;
     if (n_seqs > 65535 || n_kv_heads > 65535) return kErrUnsupportedSize;
@@ -640,14 +643,14 @@ static int launch_attention_decode(const void* q, int q_row_stride, void* out, c
     auto vv = (__nv_bfloat16*)v_pool;
     auto oo = (__nv_bfloat16*)out;
     int st = 0;
-    const bool any_term = terms.keep_first > 0 || terms.chunk > 0 || terms.slopes || terms.sinks || terms.gate || terms.softcap > 0.f;
-    if (any_term && fused) return kErrBadArgument;   // (the fused variant is not built with the terms)
-#define B200_LAUNCH(KB, F) do { if (group > 8) B200_LAUNCH_T(KB, F, true); else B200_LAUNCH_T(KB, F, false); } while (0)
     // Steps of more than 16 sequences run between products that keep nearly all of an SM's memory as shared memory (8B shape, 64
     // sequences of 512 keys: 5.42 -> 4.88 ms a step); up to 16 the products stream through L1 as this kernel does.
     LaunchForm form;
     form.early_start = early_start;
     if (n_seqs > 16 && group <= 8) form.shared_percent = kStreamingSharedPercent;
+    const bool any_term = terms.keep_first > 0 || terms.chunk > 0 || terms.slopes || terms.sinks || terms.gate || terms.softcap > 0.f;
+    if (any_term && fused) return kErrBadArgument;   // (the fused variant is not built with the terms)
+#define B200_LAUNCH(KB, F) do { if (group > 8) B200_LAUNCH_T(KB, F, true); else B200_LAUNCH_T(KB, F, false); } while (0)
 #define B200_LAUNCH_T(KB, F, HI) do { if (!F && any_term) B200_LAUNCH_H(KB, F, HI, !F); else B200_LAUNCH_H(KB, F, HI, false); } while (0)
 #define B200_LAUNCH_H(KB, F, HI, TM)                                                                                \
     do {                                                                                                            \
@@ -662,7 +665,7 @@ static int launch_attention_decode(const void* q, int q_row_stride, void* out, c
         }                                                                                                           \
         st = launch_pdl_as(kernel, grid, dim3(kAttnDecodeThreads), smem, stream, form, qq,                              \
                                 q_row_stride, oo, kv_lens, page_table, table_stride, kk, vv, part_o, part_ml, n_heads,  \
-                                n_kv_heads, window, n_splits, rope, terms);                                          \
+                                n_kv_heads, window, n_splits, rope, terms, pool_heads);                                          \
     } while (0)
 #define B200_PICK(KB) do { if (fused) B200_LAUNCH(KB, true); else B200_LAUNCH(KB, false); } while (0)
     switch (head_dim / 32) {
@@ -738,6 +741,22 @@ extern "C" int b200_attention_decode_terms(const void* q, int q_row_stride, void
                                          const_cast<void*>(v_pool), scratch, scratch_floats, n_seqs, n_heads, n_kv_heads,
                                          head_dim, window, n_splits, false, b200::RopeArgs{nullptr, 0, 0}, early_start != 0, stream,
                                          b200::DecodeTerms{keep_first, chunk, slopes, sinks, (const __nv_bfloat16*)gate, ld_gate, softcap});
+}
+
+// The same for more query heads to a key/value head than the kernel's 16: the pools hold `pool_heads` kv heads, and the queries
+// come in n_kv_heads groups, group i over kv head i % pool_heads (n_kv_heads a multiple of pool_heads).
+extern "C" int b200_attention_decode_shared(const void* q, int q_row_stride, void* out, const int* kv_lens,
+                                            const int* page_table, int table_stride, const void* k_pool, const void* v_pool,
+                                            float* scratch, long long scratch_floats, int n_seqs, int n_heads, int n_kv_heads,
+                                            int pool_heads, int head_dim, int window, int n_splits, int early_start, int keep_first,
+                                            int chunk, const float* slopes, const float* sinks, const void* gate, int ld_gate,
+                                            float softcap, cudaStream_t stream) {
+    if (pool_heads <= 0) return b200::kErrBadArgument;
+    return b200::launch_attention_decode(q, q_row_stride, out, kv_lens, page_table, table_stride, const_cast<void*>(k_pool),
+                                         const_cast<void*>(v_pool), scratch, scratch_floats, n_seqs, n_heads, n_kv_heads,
+                                         head_dim, window, n_splits, false, b200::RopeArgs{nullptr, 0, 0}, early_start != 0, stream,
+                                         b200::DecodeTerms{keep_first, chunk, slopes, sinks, (const __nv_bfloat16*)gate, ld_gate, softcap},
+                                         pool_heads);
 }
 
 // The fused variant: `qkv` holds the step's raw projections [n_seqs, (n_heads + 2 n_kv_heads) head_dim]; queries

@@ -79,6 +79,10 @@ _SIGNATURES = {
     "b200_attention_decode_rope": ("attention_decode", [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
                                                         c_void_p, c_void_p, ctypes.c_longlong, c_int, c_int, c_int,
                                                         c_int, c_int, c_int, c_void_p, c_int, c_int, c_int]),
+    "b200_attention_decode_shared": ("attention_decode", [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
+                                                          c_void_p, c_void_p, ctypes.c_longlong, c_int, c_int, c_int, c_int,
+                                                          c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
+                                                          c_int, c_float]),
     "b200_attention_prefill_f32": ("attention_prefill_f32", [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
                                                              c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                                                              c_void_p, c_void_p, c_void_p, c_int, c_float, c_int, c_int, c_void_p]),
@@ -877,11 +881,12 @@ def attention_decode(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, kv_l
                      n_kv_heads: int, head_dim: int, window: int, n_splits: int,
                      scratch: torch.Tensor | None = None, early_start: bool = True, *, keep_first: int = 0, chunk: int = 0,
                      slopes: torch.Tensor | None = None, sinks: torch.Tensor | None = None,
-                     gate: torch.Tensor | None = None, softcap: float = 0.0) -> None:
+                     gate: torch.Tensor | None = None, softcap: float = 0.0, pool_heads: int | None = None) -> None:
     """One query token per sequence (row i of q belongs to sequence i) over kv_lens[i] cached keys.
     ``scratch``: float32 workspace for the spans' partial results (allocated here when absent).
     ``early_start``: see ``attention_decode_early_start``.  ``keep_first``, ``chunk``, ``slopes``, ``sinks``, ``gate``,
-    ``softcap``: as for ``attention_paged``."""
+    ``softcap``: as for ``attention_paged``.  ``pool_heads``: the kv heads of the pools, where the queries' ``n_kv_heads`` groups
+    share them (group i reads kv head i % pool_heads)."""
     _dev(q, out, kv_lens, page_table, k_pool, v_pool)
     n_seqs = out.shape[0]
     assert q.dtype == out.dtype == k_pool.dtype == torch.bfloat16 and out.is_contiguous()
@@ -946,8 +951,9 @@ def attention_prefill_tc(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, 
     assert gate is None or (gate.dtype == torch.bfloat16 and gate.stride(1) == 1 and gate.shape[1] >= n_heads)
     assert sinks is None or (sinks.dtype == torch.float32 and sinks.is_contiguous() and sinks.numel() == n_heads)
     assert out.dtype == k_pool.dtype == torch.bfloat16 and out.is_contiguous() and k_pool.is_contiguous()
-    assert tuple(k_pool.shape[1:]) == (n_kv_heads, PAGE_TOKENS, head_dim)
-    assert tuple(v_pool.shape[1:]) == (n_kv_heads, head_dim, PAGE_TOKENS)
+    kept_heads = n_kv_heads if pool_heads is None else pool_heads
+    assert tuple(k_pool.shape[1:]) == (kept_heads, PAGE_TOKENS, head_dim) and n_kv_heads % kept_heads == 0
+    assert tuple(v_pool.shape[1:]) == (kept_heads, head_dim, PAGE_TOKENS)
     _check(_fn("b200_attention_prefill_tc")(
         q.data_ptr(), q_row_stride, out.shape[0], out.data_ptr(), cu_seqlens.data_ptr(), kv_lens.data_ptr(),
         page_table.data_ptr(), page_table.shape[1], k_pool.data_ptr(), v_pool.data_ptr(), k_pool.shape[0], n_seqs,
@@ -974,6 +980,19 @@ def random_fill(out: torch.Tensor, key: int, scale: float, offset: float) -> Non
 
 
 # --------------------------------------------------------------------------- sampling
+    if kept_heads != n_kv_heads:
+        _dev(slopes, sinks, gate)
+        for t in (slopes, sinks):
+            assert t is None or (t.dtype == torch.float32 and t.is_contiguous() and t.numel() == n_heads)
+        assert gate is None or (gate.dtype == torch.bfloat16 and gate.stride(1) == 1 and gate.shape[1] >= n_heads)
+        ptr = lambda t: t.data_ptr() if t is not None else None
+        _check(_fn("b200_attention_decode_shared")(
+            q.data_ptr(), q_row_stride, out.data_ptr(), kv_lens.data_ptr(), page_table.data_ptr(), page_table.shape[1],
+            k_pool.data_ptr(), v_pool.data_ptr(), scratch.data_ptr() if need else None, scratch.numel() if need else 0,
+            n_seqs, n_heads, n_kv_heads, kept_heads, head_dim, int(window), n_splits, 1 if early_start else 0, int(keep_first), int(chunk),
+            ptr(slopes), ptr(sinks), ptr(gate), gate.stride(0) if gate is not None else 0, float(softcap), _stream()),
+            "attention_decode" if early_start else "attention_decode:late")
+        return
 def argmax_rows(logits: torch.Tensor, out: torch.Tensor) -> None:
     """out[r] = index of the first maximum of logits[r] (float32 [R, V]); out int32 [R]."""
     _dev(logits, out)

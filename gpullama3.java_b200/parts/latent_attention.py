@@ -98,13 +98,13 @@ class LatentAttention(Mixer, OpenEnded):
     def cache_need(self):
         return KVCacheNeed(1, self.head_dim, self.window)
 
-    def plan_decode(self, ctx: StepContext, cache: KVView) -> tuple[int, bool]:
+    def plan_decode(self, ctx: StepContext, cache: KVView, groups: int = 1) -> tuple[int, bool]:
         capacity = ctx.capacity(cache.group)
         if self.window:
             capacity = min(capacity, self.window)
         resident = ops.resident_ctas(ctx.device, self.head_dim, min(self.n_heads, self.DECODE_GROUP))
-        splits = ops.attention_decode_splits(ctx.n_seqs, 1, capacity, resident)
-        return splits, ops.attention_decode_early_start(ctx.n_seqs, 1, capacity, splits)
+        splits = ops.attention_decode_splits(ctx.n_seqs, groups, capacity, resident)
+        return splits, ops.attention_decode_early_start(ctx.n_seqs, groups, capacity, splits)
 
     def load(self, tensors, dtype, device):
         H, dk, dv, R, D, dr = self.n_heads, self.key_dim, self.value_dim, self.kv_rank, self.head_dim, self.rot_dim
@@ -199,9 +199,17 @@ class LatentAttention(Mixer, OpenEnded):
         carried = ctx.empty((T, H * D), ctx.dtype)                            # queries in the latent space
         ops.gemm_per_head(q, self.carry_in, carried)
         gate = raw[:, self.gate_at:self.gate_at + H] if self.head_gate else None
-        if ctx.all_decode and H > self.DECODE_GROUP and ops.attention_decode_supported(ctx.dtype, self.DECODE_GROUP, 1, D):
-            # the decode kernel takes up to DECODE_GROUP query heads per key/value head: the heads go in groups, each
-            # group over the same cached latents
+        groups = -(-H // self.DECODE_GROUP)
+        grouped = ctx.all_decode and groups > 1 and ops.attention_decode_supported(ctx.dtype, self.DECODE_GROUP, 1, D)
+        # the decode kernel takes up to DECODE_GROUP query heads per key/value head: the heads go in groups, each
+        # group over the same cached latents; equal groups in one launch
+        if grouped and H % self.DECODE_GROUP == 0:
+            splits, early = self.plan_decode(ctx, cache, groups)
+            out = ctx.empty((T, H * D), ctx.dtype)
+            ops.attention_decode(carried, carried.stride(0), out, ctx.kv_lens, table, cache.k, cache.v, H, groups, D, self.window or 0,
+                                 splits, early_start=early, sinks=self.sinks if self.sink else None, gate=gate, pool_heads=1)
+            ops.gemm_per_head(out, self.carry_out, rows)
+        elif grouped:
             splits, early = self.plan_decode(ctx, cache)
             for g in range(0, H, self.DECODE_GROUP):
                 n = min(self.DECODE_GROUP, H - g)
