@@ -76,13 +76,13 @@ _SIGNATURES = {
     "b200_attention_prefill": ("attention_prefill", [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                                                      c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                                                      c_int, c_void_p, c_void_p, c_void_p, c_int, c_float]),
-    "b200_attention_decode_rope": ("attention_decode", [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
-                                                        c_void_p, c_void_p, ctypes.c_longlong, c_int, c_int, c_int,
-                                                        c_int, c_int, c_int, c_void_p, c_int, c_int, c_int]),
     "b200_attention_decode_shared": ("attention_decode", [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
                                                           c_void_p, c_void_p, ctypes.c_longlong, c_int, c_int, c_int, c_int,
                                                           c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
                                                           c_int, c_float]),
+    "b200_attention_decode_rope": ("attention_decode", [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
+                                                        c_void_p, c_void_p, ctypes.c_longlong, c_int, c_int, c_int,
+                                                        c_int, c_int, c_int, c_void_p, c_int, c_int, c_int]),
     "b200_attention_prefill_f32": ("attention_prefill_f32", [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
                                                              c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                                                              c_void_p, c_void_p, c_void_p, c_int, c_float, c_int, c_int, c_void_p]),
@@ -136,6 +136,9 @@ _SIGNATURES = {
     "b200_layernorm": ("norm", [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_float]),
     "b200_causal_conv_silu": ("delta_rule", [c_void_p, c_int, c_void_p, c_void_p, ctypes.c_longlong, c_void_p, c_void_p,
                                              c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int]),
+    "b200_delta_rule_step": ("delta_rule", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p,
+                                            ctypes.c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
+                                            c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int]),
     "b200_delta_rule_scan": ("delta_rule", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                                             ctypes.c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
                                             c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_int]),
@@ -146,9 +149,6 @@ _SIGNATURES = {
     "b200_moe_group": ("moe", [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p]),
     "b200_moe_gather": ("moe", [c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int]),
     "b200_moe_combine": ("moe", [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int]),
-    "b200_delta_rule_step": ("delta_rule", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p,
-                                            ctypes.c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
-                                            c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int]),
     "b200_differential_heads": ("elementwise", [c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                                                 c_float, c_float, c_float]),
     "b200_gated_norm_step": ("gated_residual", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -890,11 +890,25 @@ def attention_decode(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, kv_l
     _dev(q, out, kv_lens, page_table, k_pool, v_pool)
     n_seqs = out.shape[0]
     assert q.dtype == out.dtype == k_pool.dtype == torch.bfloat16 and out.is_contiguous()
-    assert tuple(k_pool.shape[1:]) == (n_kv_heads, PAGE_TOKENS, head_dim)
-    assert tuple(v_pool.shape[1:]) == (n_kv_heads, head_dim, PAGE_TOKENS)
+    kept_heads = n_kv_heads if pool_heads is None else pool_heads
+    assert tuple(k_pool.shape[1:]) == (kept_heads, PAGE_TOKENS, head_dim) and n_kv_heads % kept_heads == 0
+    assert tuple(v_pool.shape[1:]) == (kept_heads, head_dim, PAGE_TOKENS)
     need = n_seqs * n_heads * n_splits * (head_dim + 2) if n_splits > 1 else 0
     if need and (scratch is None or scratch.numel() < need):
         scratch = torch.empty(need, dtype=torch.float32, device=q.device)
+    if kept_heads != n_kv_heads:
+        _dev(slopes, sinks, gate)
+        for t in (slopes, sinks):
+            assert t is None or (t.dtype == torch.float32 and t.is_contiguous() and t.numel() == n_heads)
+        assert gate is None or (gate.dtype == torch.bfloat16 and gate.stride(1) == 1 and gate.shape[1] >= n_heads)
+        ptr = lambda t: t.data_ptr() if t is not None else None
+        _check(_fn("b200_attention_decode_shared")(
+            q.data_ptr(), q_row_stride, out.data_ptr(), kv_lens.data_ptr(), page_table.data_ptr(), page_table.shape[1],
+            k_pool.data_ptr(), v_pool.data_ptr(), scratch.data_ptr() if need else None, scratch.numel() if need else 0,
+            n_seqs, n_heads, n_kv_heads, kept_heads, head_dim, int(window), n_splits, 1 if early_start else 0, int(keep_first), int(chunk),
+            ptr(slopes), ptr(sinks), ptr(gate), gate.stride(0) if gate is not None else 0, float(softcap), _stream()),
+            "attention_decode" if early_start else "attention_decode:late")
+        return
     if keep_first or chunk or slopes is not None or sinks is not None or gate is not None or softcap:
         _dev(slopes, sinks, gate)
         for t in (slopes, sinks):
@@ -951,9 +965,8 @@ def attention_prefill_tc(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, 
     assert gate is None or (gate.dtype == torch.bfloat16 and gate.stride(1) == 1 and gate.shape[1] >= n_heads)
     assert sinks is None or (sinks.dtype == torch.float32 and sinks.is_contiguous() and sinks.numel() == n_heads)
     assert out.dtype == k_pool.dtype == torch.bfloat16 and out.is_contiguous() and k_pool.is_contiguous()
-    kept_heads = n_kv_heads if pool_heads is None else pool_heads
-    assert tuple(k_pool.shape[1:]) == (kept_heads, PAGE_TOKENS, head_dim) and n_kv_heads % kept_heads == 0
-    assert tuple(v_pool.shape[1:]) == (kept_heads, head_dim, PAGE_TOKENS)
+    assert tuple(k_pool.shape[1:]) == (n_kv_heads, PAGE_TOKENS, head_dim)
+    assert tuple(v_pool.shape[1:]) == (n_kv_heads, head_dim, PAGE_TOKENS)
     _check(_fn("b200_attention_prefill_tc")(
         q.data_ptr(), q_row_stride, out.shape[0], out.data_ptr(), cu_seqlens.data_ptr(), kv_lens.data_ptr(),
         page_table.data_ptr(), page_table.shape[1], k_pool.data_ptr(), v_pool.data_ptr(), k_pool.shape[0], n_seqs,
@@ -980,19 +993,6 @@ def random_fill(out: torch.Tensor, key: int, scale: float, offset: float) -> Non
 
 
 # --------------------------------------------------------------------------- sampling
-    if kept_heads != n_kv_heads:
-        _dev(slopes, sinks, gate)
-        for t in (slopes, sinks):
-            assert t is None or (t.dtype == torch.float32 and t.is_contiguous() and t.numel() == n_heads)
-        assert gate is None or (gate.dtype == torch.bfloat16 and gate.stride(1) == 1 and gate.shape[1] >= n_heads)
-        ptr = lambda t: t.data_ptr() if t is not None else None
-        _check(_fn("b200_attention_decode_shared")(
-            q.data_ptr(), q_row_stride, out.data_ptr(), kv_lens.data_ptr(), page_table.data_ptr(), page_table.shape[1],
-            k_pool.data_ptr(), v_pool.data_ptr(), scratch.data_ptr() if need else None, scratch.numel() if need else 0,
-            n_seqs, n_heads, n_kv_heads, kept_heads, head_dim, int(window), n_splits, 1 if early_start else 0, int(keep_first), int(chunk),
-            ptr(slopes), ptr(sinks), ptr(gate), gate.stride(0) if gate is not None else 0, float(softcap), _stream()),
-            "attention_decode" if early_start else "attention_decode:late")
-        return
 def argmax_rows(logits: torch.Tensor, out: torch.Tensor) -> None:
     """out[r] = index of the first maximum of logits[r] (float32 [R, V]); out int32 [R]."""
     _dev(logits, out)
@@ -1668,6 +1668,29 @@ def delta_rule_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, 
                                        1 if decay_per_head else 0, _stream()), "delta_rule_scan")
 
 
+def delta_rule_step(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor,
+                    state: torch.Tensor, slots: torch.Tensor, norm_weight: torch.Tensor, gate: torch.Tensor, out: torch.Tensor, heads: int,
+                    kv_heads: int, d_k: int, d_v: int, q_scale: float, unit_eps: float, eps: float, decay_per_head: bool = False,
+                    activation: str = "sigmoid") -> bool:
+    """``delta_rule_scan`` of one token per sequence and ``gated_rmsnorm`` of its results, out [T, heads d_v] of qkv's type, in one
+    launch.  Returns False, having done nothing, for sizes it does not take (heads other than 64 by 64)."""
+    if d_k != 64 or d_v != 64:
+        return False
+    _dev(qkv, beta, decay, dt_bias, a_log, state, slots, norm_weight, gate, out)
+    T = qkv.shape[0]
+    assert slots.numel() == T == out.shape[0] == gate.shape[0] and out.shape[1] == heads * d_v and out.stride(1) == gate.stride(1) == 1
+    assert qkv.dtype == beta.dtype == decay.dtype == gate.dtype == out.dtype and qkv.stride(1) == beta.stride(1) == decay.stride(1) == 1
+    assert dt_bias.dtype == a_log.dtype == state.dtype == norm_weight.dtype == torch.float32 and norm_weight.numel() == d_v
+    assert dt_bias.numel() == (heads if decay_per_head else heads * d_k) and a_log.numel() == heads and state.stride(1) == 1
+    assert decay.shape[1] >= (heads if decay_per_head else heads * d_k) and state.shape[1] >= heads * d_k * d_v and gate.shape[1] >= heads * d_v
+    _check(_fn("b200_delta_rule_step")(
+        qkv.data_ptr(), qkv.stride(0), beta.data_ptr(), beta.stride(0), decay.data_ptr(), decay.stride(0), dtype_code(qkv.dtype),
+        dt_bias.data_ptr(), a_log.data_ptr(), state.data_ptr(), state.stride(0), slots.data_ptr(), norm_weight.data_ptr(), gate.data_ptr(),
+        gate.stride(0), out.data_ptr(), out.stride(0), T, heads, kv_heads, d_k, d_v, float(q_scale), float(unit_eps), float(eps),
+        1 if decay_per_head else 0, GATE_ACTIVATIONS[activation], _stream()), "delta_rule_step")
+    return True
+
+
 # --------------------------------------------------------------------------- routed feed-forward (mixture of experts)
 MAX_EXPERTS, MAX_EXPERTS_PER_TOKEN = 1024, 32   # moe.cu
 ROUTER_SCORES = {"softmax": 0, "sigmoid": 1}
@@ -1765,26 +1788,3 @@ def moe_combine(o: torch.Tensor, place: torch.Tensor, weights: torch.Tensor, res
     assert o.shape[0] == T * top and o.shape[1] == residual.shape[1] and residual.shape[0] == T
     _check(_fn("b200_moe_combine")(o.data_ptr(), place.data_ptr(), weights.data_ptr(), residual.data_ptr(), T,
                                    residual.shape[1], top, _stream()), "moe_combine")
-def delta_rule_step(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor,
-                    state: torch.Tensor, slots: torch.Tensor, norm_weight: torch.Tensor, gate: torch.Tensor, out: torch.Tensor, heads: int,
-                    kv_heads: int, d_k: int, d_v: int, q_scale: float, unit_eps: float, eps: float, decay_per_head: bool = False,
-                    activation: str = "sigmoid") -> bool:
-    """``delta_rule_scan`` of one token per sequence and ``gated_rmsnorm`` of its results, out [T, heads d_v] of qkv's type, in one
-    launch.  Returns False, having done nothing, for sizes it does not take (heads other than 64 by 64)."""
-    if d_k != 64 or d_v != 64:
-        return False
-    _dev(qkv, beta, decay, dt_bias, a_log, state, slots, norm_weight, gate, out)
-    T = qkv.shape[0]
-    assert slots.numel() == T == out.shape[0] == gate.shape[0] and out.shape[1] == heads * d_v and out.stride(1) == gate.stride(1) == 1
-    assert qkv.dtype == beta.dtype == decay.dtype == gate.dtype == out.dtype and qkv.stride(1) == beta.stride(1) == decay.stride(1) == 1
-    assert dt_bias.dtype == a_log.dtype == state.dtype == norm_weight.dtype == torch.float32 and norm_weight.numel() == d_v
-    assert dt_bias.numel() == (heads if decay_per_head else heads * d_k) and a_log.numel() == heads and state.stride(1) == 1
-    assert decay.shape[1] >= (heads if decay_per_head else heads * d_k) and state.shape[1] >= heads * d_k * d_v and gate.shape[1] >= heads * d_v
-    _check(_fn("b200_delta_rule_step")(
-        qkv.data_ptr(), qkv.stride(0), beta.data_ptr(), beta.stride(0), decay.data_ptr(), decay.stride(0), dtype_code(qkv.dtype),
-        dt_bias.data_ptr(), a_log.data_ptr(), state.data_ptr(), state.stride(0), slots.data_ptr(), norm_weight.data_ptr(), gate.data_ptr(),
-        gate.stride(0), out.data_ptr(), out.stride(0), T, heads, kv_heads, d_k, d_v, float(q_scale), float(unit_eps), float(eps),
-        1 if decay_per_head else 0, GATE_ACTIVATIONS[activation], _stream()), "delta_rule_step")
-    return True
-
-
