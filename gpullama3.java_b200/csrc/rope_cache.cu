@@ -27,7 +27,7 @@ __global__ void rope_cache_write_kernel(T* __restrict__ qkv, const int* __restri
                                         T* __restrict__ v_pool, int n_heads, int n_kv_heads, int head_dim,
                                         int rotary_dim, int pairing, int write_cache) {
     pdl_launch_dependents();
-    pdl_wait();
+    // positions, sequences and page tables were copied in before the step's first kernel: places and angles are made before the wait
     const int t = blockIdx.x;
     const int pos = positions[t];
     const int q_dim = n_heads * head_dim, kv_dim = n_kv_heads * head_dim;
@@ -46,10 +46,13 @@ __global__ void rope_cache_write_kernel(T* __restrict__ qkv, const int* __restri
     __shared__ float sin_s[kMaxRotaryPairs], cos_s[kMaxRotaryPairs];
     for (int j = threadIdx.x; j < half; j += blockDim.x) sincosf((float)pos * inv_freq[j], &sin_s[j], &cos_s[j]);
     __syncthreads();
+    pdl_wait();
+    // (a token's rows are shared out among gridDim.y CTAs)
+    const int first = (int)(blockIdx.y * blockDim.x + threadIdx.x), step = (int)(gridDim.y * blockDim.x);
 
     // rotated pairs of queries (in place) and keys (into the cache)
     const int n_units = (n_heads + n_kv_heads) * half;
-    for (int u = threadIdx.x; u < n_units; u += blockDim.x) {
+    for (int u = first; u < n_units; u += step) {
         const int h = u / half, j = u % half;
         const int i0 = pairing == 0 ? 2 * j : j;
         const int i1 = pairing == 0 ? 2 * j + 1 : j + half;
@@ -71,11 +74,11 @@ __global__ void rope_cache_write_kernel(T* __restrict__ qkv, const int* __restri
     if (!write_cache) return;
     // unrotated tail of the keys, and the values
     const int tail = head_dim - rotary_dim;
-    for (int u = threadIdx.x; u < n_kv_heads * tail; u += blockDim.x) {
+    for (int u = first; u < n_kv_heads * tail; u += step) {
         const int g = u / tail, d = rotary_dim + u % tail;
         k_pool[cache_base + g * head_stride + d] = row[q_dim + g * head_dim + d];
     }
-    for (int u = threadIdx.x; u < kv_dim; u += blockDim.x) {
+    for (int u = first; u < kv_dim; u += step) {
         const int g = u / head_dim, d = u % head_dim;
         v_pool[v_base + g * head_stride + (size_t)d * kPageTokens] = row[q_dim + kv_dim + u];
     }
@@ -276,8 +279,13 @@ extern "C" int b200_rope_cache_write(void* qkv, int dtype, const int* positions,
                                         (T*)k_pool, (T*)v_pool, n_tokens, n_heads, n_kv_heads, head_dim, pairing, write_cache));
         }
     }
+    // few tokens: a thread per pair, as long as that makes no more CTAs than the GPU holds at once (8 tokens, 40 heads of 64,
+    // float32: 4.8 us with a CTA a token that looked its place up after the wait)
+    const long long pairs = (long long)(n_heads + n_kv_heads) * (rotary_dim / 2);
+    const long long room = 4ll * b200::device_sm_count() / n_tokens, want = (pairs + 255) / 256;
+    const int slices = (int)(room < 1 ? 1 : want < 1 ? 1 : want < room ? want : room);
     B200_DISPATCH_DTYPE(dtype, T,
-        return b200::launch_pdl(b200::rope_cache_write_kernel<T>, dim3(n_tokens), dim3(256), 0, stream, (T*)qkv,
+        return b200::launch_pdl(b200::rope_cache_write_kernel<T>, dim3(n_tokens, slices), dim3(256), 0, stream, (T*)qkv,
                                 positions, seq_ids, page_table, table_stride, inv_freq, (T*)k_pool, (T*)v_pool, n_heads,
                                 n_kv_heads, head_dim, rotary_dim, pairing, write_cache));
     return b200::launch_status();
