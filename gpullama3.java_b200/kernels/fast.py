@@ -42,11 +42,13 @@ def try_projection_with_rope(x: torch.Tensor, w: torch.Tensor, qkv: torch.Tensor
     if (ctx.all_decode or x.dtype != torch.bfloat16 or pos.rotary_dim != mixer.head_dim or mixer.head_dim not in (64, 128)
             or not hasattr(pos, "angles")):
         return False
-    if ops.gemm_tcgen05_k_spans(x.shape[0], w.shape[0], x.shape[1]) != 1:
+    few = 16 < x.shape[0] <= 128
+    whole_k = ops.gemm_tcgen05_k_spans(x.shape[0], w.shape[0], x.shape[1]) == 1
+    if not few and not whole_k:
         return False
-    return ops.gemm_tcgen05_qkv_rope(x, w, qkv, ctx.positions, ctx.seq_ids, page_table, pos.angles(ctx),
-                                     cache.k if writes_cache else None, cache.v if writes_cache else None,
-                                     mixer.n_heads, mixer.n_kv_heads, mixer.head_dim, pos.pairing, writes_cache)
+    operands = (x, w, qkv, ctx.positions, ctx.seq_ids, page_table, pos.angles(ctx), cache.k if writes_cache else None,
+                cache.v if writes_cache else None, mixer.n_heads, mixer.n_kv_heads, mixer.head_dim, pos.pairing, writes_cache)
+    return (few and ops.gemm_skinny_qkv_rope(*operands)) or (whole_k and ops.gemm_tcgen05_qkv_rope(*operands))
 
 
 def try_decode_attention_with_rope(qkv, out, ctx, page_table, cache, mixer, writes_cache: bool) -> bool:

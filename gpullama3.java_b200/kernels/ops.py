@@ -66,6 +66,9 @@ _SIGNATURES = {
     "b200_rope_angles": ("rope_cache", [c_void_p, c_void_p, c_void_p, c_int, c_int]),
     "b200_gemm_skinny": ("gemm_skinny_tcgen05", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int,
                                                  c_int, c_int, c_int]),
+    "b200_gemm_skinny_qkv_rope": ("gemm_skinny_tcgen05", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p,
+                                                          c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int,
+                                                          c_int, c_int, c_int]),
     "b200_attention_decode": ("attention_decode", [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
                                                    c_void_p, c_void_p, ctypes.c_longlong, c_int, c_int, c_int, c_int,
                                                    c_int, c_int, c_int]),
@@ -716,6 +719,19 @@ def gemm_tcgen05_qkv_rope(a: torch.Tensor, w: torch.Tensor, qkv: torch.Tensor, p
     unwritten), rotated keys and the values go to the cache pages of their positions.  ``angles``: ``rope_angles`` of
     the pass.  Returns False, having done nothing, for shapes it does not take (head sizes other than 64 and 128, a
     product of few tiles): the caller then runs the product and ``rope_cache_write``."""
+    return _qkv_rope("gemm_tcgen05_qkv_rope", a, w, qkv, positions, seq_ids, page_table, angles, k_pool, v_pool, n_heads, n_kv_heads,
+                     head_dim, pairing, write_cache)
+
+
+def gemm_skinny_qkv_rope(a, w, qkv, positions, seq_ids, page_table, angles, k_pool, v_pool, n_heads: int, n_kv_heads: int, head_dim: int,
+                         pairing: int, write_cache: bool = True) -> bool:
+    """``gemm_tcgen05_qkv_rope`` for at most 128 tokens, by the few-token product; declines products whose K that does not cut."""
+    return a.shape[0] <= 128 and _qkv_rope("gemm_skinny_qkv_rope", a, w, qkv, positions, seq_ids, page_table, angles, k_pool, v_pool,
+                                           n_heads, n_kv_heads, head_dim, pairing, write_cache)
+
+
+def _qkv_rope(name, a, w, qkv, positions, seq_ids, page_table, angles, k_pool, v_pool, n_heads, n_kv_heads, head_dim, pairing,
+              write_cache) -> bool:
     M, K = a.shape
     N = (n_heads + 2 * n_kv_heads) * head_dim
     if (a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or qkv.dtype != torch.bfloat16 or head_dim not in (64, 128)
@@ -731,14 +747,14 @@ def gemm_tcgen05_qkv_rope(a: torch.Tensor, w: torch.Tensor, qkv: torch.Tensor, p
         assert k_pool.dtype == v_pool.dtype == torch.bfloat16 and k_pool.is_contiguous() and v_pool.is_contiguous()
         assert tuple(k_pool.shape[1:]) == (n_kv_heads, PAGE_TOKENS, head_dim)
         assert tuple(v_pool.shape[1:]) == (n_kv_heads, head_dim, PAGE_TOKENS)
-    status = _fn("b200_gemm_tcgen05_qkv_rope")(
+    status = _fn("b200_" + name)(
         a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), qkv.data_ptr(), qkv.stride(0), M, K, positions.data_ptr(),
         seq_ids.data_ptr(), page_table.data_ptr(), page_table.shape[1], angles.data_ptr(),
         k_pool.data_ptr() if write_cache else None, v_pool.data_ptr() if write_cache else None, n_heads, n_kv_heads,
         head_dim, pairing, 1 if write_cache else 0, _stream())
     if status == _UNSUPPORTED:
         return False
-    _check(status, "gemm_tcgen05_qkv_rope")
+    _check(status, name)
     return True
 
 
