@@ -28,7 +28,9 @@
 // Terms as in the plain kernel (window, chunk, slopes, sinks, gate, softcap; not keep_first).  Values of keys past a
 // sequence's end are read as zeros.  A key that some row of the tile must not see has probability 0 there, and 0 times a value that is
 // not finite is not 0: a page with such keys and such values is summed key by key, over the keys each row sees.
-#include "common.cuh"
+#include <type_traits>
+
+#include "tcgen05.cuh"
 
 namespace b200 {
 
@@ -50,6 +52,7 @@ struct PrefillF32Args {
     float softcap;
     float* part_o;          // with spans: [row][span][D] sums, row = token * n_heads + head
     float* part_ml;         // with spans: [row][span][2] maximum and sum of exponentials
+    const int* only_if;     // a word that must not be 0 for the kernel to do anything (null: no such word)
 };
 
 __device__ __forceinline__ void fma_pair(float2& acc, float ax, float ay, float bx, float by) {
@@ -84,6 +87,7 @@ attention_prefill_f32_kernel(const PrefillF32Args a) {
     const int g = blockIdx.x % a.n_kv_heads, seq = blockIdx.y, group = a.n_heads / a.n_kv_heads;
     pdl_launch_dependents();
     pdl_wait();
+    if (a.only_if != nullptr && *a.only_if == 0) return;
     const int begin = a.cu_seqlens[seq], q_len = a.cu_seqlens[seq + 1] - begin, kv_len = a.kv_lens[seq];
     const int n_rows = q_len * group;
     const int row0 = ((int)gridDim.x / a.n_kv_heads - 1 - (int)blockIdx.x / a.n_kv_heads) * BQ;
@@ -368,6 +372,437 @@ static int prefill_f32_of(const PrefillF32Args& a, int n_seqs, int max_q_len, in
     return kErrBadArgument;
 }
 
+// ---------------------------------------------------------------------------------------------
+// The same on the tensor cores, for prompts (head_dim 64, an even number of query heads to a kv head, causal and nothing more).
+//
+// A float32 number is the sum of three bfloat16 numbers exactly: x0 = bf16(x), x1 = bf16(x - x0), x2 = x - x0 - x1.  A product of
+// two such sums is formed as six of its nine products (those left out are below 2^-24 of it), smallest first, by tcgen05.mma with
+// float32 accumulators.  The accumulators cut off what does not fit where an addition rounds, so sums stay short: a score's over 32
+// dimensions, an output's over 32 keys, two of each added in registers, and a page's output then to its row's with what that rounds
+// off kept (sums of 64: 172 us in place of 240, errors a fifth above the kernel's above).  Keys and values are split once a launch
+// (split_pages_kernel, into scratch memory, values times 2^24 so that the parts of small ones keep their bits), queries by the softmax
+// threads, probabilities in registers.
+// Probabilities are in [0, 1] and keys within the mask only, so numbers of ordinary size are all that occurs; a query or key of 2^60 or
+// more, a value of 2^100 or more, or one that is not finite raises a flag, and the kernel above then does the launch over.
+//
+// A CTA owns two tiles of 128 rows, the same tokens of two neighbouring heads, so that a page's parts serve both; warps 0 to 3 and 4
+// to 7 are their softmax threads (a row each), one warp fetches, one issues each tile's products.  A tile's next scores are formed
+// behind its outputs' products, while the other's softmax runs.  CTAs take tiles from a list by falling number, forwards and backwards
+// in turn.
+// Bound by the chain from a page's scores over its softmax to its outputs, 7 us a page with two tiles taking turns.  2,048 tokens, 32 heads
+// of 64: 577 us with multiply-adds, 240 so, at the same error (1.32e-7 and 1.33e-7 of the norm; peaked scores 3.16e-7 and 2.70e-7, 200
+// tokens behind 1,600 1.67e-7 and 1.63e-7).
+constexpr int kTcRows = 128, kTcD = 64, kTcStages = 2, kTcThreads = 384;
+constexpr int kTcTmaWarp = 8, kTcMmaWarp0 = 9, kTcMmaWarp1 = 10, kTcFlagWarp = 11;
+constexpr int kTcRegsIssuers = 40, kTcRegsSoftmax = 232;   // 128 x 40 + 256 x 232 = 64,512 = 384 x 168, the launch's registers
+constexpr int kTcPart = kPageTokens * kTcD;                // elements of one part of a page's keys or values
+constexpr float kTcValueScale = 16777216.f;                // 2^24
+
+__device__ int g_f32_tc_status = 0;
+
+struct TcF32Args {
+    PrefillF32Args f;
+    __nv_bfloat16* parts;   // [2: keys, values][slot][kv head][3][64][64]; slot = sequence * table_stride + page of the sequence
+    int* flags;             // [0]: raised, [1 ..]: per (sequence, page, kv head) of the split
+    int n_seqs, n_tiles, n_split;
+};
+
+struct TcF32Smem {
+    alignas(1024) __nv_bfloat16 q[2][3][kTcRows * kTcD];
+    alignas(1024) __nv_bfloat16 k[kTcStages][3][kTcPart];
+    alignas(1024) __nv_bfloat16 v[kTcStages][3][kTcPart];
+    alignas(8) uint64_t k_full[kTcStages];
+    uint64_t k_empty[kTcStages], v_full[kTcStages], v_empty[kTcStages];
+    uint64_t q_full[2], s_full[2], p_full[2], pv_done[2];
+    uint32_t tmem_base;
+    int abort_flag;
+    float rest[2][32][kTcRows];   // what additions into the outputs' last 32 dimensions have rounded off
+};
+
+// a number as the sum of three bfloat16 numbers
+__device__ __forceinline__ void split3(float x, float& a, float& b, float& c) {
+    a = __bfloat162float(__float2bfloat16_rn(x));
+    const float r = x - a;
+    b = __bfloat162float(__float2bfloat16_rn(r));
+    c = r - b;
+}
+__device__ __forceinline__ uint32_t two_bf16(float lo, float hi) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+// eight numbers into three 16-byte pieces of their parts
+__device__ __forceinline__ void split8(const float (&x)[8], uint4 (&piece)[3]) {
+    uint32_t w[3][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        float a0, b0, c0, a1, b1, c1;
+        split3(x[2 * i], a0, b0, c0);
+        split3(x[2 * i + 1], a1, b1, c1);
+        w[0][i] = two_bf16(a0, a1); w[1][i] = two_bf16(b0, b1); w[2][i] = two_bf16(c0, c1);
+    }
+#pragma unroll
+    for (int p = 0; p < 3; ++p) piece[p] = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+}
+
+// A CTA per (page of a sequence, kv head): keys [64][D] and values [D][64] into their parts; what lies beyond the sequence's end is 0.
+__global__ void __launch_bounds__(128)
+split_pages_kernel(const TcF32Args a) {
+    const int page = blockIdx.x, g = blockIdx.y, seq = blockIdx.z, G = a.f.n_kv_heads, W = a.f.table_stride;
+    const size_t slot = (size_t)seq * W + page;
+    pdl_launch_dependents();
+    pdl_wait();
+    if (page == 0 && g == 0 && seq == 0 && threadIdx.x == 0) a.flags[0] = 0;
+    const int valid = a.f.kv_lens[seq] - page * kPageTokens;
+    bool bad = false;
+    if (valid > 0) {
+        const size_t src = ((size_t)a.f.page_table[slot] * G + g) * kTcPart;
+        const size_t dst = (slot * G + g) * 3 * kTcPart, values = (size_t)a.n_seqs * W * G * 3 * kTcPart;
+#pragma unroll
+        for (int i = 0; i < kTcPart / 8 / 128; ++i) {
+            const int c = (i * 128 + threadIdx.x) * 8, row = c / 64, col = c % 64;
+            float k[8], v[8];
+            uint4 piece[3];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                *reinterpret_cast<float4*>(k + 4 * h) = *reinterpret_cast<const float4*>(a.f.k_pool + src + c + 4 * h);
+                *reinterpret_cast<float4*>(v + 4 * h) = *reinterpret_cast<const float4*>(a.f.v_pool + src + c + 4 * h);
+            }
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                k[e] = row < valid ? k[e] : 0.f;
+                v[e] = col + e < valid ? v[e] : 0.f;
+                bad |= !(fabsf(k[e]) < 0x1p60f) || !(fabsf(v[e]) < 0x1p100f);
+                v[e] *= kTcValueScale;
+            }
+            split8(k, piece);
+#pragma unroll
+            for (int p = 0; p < 3; ++p) *reinterpret_cast<uint4*>(a.parts + dst + p * kTcPart + c) = piece[p];
+            split8(v, piece);
+#pragma unroll
+            for (int p = 0; p < 3; ++p) *reinterpret_cast<uint4*>(a.parts + values + dst + p * kTcPart + c) = piece[p];
+        }
+    }
+    const int any = __syncthreads_or(bad);
+    if (threadIdx.x == 0) a.flags[1 + slot * G + g] = any;
+}
+
+__device__ __forceinline__ void tc_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void tc_mma_a_tmem(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, int accumulate) {
+    asm volatile(
+        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+// sums of two times sixteen neighbouring columns of this thread's row
+__device__ __forceinline__ void tmem_sum16(uint32_t first, uint32_t second, float (&v)[16]) {
+    uint32_t a[16], b[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%32];\n"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%33];\n"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=&r"(a[0]), "=&r"(a[1]), "=&r"(a[2]), "=&r"(a[3]), "=&r"(a[4]), "=&r"(a[5]), "=&r"(a[6]), "=&r"(a[7]), "=&r"(a[8]), "=&r"(a[9]),
+          "=&r"(a[10]), "=&r"(a[11]), "=&r"(a[12]), "=&r"(a[13]), "=&r"(a[14]), "=&r"(a[15]), "=&r"(b[0]), "=&r"(b[1]), "=&r"(b[2]), "=&r"(b[3]),
+          "=&r"(b[4]), "=&r"(b[5]), "=&r"(b[6]), "=&r"(b[7]), "=&r"(b[8]), "=&r"(b[9]), "=&r"(b[10]), "=&r"(b[11]), "=&r"(b[12]), "=&r"(b[13]),
+          "=&r"(b[14]), "=&r"(b[15])
+        : "r"(first), "r"(second) : "memory");
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(a[i]) + __uint_as_float(b[i]);
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                 ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
+}
+
+__global__ void __launch_bounds__(kTcThreads, 1)
+attention_prefill_f32_tc_kernel(const __grid_constant__ CUtensorMap map_parts, const TcF32Args a) {
+    // Tensor memory, 512 columns: tile t has its scores in 256 t .. + 127 (64 for each half of the dimensions), overwritten by the
+    // three parts of its probabilities (bfloat16 pairs, 96) once its threads hold them, and a page's outputs in + 128 .. + 255 (64 for
+    // each half of the keys).
+    extern __shared__ __align__(1024) uint8_t tc_raw[];
+    TcF32Smem& sm = *reinterpret_cast<TcF32Smem*>(((uintptr_t)tc_raw + 1023) & ~(uintptr_t)1023);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // the six products, as (part of the first operand, part of the second): smallest first
+    constexpr int kFirst[6] = {0, 1, 2, 0, 1, 0}, kSecond[6] = {2, 1, 0, 1, 0, 0};
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kTcStages; ++s) {
+            mbar_init(&sm.k_full[s], 1); mbar_init(&sm.k_empty[s], 2); mbar_init(&sm.v_full[s], 1); mbar_init(&sm.v_empty[s], 2);
+        }
+        for (int t = 0; t < 2; ++t) {
+            mbar_init(&sm.q_full[t], 4); mbar_init(&sm.s_full[t], 1); mbar_init(&sm.p_full[t], 4); mbar_init(&sm.pv_done[t], 1);
+        }
+        sm.abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_parts) : "memory");
+    }
+    if (warp == kTcMmaWarp0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem_base)), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = sm.tmem_base;
+    volatile int* abort_flag = &sm.abort_flag;
+    pdl_launch_dependents();
+    pdl_wait();
+
+    const int G = a.f.n_kv_heads, group = a.f.n_heads / G, n_pairs = a.f.n_heads / 2;
+    const int total = a.n_tiles * n_pairs * a.n_seqs;
+    auto run_units = [&](auto role) {
+        constexpr int ROLE = decltype(role)::value;   // 1: softmax warps, 0: the others
+        int units_done = 0, base = 0;                 // phases of q_full; blocks of earlier units (phases of everything else)
+        for (int round = 0;; ++round) {
+            const int unit = round * (int)gridDim.x + ((round & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x);
+            if (round * (int)gridDim.x >= total || *abort_flag) break;
+            if (unit >= total) continue;
+            const int tile = a.n_tiles - 1 - unit / (n_pairs * a.n_seqs), in_tile = unit % (n_pairs * a.n_seqs);
+            const int seq = in_tile / n_pairs, head0 = in_tile % n_pairs * 2;
+            const int tok0 = a.f.cu_seqlens[seq], q_len = a.f.cu_seqlens[seq + 1] - tok0, q0 = tile * kTcRows;
+            if (q0 >= q_len) continue;
+            const int kv_len = a.f.kv_lens[seq], p_first = kv_len - q_len + q0, rows = min(kTcRows, q_len - q0);
+            const int nb = (p_first + rows - 1) / kPageTokens + 1;
+
+            if (ROLE == 0 && warp == kTcTmaWarp && lane == 0) {
+                const int row_k = ((seq * a.f.table_stride) * G + head0 / group) * 3 * 64, row_page = G * 3 * 64;
+                const int row_v = row_k + a.n_seqs * a.f.table_stride * G * 3 * 64;
+                for (int j = 0; j < nb; ++j) {
+                    const int n = base + j, s = n % kTcStages;
+                    bool ok = n < kTcStages || mbar_wait(&sm.k_empty[s], ((n / kTcStages) - 1) & 1, abort_flag);
+                    if (ok) {
+                        mbar_expect_tx(&sm.k_full[s], 3 * kTcPart * 2);
+                        for (int p = 0; p < 3; ++p) tma_load_2d(sm.k[s][p], &map_parts, 0, row_k + j * row_page + p * 64, &sm.k_full[s]);
+                        ok = n < kTcStages || mbar_wait(&sm.v_empty[s], ((n / kTcStages) - 1) & 1, abort_flag);
+                    }
+                    if (!ok) { *abort_flag = 1; atomicCAS(&g_f32_tc_status, 0, (1 << 8) | s); break; }
+                    mbar_expect_tx(&sm.v_full[s], 3 * kTcPart * 2);
+                    for (int p = 0; p < 3; ++p) tma_load_2d(sm.v[s][p], &map_parts, 0, row_v + j * row_page + p * 64, &sm.v_full[s]);
+                }
+            } else if (ROLE == 0 && (warp == kTcMmaWarp0 || warp == kTcMmaWarp1) && lane == 0) {
+                const int t = warp - kTcMmaWarp0;
+                constexpr uint32_t idesc = umma_idesc_bf16(kTcRows, 64);
+                bool ok = mbar_wait(&sm.q_full[t], units_done & 1, abort_flag);
+                if (!ok) { *abort_flag = 1; atomicCAS(&g_f32_tc_status, 0, 2 << 8); }
+                auto scores = [&](int j) {
+                    const int n = base + j, s = n % kTcStages;
+                    if (!mbar_wait(&sm.k_full[s], (n / kTcStages) & 1, abort_flag)) {
+                        *abort_flag = 1; atomicCAS(&g_f32_tc_status, 0, (3 << 8) | s); ok = false;
+                        return;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                    for (int half = 0; half < 2; ++half)
+#pragma unroll
+                        for (int i = 0; i < 6; ++i) {
+                            const uint64_t qd = umma_desc(sm.q[t][kFirst[i]]) + 4 * half, kd = umma_desc(sm.k[s][kSecond[i]]) + 4 * half;
+#pragma unroll
+                            for (int kk = 0; kk < 2; ++kk) umma_bf16(tmem + 256 * t + 64 * half, qd + 2 * kk, kd + 2 * kk, idesc, (i | kk) != 0);
+                        }
+                    umma_commit(&sm.s_full[t]);
+                    umma_commit(&sm.k_empty[s]);
+                };
+                if (ok) scores(0);
+                for (int j = 0; j < nb && ok; ++j) {
+                    const int n = base + j, s = n % kTcStages;
+                    if (!mbar_wait(&sm.p_full[t], n & 1, abort_flag) || !mbar_wait(&sm.v_full[s], (n / kTcStages) & 1, abort_flag)) {
+                        *abort_flag = 1; atomicCAS(&g_f32_tc_status, 0, (5 << 8) | t); ok = false; break;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                    for (int half = 0; half < 2; ++half)
+#pragma unroll
+                        for (int i = 0; i < 6; ++i) {
+                            const uint64_t vd = umma_desc(sm.v[s][kSecond[i]]) + 4 * half;
+#pragma unroll
+                            for (int kk = 0; kk < 2; ++kk)
+                                tc_mma_a_tmem(tmem + 256 * t + 128 + 64 * half, tmem + 256 * t + 32 * kFirst[i] + 16 * half + 8 * kk, vd + 2 * kk,
+                                              idesc, (i | kk) != 0);
+                        }
+                    umma_commit(&sm.pv_done[t]);
+                    umma_commit(&sm.v_empty[s]);
+                    if (j + 1 < nb) scores(j + 1);   // (behind the product that reads the probabilities in their place)
+                }
+            } else if (ROLE == 1) {
+                const int t = warp >> 2, quarter = warp & 3, r = quarter * 32 + lane;
+                const uint32_t mine = tmem + 256 * t + ((uint32_t)(quarter * 32) << 16);
+                const int pos = p_first + min(r, rows - 1);           // rows past the end repeat the last one and are not stored
+                // ---- this row of Q, in parts, into the swizzled layout the products read (the unit before has formed its last scores)
+                bool bad = false;
+                const float* qrow = a.f.q + (size_t)(tok0 + q0 + min(r, rows - 1)) * a.f.q_row_stride + (size_t)(head0 + t) * kTcD;
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    float x[8];
+                    uint4 piece[3];
+                    *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(qrow + 8 * c);
+                    *reinterpret_cast<float4*>(x + 4) = *reinterpret_cast<const float4*>(qrow + 8 * c + 4);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) bad |= !(fabsf(x[e]) < 0x1p60f);
+                    split8(x, piece);
+#pragma unroll
+                    for (int p = 0; p < 3; ++p)
+                        *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(sm.q[t][p]) + r * 128 + ((c ^ (r & 7)) << 4)) = piece[p];
+                }
+                if (bad) atomicOr(a.flags, 1);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) tc_arrive(&sm.q_full[t]);
+                float m = -INFINITY, l = 0.f, l_rest = 0.f;     // l_rest: what the additions into l have rounded off
+                // o: the row's outputs; what its additions round off: the first 32 dimensions' in registers, the others' in shared memory
+                float o[kTcD], rest[32];
+                float* kept = &sm.rest[t][0][r];
+#pragma unroll
+                for (int d = 0; d < kTcD; ++d) o[d] = 0.f;
+#pragma unroll
+                for (int d = 0; d < 32; ++d) rest[d] = kept[d * kTcRows] = 0.f;
+                auto add_page = [&](float corr) {   // (o += page) corr
+#pragma unroll
+                    for (int c = 0; c < kTcD; c += 16) {
+                        float v[16];
+                        tmem_sum16(mine + 128 + c, mine + 192 + c, v);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            const float add = v[i] + (c < 32 ? rest[(c + i) & 31] : kept[((c + i) & 31) * kTcRows]), sum = o[c + i] + add;
+                            const float lost = (add - (sum - o[c + i])) * corr;
+                            if (c < 32) rest[(c + i) & 31] = lost;
+                            else kept[((c + i) & 31) * kTcRows] = lost;
+                            o[c + i] = sum * corr;
+                        }
+                    }
+                };
+                auto wait = [&](uint64_t* bar, int phase, int where) {
+                    bool ok = mbar_wait(bar, phase, abort_flag);
+                    if (!ok && lane == 0) { *abort_flag = 1; atomicCAS(&g_f32_tc_status, 0, (where << 8) | warp); }
+                    ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    return ok;
+                };
+                bool ok = true;
+                for (int j = 0; j < nb; ++j) {
+                    ok = wait(&sm.s_full[t], (base + j) & 1, 6);
+                    if (!ok) break;
+                    float s[2][32];
+#pragma unroll
+                    for (int c = 0; c < 64; c += 16) {
+                        float v[16];
+                        tmem_sum16(mine + c, mine + 64 + c, v);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) s[c >> 5][(c & 31) + i] = v[i];
+                    }
+                    const int key0 = j * kPageTokens;
+                    if (key0 + kPageTokens - 1 > p_first) {
+#pragma unroll
+                        for (int c = 0; c < 2; ++c)
+#pragma unroll
+                            for (int i = 0; i < 32; ++i) s[c][i] = key0 + 32 * c + i <= pos ? s[c][i] : -INFINITY;
+                    }
+                    float top[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+                    for (int c = 0; c < 2; ++c)
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) top[i & 3] = fmaxf(top[i & 3], s[c][i]);
+                    // (the first page holds position 0, which every row sees: the maximum is finite from there on; 1 / sqrt(64) is exact)
+                    const float m_new = fmaxf(m, 0.125f * fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3])));
+                    const float corr = expf(m - m_new);
+                    m = m_new;
+                    if (j > 0) {
+                        ok = wait(&sm.pv_done[t], (base + j - 1) & 1, 7);
+                        if (!ok) break;
+                        add_page(corr);
+                    }
+                    float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {       // 16 keys: eight columns of each part
+                        uint32_t part[3][8];
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            const int at = 16 * (c & 1) + 2 * i;
+                            const float p0 = expf(fmaf(0.125f, s[c >> 1][at], -m)), p1 = expf(fmaf(0.125f, s[c >> 1][at + 1], -m));
+                            sum[i & 3] += p0 + p1;
+                            float a0, b0, c0, a1, b1, c1;
+                            split3(p0, a0, b0, c0);
+                            split3(p1, a1, b1, c1);
+                            part[0][i] = two_bf16(a0, a1); part[1][i] = two_bf16(b0, b1); part[2][i] = two_bf16(c0, c1);
+                        }
+#pragma unroll
+                        for (int p = 0; p < 3; ++p) tmem_st8(mine + 32 * p + 8 * c, part[p]);
+                    }
+                    {
+                        const float before = l * corr, add = ((sum[0] + sum[1]) + (sum[2] + sum[3])) + l_rest * corr;
+                        l = before + add;
+                        l_rest = add - (l - before);
+                    }
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) tc_arrive(&sm.p_full[t]);
+                }
+                if (ok) ok = wait(&sm.pv_done[t], (base + nb - 1) & 1, 8);
+                if (ok) {
+                    add_page(1.f);
+                    if (r < rows) {
+                        float* dst = a.f.out + ((size_t)(tok0 + q0 + r) * a.f.n_heads + head0 + t) * kTcD;
+#pragma unroll
+                        for (int d = 0; d < kTcD; d += 4) {
+                            float4 v;
+                            v.x = o[d] / l * (1.f / kTcValueScale); v.y = o[d + 1] / l * (1.f / kTcValueScale);
+                            v.z = o[d + 2] / l * (1.f / kTcValueScale); v.w = o[d + 3] / l * (1.f / kTcValueScale);
+                            *reinterpret_cast<float4*>(dst + d) = v;
+                        }
+                    }
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            }
+            ++units_done;
+            base += nb;
+        }
+    };
+    if (warp < 8) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kTcRegsSoftmax));
+        run_units(std::integral_constant<int, 1>{});
+    } else {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kTcRegsIssuers));
+        if (warp == kTcFlagWarp && blockIdx.x == 0) {
+            int bad = 0;
+            for (int i = lane; i < a.n_split; i += 32) bad |= a.flags[1 + i];
+            if (bad) atomicOr(a.flags, 1);
+        }
+        run_units(std::integral_constant<int, 0>{});
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == kTcMmaWarp0) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(sm.tmem_base), "r"(512) : "memory");
+    }
+}
+
+static int launch_prefill_f32_tc(const PrefillF32Args& f, int n_seqs, int max_q_len, void* scratch, cudaStream_t stream) {
+    TcF32Args a = {};
+    a.f = f;
+    a.n_seqs = n_seqs;
+    a.n_tiles = (max_q_len + kTcRows - 1) / kTcRows;
+    a.n_split = n_seqs * f.table_stride * f.n_kv_heads;
+    a.parts = (__nv_bfloat16*)scratch;
+    const long long rows = 2ll * a.n_split * 3 * 64;
+    a.flags = (int*)((uint8_t*)scratch + (size_t)rows * 64 * 2);
+    if (rows >= (1ll << 31) || (long long)a.n_tiles * (f.n_heads / 2) * n_seqs >= (1ll << 30)) return kErrUnsupportedSize;
+    CUtensorMap map;
+    if (!make_map(&map, scratch, (int)rows, 64, 64, 64)) return kErrUnsupportedSize;
+    const size_t smem = sizeof(TcF32Smem) + 1024;
+    if (cudaFuncSetAttribute(attention_prefill_f32_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        return (int)cudaGetLastError();
+    int st = launch_pdl(split_pages_kernel, dim3(f.table_stride, f.n_kv_heads, n_seqs), dim3(128), 0, stream, a);
+    if (st != 0) return st;
+    const int units = a.n_tiles * (f.n_heads / 2) * n_seqs, sms = device_sm_count();
+    st = launch_pdl(attention_prefill_f32_tc_kernel, dim3(units < sms ? units : sms), dim3(kTcThreads), smem, stream, map, a);
+    if (st != 0) return st;
+    PrefillF32Args again = f;
+    again.only_if = a.flags;
+    return launch_prefill_f32<kTcD, 4>(again, n_seqs, max_q_len, 0, 1, nullptr, stream);
+}
+
 }  // namespace b200
 
 // Queries: the first n_heads head_dim elements of rows of q_row_stride elements, packed sequence after sequence
@@ -398,4 +833,38 @@ extern "C" int b200_attention_prefill_f32(const void* q, int q_row_stride, void*
         case 128: return prefill_f32_of<128>(a, n_seqs, max_q_len, n_tokens, tile, n_spans, scratch, stream);
         default: return kErrUnsupportedSize;
     }
+}
+
+// Bytes of scratch that b200_attention_prefill_f32_tc needs.
+extern "C" long long b200_attention_prefill_f32_tc_scratch(int n_seqs, int table_stride, int n_kv_heads) {
+    const long long pages = (long long)n_seqs * table_stride * n_kv_heads;
+    return pages * 2 * 3 * b200::kTcPart * 2 + (pages + 1) * 4;
+}
+
+extern "C" int b200_attention_prefill_f32_tc_status() {
+    int v = 0, zero = 0;
+    if (cudaMemcpyFromSymbol(&v, b200::g_f32_tc_status, sizeof(int)) != cudaSuccess) return -1;
+    cudaMemcpyToSymbol(b200::g_f32_tc_status, &zero, sizeof(int));
+    return v;
+}
+
+// The same as b200_attention_prefill_f32 without window or terms, head_dim 64 and an even number of query heads to a kv head, on the
+// tensor cores (other operands: kErrUnsupportedSize).  scratch: 128-aligned, b200_attention_prefill_f32_tc_scratch bytes.
+extern "C" int b200_attention_prefill_f32_tc(const void* q, int q_row_stride, void* out, const int* cu_seqlens, const int* kv_lens,
+                                             const int* page_table, int table_stride, const void* k_pool, const void* v_pool,
+                                             int n_seqs, int max_q_len, int n_heads, int n_kv_heads, int head_dim, void* scratch,
+                                             long long scratch_bytes, cudaStream_t stream) {
+    using namespace b200;
+    if (n_seqs <= 0 || max_q_len <= 0) return 0;
+    if (n_kv_heads <= 0 || n_heads % n_kv_heads != 0 || table_stride <= 0) return kErrBadArgument;
+    if (head_dim != kTcD || (n_heads / n_kv_heads) % 2 != 0 || n_kv_heads > 65535 || n_seqs > 65535) return kErrUnsupportedSize;
+    if (q_row_stride % 4 != 0 || (((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)out) & 15)) return kErrUnsupportedSize;
+    if (scratch == nullptr || ((uintptr_t)scratch & 127) || scratch_bytes < b200_attention_prefill_f32_tc_scratch(n_seqs, table_stride, n_kv_heads))
+        return kErrBadArgument;
+    if ((long long)max_q_len * n_heads > 0x7fffff00ll) return kErrUnsupportedSize;
+    PrefillF32Args a = {};
+    a.q = (const float*)q; a.out = (float*)out; a.cu_seqlens = cu_seqlens; a.kv_lens = kv_lens; a.page_table = page_table;
+    a.k_pool = (const float*)k_pool; a.v_pool = (const float*)v_pool;
+    a.q_row_stride = q_row_stride; a.table_stride = table_stride; a.n_heads = n_heads; a.n_kv_heads = n_kv_heads;
+    return launch_prefill_f32_tc(a, n_seqs, max_q_len, scratch, stream);
 }

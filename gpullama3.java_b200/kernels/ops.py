@@ -89,6 +89,9 @@ _SIGNATURES = {
     "b200_attention_prefill_f32": ("attention_prefill_f32", [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
                                                              c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                                                              c_void_p, c_void_p, c_void_p, c_int, c_float, c_int, c_int, c_void_p]),
+    "b200_attention_prefill_f32_tc": ("attention_prefill_f32", [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
+                                                                c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p,
+                                                                ctypes.c_longlong]),
     "b200_attention_prefill_tc": ("attention_prefill_tcgen05", [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p,
                                                                 c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int,
                                                                 c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
@@ -447,6 +450,11 @@ def attention_f32_plan(q_lens: list[int], kv_lens: list[int], n_heads: int, n_kv
     rounds of SMs and for five, the one that the figures above say is fastest (4 % above the fastest measured on the mean, 41 % at most; 2 tokens behind 8,000,
     32 heads of 64 over 8: 24 us, one tile of 64 rows without spans 967).  The plain kernel reads keys and values for every query head anew,
     which one or two heads to a kv head can afford (8 sequences of 2,000 keys decoded, 32 heads of 64: 64 us, 97 in tiles of 8)."""
+    return _attention_f32_fastest(q_lens, kv_lens, n_heads, n_kv_heads, head_dim, reach, sms)[1:]
+
+
+def _attention_f32_fastest(q_lens, kv_lens, n_heads, n_kv_heads, head_dim, reach, sms) -> tuple[float, int, int]:
+    """``attention_f32_plan`` with the time it expects, in microseconds, in front."""
     group, wide = n_heads // n_kv_heads, head_dim / 64
     longest = -(-min(reach, max(kv_lens)) // PAGE_TOKENS)
     pages = [min(reach, kv - q / 2) / PAGE_TOKENS + 0.5 for q, kv in zip(q_lens, kv_lens)]
@@ -471,7 +479,73 @@ def attention_f32_plan(q_lens: list[int], kv_lens: list[int], n_heads: int, n_kv
             if spans > 1:   # (a twentieth more, so that what is equal by these figures stays in one launch)
                 cost = 1.05 * cost + 1.0 + (5.75e-6 * sum(q_lens) * n_heads * spans * head_dim if tile else 0.0)
             best = min(best, (cost, tile, spans if tile else 0))
-    return best[1:]
+    return best
+
+
+_F32_TC_ROWS, _F32_TC_MOST_SCRATCH = 128, 1 << 28
+_F32_TC_LAUNCHES, _F32_TC_PAGE, _F32_TC_SPLIT = 16.0, 7.0, 0.016   # microseconds: three launches; a page of two tiles; a page of a kv head
+
+
+def attention_f32_tensor_cores_pay(q_lens: list[int], kv_lens: list[int], n_heads: int, n_kv_heads: int, head_dim: int, sms: int) -> bool:
+    """Whether ``attention_prefill_f32_tc`` is expected to be faster than what ``attention_f32_plan`` says for the same pass (causal,
+    nothing more).  Its CTAs take two tiles of 128 rows each in rounds, by falling number of the tile, and a page of two tiles takes 7 us
+    whatever runs beside it: a round lasts as long as its longest tiles.  (32 heads of 64, the plan's kernel / this one, us: 256 tokens
+    32 / 46, 512 69 / 73, 1,024 163 / 129, 2,048 576 / 240, 4,096 2,198 / 855; eight of 256 118 / 73; 300, 17 behind 900, 1 and 700
+    tokens 121 / 250; 128 behind 4,000 179 / 455.)"""
+    pairs, n_seqs = n_heads // 2, len(q_lens)
+    n_tiles = -(-max(q_lens) // _F32_TC_ROWS)
+    total, pages = n_tiles * pairs * n_seqs, 0
+    for first in range(0, total, sms):
+        hi, lo = (n_tiles - 1 - u // (pairs * n_seqs) for u in (first, min(first + sms, total) - 1))
+        last = [min(hi, -(-q // _F32_TC_ROWS) - 1) for q in q_lens]
+        pages += max((-(-min(kv, kv - q + (t + 1) * _F32_TC_ROWS) // PAGE_TOKENS) for q, kv, t in zip(q_lens, kv_lens, last) if t >= lo), default=0)
+    split = sum(-(-kv // PAGE_TOKENS) for kv in kv_lens) * n_kv_heads
+    expected = _F32_TC_LAUNCHES + _F32_TC_SPLIT * split + _F32_TC_PAGE * pages
+    return expected < _attention_f32_fastest(q_lens, kv_lens, n_heads, n_kv_heads, head_dim, max(kv_lens), sms)[0]
+
+
+def attention_prefill_f32_tc(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, cu_seqlens: torch.Tensor, kv_lens: torch.Tensor,
+                             page_table: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, n_seqs: int, max_q_len: int,
+                             n_heads: int, n_kv_heads: int, head_dim: int, alloc=None) -> bool:
+    """``attention_prefill_f32`` without window or terms on the tensor cores: every number as the sum of three bfloat16 numbers, a page's
+    sums added in float32.  Heads of 64, an even number of query heads to a kv head.  ``alloc(shape, dtype)``: where the split
+    keys and values go, 12 bytes an element (None: the allocator).  Returns False, having done nothing, for operands it does not take and
+    where there is no memory for these."""
+    if (q.dtype != torch.float32 or head_dim != 64 or n_heads % (2 * n_kv_heads) or q_row_stride % 4
+            or (q.data_ptr() | out.data_ptr() | k_pool.data_ptr() | v_pool.data_ptr()) & 15):
+        return False
+    _dev(q, out, cu_seqlens, kv_lens, page_table, k_pool, v_pool)
+    assert out.is_contiguous() and out.shape[1] == n_heads * head_dim and out.dtype == q.dtype == k_pool.dtype == v_pool.dtype
+    assert k_pool.is_contiguous() and v_pool.is_contiguous() and page_table.is_contiguous() and page_table.shape[0] >= n_seqs
+    assert tuple(k_pool.shape[1:]) == (n_kv_heads, PAGE_TOKENS, head_dim)
+    assert tuple(v_pool.shape[1:]) == (n_kv_heads, head_dim, PAGE_TOKENS)
+    assert cu_seqlens.dtype == kv_lens.dtype == page_table.dtype == torch.int32 and cu_seqlens.numel() == n_seqs + 1
+    lib = library("attention_prefill_f32")
+    lib.b200_attention_prefill_f32_tc_scratch.restype = ctypes.c_longlong
+    nbytes = int(lib.b200_attention_prefill_f32_tc_scratch(n_seqs, page_table.shape[1], n_kv_heads))
+    if nbytes > _F32_TC_MOST_SCRATCH:
+        return False
+    try:
+        scratch = alloc((nbytes,), torch.uint8) if alloc is not None else torch.empty(nbytes, dtype=torch.uint8, device=q.device)
+    except torch.OutOfMemoryError:
+        scratch = None
+    if scratch is None:
+        return False
+    status = _fn("b200_attention_prefill_f32_tc")(
+        q.data_ptr(), q_row_stride, out.data_ptr(), cu_seqlens.data_ptr(), kv_lens.data_ptr(), page_table.data_ptr(),
+        page_table.shape[1], k_pool.data_ptr(), v_pool.data_ptr(), n_seqs, int(max_q_len), n_heads, n_kv_heads, head_dim,
+        scratch.data_ptr(), nbytes, _stream())
+    if status == _UNSUPPORTED:
+        return False
+    _check(status, "attention_paged")
+    return True
+
+
+def attention_prefill_f32_tc_status() -> int:
+    """Where a wait of the kernel gave up since the last call (0: nowhere)."""
+    lib = library("attention_prefill_f32")
+    lib.b200_attention_prefill_f32_tc_status.restype = c_int
+    return int(lib.b200_attention_prefill_f32_tc_status())
 
 
 # --------------------------------------------------------------------------- matrix products

@@ -248,6 +248,23 @@ def _reach(shape) -> int | None:
     return getattr(shape, "chunk", None)
 
 
+def _plain_causal(shape) -> bool:
+    """Whether the mixer's mask is causality alone and its scores have no further terms."""
+    return not (shape.window or shape.keep_first or getattr(shape, "has_terms", False) or getattr(shape, "chunk", None))
+
+
+def _tensor_cores_pay(shape, ctx: StepContext, device) -> bool:
+    """Whether a float32 pass of such a mixer is faster on the tensor cores (decided once a pass)."""
+    if shape.head_dim != 64 or shape.n_heads % (2 * shape.n_kv_heads):
+        return False
+    key = ("float32 attention on tensor cores", shape.n_heads, shape.n_kv_heads)
+    if key not in ctx.extras:
+        kv_lens = [s + q for s, q in zip(ctx.start_pos, ctx.q_lens)]
+        ctx.extras[key] = ops.attention_f32_tensor_cores_pay(ctx.q_lens, kv_lens, shape.n_heads, shape.n_kv_heads, shape.head_dim,
+                                                             ops.sm_count(device))
+    return ctx.extras[key]
+
+
 def attend(shape, qkv: torch.Tensor, out: torch.Tensor, ctx: StepContext, table: torch.Tensor, cache: KVView, gate=None) -> None:
     """Attention of the finished query rows in ``qkv`` over the paged cache into ``out``: a tensor-core kernel where one
     takes the sizes, else the plain kernel (a step of few tokens cuts their keys into spans so that the GPU has CTAs to
@@ -262,6 +279,10 @@ def attend(shape, qkv: torch.Tensor, out: torch.Tensor, ctx: StepContext, table:
         # a tile of a sequence's queries at a time, the keys of few tiles in spans of pages; a decode step's launches must be right
         # for sequences of any length up to the step's capacity
         key = ("float32 attention", shape.n_heads, shape.n_kv_heads, shape.head_dim, reach)
+        if gate is None and not ctx.all_decode and _plain_causal(shape) and _tensor_cores_pay(shape, ctx, qkv.device):
+            if ops.attention_prefill_f32_tc(qkv, qkv.shape[1], out, ctx.cu_seqlens, ctx.kv_lens, table, cache.k, cache.v, ctx.n_seqs,
+                                            ctx.max_q_len, shape.n_heads, shape.n_kv_heads, shape.head_dim, alloc=scratch_of(ctx)):
+                return
         plan = ctx.extras.get(key)
         if plan is None:
             kv_lens = [reach] * ctx.n_seqs if ctx.all_decode else [s + q for s, q in zip(ctx.start_pos, ctx.q_lens)]
