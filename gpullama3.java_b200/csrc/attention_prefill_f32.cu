@@ -382,8 +382,10 @@ static int prefill_f32_of(const PrefillF32Args& a, int n_seqs, int max_q_len, in
 // off kept (sums of 64: 172 us in place of 240, errors a fifth above the kernel's above).  Keys and values are split once a launch
 // (split_pages_kernel, into scratch memory, values times 2^24 so that the parts of small ones keep their bits), queries by the softmax
 // threads, probabilities in registers.
-// Probabilities are in [0, 1] and keys within the mask only, so numbers of ordinary size are all that occurs; a query or key of 2^60 or
-// more, a value of 2^100 or more, or one that is not finite raises a flag, and the kernel above then does the launch over.
+// Probabilities are in [0, 1] and keys within the mask only.  A query or key of 2^60 or more (a score of 64 such products would reach
+// 2^126), a value of 2^72 or more, or one that is not finite raises a flag, and the kernel above then does the launch over.  2^72: a row's
+// sums are kept unnormalised, up to one value times 2^24 for each of its keys, and the launch takes fewer than 2^29 keys a sequence:
+// 2^72 2^24 2^29 = 2^125 is finite.
 //
 // A CTA owns two tiles of 128 rows, the same tokens of two neighbouring heads, so that a page's parts serve both; warps 0 to 3 and 4
 // to 7 are their softmax threads (a row each), one warp fetches, one issues each tile's products.  A tile's next scores are formed
@@ -397,6 +399,7 @@ constexpr int kTcTmaWarp = 8, kTcMmaWarp0 = 9, kTcMmaWarp1 = 10, kTcFlagWarp = 1
 constexpr int kTcRegsIssuers = 40, kTcRegsSoftmax = 232;   // 128 x 40 + 256 x 232 = 64,512 = 384 x 168, the launch's registers
 constexpr int kTcPart = kPageTokens * kTcD;                // elements of one part of a page's keys or values
 constexpr float kTcValueScale = 16777216.f;                // 2^24
+constexpr float kTcMostScoreFactor = 0x1p60f, kTcMostValue = 0x1p72f;   // (see above)
 
 __device__ int g_f32_tc_status = 0;
 
@@ -471,7 +474,7 @@ split_pages_kernel(const TcF32Args a) {
             for (int e = 0; e < 8; ++e) {
                 k[e] = row < valid ? k[e] : 0.f;
                 v[e] = col + e < valid ? v[e] : 0.f;
-                bad |= !(fabsf(k[e]) < 0x1p60f) || !(fabsf(v[e]) < 0x1p100f);
+                bad |= !(fabsf(k[e]) < kTcMostScoreFactor) || !(fabsf(v[e]) < kTcMostValue);
                 v[e] *= kTcValueScale;
             }
             split8(k, piece);
@@ -638,7 +641,7 @@ attention_prefill_f32_tc_kernel(const __grid_constant__ CUtensorMap map_parts, c
                     *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(qrow + 8 * c);
                     *reinterpret_cast<float4*>(x + 4) = *reinterpret_cast<const float4*>(qrow + 8 * c + 4);
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) bad |= !(fabsf(x[e]) < 0x1p60f);
+                    for (int e = 0; e < 8; ++e) bad |= !(fabsf(x[e]) < kTcMostScoreFactor);
                     split8(x, piece);
 #pragma unroll
                     for (int p = 0; p < 3; ++p)

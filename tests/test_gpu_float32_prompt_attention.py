@@ -93,6 +93,26 @@ def test_numbers_without_such_parts(what):
         assert torch.equal(got.isnan(), tiles.isnan()) and torch.equal(got.nan_to_num(), tiles.nan_to_num())
 
 
+@pytest.mark.parametrize("keys", [64, 2048])
+@pytest.mark.parametrize("value", [1e30, 2.0 ** 72, 2.0 ** 71.9, -2.0 ** 71.9, 1e20], ids=["1e30", "at the bound", "below it", "negative", "1e20"])
+def test_large_values_of_equal_weight(value, keys):
+    """Scores of 0, so that a row's unnormalised sum grows with its keys: finite at every length, and from the bound on (2^72) the
+    multiply-add kernel's bits.  Below it every row is the mean of equal values: each of the twelve products that are added up for half a page cuts off at most
+    2^-23 of the sum, all to the same side where the values are equal."""
+    q_lens, behind, H, G = [128], [keys - 128], 4, 2
+    if keys < 128:
+        q_lens, behind = [keys], [0]
+    c = case(q_lens, behind, H, G, 7)
+    c[0].zero_()
+    c[5].fill_(value)
+    got, tiles = both(c, q_lens, H, G)
+    assert bool(got.isfinite().all())
+    if value >= 2.0 ** 72:
+        assert torch.equal(got, tiles)
+    else:
+        torch.testing.assert_close(got, torch.full_like(got, value), rtol=12 * 2.0 ** -23, atol=0.0)
+
+
 def test_stale_pages_are_not_read():
     """What lies behind a sequence's end in its last page, and pages it does not have, may hold anything."""
     q_lens, behind, H, G = [100], [30], 4, 2
