@@ -502,9 +502,10 @@ __device__ __forceinline__ void umma_bf16_a_tmem(uint32_t tmem_d, uint32_t tmem_
 // another in one stream.
 __device__ unsigned int g_pair_ctl[4];
 
-// WIN: compiled with a window or `chunk`.  Both tiles then start at the block that holds the first key of the pair's first row; what
-// of it lies below a row's own first key is masked as what lies above its position is (for the second tile that is a block more
-// than it needs, in nine at a window of 1,024).  2,048 tokens, 32 heads of 64, window 1,024: 62.6 us with a tile a CTA, 48.5 so.
+// WIN: compiled with a window or `chunk`.  The pair's blocks then start at the one that holds the first key of its first row, and each
+// tile's at the one that holds the first key of its own first row, as in the kernel above: a value that is not finite would reach rows whose
+// probability for it is 0 (0 times it is not 0), so no row may read a block that its tile does not see.  What of a block lies below a row's own
+// first key is masked as what lies above its position is.  2,048 tokens, 32 heads of 64, window 1,024: 61.4 us with a tile a CTA, 48.0 so.
 template <int D, bool TERMS, bool WIN>
 __global__ void __launch_bounds__(kPairThreads, 1)
 attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -584,12 +585,13 @@ attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
             const int kv_len = kv_lens[seq], start = kv_len - q_len;
             // tile t: rows q0 + 128 t .. ; its key blocks are 0 .. nb[t] - 1 (causal), nb[1] = 0 when the tile has no rows
             const int rows0 = min(kFaRows, q_len - q0), rows1 = max(0, min(kFaRows, q_len - q0 - kFaRows));
-            // (with WIN counted from block blk0, where the first row's keys start)
+            // (with WIN counted from block blk0, where the first row's keys start; the second tile's first block is then f1)
             auto first_key = [&](int pos) { return !WIN ? 0 : chunk > 0 ? pos - pos % chunk : max(0, pos - window + 1); };
             const int blk0 = WIN ? first_key(start + q0) / kFaKeys : 0;
             const int nb0 = (start + q0 + rows0 - 1) / kFaKeys + 1 - blk0;
             const int nb1 = rows1 > 0 ? (start + q0 + kFaRows + rows1 - 1) / kFaKeys + 1 - blk0 : 0;
             const int nb = max(nb0, nb1);
+            const int f1 = WIN && rows1 > 0 ? first_key(start + q0 + kFaRows) / kFaKeys - blk0 : 0;   // (<= nb0: no block lies between the tiles)
 
             if (ROLE == 0 && warp == kPairTmaWarp && lane == 0) {
                 // ---- producer: both Q tiles, then per block two K pages and two V^T pages
@@ -627,6 +629,7 @@ attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
                 // softmax of the current ones runs, and the two tiles' threads keep the pipe fed between them.
                 const int t = warp == kPairMmaWarp0 ? 0 : 1;
                 const int nbt = t == 0 ? nb0 : nb1, nb_other = t == 0 ? nb1 : nb0;
+                const int f = t == 0 ? 0 : f1;
                 constexpr uint32_t idesc_s = umma_idesc_bf16(kFaRows, kFaKeys);
                 constexpr uint32_t idesc_o = umma_idesc_bf16(kFaRows, D);
                 bool ok = nbt > 0;
@@ -655,19 +658,23 @@ attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
                     umma_commit(&sm.s_full[t]);
                 };
                 if (ok) {
-                    need_block(0);
-                    if (ok) scores(0);
+                    for (int i = 0; i < f && ok; ++i) {   // blocks of the other tile alone: let go as they land, to stay in step with the ring
+                        need_block(i);
+                        if (ok) mbar_arrive_fa(&sm.kv_empty[(kv_base + i) % PairStages<D>::value]);
+                    }
+                    need_block(f);
+                    if (ok) scores(f);
                 }
-                for (int i = 0; i < nbt && ok; ++i) {
+                for (int i = f; i < nbt && ok; ++i) {
                     if (kEarlyScores && i + 1 < nbt) {
-                        if (!mbar_wait(&sm.s_free[t], (tile_blocks[t] + i) & 1, abort_flag)) {
+                        if (!mbar_wait(&sm.s_free[t], (tile_blocks[t] + i - f) & 1, abort_flag)) {
                             *abort_flag = 1; atomicCAS(&g_fa_status, 0, (17 << 8) | t); ok = false; break;
                         }
                         need_block(i + 1);
                         if (!ok) break;
                         scores(i + 1);
                     }
-                    if (!mbar_wait(&sm.p_full[t], (tile_blocks[t] + i) & 1, abort_flag)) {
+                    if (!mbar_wait(&sm.p_full[t], (tile_blocks[t] + i - f) & 1, abort_flag)) {
                         *abort_flag = 1; atomicCAS(&g_fa_status, 0, (14 << 8) | t); ok = false; break;
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -676,7 +683,7 @@ attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
 #pragma unroll
                     for (int kk = 0; kk < kFaKeys / 16; ++kk)  // O += P V_i; 16 keys = 8 columns of P
                         umma_bf16_a_tmem(tmem + 256 + D * t, tmem + (D == 64 ? 384 + 64 * t : 128 * t) + 8 * kk,
-                                         (kk < 4 ? vd0 : vd1) + 2 * (kk % 4), idesc_o, (i | kk) != 0);
+                                         (kk < 4 ? vd0 : vd1) + 2 * (kk % 4), idesc_o, ((i - f) | kk) != 0);
                     umma_commit(&sm.pv_done[t]);
                     if (!kEarlyScores && i + 1 < nbt) {  // P lies where the next scores go: they follow the product that reads it
                         need_block(i + 1);
@@ -692,7 +699,7 @@ attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
                 const int t = warp >> 2, quarter = warp & 3;
                 const int r = quarter * 32 + lane;
                 const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-                const int rows_t = t == 0 ? rows0 : rows1, nbt = t == 0 ? nb0 : nb1;
+                const int rows_t = t == 0 ? rows0 : rows1, nbt = t == 0 ? nb0 : nb1, f = t == 0 ? 0 : f1;
                 const int p_first = start + q0 + kFaRows * t;
                 const int pos = p_first + min(r, max(rows_t, 1) - 1);  // rows past the end mirror the last one (never stored)
                 const int lo_key = first_key(pos), lo_last = first_key(p_first + max(rows_t, 1) - 1);
@@ -701,8 +708,17 @@ attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
                 const float cap_qk = TERMS ? terms.softcap * sqrtf((float)D) : 0.f, cap_log2 = TERMS && cap_qk > 0.f ? 2.885390081777927f / cap_qk : 0.f;
                 float m_ref = -INFINITY, l = 0.f;
                 bool ok = true;
-                for (int j = 0; j < nbt; ++j) {
-                    ok = mbar_wait(&sm.s_full[t], (tile_blocks[t] + j) & 1, abort_flag);
+                if constexpr (WIN) {
+                    for (int j = 0; j < f && ok; ++j) {  // rounds ahead of this tile's blocks: pass the turn on
+                        ok = mbar_wait(&sm.exp_turn[t], (kv_base + j) & 1, abort_flag);
+                        if (!ok && lane == 0) { *abort_flag = 1; atomicCAS(&g_fa_status, 0, (20 << 8) | (t * 4 + quarter)); }
+                        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+                        __syncwarp();
+                        if (ok && lane == 0) mbar_arrive_fa(&sm.exp_turn[1 - t]);
+                    }
+                }
+                for (int j = f; j < nbt && (!WIN || ok); ++j) {
+                    ok = mbar_wait(&sm.s_full[t], (tile_blocks[t] + j - f) & 1, abort_flag);
                     if (!ok && lane == 0) { *abort_flag = 1; atomicCAS(&g_fa_status, 0, (15 << 8) | (t * 4 + quarter)); }
                     ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
                     if (!ok) break;
@@ -738,8 +754,8 @@ attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
                     }
                     if (TERMS && cap_qk > 0.f && m_blk > -INFINITY) m_blk = soft_capped_fast(m_blk, cap_qk, cap_log2);
                     // the block before must have left P and O alone before either is touched (it has, long ago, as a rule)
-                    if (j > 0) {
-                        ok = mbar_wait(&sm.pv_done[t], (tile_blocks[t] + j - 1) & 1, abort_flag);
+                    if (j > f) {
+                        ok = mbar_wait(&sm.pv_done[t], (tile_blocks[t] + j - f - 1) & 1, abort_flag);
                         if (!ok && lane == 0) { *abort_flag = 1; atomicCAS(&g_fa_status, 0, (18 << 8) | (t * 4 + quarter)); }
                         ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
                         if (!ok) break;
@@ -751,7 +767,7 @@ attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
                         const float m_new = move ? m_blk : m_ref;
                         const float corr = (m_ref == -INFINITY) ? 0.f : ex2((m_ref - m_new) * scale_log2);
                         l *= corr;
-                        if (j > 0) {  // O holds earlier blocks: rescale this row (whole warps take part in the TMEM access)
+                        if (j > f) {  // O holds earlier blocks: rescale this row (whole warps take part in the TMEM access)
 #pragma unroll 1
                             for (int c0 = 0; c0 < D; c0 += 32) {
                                 float o[32];
@@ -860,7 +876,7 @@ attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
                     if (ok && lane == 0) mbar_arrive_fa(&sm.exp_turn[1 - t]);
                 }
                 if (ok && nbt > 0) {
-                    ok = mbar_wait(&sm.pv_done[t], (tile_blocks[t] + nbt - 1) & 1, abort_flag);
+                    ok = mbar_wait(&sm.pv_done[t], (tile_blocks[t] + nbt - f - 1) & 1, abort_flag);
                     if (!ok && lane == 0) { *abort_flag = 1; atomicCAS(&g_fa_status, 0, (16 << 8) | (t * 4 + quarter)); }
                     ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
                     if (ok) {
@@ -893,7 +909,7 @@ attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
             ++units_done;
             kv_base += nb;
             tile_blocks[0] += nb0;
-            tile_blocks[1] += nb1;
+            tile_blocks[1] += nb1 - f1;
         }
     };
     if (warp < 8) {
@@ -1022,10 +1038,10 @@ extern "C" int b200_attention_prefill_tc(const void* q, int q_row_stride, int n_
     const bool more = softcap > 0.f || gate != nullptr;
 #define B200_GO(F, D, T, ...)                                                                                                  \
     F<D, T>(mq, mk, mv, out, cu_seqlens, kv_lens, page_table, table_stride, n_seqs, max_q_len, n_heads, n_kv_heads, __VA_ARGS__, stream)
-    // Tiles in pairs when there are enough pairs to give every SM one (fewer: the single-tile kernel fills more SMs).  A mask that hides
-    // early keys costs a pair its second tile's first block, which counts where few blocks are seen; heads of 64, two of whose
-    // single-tile CTAs share an SM, go in pairs from 768 keys on (2,048 tokens, 32 heads, a tile a CTA / in pairs: window 512 42.9 / 45.5 us,
-    // 1,024 62.6 / 48.5; 8,192 tokens, window 4,096: 568 / 363), heads of 128 always (window 128: 43.9 / 38.9, 1,024: 92.7 / 60.9).
+    // Tiles in pairs when there are enough pairs to give every SM one (fewer: the single-tile kernel fills more SMs).  Under a mask that hides
+    // early keys few blocks are seen, and two single-tile CTAs with heads of 64 share an SM, so these go in pairs from 768 keys on (2,048 tokens,
+    // 32 heads, us with a tile a CTA / in pairs: window 512 41.9 / 44.4, 768 52.1 / 49.2, 1,024 61.4 / 48.0; 8,192 tokens, window 4,096: 568 / 363,
+    // runs of 2,048: 251 / 168), heads of 128 always (window 128: 44.0 / 37.7, 1,024: 92.5 / 61.6).
     const int reach = window > 0 ? window : chunk;
     const bool pairs = reach == 0 || head_dim == 128 || reach >= 768;
     if (pairs && (long long)((max_q_len + 2 * kFaRows - 1) / (2 * kFaRows)) * n_heads * n_seqs >= device_sm_count()) {

@@ -117,3 +117,37 @@ def test_windows_over_pairs_of_tiles(D, T, start, window, chunk):
         want[:, h] = s.softmax(-1) @ v[h // 5]
     # probabilities and results rounded to bfloat16: 2^-9 each of the values' unit spread, a little more where few keys are seen
     torch.testing.assert_close(out.double(), want.reshape(T, -1), rtol=2.0 ** -7, atol=2.0 ** -7)
+
+
+@pytest.mark.parametrize("D, window, chunk", [(64, 1000, 0), (64, 0, 1024), (64, 300, 0), (128, 300, 0), (128, 0, 300), (128, 128, 0)])
+def test_values_that_a_tile_does_not_read(D, window, chunk):
+    """An infinite value reaches the rows whose tile of 128 reads its block of 128 keys, and no others: theirs are the bits without it.
+    (Behind 200 positions the second tile of a pair starts up to eight blocks behind the first.)"""
+    o = ops()
+    H, G, T, start = 40, 8, 1300, 200
+    kv = start + T
+    g = torch.Generator("cuda").manual_seed(D + window + chunk)
+    randn = lambda *s: torch.randn(*s, generator=g, device="cuda").to(torch.bfloat16)
+    W = -(-kv // 64)
+    table = torch.randperm(W, generator=torch.Generator().manual_seed(D)).to(torch.int32).view(1, W).cuda()
+    q, k_pool, v_pool = randn(T, H * D), randn(W, G, 64, D), randn(W, G, D, 64)
+    cu, kl = torch.tensor([0, T], dtype=torch.int32, device="cuda"), torch.tensor([kv], dtype=torch.int32, device="cuda")
+
+    def run(values):
+        out = torch.empty(T, H * D, dtype=torch.bfloat16, device="cuda")
+        assert o.attention_prefill_tc(q, H * D, out, cu, kl, table, k_pool, values, 1, T, H, G, D, window, chunk=chunk)
+        assert o.attention_prefill_tc_status() == 0
+        return out
+    clean = run(v_pool)
+    first = torch.tensor([start + r - r % 128 for r in range(T)])                  # position of the first row of a row's tile
+    lowest = first - first % chunk if chunk else (first - window + 1).clamp(min=0)
+    assert bool((lowest >= 128).any())
+    for at in (10, 200, 400, 1023):
+        poisoned = v_pool.clone()
+        poisoned[int(table[0, at // 64]), :, :, at % 64] = math.inf
+        got = run(poisoned)
+        unread = (at // 128 < lowest // 128).cuda()
+        assert torch.equal(got[unread], clean[unread])
+        pos = torch.arange(start, kv)
+        sees = (pos >= at) & ((at >= pos - pos % chunk) if chunk else (at > pos - window))
+        assert not bool(got[sees.cuda()].isfinite().any())
