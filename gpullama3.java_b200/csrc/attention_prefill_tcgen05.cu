@@ -231,8 +231,10 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             mbar_expect_tx(&sm.kv_full[s], 2 * (64 * D * 2) + 2 * (D * 64 * 2));
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const int lp = blk * 2 + h;  // logical page; pages the sequence does not have are read as zeros
-                const bool have = lp < n_pages_seq;
+                // logical page; pages the sequence does not have are read as zeros, and so are those that lie wholly below the
+                // first key: a windowed cache has let them go, and its table names another sequence's page in their place
+                const int lp = blk * 2 + h;
+                const bool have = lp < n_pages_seq && (lp + 1) * kPageTokens > key_lo;
                 const int page = have ? pages[lp] : 0;
 #pragma unroll
                 for (int a = 0; a < kAtoms; ++a)  // keys 64 h .. of atom a (dims 64 a ..)
@@ -587,7 +589,7 @@ attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
             const int rows0 = min(kFaRows, q_len - q0), rows1 = max(0, min(kFaRows, q_len - q0 - kFaRows));
             // (with WIN counted from block blk0, where the first row's keys start; the second tile's first block is then f1)
             auto first_key = [&](int pos) { return !WIN ? 0 : chunk > 0 ? pos - pos % chunk : max(0, pos - window + 1); };
-            const int blk0 = WIN ? first_key(start + q0) / kFaKeys : 0;
+            const int key_lo = first_key(start + q0), blk0 = key_lo / kFaKeys;
             const int nb0 = (start + q0 + rows0 - 1) / kFaKeys + 1 - blk0;
             const int nb1 = rows1 > 0 ? (start + q0 + kFaRows + rows1 - 1) / kFaKeys + 1 - blk0 : 0;
             const int nb = max(nb0, nb1);
@@ -611,8 +613,8 @@ attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
                     mbar_expect_tx(&sm.kv_full[s], 2 * (64 * D * 2) + 2 * (D * 64 * 2));
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
-                        const int lp = (blk0 + j) * 2 + h;  // logical page; pages the sequence does not have are read as zeros
-                        const bool have = lp < n_pages_seq;
+                        const int lp = (blk0 + j) * 2 + h;  // logical page; see the producer above
+                        const bool have = lp < n_pages_seq && (!WIN || (lp + 1) * kPageTokens > key_lo);
                         const int page = have ? pages[lp] : 0;
 #pragma unroll
                         for (int a = 0; a < kAtoms; ++a)

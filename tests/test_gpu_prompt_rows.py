@@ -151,3 +151,27 @@ def test_values_that_a_tile_does_not_read(D, window, chunk):
         pos = torch.arange(start, kv)
         sees = (pos >= at) & ((at >= pos - pos % chunk) if chunk else (at > pos - window))
         assert not bool(got[sees.cuda()].isfinite().any())
+
+
+@pytest.mark.parametrize("D, window, start", [(64, 1000, 1200), (64, 300, 500), (128, 300, 500), (128, 130, 1230), (128, 1, 192)])
+def test_pages_that_a_window_has_let_go(D, window, start):
+    """The table names page 0 in their place, which may hold anything of another sequence's: the bits with zeros in it."""
+    o = ops()
+    H, G, T = 40, 8, 1100
+    kv = start + T
+    gone = max(0, start - window + 1) // 64
+    assert gone % 2 == 1                     # (the first block of 128 keys begins with a page that is gone)
+    g = torch.Generator("cuda").manual_seed(D + window)
+    randn = lambda *s: torch.randn(*s, generator=g, device="cuda").to(torch.bfloat16)
+    W = -(-kv // 64)
+    table = (1 + torch.randperm(W, generator=torch.Generator().manual_seed(D))).to(torch.int32).view(1, W).cuda()
+    table[0, :gone] = 0
+    q, k_pool, v_pool = randn(T, H * D), randn(W + 1, G, 64, D), randn(W + 1, G, D, 64)
+    cu, kl = torch.tensor([0, T], dtype=torch.int32, device="cuda"), torch.tensor([kv], dtype=torch.int32, device="cuda")
+    outs = []
+    for keys, values in ((0.0, 0.0), (math.nan, math.inf), (math.inf, math.nan)):
+        k_pool[0], v_pool[0] = keys, values
+        outs.append(torch.empty(T, H * D, dtype=torch.bfloat16, device="cuda"))
+        assert o.attention_prefill_tc(q, H * D, outs[-1], cu, kl, table, k_pool, v_pool, 1, T, H, G, D, window)
+        assert o.attention_prefill_tc_status() == 0
+    assert bool(outs[0].isfinite().all()) and torch.equal(outs[1], outs[0]) and torch.equal(outs[2], outs[0])
