@@ -49,7 +49,8 @@ __device__ __forceinline__ void skinny_rope_emit(const SkinnyRope& p, __nv_bfloa
     float v = __bfloat162float(__float2bfloat16_rn(own));
     if (h < p.n_heads + p.n_kv_heads) {
         const float o = __bfloat162float(__float2bfloat16_rn(other));
-        v = first ? v * a.x - o * a.y : o * a.y + v * a.x;
+        // (v0 c - v1 s and v0 s + v1 c with the second product rounded by itself, as rope_cache.cu's kernels have them: the same bits)
+        v = __fmaf_rn(first ? v : o, first ? a.x : a.y, __fmul_rn(first ? o : v, first ? -a.y : a.x));
     }
     if (h < p.n_heads) {
         C[(size_t)token * ldc + n] = __float2bfloat16_rn(v);

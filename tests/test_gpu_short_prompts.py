@@ -19,8 +19,7 @@ def ops():
 @pytest.mark.parametrize("write_cache", [True, False], ids=["writes", "reads_only"])
 def test_few_token_projection_with_rotation_and_cache_write(H, KVH, D, M, K, pairing, write_cache):
     """Two sequences in one pass, the second behind 77 positions, pages scattered.  Both round the same sums to bfloat16 before they turn
-    them by the same angles, and then round a 32-bit turn whose two products the compiler may join in either order: a result may fall
-    on the other side of a rounding (one unit of 2^-8), rarely.  Values, which are not turned, and what is not written have the same bits."""
+    them by the same angles in the same order of roundings: the same bits, and what is not written is untouched."""
     o = ops()
     g = torch.Generator().manual_seed(H * D + M + pairing)
     N = (H + 2 * KVH) * D
@@ -44,7 +43,5 @@ def test_few_token_projection_with_rotation_and_cache_write(H, KVH, D, M, K, pai
                                   H, KVH, D, pairing, write_cache)
     assert o.gemm_skinny_status() == 0
     assert torch.equal(v_got, v_want)
-    for a, b in ((got[:, :H * D], want[:, :H * D]), (k_got, k_want)):
-        torch.testing.assert_close(a, b, rtol=2.0 ** -7, atol=1e-6)
-        assert float((a != b).float().mean()) < 1e-3
+    assert torch.equal(got[:, :H * D], want[:, :H * D]) and torch.equal(k_got, k_want)
     assert bool((got[:, H * D:] == 7.0).all())
