@@ -154,8 +154,8 @@ template <> struct StreamVec<1> {
 // asks for everything it reads of up to kStepKeep accesses before it writes anything (x is read and written through one pointer,
 // so the compiler cannot), keeps their u in registers (widths up to kStepKeep * VEC * kStepThreads) and forms u again from
 // the new streams beyond that.  S: the number of streams, or 0 for a number given at run time.
-// Bound by its bytes (2,048 tokens, three streams of 2,048: 142 MB in 36 us, launches by event; 50 us with 256 threads whose loads waited
-// for the stores before them).
+// Bound by its bytes (2,048 tokens, three streams of 2,048: 142 MB in 29.5 us, launches back to back; 1.4 times as long with 256 threads
+// whose loads waited for the stores before them).
 constexpr int kStepKeep = 2, kStepThreads = 512;
 
 template <typename TO, int VEC, int S>
@@ -271,7 +271,9 @@ streams_step_kernel(float* __restrict__ x, const float* __restrict__ mix, const 
 // The same for prompts: persistent CTAs, two an SM, whose tokens arrive through a ring of shared-memory stages (bulk copies, up to
 // kRingStages tokens ahead), so that an SM's loads never wait for the stores before them.  A thread keeps its u in registers
 // (widths up to kStepKeep * 4 * kStepThreads); one barrier a token, behind which its stage is filled again.  2,048 tokens, three streams of
-// 2,048 (142 MB, a part of them in L2): 38 us as above, 20 so.  For prompts of four tokens a CTA and more; fewer leave nothing to run ahead.
+// 2,048 (142 MB, a part of them in L2), launches back to back: 29.5 us as above, 18.2 so.  For prompts of four tokens a CTA and more;
+// fewer leave nothing to run ahead.  A copy that does not arrive within mbar_wait's two seconds is recorded in g_streams_status, with the
+// step's streams half updated.
 constexpr int kRingStages = 4, kRingBytes = 112 * 1024;
 
 __device__ int g_streams_status = 0;

@@ -1163,6 +1163,14 @@ def streams_step(x: torch.Tensor, mix: torch.Tensor, write: torch.Tensor, y: tor
            "streams_step")
 
 
+def streams_status() -> int:
+    """0 when every copy that ``streams_step`` waited for has arrived since the last call (1: a launch of many tokens gave up after two
+    seconds and left its streams half updated); synchronises."""
+    lib = library("streams")
+    lib.b200_streams_status.restype = c_int
+    return int(lib.b200_streams_status())
+
+
 # --------------------------------------------------------------------------- rows of a projection, per head
 TO_ROWS, TO_CACHE_KEYS, TO_CACHE_VALUES = 0, 1, 2
 

@@ -13,6 +13,7 @@ import torch
 import plain_guduzen
 from conftest import random_prompts
 from guduzen_helpers import assert_logits, make_guduzen_dir, plain_inputs
+from gpullama3.java_b200.kernels import ops
 
 pytestmark = pytest.mark.gpu
 DTYPES = pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
@@ -100,5 +101,6 @@ def test_far_keys_and_long_memory(session_tmp, dtype, prompt_len, chunk):
     moved = _moved(late[250:], full[550:], float(full.abs().max()))
     assert float((moved > 20).float().mean()) > 0.9, moved.median()
     got = _run(d, dtype, tokens, prompt_len, chunk)
+    assert ops.streams_status() == 0
     assert_logits(got, ref, dtype, f"far keys, prompt of {prompt_len}")
     assert_logits(got[:4], ref[:4], dtype, "the first tokens")

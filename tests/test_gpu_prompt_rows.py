@@ -32,8 +32,7 @@ def test_streams_step_through_a_ring(streams, width, T, reads):
     for a, b in zip(whole, pieces):
         assert torch.equal(a, b)
     assert not whole[1].any()
-    from gpullama3.java_b200.kernels.build import library
-    assert library("streams").b200_streams_status() == 0
+    assert o.streams_status() == 0
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32], ids=["bf16", "f32"])
