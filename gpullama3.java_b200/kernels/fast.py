@@ -42,7 +42,7 @@ def try_projection_with_rope(x: torch.Tensor, w: torch.Tensor, qkv: torch.Tensor
     if (ctx.all_decode or x.dtype != torch.bfloat16 or pos.rotary_dim != mixer.head_dim or mixer.head_dim not in (64, 128)
             or not hasattr(pos, "angles")):
         return False
-    few = 16 < x.shape[0] <= 128
+    few = 16 < x.shape[0] <= 128 and ops.gemm_skinny_k_spans(x.shape[0], w.shape[0], x.shape[1], x.device) > 1
     whole_k = ops.gemm_tcgen05_k_spans(x.shape[0], w.shape[0], x.shape[1]) == 1
     if not few and not whole_k:
         return False

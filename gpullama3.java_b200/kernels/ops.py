@@ -837,6 +837,11 @@ def gemm_tcgen05_k_spans(M: int, N: int, K: int) -> int:
     return int(library("gemm_tcgen05").b200_gemm_tcgen05_k_spans(M, N, K))
 
 
+def gemm_skinny_k_spans(M: int, N: int, K: int, device) -> int:
+    """Into how many spans ``gemm_skinny`` cuts K for this shape when it is left the choice (1: it does not)."""
+    return int(library("gemm_skinny_tcgen05").b200_gemm_skinny_splits(M, N, K, sm_count(device)))
+
+
 def gemm_skinny(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, epilogue: int = EPILOGUE_STORE,
                 k_splits: int | None = None) -> bool:
     """The few-token matrix product on tcgen05 tensor cores (bfloat16 operands, at most 128 tokens,
@@ -853,7 +858,7 @@ def gemm_skinny(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, epilogue: int
     assert c.shape[1] == (N // 2 if epilogue in GATED_EPILOGUES else N)
     fn = _fn("b200_gemm_skinny")
     if k_splits is None:
-        k_splits = library("gemm_skinny_tcgen05").b200_gemm_skinny_splits(M, N, K, sm_count(a.device))
+        k_splits = gemm_skinny_k_spans(M, N, K, a.device)
     _check(fn(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), c.data_ptr(), dtype_code(c.dtype), c.stride(0), M, N,
               K, epilogue, k_splits, _stream()), "gemm_skinny")
     return True
