@@ -643,11 +643,16 @@ static int launch_attention_decode(const void* q, int q_row_stride, void* out, c
     auto vv = (__nv_bfloat16*)v_pool;
     auto oo = (__nv_bfloat16*)out;
     int st = 0;
-    // Steps of more than 16 sequences run between products that keep nearly all of an SM's memory as shared memory (8B shape, 64
-    // sequences of 512 keys: 5.42 -> 4.88 ms a step); up to 16 the products stream through L1 as this kernel does.
+    // Steps of more than 16 sequences run between products that keep most of an SM's memory as shared memory (two CTAs of a ring: 160 KB in tiles
+    // of 32 tokens, 192 in tiles of 64); up to 16 the products stream through L1 as this kernel does.  Asking for L1 costs a change of split on
+    // either side, which pays where the rings leave little: from 33 tokens on with heads of 64, and already from 20 on with wider ones, whose
+    // pages need more in flight.  A step in us, not asking / asking: 1B shape 17 x 512 keys 956 / 986, 32 x 512 1,110 / 1,133, 33 x 512 1,217 /
+    // 1,191, 64 x 512 1,385 / 1,243; 3B 17 x 512 2,183 / 2,201, 20 x 512 2,264 / 2,246, 24 x 1,500 3,009 / 2,924; 8B 20 x 512 3,805 / 3,830,
+    // 24 x 1,500 4,649 / 4,643, 48 x 512 5,197 / 4,794, 64 x 512 5,417 / 4,880.  Groups of more than 8 heads keep more of their own in shared
+    // memory and never gain (Guduzen's latent attention, 32 x 512: 1,487 / 1,518).
     LaunchForm form;
     form.early_start = early_start;
-    if (n_seqs > 16 && group <= 8) form.shared_percent = kStreamingSharedPercent;
+    if (n_seqs >= (head_dim > 64 ? 20 : 33) && group <= 8) form.shared_percent = kStreamingSharedPercent;
     const bool any_term = terms.keep_first > 0 || terms.chunk > 0 || terms.slopes || terms.sinks || terms.gate || terms.softcap > 0.f;
     if (any_term && fused) return kErrBadArgument;   // (the fused variant is not built with the terms)
 #define B200_LAUNCH(KB, F) do { if (group > 8) B200_LAUNCH_T(KB, F, true); else B200_LAUNCH_T(KB, F, false); } while (0)
