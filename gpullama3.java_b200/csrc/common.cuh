@@ -127,6 +127,11 @@ struct LaunchForm {
     int shared_percent = -1;
 };
 constexpr int kStreamingSharedPercent = 28;   // 64 KB of shared memory: the resident CTAs of the streaming kernels; the rest is L1
+// Weight rows from which a product counts as an output head (no other product of the configurations has as many): its launch asks for that
+// split.  It reads long enough to be worth an SM's change from a prompt kernel's split, which leaves L1 a few KB (128,256 x 2,048 behind
+// a prompt of 45 tokens: 120 us without, 79 with), and in decode steps, whose kernels stream as it does, asking costs nothing (a step of
+// the 1B shape alone 662 us with and 663 without, 8 sequences 925 and 926; in float32 1,791 and 1,801).
+constexpr int kHeadRows = 32768;
 
 template <typename... KArgs, typename... Args>
 inline int launch_pdl_as(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const LaunchForm& form, Args... args) {

@@ -34,7 +34,6 @@ namespace b200 {
 
 constexpr int kDecodeWarps = 8;
 constexpr int kDecodeThreads = kDecodeWarps * 32;
-constexpr int kHeadRows = 32768;   // weight rows from which a product counts as an output head
 
 __device__ __forceinline__ uint4 load_stream(const void* p) {
     uint4 v;
@@ -270,8 +269,8 @@ static int launch_u(const __nv_bfloat16* a, int lda, const __nv_bfloat16* w, int
             configured = true;
         }
     }
-    // An output head reads long enough to be worth an SM's change from the prompt kernels' split of its memory, which leaves L1, where
-    // this kernel's loads are, a few KB (128,256 x 2,048 behind a prompt of 45 tokens: 120 us without, 79 with).
+    // An output head asks for L1, where this kernel's loads are (see kHeadRows), as long as the CTAs that an SM holds (up to four) fit the
+    // 64 KB of shared memory which that leaves: up to 12 KB each, which is up to 16 tokens.
     LaunchForm form;
     if (N >= kHeadRows && smem <= 12 * 1024) form.shared_percent = kStreamingSharedPercent;
     return launch_pdl_as(kernel, dim3((N + ROWS - 1) / ROWS), dim3(kDecodeThreads), smem, stream, form, a, lda, w, ldw, (TC*)C, ldc,

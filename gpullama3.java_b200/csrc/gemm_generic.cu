@@ -428,8 +428,8 @@ static int launch_fewrows(const void* A, int lda, const void* W, int ldw, void* 
                                   (const TA*)A, lda, (const TW*)W, ldw, (TC*)C, ldc, M, N, K, epilogue, batch);
     }
     const dim3 grid((N + kFewRows - 1) / kFewRows, 1, n_batch);
-    LaunchForm form;   // (an output head: as gemm_decode.cu's)
-    if (N >= 32768) form.shared_percent = kStreamingSharedPercent;
+    LaunchForm form;
+    if (N >= kHeadRows) form.shared_percent = kStreamingSharedPercent;
     auto go = [&](auto kernel) {
         return launch_pdl_as(kernel, grid, dim3(kFewThreads), 0, stream, form, (const TA*)A, lda, (const TW*)W, ldw, (TC*)C, ldc, M, N, K, epilogue, batch);
     };
