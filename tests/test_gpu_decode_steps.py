@@ -1,5 +1,5 @@
-"""Decode-step forms: a delta-rule token with its output norm in one launch, attention groups that share a key/value head, spans of
-unequal sequences, and float32 products of few rows on the tensor cores."""
+"""Decode-step forms: a delta-rule token with its output norm in one launch, attention groups that share a key/value head, and spans of
+unequal sequences."""
 import math
 
 import pytest

@@ -174,3 +174,82 @@ def test_pages_that_a_window_has_let_go(D, window, start):
         assert o.attention_prefill_tc(q, H * D, outs[-1], cu, kl, table, k_pool, v_pool, 1, T, H, G, D, window)
         assert o.attention_prefill_tc_status() == 0
     assert bool(outs[0].isfinite().all()) and torch.equal(outs[1], outs[0]) and torch.equal(outs[2], outs[0])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32], ids=["bf16", "f32"])
+@pytest.mark.parametrize("G, a, b, D, T", [(1, 64, 32, 128, 300), (3, 40, 40, 96, 257), (2, 128, 64, 192, 2048)])
+@pytest.mark.parametrize("turned", [False, True])
+def test_key_rows_of_two_segments_of_many_tokens(G, a, b, D, T, turned, dtype):
+    """A cached key row from two places of the projection (a normed part, then one that is turned or not and widened with zeros) and a value
+    row: against the same launch in pieces of fewer tokens than the tile kernel takes, which differs in the order of the norm's sum."""
+    o = ops()
+    g = torch.Generator("cuda").manual_seed(T + D)
+    raw = torch.randn(T, G * (2 * a + b) + 4, generator=g, device="cuda").to(dtype)
+    weight = torch.randn(a, generator=g, device="cuda")
+    W = -(-(T + 9) // 64)
+    table = torch.randperm(W + 1, generator=torch.Generator().manual_seed(T))[:W].to(torch.int32).view(1, W).cuda()
+    positions = torch.arange(9, T + 9, dtype=torch.int32, device="cuda")
+    inv_freq = 1.0 / 10000.0 ** (torch.arange(b // 2, device="cuda").float() / (b // 2))
+    seg = o.head_row_segment
+    turn = {"half_pairs": b // 2, "turn_mul": 0.75} if turned else {}
+    segments = o.head_row_segments(seg(4, G, a, 0, a, -1, True, 0, target=o.TO_CACHE_KEYS, cache_dim=D),
+                                   seg(4 + G * a, G, b, a, D - a, mul=0.5, target=o.TO_CACHE_KEYS, cache_dim=D, **turn),
+                                   seg(4 + G * (a + b), G, a, 0, D, target=o.TO_CACHE_VALUES))
+
+    def run(piece):
+        pools = [torch.full(s, 3.0, dtype=dtype, device="cuda") for s in ((W + 1, G, 64, D), (W + 1, G, D, 64))]
+        for at in range(0, T, piece):
+            part = slice(at, min(T, at + piece))
+            pos = positions[part]
+            o.head_rows(raw[part], None, segments, 1e-6, None, weight, cache=(pos, torch.zeros_like(pos), table, *pools),
+                        rotary=(pos, inv_freq) if turned else None)
+        return pools
+    whole, pieces = run(T), run(100)
+    assert torch.equal(whole[1], pieces[1])
+    tol = dict(rtol=2.0 ** -7, atol=1e-6) if dtype == torch.bfloat16 else dict(rtol=2e-6, atol=2e-6)   # (one rounding to the type)
+    torch.testing.assert_close(whole[0], pieces[0], **tol)
+    page, at = table[0].long()[positions.long() // 64], positions.long() % 64
+    first = raw[:, 4:4 + G * a].double().view(T, G, a)
+    unit = first * torch.rsqrt((first * first).mean(-1, keepdim=True) + 1e-6) * weight.double()
+    torch.testing.assert_close(whole[0][page, :, at, :a].double(), unit, **tol)
+    assert not bool(whole[0][page, :, at, a + b:].any())
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("window, chunk", [(1000, 0), (777, 0), (0, 768), (0, 1000), (300, 0), (0, 130)])
+@pytest.mark.parametrize("softcap, sink, gated", [(0.0, None, False), (2.0, 0.7, True), (0.0, 1.5, False), (30.0, None, True)])
+def test_windows_with_terms_over_pairs_of_unequal_sequences(D, window, chunk, softcap, sink, gated):
+    """Enough tiles for pairs of them (heads of 64 below 768 keys go a tile a CTA), sequences that end in a pair's first and second tile, behind nothing
+    and behind prefixes that end inside a block."""
+    o = ops()
+    H, G, q_lens, behind = 20, 4, [700, 33, 1100], [0, 900, 77]
+    kv = [q + b for q, b in zip(q_lens, behind)]
+    g = torch.Generator("cuda").manual_seed(D + window + chunk)
+    randn = lambda *s: torch.randn(*s, generator=g, device="cuda").to(torch.bfloat16)
+    W, T = -(-max(kv) // 64), sum(q_lens)
+    table = torch.randperm(3 * W + 1, generator=torch.Generator().manual_seed(D))[:3 * W].to(torch.int32).view(3, W).cuda()
+    q, k_pool, v_pool = randn(T, H * D), randn(3 * W + 1, G, 64, D), randn(3 * W + 1, G, D, 64)
+    gate = randn(T, H + 3)[:, :H]
+    sinks = sink + 0.1 * torch.arange(H, device="cuda") if sink is not None else None
+    cu = torch.tensor([0, 700, 733, T], dtype=torch.int32, device="cuda")
+    out = torch.empty(T, H * D, dtype=torch.bfloat16, device="cuda")
+    assert o.attention_prefill_tc(q, H * D, out, cu, torch.tensor(kv, dtype=torch.int32, device="cuda"), table, k_pool, v_pool, 3, max(q_lens), H, G, D,
+                                  window, chunk=chunk, sinks=sinks, gate=gate if gated else None, softcap=softcap)
+    assert o.attention_prefill_tc_status() == 0
+    want = torch.empty(T, H, D, dtype=torch.float64, device="cuda")
+    for s in range(3):
+        k = k_pool[table[s].long()].permute(1, 0, 2, 3).reshape(G, W * 64, D)[:, :kv[s]].double()
+        v = v_pool[table[s].long()].permute(1, 0, 3, 2).reshape(G, W * 64, D)[:, :kv[s]].double()
+        pos, key = torch.arange(behind[s], kv[s], device="cuda")[:, None], torch.arange(kv[s], device="cuda")[None]
+        hidden = (key > pos) | ((key < pos - pos % chunk) if chunk else (key <= pos - window))
+        rows = slice(int(cu[s]), int(cu[s + 1]))
+        for h in range(H):
+            x = q[rows, h * D:(h + 1) * D].double() @ k[h * G // H].T / math.sqrt(D)
+            x = (softcap * torch.tanh(x / softcap) if softcap else x).masked_fill(hidden, -math.inf)
+            if sink is not None:
+                x = torch.cat([x, sinks[h].double().expand(x.shape[0], 1)], 1)
+            want[rows, h] = x.softmax(-1)[:, :kv[s]] @ v[h * G // H]
+    if gated:
+        want *= torch.sigmoid(gate.double())[:, :, None]
+    # (probabilities and results rounded to bfloat16)
+    torch.testing.assert_close(out.double(), want.reshape(T, -1), rtol=2.0 ** -7, atol=2.0 ** -7)
