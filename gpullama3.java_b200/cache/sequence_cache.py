@@ -166,6 +166,7 @@ class KVView:
     k: torch.Tensor  # [n_pages, kv_heads, PAGE_TOKENS, head_dim]
     v: torch.Tensor  # [n_pages, kv_heads, head_dim, PAGE_TOKENS]
     window: int | None
+    work_counters: torch.Tensor | None = None   # int32 [4] of the group's own: by which a prompt attention's CTAs share out its tiles
 
 
 class KVGroup(PagedGroup):
@@ -177,10 +178,11 @@ class KVGroup(PagedGroup):
                              device=sizes.device)
         self.v = torch.zeros((len(self.entries), n, need.n_kv_heads, need.head_dim, PAGE_TOKENS), dtype=sizes.dtype,
                              device=sizes.device)
+        self.work_counters = torch.zeros(4, dtype=torch.int32, device=sizes.device)
 
     def view(self, entry):
         i = self.entry_pos[entry]
-        return KVView(group=self.index, k=self.k[i], v=self.v[i], window=self.need.window)
+        return KVView(group=self.index, k=self.k[i], v=self.v[i], window=self.need.window, work_counters=self.work_counters)
 
     def bytes_per_token(self):
         return 2 * len(self.entries) * self.need.n_kv_heads * self.need.head_dim * self.k.element_size()

@@ -459,6 +459,7 @@ struct PairSmem {
     uint32_t tmem_base;
     int abort_flag;
     int unit;  // the unit of work the CTA is on
+    int round; // without work counters: how many units the CTA has been given
 };
 
 __device__ __forceinline__ void tmem_ld32_issue(uint32_t taddr, uint32_t (&r)[32]) {
@@ -497,12 +498,13 @@ __device__ __forceinline__ void umma_bf16_a_tmem(uint32_t tmem_d, uint32_t tmem_
         ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
-// Work counters, kept on the device so that a launch needs nothing from the host (it may be replayed from a
-// graph): words 0 and 1 count units, word 2 is the number of launches that have ended, word 3 counts the CTAs of
+// Work counters (`ctl`, four words that begin as zeros), kept on the device so that a launch needs nothing from the host (it may be
+// replayed from a graph): words 0 and 1 count units, word 2 is the number of launches that have ended, word 3 counts the CTAs of
 // the running launch that have ended.  A launch takes its units from word (launches ended) % 2 and zeroes the
-// other word for the launch after it; its last CTA advances word 2.  Launches on a device must follow one
-// another in one stream.
-__device__ unsigned int g_pair_ctl[4];
+// other word for the launch after it; its last CTA advances word 2.  Launches over the same words must follow one
+// another; a cache keeps its own, whose pages are subject to that in any case.  Without words a CTA takes every gridDim.x-th unit, forwards
+// and backwards in turn, and launches share nothing (2,048 tokens, 32 heads of 64, window 1,024: 47.7 us with words, 51.8 without;
+// 8,192 tokens in runs of 2,048: 168 and 213).
 
 // WIN: compiled with a window or `chunk`.  The pair's blocks then start at the one that holds the first key of its first row, and each
 // tile's at the one that holds the first key of its own first row, as in the kernel above: a value that is not finite would reach rows whose
@@ -515,7 +517,7 @@ attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
                               const int* __restrict__ cu_seqlens, const int* __restrict__ kv_lens,
                               const int* __restrict__ page_table, int table_stride, int n_heads, int n_kv_heads,
                               int k_rows_total, int v_rows_total, int n_seqs, int n_pairs, const float* __restrict__ sinks, FaTerms terms,
-                              int window, int chunk) {
+                              int window, int chunk, unsigned int* ctl) {
     static_assert(D == 64 || D == 128, "the pair kernel is laid out for head_dim 64 and 128");
     // Tensor memory, 512 columns.  Tile t: S in columns 128 t, O in 256 + D t.  P (bfloat16 pairs, 64 columns): with
     // head_dim 64 in columns 384 + 64 t; with head_dim 128 nothing is left, so P overwrites the first half of S, which
@@ -534,6 +536,7 @@ attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
             mbar_init(&sm.exp_turn[t], 4);
         }
         sm.abort_flag = 0;
+        sm.round = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_q) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
@@ -550,9 +553,9 @@ attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
     volatile int* abort_flag = &sm.abort_flag;
     pdl_launch_dependents();
     pdl_wait();  // the set-up above overlapped the kernel before; its results are read from here on
-    const unsigned int launches_ended = *reinterpret_cast<volatile unsigned int*>(&g_pair_ctl[2]);
+    const unsigned int launches_ended = ctl != nullptr ? *reinterpret_cast<volatile unsigned int*>(&ctl[2]) : 0;
     const int counter = (int)(launches_ended & 1u);
-    if (blockIdx.x == 0 && threadIdx.x == 0) g_pair_ctl[counter ^ 1] = 0;
+    if (ctl != nullptr && blockIdx.x == 0 && threadIdx.x == 0) ctl[counter ^ 1] = 0;
     // The exponentials of a block keep the special-function units busy; reading S, the maximum and the hand-over
     // do not.  So the two tiles' softmax threads alternate: a tile computes its exponentials only while it holds
     // the turn, and the other tile's remaining work runs meanwhile.  Tile 0 has the first turn.
@@ -574,7 +577,14 @@ attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
         constexpr int ROLE = decltype(role)::value;   // 1: softmax warps, 0: TMA and MMA warps (and the idle one)
         for (;;) {
             __syncthreads();  // the unit before is finished everywhere: tensor memory, Q and the unit number are free
-            if (threadIdx.x == 0) sm.unit = (int)atomicAdd(&g_pair_ctl[counter], 1u);
+            if (threadIdx.x == 0) {
+                if (ctl != nullptr) {
+                    sm.unit = (int)atomicAdd(&ctl[counter], 1u);
+                } else {
+                    const int round = sm.round++, place = round % 2 == 0 ? (int)blockIdx.x : (int)gridDim.x - 1 - (int)blockIdx.x;
+                    sm.unit = round * (int)gridDim.x + place;
+                }
+            }
             __syncthreads();
             const int unit = sm.unit;
             if (unit >= total_units || *abort_flag) break;
@@ -927,12 +937,12 @@ attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(sm.tmem_base), "r"(512) : "memory");
     }
-    if (threadIdx.x == 0) {  // the last CTA to end hands the counters over to the next launch
+    if (ctl != nullptr && threadIdx.x == 0) {  // the last CTA to end hands the counters over to the next launch
         __threadfence();
-        if (atomicAdd(&g_pair_ctl[3], 1u) == gridDim.x - 1) {
-            g_pair_ctl[3] = 0;
+        if (atomicAdd(&ctl[3], 1u) == gridDim.x - 1) {
+            ctl[3] = 0;
             __threadfence();
-            g_pair_ctl[2] = launches_ended + 1;
+            ctl[2] = launches_ended + 1;
         }
     }
 }
@@ -982,7 +992,7 @@ namespace b200 {
 template <int D, bool TERMS, bool WIN>
 static int launch_pair_of(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, void* out, const int* cu_seqlens,
                        const int* kv_lens, const int* page_table, int table_stride, int n_seqs, int max_q_len, int n_heads,
-                       int n_kv_heads, int k_rows, int v_rows, const float* sinks, FaTerms terms, int window, int chunk, cudaStream_t stream) {
+                       int n_kv_heads, int k_rows, int v_rows, const float* sinks, FaTerms terms, int window, int chunk, unsigned int* ctl, cudaStream_t stream) {
     const size_t smem = sizeof(PairSmem<D>) + 1024;
     static bool configured = false;
     if (!configured) {
@@ -1001,28 +1011,28 @@ static int launch_pair_of(const CUtensorMap& mq, const CUtensorMap& mk, const CU
     const int grid = (int)(units < n_sms ? units : n_sms);  // one CTA per SM; each takes units until none are left
     return launch_pdl(attention_prefill_pair_kernel<D, TERMS, WIN>, dim3(grid), dim3(kPairThreads), smem, stream, mq, mk, mv,
                       (__nv_bfloat16*)out, cu_seqlens, kv_lens, page_table, table_stride, n_heads, n_kv_heads, k_rows, v_rows,
-                      n_seqs, n_pairs, sinks, terms, window, chunk);
+                      n_seqs, n_pairs, sinks, terms, window, chunk, ctl);
 }
 
 template <int D, bool TERMS>
 static int launch_pair(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, void* out, const int* cu_seqlens,
                        const int* kv_lens, const int* page_table, int table_stride, int n_seqs, int max_q_len, int n_heads,
-                       int n_kv_heads, int k_rows, int v_rows, const float* sinks, FaTerms terms, int window, int chunk, cudaStream_t stream) {
+                       int n_kv_heads, int k_rows, int v_rows, const float* sinks, FaTerms terms, int window, int chunk, unsigned int* ctl, cudaStream_t stream) {
     auto go = window > 0 || chunk > 0 ? launch_pair_of<D, TERMS, true> : launch_pair_of<D, TERMS, false>;
     return go(mq, mk, mv, out, cu_seqlens, kv_lens, page_table, table_stride, n_seqs, max_q_len, n_heads, n_kv_heads, k_rows, v_rows,
-              sinks, terms, window, chunk, stream);
+              sinks, terms, window, chunk, ctl, stream);
 }
 }  // namespace b200
 
 // q: packed rows of q_row_stride elements whose first n_heads * head_dim are the rotated queries (n_rows of them);
 // k_pool [n_pages][n_kv_heads][64][head_dim], v_pool [n_pages][n_kv_heads][head_dim][64] (values transposed).
 // head_dim 64 or 128.  window, or chunk (not both; 0: none); sinks: float32 [n_heads] or null; gate bfloat16 [T][ld_gate] or null;
-// softcap 0: none.
+// softcap 0: none.  ctl: four words that began as zeros and that only launches which follow one another use, or null.
 extern "C" int b200_attention_prefill_tc(const void* q, int q_row_stride, int n_rows, void* out, const int* cu_seqlens,
                                          const int* kv_lens, const int* page_table, int table_stride,
                                          const void* k_pool, const void* v_pool, int n_pages, int n_seqs, int max_q_len,
                                          int n_heads, int n_kv_heads, int head_dim, int window, int chunk, const float* sinks,
-                                         const void* gate, int ld_gate, float softcap, cudaStream_t stream) {
+                                         const void* gate, int ld_gate, float softcap, unsigned int* ctl, cudaStream_t stream) {
     using namespace b200;
     if (n_seqs <= 0 || max_q_len <= 0) return 0;
     if (n_kv_heads <= 0 || n_heads % n_kv_heads != 0 || chunk < 0 || (chunk > 0 && window > 0) || !(softcap >= 0.f)) return kErrBadArgument;
@@ -1048,10 +1058,10 @@ extern "C" int b200_attention_prefill_tc(const void* q, int q_row_stride, int n_
     const bool pairs = reach == 0 || head_dim == 128 || reach >= 768;
     if (pairs && (long long)((max_q_len + 2 * kFaRows - 1) / (2 * kFaRows)) * n_heads * n_seqs >= device_sm_count()) {
         if (head_dim == 64)
-            return more || sinks != nullptr ? B200_GO(launch_pair, 64, true, (int)k_rows, (int)v_rows, sinks, terms, window, chunk)
-                                            : B200_GO(launch_pair, 64, false, (int)k_rows, (int)v_rows, sinks, terms, window, chunk);
-        return more || sinks != nullptr ? B200_GO(launch_pair, 128, true, (int)k_rows, (int)v_rows, sinks, terms, window, chunk)
-                                        : B200_GO(launch_pair, 128, false, (int)k_rows, (int)v_rows, sinks, terms, window, chunk);
+            return more || sinks != nullptr ? B200_GO(launch_pair, 64, true, (int)k_rows, (int)v_rows, sinks, terms, window, chunk, ctl)
+                                            : B200_GO(launch_pair, 64, false, (int)k_rows, (int)v_rows, sinks, terms, window, chunk, ctl);
+        return more || sinks != nullptr ? B200_GO(launch_pair, 128, true, (int)k_rows, (int)v_rows, sinks, terms, window, chunk, ctl)
+                                        : B200_GO(launch_pair, 128, false, (int)k_rows, (int)v_rows, sinks, terms, window, chunk, ctl);
     }
     if (head_dim == 64)
         return more ? B200_GO(launch_fa, 64, true, window, chunk, sinks, (int)k_rows, (int)v_rows, terms)

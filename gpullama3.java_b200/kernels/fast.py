@@ -83,7 +83,7 @@ def try_attention(qkv, out, ctx, page_table, cache, mixer, gate=None) -> bool:
         if not mixer.keep_first and mixer.slopes is None and ops.attention_prefill_tc(
                 qkv, qkv.shape[1], out, ctx.cu_seqlens, ctx.kv_lens, page_table, cache.k, cache.v, ctx.n_seqs, ctx.max_q_len,
                 mixer.n_heads, mixer.n_kv_heads, mixer.head_dim, mixer.window or 0, chunk=chunk, sinks=mixer.sinks, gate=gate,
-                softcap=terms["softcap"]):
+                softcap=terms["softcap"], work_counters=getattr(cache, "work_counters", None)):
             return True
         ops.attention_prefill(qkv, qkv.shape[1], out, ctx.cu_seqlens, ctx.kv_lens, page_table, cache.k, cache.v,
                               ctx.n_seqs, ctx.max_q_len, mixer.n_heads, mixer.n_kv_heads, mixer.head_dim,
@@ -96,7 +96,8 @@ def try_attention(qkv, out, ctx, page_table, cache, mixer, gate=None) -> bool:
         return True
     if qkv.dtype == torch.bfloat16 and ops.attention_prefill_tc(
             qkv, qkv.shape[1], out, ctx.cu_seqlens, ctx.kv_lens, page_table, cache.k, cache.v, ctx.n_seqs,
-            ctx.max_q_len, mixer.n_heads, mixer.n_kv_heads, mixer.head_dim, mixer.window or 0):
+            ctx.max_q_len, mixer.n_heads, mixer.n_kv_heads, mixer.head_dim, mixer.window or 0,
+            work_counters=getattr(cache, "work_counters", None)):
         return True
     if qkv.dtype == torch.bfloat16 and mixer.head_dim in (32, 64, 96, 128):
         ops.attention_prefill(qkv, qkv.shape[1], out, ctx.cu_seqlens, ctx.kv_lens, page_table, cache.k, cache.v,

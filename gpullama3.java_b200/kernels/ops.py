@@ -95,7 +95,7 @@ _SIGNATURES = {
     "b200_attention_prefill_tc": ("attention_prefill_tcgen05", [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p,
                                                                 c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int,
                                                                 c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
-                                                                c_float]),
+                                                                c_float, c_void_p]),
     "b200_random_fill": ("random_init", [c_void_p, c_int, ctypes.c_longlong, ctypes.c_ulonglong, c_float, c_float]),
     "b200_streams_combine": ("streams", [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int]),
     "b200_streams_read_norm": ("streams", [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
@@ -1051,12 +1051,15 @@ def attention_prefill_tc(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, 
                          kv_lens: torch.Tensor, page_table: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
                          n_seqs: int, max_q_len: int, n_heads: int, n_kv_heads: int, head_dim: int, window: int, *,
                          chunk: int = 0, sinks: torch.Tensor | None = None, gate: torch.Tensor | None = None,
-                         softcap: float = 0.0) -> bool:
+                         softcap: float = 0.0, work_counters: torch.Tensor | None = None) -> bool:
     """``attention_prefill`` on tcgen05 tensor cores (head_dim 64 or 128), with ``chunk``, ``sinks``, ``gate`` and ``softcap`` but
-    none of the other terms.  Returns False, having done nothing, for sizes it does not take."""
+    none of the other terms.  ``work_counters``: int32 [4] that began as zeros, by which a launch's CTAs share its tiles out as they get
+    done; only for launches that follow one another (a cache's).  Without it they are shared out beforehand, and launches may run side by side.
+    Returns False, having done nothing, for sizes it does not take."""
     if head_dim not in (64, 128) or q.dtype != torch.bfloat16 or q_row_stride % 8 or (q.data_ptr() | out.data_ptr()) & 15:
         return False
-    _dev(q, out, cu_seqlens, kv_lens, page_table, k_pool, v_pool, sinks, gate)
+    _dev(q, out, cu_seqlens, kv_lens, page_table, k_pool, v_pool, sinks, gate, work_counters)
+    assert work_counters is None or (work_counters.dtype == torch.int32 and work_counters.is_contiguous() and work_counters.numel() == 4)
     assert gate is None or (gate.dtype == torch.bfloat16 and gate.stride(1) == 1 and gate.shape[1] >= n_heads)
     assert sinks is None or (sinks.dtype == torch.float32 and sinks.is_contiguous() and sinks.numel() == n_heads)
     assert out.dtype == k_pool.dtype == torch.bfloat16 and out.is_contiguous() and k_pool.is_contiguous()
@@ -1066,8 +1069,8 @@ def attention_prefill_tc(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, 
         q.data_ptr(), q_row_stride, out.shape[0], out.data_ptr(), cu_seqlens.data_ptr(), kv_lens.data_ptr(),
         page_table.data_ptr(), page_table.shape[1], k_pool.data_ptr(), v_pool.data_ptr(), k_pool.shape[0], n_seqs,
         max_q_len, n_heads, n_kv_heads, head_dim, int(window), int(chunk), sinks.data_ptr() if sinks is not None else None,
-        gate.data_ptr() if gate is not None else None, gate.stride(0) if gate is not None else 0, float(softcap), _stream()),
-        "attention_prefill_tc")
+        gate.data_ptr() if gate is not None else None, gate.stride(0) if gate is not None else 0, float(softcap),
+        work_counters.data_ptr() if work_counters is not None else None, _stream()), "attention_prefill_tc")
     return True
 
 

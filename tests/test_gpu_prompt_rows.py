@@ -253,3 +253,35 @@ def test_windows_with_terms_over_pairs_of_unequal_sequences(D, window, chunk, so
         want *= torch.sigmoid(gate.double())[:, :, None]
     # (probabilities and results rounded to bfloat16)
     torch.testing.assert_close(out.double(), want.reshape(T, -1), rtol=2.0 ** -7, atol=2.0 ** -7)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("window, chunk", [(900, 0), (0, 1000), (0, 0)])
+@pytest.mark.parametrize("counted", [False, True], ids=["shared out beforehand", "by counters"])
+def test_pairs_of_tiles_on_two_streams(D, window, chunk, counted):
+    """Launches without counters share nothing, and those with counters only with launches over the same ones: what two streams run at a
+    time has the bits of each launch by itself, launch after launch, and the counters count the launches."""
+    o = ops()
+    H, G, T = 40, 8, 1500
+    g = torch.Generator("cuda").manual_seed(D)
+    randn = lambda *s: torch.randn(*s, generator=g, device="cuda").to(torch.bfloat16)
+    W = -(-T // 64)
+    table = torch.arange(W, dtype=torch.int32, device="cuda").view(1, W)
+    q, k_pool, v_pool = randn(T, H * D), randn(W, G, 64, D), randn(W, G, D, 64)
+    cu, kl = torch.tensor([0, T], dtype=torch.int32, device="cuda"), torch.tensor([T], dtype=torch.int32, device="cuda")
+    counters = torch.zeros(2, 4, dtype=torch.int32, device="cuda")
+
+    def run(out, words):
+        assert o.attention_prefill_tc(q, H * D, out, cu, kl, table, k_pool, v_pool, 1, T, H, G, D, window, chunk=chunk, work_counters=words)
+    want, outs = torch.empty(T, H * D, dtype=torch.bfloat16, device="cuda"), torch.zeros(2, 20, T, H * D, dtype=torch.bfloat16, device="cuda")
+    run(want, None)
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    for i in range(20):
+        for out, stream, words in zip(outs, streams, counters):
+            with torch.cuda.stream(stream):
+                run(out[i], words if counted else None)
+    torch.cuda.synchronize()
+    assert o.attention_prefill_tc_status() == 0
+    assert bool((outs == want).all())
+    assert counters[:, 2:].tolist() == [[20, 0] if counted else [0, 0]] * 2
