@@ -373,7 +373,9 @@ static int prefill_f32_of(const PrefillF32Args& a, int n_seqs, int max_q_len, in
 }
 
 // ---------------------------------------------------------------------------------------------
-// The same on the tensor cores, for prompts (head_dim 64, an even number of query heads to a kv head, causal and nothing more).
+// The same on the tensor cores, for prompts (head_dim 64, an even number of query heads to a kv head, causal and nothing more).  Heads of
+// 128 are not taken: the parts of two tiles of queries alone would fill 192 of the 227 KB of shared memory, and one tile leaves nothing to run
+// during its softmax.
 //
 // A float32 number is the sum of three bfloat16 numbers exactly: x0 = bf16(x), x1 = bf16(x - x0), x2 = x - x0 - x1.  A product of
 // two such sums is formed as six of its nine products (those left out are below 2^-24 of it), smallest first, by tcgen05.mma with

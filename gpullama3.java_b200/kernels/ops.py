@@ -482,6 +482,8 @@ def _attention_f32_fastest(q_lens, kv_lens, n_heads, n_kv_heads, head_dim, reach
     return best
 
 
+# (the parts of a page of a kv head take 48 KB.  A pass's workspace keeps what its largest pass took, so at most a quarter of a gigabyte of it goes
+# here, 43,690 cached tokens over 8 kv heads; batches beyond that keep the multiply-add kernel)
 _F32_TC_ROWS, _F32_TC_MOST_SCRATCH = 128, 1 << 28
 _F32_TC_LAUNCHES, _F32_TC_PAGE, _F32_TC_SPLIT = 16.0, 7.0, 0.016   # microseconds: three launches; a page of two tiles; a page of a kv head
 
