@@ -72,6 +72,7 @@ def test_entry_point_without_allocation_matches_the_regular_one():
         # The lengths reach the device through a kernel that runs right before the call, as they would in a
         # serving loop that keeps them on the device: the entry point must not read them before that kernel is done.
         lens_late = torch.zeros_like(lens)
+        lens_late.add_(lens).zero_()                    # (a kernel's code is loaded at its first launch, which may take device memory)
         torch.cuda.synchronize()
         free_before, _ = torch.cuda.mem_get_info()      # the driver's own count: sees any cudaMalloc, not only torch's
         lens_late.add_(lens)
